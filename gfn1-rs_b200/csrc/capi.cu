@@ -30,11 +30,11 @@ cudaError_t launch_setup(int max_l, dim3 grid, int nt, size_t smem, cudaStream_t
 cudaError_t launch_grad(int max_l, dim3 grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
                         const int* mols, int phases);
 long long scc_workspace_doubles(int maxn, int maxnsh, int cap, int maxnat);
-size_t scc_smem_bytes(int maxnsh, int maxn, int maxnat, int matrix_n);
-size_t scc_max_dynamic_smem(int nt);
-cudaError_t launch_scc(int nt, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
+int scc_kind(int N);
+size_t scc_smem_bytes(int kind, int maxnsh, int maxn, int maxnat);
+cudaError_t launch_scc(int kind, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
                        const SccOptions& opt, const SccLaunch& SL);
-cudaError_t launch_scc_robust(int nt, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
+cudaError_t launch_scc_robust(int kind, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
                               const SccOptions& opt, const SccLaunch& SL);
 // large molecules on many SMs (wide.cuh)
 struct WideRuntime;
@@ -290,16 +290,16 @@ struct gfn1_batch {
   long long natoms = 0, nshells = 0, naos = 0, mat_total = 0, gam_total = 0, pair_total = 0;
   int max_nat = 0, max_nsh = 0, max_n = 0, cap = 0;
   int max_l = 0;  // highest shell angular momentum of the batch (selects the s/p setup and gradient kernels)
-  // SCC size classes: [0] molecules above the split size, [1] the rest
+  // SCC size classes, largest molecules first: the molecules of each kernel
   struct SccClass {
-    int q_begin = 0, q_end = 0, n_cta = 0, nt = 256, maxn = 0, maxnsh = 0, maxnat = 0;
+    int q_begin = 0, q_end = 0, n_cta = 0, kind = 0, maxn = 0, maxnsh = 0, maxnat = 0;
     long long ws_offset = 0, ws_stride = 0;
     size_t smem = 0;
-  } cls[2];
+  } cls[3];
   SccClass robust;  // fallback ladder: workspace for the batch's largest molecule, a few CTAs
   DevBuf<int> failed;
-  cudaStream_t side = nullptr;  // second stream for the concurrent class launch
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t side[2] = {nullptr, nullptr};  // streams of the second and third class
+  cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
   gfn1_options opt;
   bool has_init_q = false;
   bool profiling = false;
@@ -417,10 +417,13 @@ struct gfn1_batch {
     if (wide) wide_runtime_delete(wide);
     wide = nullptr;
     if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
-    ev_fork = ev_join = nullptr;
-    side = nullptr;
+    ev_fork = nullptr;
+    for (int c = 0; c < 2; ++c) {
+      if (ev_join[c]) cudaEventDestroy(ev_join[c]);
+      if (side[c]) cudaStreamDestroy(side[c]);
+      ev_join[c] = nullptr;
+      side[c] = nullptr;
+    }
   }
 };
 
@@ -645,12 +648,12 @@ namespace {
 // Fills the topology part of a batch (sizes, offsets, order, element check,
 // electron count) into the pinned input blob and grows every buffer.  Buffers
 // are never shrunk, so a reused batch allocates only when a larger batch comes.
-// Molecules above this many AOs run on groups of SMs (wide.cuh); GFN1_DENSE_N
-// overrides the default of 256.
+// Molecules above this many AOs run on groups of SMs (wide.cuh): the largest
+// matrix one SM's registers hold, or fewer with GFN1_DENSE_N.
 int dense_threshold() {
-  int n = 256;
+  int n = kSccKinds[2].p;
   if (const char* dn = std::getenv("GFN1_DENSE_N"))
-    if (*dn) n = std::max(2, std::atoi(dn));
+    if (*dn) n = std::min(n, std::max(2, std::atoi(dn)));
   return n;
 }
 
@@ -801,15 +804,6 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   for (int m = 0; m < nmol; ++m) h_order[m] = m;
   std::stable_sort(h_order, h_order + nmol, [&](int x, int y) { return n_m[x] > n_m[y]; });
   b->cap = std::max(1, std::min(std::max(o.scc_broyden_size, 2), o.max_scc));
-  // two size classes over the sorted order (class 0: N > kSplitN), each with its
-  // CTA size; 512 / nt CTAs share an SM, so several molecules interleave on it.
-  // Measured on the 4096-molecule batch (SCC stage, zero guess): one 512-thread
-  // CTA per SM above 96 AOs 141 ms, 256 threads 126 ms, 128 threads 113 ms,
-  // 64 threads 139 ms: four molecules per SM hide each other's barrier and
-  // latency stalls, while smaller CTAs lose too much per-molecule parallelism.
-  // A class whose vectors do not fit the per-CTA shared memory gets larger CTAs.
-  const int kSplitN = 96;
-  const int kClassNt[2] = {128, 128};
   // above kDenseN AOs one SM per molecule is too slow: those molecules run on
   // groups of SMs (wide.cuh).  GFN1_DENSE_N overrides the threshold (the tests
   // use it to run both paths on the same molecules).
@@ -857,64 +851,58 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   b->host_err_mol = -1;
   for (int m = 0; m < nmol && b->host_err_mol < 0; ++m)
     if (h_st[m] != GFN1_OK) b->host_err_mol = m;
-  int n_large = n_dense;
-  while (n_large < nmol && n_m[h_order[n_large]] > kSplitN) ++n_large;
   long long ws_total = 0;
-  for (int c = 0; c < 2; ++c) {
+  int q = n_dense;
+  for (int c = 0; c < 3; ++c) {  // one class per kernel, the largest molecules first
     gfn1_batch::SccClass& K = b->cls[c];
-    K.q_begin = c == 0 ? n_dense : n_large;
-    K.q_end = c == 0 ? n_large : nmol;
-    K.nt = kClassNt[c];
+    K.kind = 2 - c;
+    K.q_begin = q;
+    while (q < nmol && scc_kind(n_m[h_order[q]]) == K.kind) ++q;
+    K.q_end = q;
+    const int count = K.q_end - K.q_begin;
     K.maxn = K.maxnsh = K.maxnat = 0;
-    for (int q = K.q_begin; q < K.q_end; ++q) {
-      const int mm = h_order[q];
+    for (int i = K.q_begin; i < K.q_end; ++i) {
+      const int mm = h_order[i];
       K.maxn = std::max(K.maxn, n_m[mm]);
       K.maxnsh = std::max(K.maxnsh, nsh_m[mm]);
       K.maxnat = std::max(K.maxnat, atom_offsets[mm + 1] - atom_offsets[mm]);
     }
-    const int count = K.q_end - K.q_begin;
-    const size_t fixed = scc_smem_bytes(K.maxnsh, K.maxn, K.maxnat, 0);
-    while (K.nt < 512 && fixed > scc_max_dynamic_smem(K.nt)) K.nt *= 2;  // vectors of big molecules need room
-    K.n_cta = count == 0 ? 0 : std::max(1, std::min(count, (kSccThreadsPerSm / K.nt) * eng->num_sms));
+    // few small molecules: wider CTAs, as many as there are SM halves
+    if (K.kind == 0 && count <= kSccKinds[1].ctas * eng->num_sms) K.kind = 1;
+    K.n_cta = std::min(count, kSccKinds[K.kind].ctas * eng->num_sms);
     K.ws_stride = count == 0 ? 0 : scc_workspace_doubles(std::max(K.maxn, 1), std::max(K.maxnsh, 1), b->cap,
                                                            std::max(K.maxnat, 1));
     K.ws_offset = ws_total;
     ws_total += K.ws_stride * K.n_cta;
-    // Shared memory holds the index tables and vectors only; the working matrix
-    // stays in global memory, cached by the L1 that the small carve-out leaves
-    // (with four CTAs per SM this measured faster than giving each CTA room for
-    // the matrix: 98 vs 105 ms for the SCC stage of the 4096-molecule batch).
-    K.smem = fixed;
+    K.smem = scc_smem_bytes(K.kind, K.maxnsh, K.maxn, K.maxnat);
   }
   {  // fallback ladder: molecules the rung-0 launches leave unconverged, rerun by a few CTAs
     gfn1_batch::SccClass& R = b->robust;
     R.maxn = R.maxnsh = R.maxnat = 0;
-    for (int q = n_dense; q < nmol; ++q) {
-      const int mm = h_order[q];
+    for (int i = n_dense; i < nmol; ++i) {
+      const int mm = h_order[i];
       R.maxn = std::max(R.maxn, n_m[mm]);
       R.maxnsh = std::max(R.maxnsh, nsh_m[mm]);
       R.maxnat = std::max(R.maxnat, atom_offsets[mm + 1] - atom_offsets[mm]);
     }
     const int count = nmol - n_dense;
-    R.nt = 128;
-    const size_t fixed = scc_smem_bytes(R.maxnsh, R.maxn, R.maxnat, 0);
-    while (R.nt < 512 && fixed > scc_max_dynamic_smem(R.nt)) R.nt *= 2;
+    R.kind = scc_kind(R.maxn);
     // a requested level shift runs every molecule on this kernel: full width
-    const int width = o.level_shift != 0.0 ? (kSccThreadsPerSm / R.nt) * eng->num_sms : 64;
+    const int width = o.level_shift != 0.0 ? kSccKinds[R.kind].ctas * eng->num_sms : 64;
     R.n_cta = count == 0 ? 0 : std::min(count, width);
     R.ws_stride = count == 0 ? 0 : scc_workspace_doubles(std::max(R.maxn, 1), std::max(R.maxnsh, 1), b->cap,
                                                            std::max(R.maxnat, 1));
     R.ws_offset = ws_total;
     ws_total += R.ws_stride * R.n_cta;
-    R.smem = fixed;
+    R.smem = scc_smem_bytes(R.kind, R.maxnsh, R.maxn, R.maxnat);
   }
-  if (!b->side) {
-    if (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess)
+  if (!b->ev_fork && cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess)
+    return fail(eng, GFN1_E_DEVICE, "event creation failed");
+  for (int c = 0; c < 2; ++c)
+    if ((!b->side[c] && cudaStreamCreateWithFlags(&b->side[c], cudaStreamNonBlocking) != cudaSuccess) ||
+        (!b->ev_join[c] && cudaEventCreateWithFlags(&b->ev_join[c], cudaEventDisableTiming) != cudaSuccess))
       return fail(eng, GFN1_E_DEVICE, "stream creation failed");
-  }
-  bool ok = b->d_in.ensure(L.in_bytes) && b->d_out.ensure(L.out_bytes) && b->queue.ensure(4) &&
+  bool ok = b->d_in.ensure(L.in_bytes) && b->d_out.ensure(L.out_bytes) && b->queue.ensure(5) &&
             b->failed.ensure((size_t)nmol) &&
             b->stage.ensure(kStages) && b->S.ensure(mat_total) && b->H0.ensure(mat_total) && b->P.ensure(mat_total) &&
             b->W.ensure(mat_total) && b->ws.ensure((size_t)std::max<long long>(ws_total, 1)) && b->gam.ensure(gam_total) &&
@@ -966,7 +954,7 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
     // reset status from the host-validated copy and the work counter
     if ((e = cudaMemcpyAsync(B.status, b->din<int>(b->lay.status0), sizeof(int) * b->nmol, cudaMemcpyDeviceToDevice,
                              st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 4, st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b->queue.p, 0, sizeof(int) * 5, st)) != cudaSuccess ||
         (e = cudaMemsetAsync(B.rung, 0, sizeof(int) * b->nmol, st)) != cudaSuccess)
       return cuda_fail(eng, e, "batch reset");
     if (b->opt_skip && (e = launch_opt_skip(b->nmol, b->opt_skip, B.status, st)) != cudaSuccess)
@@ -1006,22 +994,23 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
     so.etemp = b->opt.electronic_temperature;
     so.spin_mult = b->opt.spin_multiplicity;
     so.level_shift = b->opt.level_shift;
-    // fork: the small-molecule class runs on the side stream next to the large one
-    if ((e = cudaEventRecord(b->ev_fork, st)) != cudaSuccess || (e = cudaStreamWaitEvent(b->side, b->ev_fork, 0)) != cudaSuccess)
-      return cuda_fail(eng, e, "stream fork");
+    // the first class with molecules runs on `st`, the others next to it on the
+    // side streams, which start after what `st` has so far
+    bool forked = false;
+    int used = 0;
     if (so.level_shift != 0.0 && b->n_shift > 0) {  // every molecule to the ladder kernel, from rung 0
       if ((e = cudaMemcpyAsync(b->failed.p, b->shift_list.p, sizeof(int) * b->n_shift, cudaMemcpyDeviceToDevice, st)) !=
               cudaSuccess ||
           (e = cudaMemcpyAsync(b->queue.p + 3, b->shift_count.p, sizeof(int), cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
         return cuda_fail(eng, e, "level-shift list");
     }
-    for (int c = 0; c < 2 && so.level_shift == 0.0; ++c) {
+    for (int c = 0; c < 3 && so.level_shift == 0.0; ++c) {
       const gfn1_batch::SccClass& K = b->cls[c];
       if (K.n_cta == 0) continue;
       SccLaunch SL;
       SL.q_begin = K.q_begin;
       SL.q_end = K.q_end;
-      SL.counter = b->queue.p + c;
+      SL.counter = b->queue.p + (c < 2 ? c : 4);
       SL.ws = b->ws.p + K.ws_offset;
       SL.ws_stride = K.ws_stride;
       SL.maxn = K.maxn;
@@ -1029,11 +1018,22 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
       SL.maxnat = K.maxnat;
       SL.cap = b->cap;
       SL.smem_bytes = (int)K.smem;
-      if ((e = launch_scc(K.nt, K.n_cta, K.smem, c == 0 ? st : b->side, B, M, so, SL)) != cudaSuccess)
+      bool more = false;
+      for (int c2 = c + 1; c2 < 3; ++c2) more = more || b->cls[c2].n_cta > 0;
+      if (!forked && more) {
+        if ((e = cudaEventRecord(b->ev_fork, st)) != cudaSuccess) return cuda_fail(eng, e, "stream fork");
+        forked = true;
+      }
+      cudaStream_t ks = used == 0 ? st : b->side[used - 1];
+      if (used > 0 && (e = cudaStreamWaitEvent(ks, b->ev_fork, 0)) != cudaSuccess) return cuda_fail(eng, e, "stream fork");
+      if ((e = launch_scc(K.kind, K.n_cta, K.smem, ks, B, M, so, SL)) != cudaSuccess)
         return cuda_fail(eng, e, "scc launch");
+      if (used > 0 && (e = cudaEventRecord(b->ev_join[used - 1], ks)) != cudaSuccess)
+        return cuda_fail(eng, e, "stream join");
+      ++used;
     }
-    if ((e = cudaEventRecord(b->ev_join, b->side)) != cudaSuccess || (e = cudaStreamWaitEvent(st, b->ev_join, 0)) != cudaSuccess)
-      return cuda_fail(eng, e, "stream join");
+    for (int c = 0; c + 1 < used; ++c)
+      if ((e = cudaStreamWaitEvent(st, b->ev_join[c], 0)) != cudaSuccess) return cuda_fail(eng, e, "stream join");
     if (b->robust.n_cta > 0) {  // rungs 1-3 for whatever rung 0 left unconverged (exits at once if nothing)
       const gfn1_batch::SccClass& R = b->robust;
       SccLaunch SL;
@@ -1047,7 +1047,7 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
       SL.maxnat = R.maxnat;
       SL.cap = b->cap;
       SL.smem_bytes = (int)R.smem;
-      if ((e = launch_scc_robust(R.nt, R.n_cta, R.smem, st, B, M, so, SL)) != cudaSuccess)
+      if ((e = launch_scc_robust(R.kind, R.n_cta, R.smem, st, B, M, so, SL)) != cudaSuccess)
         return cuda_fail(eng, e, "scc fallback launch");
     }
     if (!b->wide_ids.empty()) {  // large molecules on groups of SMs, after the one-SM classes
@@ -1357,7 +1357,7 @@ int gfn1_batch_info(const gfn1_batch* b, int64_t* natoms, int64_t* nshells, int6
   if (naos) *naos = b->naos;
   if (launches) {  // setup, one SCC launch per non-empty size class, the fallback ladder, gradient, learned guess
     const int nd = b->n_dense, ns = b->nmol - nd;  // (the large-molecule SCC launches vary with its iterations)
-    *launches = (ns > 0) + (nd > 0) + (b->cls[0].n_cta > 0) + (b->cls[1].n_cta > 0) + (b->robust.n_cta > 0) +
+    *launches = (ns > 0) + (nd > 0) + (b->cls[0].n_cta > 0) + (b->cls[1].n_cta > 0) + (b->cls[2].n_cta > 0) + (b->robust.n_cta > 0) +
                 (b->opt.compute_gradient ? (ns > 0) + 2 * (nd > 0) : 0) + (b->guess && !b->has_init_q ? 3 : 0);
   }
   return GFN1_OK;
@@ -1825,8 +1825,9 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   so.spin_mult = o.spin_multiplicity;
   so.level_shift = 0.0;
   const size_t sm_setup = sizeof(double) * (16 * (size_t)nat + 32) + sizeof(int) * (3 * (size_t)nat + 2 + 2 * (size_t)nsh);
-  const size_t sm_scc = std::max(scc_smem_bytes(nsh, n, nat, 0),
-                                 std::min(scc_smem_bytes(nsh, n, nat, n), scc_max_dynamic_smem(n > 96 ? 512 : 256)));
+  constexpr int kNaKind = 1;  // 256 threads, up to 128 AOs in registers
+  static_assert(kSccKinds[kNaKind].p >= kNaMaxAo, "the no-allocation path's largest molecule");
+  const size_t sm_scc = scc_smem_bytes(kNaKind, nsh, n, nat);
   const size_t sm_grad = sizeof(double) * 7 * (size_t)nat + sizeof(int) * (3 * (size_t)nat + 2);
   if (use_guess) {  // predicted shell charges into the initial-charge slot of the input region
     const GuessModel& g = eng->guess->model;
@@ -1852,7 +1853,7 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   SL.maxnat = nat;
   SL.cap = cap;
   SL.smem_bytes = (int)sm_scc;
-  if ((e = launch_scc(n > 96 ? 512 : 256, 1, sm_scc, st, B, M, so, SL)) != cudaSuccess)
+  if ((e = launch_scc(kNaKind, 1, sm_scc, st, B, M, so, SL)) != cudaSuccess)
     return cuda_fail(eng, e, "scc launch");
   if (o.compute_gradient && (e = launch_grad(2, dim3(1), sm_grad, st, B, M, nullptr, 3)) != cudaSuccess)
     return cuda_fail(eng, e, "gradient launch");

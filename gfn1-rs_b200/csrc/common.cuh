@@ -127,17 +127,18 @@ struct Batch {
   int* rung;                // [nmol] fallback-ladder rung whose SCC converged (-1: none), or null
   double* orb_eps;          // [naos] orbital energies of the last diagonalisation (offset ao_off[m]), or null
   double* orb_occ;          // [naos] their occupations, or null
-  int* queue;               // work counters: [0], [1] size classes, [2] fallback ladder, [3] failed count
+  int* queue;               // work counters: [0], [1], [4] size classes, [2] fallback ladder, [3] failed count
   int* failed;              // [nmol] molecules whose first SCC attempt did not converge, or null
   unsigned long long* stage_cycles;  // [kStages] per-stage clock totals, or null
 };
 
-// Threads of the persistent SCC kernel resident per SM: 128-thread CTAs run
-// kSccThreadsPerSm / 128 to an SM (the register budget per thread follows).
-#ifndef GFN1_SCC_THREADS_PER_SM
-#define GFN1_SCC_THREADS_PER_SM 512
-#endif
-constexpr int kSccThreadsPerSm = GFN1_SCC_THREADS_PER_SM;
+// Instantiations of the persistent SCC kernel: threads per CTA, the largest
+// matrix whose Householder reduction the CTA keeps on chip, and the CTAs per SM the register budget is sized for (512 threads at 128 registers, or 256
+// threads at 255).  A molecule runs on the first one that holds its matrix.
+struct SccKind {
+  int nt, p, ctas;
+};
+constexpr SccKind kSccKinds[3] = {{128, 64, 4}, {256, 128, 2}, {256, 192, 1}};
 
 // SCC stages timed when Batch::stage_cycles is set (the device counterpart of
 // the reference's GFN1_PROFILE scopes, src/electronic.rs:1448, :2089-2157).

@@ -1,15 +1,19 @@
 // Persistent SCC kernel: each CTA pulls molecules from a work queue (most
 // expensive first) and runs the complete self-consistent-charge loop of
 // gfn1-rs `run_scc_with_core` (src/electronic.rs:849-2054, plain charge-vector
-// branch, ladder rung 0) on the device.  The batch path launches two size
-// classes concurrently (above and below 96 AOs), both with 128-thread CTAs and
-// four CTAs per SM; shared memory holds the index tables and N-vectors, and the
-// eigensolver's working matrix lives in the CTA's global workspace slot, cached
-// by L1.  Up to 193 AOs the Householder reduction is blocked (8-column panels,
-// tensor-core trailing updates); the prologue's Cholesky is left-looking over
-// 8-column panels.  Wider CTAs (256/512 threads) and a working
-// matrix in shared memory are used only by the allocation-free single-molecule
-// entry point, which passes the room for it in the launch's shared memory.
+// branch, ladder rung 0) on the device.  Three instantiations run side by side,
+// each with the molecules whose matrix its CTA keeps on chip for the Householder
+// reduction (kSccKinds in common.cuh): up to 64 AOs on 128-thread CTAs, four per
+// SM; up to 128 on 256 threads, two per SM; up to 192 on 256 threads, one per SM
+// (more CTAs per SM hide barriers and latencies better, but a reduction that
+// fetches its matrix from L1 per column costs more: 128-thread CTAs, four per SM
+// at every size, took 60.5 ms for the SCC of the 4096-molecule batch, these
+// 42.4).  A batch with few small molecules runs them on 256 threads.  Shared
+// memory holds the molecule's state, the index tables, the N-vectors and the
+// scratch of the reduction and of the back-transformation; the matrices live in
+// the CTA's global workspace slot.  The stages are functions of their own that
+// read the molecule's state from shared memory, so that each has the whole
+// register budget.
 //
 // Algorithmic choices that differ from the reference but give the same results
 // up to FP64 rounding:
@@ -19,12 +23,13 @@
 //    the potential term  -1/2 (M + M^T),  M = L^-1 diag(v) L  (lower triangular),
 //    because  L^-1 (S o V) L^-T = L^-1 diag(v) L + (L^-1 diag(v) L)^T  for
 //    V_mu,nu = v_mu + v_nu (src/electronic.rs:3133-3158).
-//  * eigensolver: Householder tridiagonalisation (three barriers per column in
-//    the blocked form), Sturm counts plus Laguerre steps, warm-started from
-//    the previous iteration, for the eigenvalues the occupations need,
-//    inverse iteration (with modified Gram-Schmidt inside eigenvalue clusters)
-//    for the occupied eigenvectors only, and a blocked (compact-WY)
-//    back-transformation (replaces faer's self_adjoint_eigen, src/linalg.rs:153-191).
+//  * eigensolver: Householder tridiagonalisation with the matrix on chip
+//    (tridiag.cuh), Sturm counts shared by the CTA plus Laguerre steps,
+//    warm-started from the previous iteration, for the eigenvalues the
+//    occupations need, twisted factorisations (inverse iteration with modified
+//    Gram-Schmidt inside eigenvalue clusters) for the occupied eigenvectors only,
+//    and a compact-WY back-transformation with the orbitals in registers
+//    (orbitals.cuh; replaces faer's self_adjoint_eigen, src/linalg.rs:153-191).
 //  * electronic energy: tr(H0 P) = sum_i f_i eps_i + sum_mu v_mu (S P)_mu,mu,
 //    which holds exactly for the F that was diagonalised, so P is only formed once
 //    the SCC has converged (src/electronic.rs:3182-3188, :2173-2191).
@@ -37,19 +42,20 @@
 
 #include "common.cuh"
 #include "model.cuh"
+#include "orbitals.cuh"
+#include "tridiag.cuh"
 
 namespace gfn1 {
 
 constexpr double kBoltzmann = 3.1668115634556e-6;  // src/constants.rs:26
-constexpr int kVecSlots = 9;                          // N-length vectors kept in shared memory
-constexpr int kBackNB = 16;                           // reflectors per compact-WY block
+constexpr int kVecSlots = 8;  // N-length vectors kept in shared memory
 
 struct SccShared {
   double red[32];
   double scal[16];
   int iscal[16];
-  double Tm[kBackNB][kBackNB];
-  double VtV[kBackNB][kBackNB];
+  double Ld[8][9];      // Cholesky: diagonal block and reciprocal pivots
+  int first[2][16];     // occupations: each warp's first trial level that holds the electrons
 };
 
 // Per-stage clock accounting by thread 0 of the CTA (no-op without a buffer).
@@ -75,38 +81,37 @@ struct StageClock {
 
 // Layout of one CTA's global workspace slot (doubles).
 struct CtaWs {
-  double *L, *Li, *Hp, *A, *Z, *C, *D, *iw, *W1, *W2;
+  double *L, *LiT, *Hp, *F, *Z, *Ct, *V, *iw, *popw;
   double *df, *u, *dots, *omega, *beta, *cvec, *qin, *qout, *vsh, *qlast, *dqlast, *qnext, *vout, *qat;
 };
-// Leading dimension of the working matrix: odd in shared memory (strided
-// column accesses spread over the banks), a multiple of four doubles in global
-// memory (every row starts on a 32-byte sector).
-__host__ __device__ inline int work_lda(int n) { return (n & 1) ? n : n + 1; }
-__host__ __device__ inline int work_lda_global(int n) { return (n + 3) & ~3; }
+// Leading dimension of the matrices: whole 8 x 8 tiles.
+__host__ __device__ inline int work_ld(int n) { return (n + 7) & ~7; }
+// Reflectors of the register-resident reduction: rows padded to 32 columns, and
+// room for zero rows up to a multiple of 16.
+__host__ __device__ inline int refl_ld(int n) { return (n + 31) & ~31; }
+__host__ __device__ inline long long refl_size(int n) { return (long long)(n + 16) * refl_ld(n); }
+constexpr int kMaxSccWarps = 8;
 
-// Slot sizes in doubles; the slot size is a multiple of four and the working
-// matrix A starts on a multiple of four (slots start 32-byte aligned).
+// Slot sizes in doubles; every matrix starts on a 32-byte boundary.
 __host__ __device__ inline long long cta_ws_size(int maxn, int maxnsh, int cap, int maxnat) {
-  const long long n2 = (long long)maxn * (maxn + 1);
-  const long long na = (long long)maxn * work_lda_global(maxn);
-  const long long t = 11 * n2 + na + 4 + 2LL * kBackNB * maxn + 2LL * cap * maxnsh + 2LL * cap * cap + 2LL * cap +
-                      8LL * maxnsh + maxnat + 64;
+  const long long n2 = (long long)work_ld(maxn) * work_ld(maxn);
+  const long long t = 11 * n2 + refl_size(maxn) + (long long)kMaxSccWarps * work_ld(maxn) + 2LL * cap * maxnsh +
+                      2LL * cap * cap + 2LL * cap + 8LL * maxnsh + maxnat + 64;
   return (t + 3) & ~3LL;
 }
 __device__ __forceinline__ CtaWs cta_ws(double* base, int maxn, int maxnsh, int cap) {
   CtaWs w;
-  const long long n2 = (long long)maxn * (maxn + 1);
+  const long long n2 = (long long)work_ld(maxn) * work_ld(maxn);
   w.L = base;
-  w.Li = w.L + n2;
-  w.Hp = w.Li + n2;
-  w.A = base + ((3 * n2 + 3) & ~3LL);
-  w.Z = w.A + (long long)maxn * work_lda_global(maxn);
-  w.C = w.Z + n2;
-  w.D = w.C + n2;
-  w.iw = w.D + n2;  // 5 * n2
-  w.W1 = w.iw + 5 * n2;
-  w.W2 = w.W1 + (long long)kBackNB * maxn;
-  w.df = w.W2 + (long long)kBackNB * maxn;
+  w.LiT = w.L + n2;
+  w.Hp = w.LiT + n2;
+  w.F = w.Hp + n2;
+  w.Z = w.F + n2;
+  w.Ct = w.Z + n2;
+  w.iw = w.Ct + n2;  // 5 * n2
+  w.V = w.iw + 5 * n2;
+  w.popw = w.V + refl_size(maxn);
+  w.df = w.popw + (long long)kMaxSccWarps * work_ld(maxn);
   w.u = w.df + (long long)cap * maxnsh;
   w.dots = w.u + (long long)cap * maxnsh;
   w.beta = w.dots + (long long)cap * cap;
@@ -126,9 +131,16 @@ __device__ __forceinline__ CtaWs cta_ws(double* base, int maxn, int maxnsh, int 
 __host__ __device__ inline int scc_ints(int maxnsh, int maxn, int maxnat) {
   return 3 * maxnsh + maxn + maxnat + 1;
 }
+// Byte offset of the N-vectors in the SCC kernel's dynamic shared memory: after
+// the CTA's state and the index tables.
+struct SccCta;
+__host__ __device__ constexpr size_t scc_cta_bytes();
+__host__ __device__ inline size_t scc_vec_bytes(int maxnsh, int maxn, int maxnat) {
+  return (scc_cta_bytes() + (size_t)4 * scc_ints(maxnsh, maxn, maxnat) + 15) & ~(size_t)15;
+}
 __host__ __device__ inline size_t scc_smem_fixed(int maxnsh, int maxn, int maxnat) {
-  const size_t ib = ((size_t)4 * scc_ints(maxnsh, maxn, maxnat) + 15) & ~(size_t)15;
-  return ib + sizeof(double) * kVecSlots * (size_t)maxn;
+  const size_t ib = scc_vec_bytes(maxnsh, maxn, maxnat);
+  return ib + sizeof(double) * ((kVecSlots * (size_t)maxn + 1) & ~(size_t)1);
 }
 
 // Sturm count and characteristic polynomial at x for the symmetric tridiagonal
@@ -138,7 +150,7 @@ __host__ __device__ inline size_t scc_smem_fixed(int maxnsh, int maxn, int maxna
 // is LAPACK dlaebz's ratio recurrence q_i = p_i / p_{i-1} multiplied through by
 // p_{i-1}, so the count (the number of negative q_i) is the same but the loop
 // needs no division.  The pair (p_i, p_{i-1}) and its derivatives are rescaled
-// by an exact power of two every 4 steps.  The pivot guard |q_i| < pivmin sets
+// by an exact power of two every 8 steps.  The pivot guard |q_i| < pivmin sets
 // q_i = -2^-600 (LAPACK: -pivmin; the two differ only when e_i^2 < 2^-600 |d_i -
 // x|, an exact split) and moves the pair to a scale where |p_i| is near 1.  The
 // derivatives may overflow; they only steer the Laguerre step.
@@ -147,59 +159,140 @@ __device__ __forceinline__ double pow2_inv_scale(double m) {  // 2^-floor(log2 m
   const long long sc = 1023 - (ex < -1000 ? -1000 : (ex > 1000 ? 1000 : ex));
   return __longlong_as_double(sc << 52);
 }
+struct SturmState {
+  double p, pm, dp, dpm, ddp, ddpm;
+  int c;
+};
+// One step with the pivot guard.
+__device__ __forceinline__ void sturm_step(SturmState& s, double t, double e2, double pivmin) {
+  constexpr double kGuardScale = 0x1p600;
+  double pn = fma(t, s.p, -(e2 * s.pm));
+  double dpn = fma(t, s.dp, fma(-e2, s.dpm, -s.p));
+  double ddpn = fma(t, s.ddp, fma(-e2, s.ddpm, -2.0 * s.dp));
+  if (fabs(pn) <= pivmin * fabs(s.p)) {
+    const double sc = pow2_inv_scale(fabs(s.p)) * kGuardScale;
+    pn = s.p * -pow2_inv_scale(fabs(s.p));
+    s.p = pn * -kGuardScale;
+    s.dp *= sc;
+    dpn *= sc;
+    s.ddp *= sc;
+    ddpn *= sc;
+  }
+  s.c += (pn > 0.0) != (s.p > 0.0);
+  s.pm = s.p;
+  s.p = pn;
+  s.dpm = s.dp;
+  s.dp = dpn;
+  s.ddpm = s.ddp;
+  s.ddp = ddpn;
+}
+__device__ __forceinline__ int exp_bits(double x) { return __double2hiint(x) & 0x7ff00000; }
+// G steps and a rescale.  The guard's test and branch after every step would
+// take most of the time (96 cycles a step, where a multiply-add's latency is 8).
+// The pair (p, pm) starts a group at a scale near 1 and the guard needs
+// |pn| <= pivmin |p| ~ 2^-1022, so a group whose values all stay above 2^-700 has
+// none; otherwise the group is done step by step.
+template <int G>
+__device__ __forceinline__ void sturm_group(SturmState& s, const double (&t)[8], const double (&e2)[8], double pivmin) {
+  double a = s.p, b = s.pm, da = s.dp, db = s.dpm, va = s.ddp, vb = s.ddpm;
+  int low = 0x7ff00000, c = 0;
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    const double q = fma(t[i], a, -(e2[i] * b));
+    const double u = fma(t[i], da, fma(-e2[i], db, -a));
+    const double v = fma(t[i], va, fma(-e2[i], vb, -2.0 * da));
+    c += (unsigned)(__double2hiint(q) ^ __double2hiint(a)) >> 31;
+    low = min(low, exp_bits(q));
+    b = a;
+    a = q;
+    db = da;
+    da = u;
+    vb = va;
+    va = v;
+  }
+  if (low >= (1023 - 700) << 20) {
+    s.p = a;
+    s.pm = b;
+    s.dp = da;
+    s.dpm = db;
+    s.ddp = va;
+    s.ddpm = vb;
+    s.c += c;
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < G; ++i) {
+      double ti = t[0], ei = e2[0];
+#pragma unroll
+      for (int j = 1; j < G; ++j)
+        if (j == i) {
+          ti = t[j];
+          ei = e2[j];
+        }
+      sturm_step(s, ti, ei, pivmin);
+    }
+  }
+  // exact power of two; (p, pm) is never zero
+  const int ex = max(exp_bits(s.p), exp_bits(s.pm));
+  const double sc = __hiloint2double(min(max(0x7fe00000 - ex, 23 << 20), 2023 << 20), 0);
+  s.p *= sc;
+  s.pm *= sc;
+  s.dp *= sc;
+  s.dpm *= sc;
+  s.ddp *= sc;
+  s.ddpm *= sc;
+}
 __device__ __forceinline__ int sturm_poly(const double* d, const double* esq, int n, double x, double pivmin,
                                           double& pout, double& dpout, double& ddpout) {
-  constexpr double kGuardScale = 0x1p600;
-  double pm = 1.0, p = d[0] - x, dpm = 0.0, dp = -1.0, ddpm = 0.0, ddp = 0.0;
-  if (fabs(p) < pivmin) {
-    p = -1.0;
-    pm = kGuardScale;
-    dp = -kGuardScale;
+  SturmState s{d[0] - x, 1.0, -1.0, 0.0, 0.0, 0.0, 0};
+  if (fabs(s.p) < pivmin) {
+    constexpr double kGuardScale = 0x1p600;
+    s.p = -1.0;
+    s.pm = kGuardScale;
+    s.dp = -kGuardScale;
   }
-  int c = p <= 0.0;
-  auto step = [&](double t, double e2) {
-    double pn = t * p - e2 * pm;
-    double dpn = t * dp - p - e2 * dpm;
-    double ddpn = t * ddp - 2.0 * dp - e2 * ddpm;
-    if (fabs(pn) <= pivmin * fabs(p)) {
-      const double s = pow2_inv_scale(fabs(p)) * kGuardScale;
-      pn = p * -pow2_inv_scale(fabs(p));
-      p = pn * -kGuardScale;
-      dp *= s;
-      dpn *= s;
-      ddp *= s;
-      ddpn *= s;
+  s.c = s.p <= 0.0;
+  double t[8], e2[8], tn[8], en[8];
+  auto load = [&](int i, double (&tt)[8], double (&ee)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = min(i + j, n - 1);
+      tt[j] = d[k] - x;
+      ee[j] = esq[max(k, 1) - 1];
     }
-    c += (pn > 0.0) != (p > 0.0);
-    pm = p;
-    p = pn;
-    dpm = dp;
-    dp = dpn;
-    ddpm = ddp;
-    ddp = ddpn;
   };
   int i = 1;
-  // groups of four steps with the loads issued first, then a rescale
-  for (; i + 3 < n; i += 4) {
-    const double t0 = d[i] - x, t1 = d[i + 1] - x, t2 = d[i + 2] - x, t3 = d[i + 3] - x;
-    const double e0 = esq[i - 1], e1 = esq[i], e2 = esq[i + 1], e3 = esq[i + 2];
-    step(t0, e0);
-    step(t1, e1);
-    step(t2, e2);
-    step(t3, e3);
-    const double sc = pow2_inv_scale(fmax(fabs(p), fabs(pm)));
-    p *= sc;
-    pm *= sc;
-    dp *= sc;
-    dpm *= sc;
-    ddp *= sc;
-    ddpm *= sc;
+  load(1, t, e2);
+  for (; i + 7 < n; i += 8) {  // the next group's entries are fetched before this one's steps
+    load(i + 8, tn, en);
+    sturm_group<8>(s, t, e2, pivmin);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      t[j] = tn[j];
+      e2[j] = en[j];
+    }
   }
-  for (; i < n; ++i) step(d[i] - x, esq[i - 1]);
-  pout = p;
-  dpout = dp;
-  ddpout = ddp;
-  return c;
+  if (i + 3 < n) {
+    sturm_group<4>(s, t, e2, pivmin);
+    i += 4;
+    t[0] = t[4];
+    t[1] = t[5];
+    t[2] = t[6];
+    e2[0] = e2[4];
+    e2[1] = e2[5];
+    e2[2] = e2[6];
+  }
+#pragma unroll 1
+  for (; i < n; ++i) {  // at most three
+    sturm_step(s, t[0], e2[0], pivmin);
+    t[0] = t[1];
+    e2[0] = e2[1];
+    t[1] = t[2];
+    e2[1] = e2[2];
+  }
+  pout = s.p;
+  dpout = s.dp;
+  ddpout = s.ddp;
+  return s.c;
 }
 
 __device__ __forceinline__ double hash_unit(unsigned a, unsigned b) {
@@ -391,417 +484,6 @@ __device__ double tri_factor_rhs(const double* d, const double* e, int n, double
 
 // ---------------------------------------------------------------- stages
 
-// Householder reduction of the symmetric A (full storage, leading dimension lda)
-// to tridiagonal (d, e); reflector k is kept in row k right of the diagonal
-// with its factor in tau[k] (H_k = I - tau_k v v^T).  Two barriers per column:
-// the matrix-vector product and the p.v partial sums, then the rank-2 update,
-// during which warp 0 also forms the norm of the next pivot row.
-// Four interleaved warp reductions (their shuffle latencies overlap).
-__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-    d += __shfl_xor_sync(0xffffffffu, d, o);
-  }
-}
-
-// D += A B for one 8x8x4 FP64 tile on the tensor cores (PTX mma.m8n8k4 .f64,
-// row-major A, column-major B): lane l holds A[l/4][l%4], B[l%4][l/4] and
-// D[l/4][2(l%4)], D[l/4][2(l%4)+1].
-__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
-// Householder reduction of the symmetric A (full storage, leading dimension
-// lda) to tridiagonal form: d, e, reflector scalars tau, and the reflector of
-// column k in row k (entries k+1..N-1).  Per column: p = beta A22 v by warps
-// over rows (four rows at a time, lanes over columns), one barrier, then the
-// rank-2 update A22 -= v w^T + w v^T with w = p - K v, which also yields the
-// norm of the next column; a second barrier.  While the trailing size is at
-// most 32 * kCols, each lane keeps v_j and w_j of its columns in registers, so
-// the update reads and writes each element once.
-// One column of the Householder reduction after its reflector (v0, beta,
-// alpha) is known: p = beta A22 v, the rank-2 update and the norm of the next
-// column, which it returns.  Cached: the trailing size fits 32 * kCols and each
-// lane keeps its columns of v and w in registers.
-template <int NT, bool Cached>
-__device__ __forceinline__ double householder_column(double* A, int lda, int N, int k, double v0, double beta,
-                                                     double alpha, double* d, double* e, double* tau, double* pvec,
-                                                     SccShared& sh) {
-  constexpr int NW = NT / 32;
-  constexpr int kCols = 6;
-  constexpr bool cached = Cached;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int m = N - k - 1;
-  double* rowk = A + (long long)k * lda + (k + 1);
-  double* a22 = A + (long long)(k + 1) * lda + (k + 1);
-  double vreg[kCols], wreg[kCols];
-#pragma unroll
-  for (int c = 0; c < kCols; ++c) {
-    const int j = lane + 32 * c;
-    vreg[c] = (cached && j < m) ? (j == 0 ? v0 : rowk[j]) : 0.0;
-  }
-  // p = beta A22 v
-  double pv_part = 0.0;
-  for (int i0 = wid; i0 < m; i0 += 4 * NW) {
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    if (cached) {
-#pragma unroll
-      for (int c = 0; c < kCols; ++c) {
-        const int j = lane + 32 * c;
-        if (j < m) {
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int i = i0 + r * NW;
-            if (i < m) s[r] += a22[(long long)i * lda + j] * vreg[c];
-          }
-        }
-      }
-    } else {
-      for (int j = lane; j < m; j += 32) {
-        const double v = (j == 0) ? v0 : rowk[j];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int i = i0 + r * NW;
-          if (i < m) s[r] += a22[(long long)i * lda + j] * v;
-        }
-      }
-    }
-    warp_sum4(s[0], s[1], s[2], s[3]);
-    if (lane == 0) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = i0 + r * NW;
-        if (i < m) {
-          const double pi = beta * s[r];
-          pvec[i] = pi;
-          pv_part += pi * (i == 0 ? v0 : rowk[i]);
-        }
-      }
-    }
-  }
-  if (lane == 0) sh.red[wid] = pv_part;
-  __syncthreads();
-  double pv = 0.0;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) pv += sh.red[w];
-  const double K = 0.5 * beta * pv;
-  if (tid == 0) {
-    d[k] = A[(long long)k * lda + k];
-    e[k] = alpha;
-    tau[k] = beta;
-  }
-#pragma unroll
-  for (int c = 0; c < kCols; ++c) {
-    const int j = lane + 32 * c;
-    wreg[c] = (cached && j < m) ? pvec[j] - K * vreg[c] : 0.0;
-  }
-  // A22 -= v w^T + w v^T; warp 0 also takes the norm of the next column (row 1 of A22 from entry 1)
-  double nrm = 0.0;
-  for (int i = wid; i < m; i += NW) {
-    double* brow = a22 + (long long)i * lda;
-    const double vi = (i == 0) ? v0 : rowk[i];
-    const double wi = pvec[i] - K * vi;
-    if (cached) {
-#pragma unroll
-      for (int c = 0; c < kCols; ++c) {
-        const int j = lane + 32 * c;
-        if (j < m) {
-          const double nb = brow[j] - (vi * wreg[c] + wi * vreg[c]);
-          brow[j] = nb;
-          if (i == 0 && j >= 1) nrm += nb * nb;
-        }
-      }
-    } else {
-      for (int j = lane; j < m; j += 32) {
-        const double vj = (j == 0) ? v0 : rowk[j];
-        const double wj = pvec[j] - K * vj;
-        const double nb = brow[j] - (vi * wj + wi * vj);
-        brow[j] = nb;
-        if (i == 0 && j >= 1) nrm += nb * nb;
-      }
-    }
-  }
-  if (wid == 0) {
-    nrm = warp_sum(nrm);
-    if (lane == 0) sh.scal[3] = nrm;
-  }
-  __syncthreads();
-  if (tid == 0) rowk[0] = v0;  // the reflector of column k is row k from entry k+1
-  return sh.scal[3];
-}
-
-// The large-trailing-size column out of line, so that the hot loop of the
-// usual sizes stays compact.
-template <int NT>
-__device__ __noinline__ double householder_column_wide(double* A, int lda, int N, int k, double v0, double beta,
-                                                       double alpha, double* d, double* e, double* tau, double* pvec,
-                                                       SccShared& sh) {
-  return householder_column<NT, false>(A, lda, N, k, v0, beta, alpha, d, e, tau, pvec, sh);
-}
-
-template <int NT>
-__device__ void tridiagonalize(double* A, int lda, int N, double* d, double* e, double* tau, double* pvec,
-                               SccShared& sh) {
-  constexpr int kCols = 6;
-  const int tid = threadIdx.x;
-  double part = 0.0;
-  if (N >= 3)
-    for (int j = 1 + tid; j < N; j += NT) part += A[j] * A[j];
-  double xn2 = block_sum(part, sh.red);
-  for (int k = 0; k < N - 2; ++k) {
-    const int m = N - k - 1;
-    const double* rowk = A + (long long)k * lda + (k + 1);
-    const double x0 = rowk[0];
-    const double tail = xn2 - x0 * x0;
-    if (tail == 0.0) {  // column already reduced
-      __syncthreads();
-      if (tid == 0) {
-        d[k] = A[(long long)k * lda + k];
-        e[k] = x0;
-        tau[k] = 0.0;
-      }
-      double p2 = 0.0;
-      const double* nrow = A + (long long)(k + 1) * lda;
-      for (int j = k + 2 + tid; j < N; j += NT) p2 += nrow[j] * nrow[j];
-      xn2 = block_sum(p2, sh.red);
-      continue;
-    }
-    const double xn = sqrt(xn2);
-    const double alpha = x0 >= 0.0 ? -xn : xn;
-    const double v0 = x0 - alpha;
-    const double beta = 2.0 / (v0 * v0 + tail);
-    xn2 = (m <= 32 * kCols) ? householder_column<NT, true>(A, lda, N, k, v0, beta, alpha, d, e, tau, pvec, sh)
-                            : householder_column_wide<NT>(A, lda, N, k, v0, beta, alpha, d, e, tau, pvec, sh);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    if (N >= 2) {
-      d[N - 2] = A[(long long)(N - 2) * lda + (N - 2)];
-      e[N - 2] = A[(long long)(N - 1) * lda + (N - 2)];
-      tau[N - 2] = 0.0;
-    }
-    d[N - 1] = A[(long long)(N - 1) * lda + (N - 1)];
-    e[N - 1] = 0.0;
-    tau[N - 1] = 0.0;
-  }
-  __syncthreads();
-}
-
-// Blocked Householder reduction (panels of kPanel columns, four-warp CTAs, at
-// most 32 * 6 + 1 rows): the same reflectors as tridiagonalize, but the rank-2
-// updates of a panel are applied lazily to each panel column and, at the end
-// of the panel, to the trailing matrix in one FP64 tensor-core pass,
-// A22 -= V W^T + W V^T.  Per column: the column with the panel's earlier
-// updates (x), its reflector (stored in row k as before), p = beta (A22 v -
-// V (W^T v) - W (V^T v)) with A22 as of the panel start, and w = p - K v kept
-// in Wp (kPanel x N, row l for the panel's column l).  V is read from the
-// reflector rows of A.  xs and pvec are N-vectors of scratch.  A is the
-// global working matrix (32-byte aligned, lda a multiple of four).
-constexpr int kPanel = 8;
-template <int NT>
-__device__ void tridiagonalize_blocked(double* A, int lda, int N, double* d, double* e, double* tau, double* pvec,
-                                       double* xs, double* Wp, SccShared& sh) {
-  constexpr int NW = NT / 32;
-  constexpr int kCols = 6;
-  static_assert(NW == 4, "four warps");
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
-  for (int k0 = 0; k0 < N - 2; k0 += kPanel) {
-    const int nbp = min(kPanel, N - 2 - k0);
-    // W of the previous column at row k, which thread 0 wrote: every thread
-    // forms it itself, so that the column needs no barrier after W is stored
-    double w_last = 0.0;
-    for (int j = 0; j < nbp; ++j) {
-      const int k = k0 + j, m = N - k - 1;
-      // x: row k (= column k) from the diagonal, with the panel's earlier updates
-      double part = 0.0;
-      for (int t = tid; t <= m; t += NT) {
-        const int i = k + t;
-        double x = A[(long long)k * lda + i];
-#pragma unroll 4
-        for (int l = 0; l < j; ++l) {
-          const double* vl = A + (long long)(k0 + l) * lda;
-          const double* wl = Wp + (long long)l * N;
-          const double wk = (l == j - 1) ? w_last : wl[k];
-          x -= vl[k] * wl[i] + wk * vl[i];
-        }
-        xs[t] = x;
-        if (t >= 1) part += x * x;
-      }
-      part = warp_sum(part);
-      if (lane == 0) sh.red[wid] = part;
-      __syncthreads();
-      const double xn2 = (sh.red[0] + sh.red[1]) + (sh.red[2] + sh.red[3]);
-      const double x0 = xs[1];
-      const double tail = xn2 - x0 * x0;
-      if (tid == 0) d[k] = xs[0];
-      if (tail == 0.0) {  // column already reduced: no reflector, W column zero
-        for (int t = tid; t < m; t += NT) {
-          A[(long long)k * lda + k + 1 + t] = xs[1 + t];
-          Wp[(long long)j * N + k + 1 + t] = 0.0;
-        }
-        if (tid == 0) {
-          e[k] = x0;
-          tau[k] = 0.0;
-        }
-        w_last = 0.0;
-        __syncthreads();
-        continue;
-      }
-      const double xn = sqrt(xn2);
-      const double alpha = x0 >= 0.0 ? -xn : xn;
-      const double v0 = x0 - alpha;
-      const double beta = 2.0 / (v0 * v0 + tail);
-      double vreg[kCols];
-#pragma unroll
-      for (int c = 0; c < kCols; ++c) {
-        const int jj = lane + 32 * c;
-        vreg[c] = jj < m ? (jj == 0 ? v0 : xs[1 + jj]) : 0.0;
-      }
-      if (wid == 0) {  // the reflector of column k is row k from entry k+1
-#pragma unroll
-        for (int c = 0; c < kCols; ++c) {
-          const int jj = lane + 32 * c;
-          if (jj < m) A[(long long)k * lda + k + 1 + jj] = vreg[c];
-        }
-      }
-      // raw A22 v: A22 is kept symmetric, so entry t is column t of A22
-      // dotted with v, and each row of A22 read across the threads is
-      // contiguous (no cross-lane sums); v from shared memory.  Each thread
-      // takes two adjacent columns with 16-byte loads: the pair of absolute
-      // columns (c, c + 1), c even, so that every load is aligned (A starts on
-      // 32 bytes, lda is a multiple of four); a pair may reach column k (left
-      // of A22) or column N (the row's padding), whose sums are dropped.  Per
-      // column, two partial sums over odd and even rows, eight rows in
-      // flight.
-      {
-        const int u0 = (k + 1) >> 1, np = ((N - 1) >> 1) - u0 + 1, ld2 = lda >> 1;
-        const double2* rowk = reinterpret_cast<const double2*>(A + (long long)(k + 1) * lda) + u0;
-        for (int p = tid; p < np; p += NT) {
-          const double2* col = rowk + p;
-          const double2 a0 = col[0];
-          double s0 = a0.x * v0, s1 = 0.0, q0 = a0.y * v0, q1 = 0.0;
-          int r = 1;
-          for (; r + 7 < m; r += 8) {
-            double2 a[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = col[(long long)(r + u) * ld2];
-#pragma unroll
-            for (int u = 0; u < 8; u += 2) {
-              const double xa = xs[1 + r + u], xb = xs[2 + r + u];
-              s0 += a[u].x * xa;
-              q0 += a[u].y * xa;
-              s1 += a[u + 1].x * xb;
-              q1 += a[u + 1].y * xb;
-            }
-          }
-          for (; r < m; ++r) {
-            const double2 a = col[(long long)r * ld2];
-            s0 += a.x * xs[1 + r];
-            q0 += a.y * xs[1 + r];
-          }
-          const int t = 2 * (u0 + p) - (k + 1);  // A22 index of the pair's first column
-          if (t >= 0) pvec[t] = s0 + s1;
-          if (t + 1 < m) pvec[t + 1] = q0 + q1;
-        }
-      }
-      for (int l = wid; l < j; l += NW) {
-        const double* vl = A + (long long)(k0 + l) * lda + (k + 1);
-        const double* wl = Wp + (long long)l * N + (k + 1);
-        double om = 0.0, nu = 0.0;
-#pragma unroll
-        for (int c = 0; c < kCols; ++c) {
-          const int jj = lane + 32 * c;
-          if (jj < m) {
-            om += wl[jj] * vreg[c];
-            nu += vl[jj] * vreg[c];
-          }
-        }
-        om = warp_sum(om);
-        nu = warp_sum(nu);
-        if (lane == 0) {
-          sh.VtV[0][l] = om;
-          sh.VtV[1][l] = nu;
-        }
-      }
-      __syncthreads();
-      // p = beta (A22 v - V (W^T v) - W (V^T v)) and p.v
-      // (at most two entries per thread: N <= 32 * kCols + 1; v kept in
-      // registers, since the next column overwrites xs without a barrier)
-      double pv_part = 0.0;
-      double vt[2] = {0.0, 0.0};
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int t = tid + u * NT;
-        if (t < m) {
-          const int i = k + 1 + t;
-          double p = pvec[t];
-#pragma unroll 4
-          for (int l = 0; l < j; ++l)
-            p -= A[(long long)(k0 + l) * lda + i] * sh.VtV[0][l] + Wp[(long long)l * N + i] * sh.VtV[1][l];
-          p *= beta;
-          pvec[t] = p;
-          vt[u] = t == 0 ? v0 : xs[1 + t];
-          pv_part += p * vt[u];
-        }
-      }
-      pv_part = warp_sum(pv_part);
-      if (lane == 0) sh.red[4 + wid] = pv_part;
-      __syncthreads();
-      const double K = 0.5 * beta * ((sh.red[4] + sh.red[5]) + (sh.red[6] + sh.red[7]));
-      // each thread stores W at the rows whose x it forms in the next column
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int t = tid + u * NT;
-        if (t < m) Wp[(long long)j * N + k + 1 + t] = pvec[t] - K * vt[u];
-      }
-      w_last = pvec[0] - K * v0;
-      if (tid == 0) {
-        e[k] = alpha;
-        tau[k] = beta;
-      }
-      if (j == nbp - 1) __syncthreads();  // the trailing update reads all of W
-    }
-    // trailing matrix: A22 -= V W^T + W V^T for rows and columns >= s0, as
-    // 8x8 tiles starting from A, k over the panel's columns
-    const int s0 = k0 + nbp, ms = N - s0;
-    const int T = (ms + 7) >> 3;
-    for (int tile = wid; tile < T * T; tile += NW) {
-      const int I = tile / T, J = tile - I * T;
-      const int i = s0 + I * 8 + g, jb = s0 + J * 8 + g, jc = s0 + J * 8 + 2 * t4;
-      double c0 = (i < N && jc < N) ? A[(long long)i * lda + jc] : 0.0;
-      double c1 = (i < N && jc + 1 < N) ? A[(long long)i * lda + jc + 1] : 0.0;
-      for (int l0 = 0; l0 < nbp; l0 += 4) {
-        const int l = l0 + t4;
-        const bool lok = l < nbp;
-        const double* vl = A + (long long)(k0 + (lok ? l : 0)) * lda;
-        const double* wl = Wp + (long long)(lok ? l : 0) * N;
-        dmma_m8n8k4(c0, c1, (lok && i < N) ? -vl[i] : 0.0, (lok && jb < N) ? wl[jb] : 0.0);
-        dmma_m8n8k4(c0, c1, (lok && i < N) ? -wl[i] : 0.0, (lok && jb < N) ? vl[jb] : 0.0);
-      }
-      if (i < N && jc < N) A[(long long)i * lda + jc] = c0;
-      if (i < N && jc + 1 < N) A[(long long)i * lda + jc + 1] = c1;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    if (N >= 2) {
-      d[N - 2] = A[(long long)(N - 2) * lda + (N - 2)];
-      e[N - 2] = A[(long long)(N - 1) * lda + (N - 2)];
-      tau[N - 2] = 0.0;
-    }
-    d[N - 1] = A[(long long)(N - 1) * lda + (N - 1)];
-    e[N - 1] = 0.0;
-    tau[N - 1] = 0.0;
-  }
-  __syncthreads();
-}
-
 // Eigenvalues k = 0..nneed-1 and N-1 of the tridiagonal, one thread each.
 // Bisection on the Sturm count until the count at the iterate x says that
 // eigenvalue k is the nearest one above (count k) or below (count k+1); from
@@ -860,16 +542,81 @@ __device__ __forceinline__ double eigenvalue_k(const double* d, const double* es
   return x;
 }
 
-// nwarm: eps[0..nwarm) and eps[N-1] hold the previous SCC iteration's
-// eigenvalues, the first iterates of their searches (0: none).
+// Eigenvalues k = 0..nneed-1 and N-1 by the whole CTA, one thread each (at most
+// NT of them).  As eigenvalue_k, but every Sturm count serves every thread: the
+// points and counts of a round are shared, so each bracket is the tightest that
+// all of them allow, and a first round of evenly spread points isolates most
+// eigenvalues of a cold start.  (One thread alone bisected its own way in from
+// the Gerschgorin interval whenever its start was not next to its eigenvalue,
+// and the slowest of a warp's 32 decided: about 30 evaluations at N = 128, here
+// 4 to 8.)  warm: eps holds the previous SCC iteration's eigenvalues, the first
+// points.  px, pc: N doubles of shared scratch.
 template <int NT>
-__device__ void eigenvalues(const double* d, const double* esq, int N, int nneed, double gl, double gu,
-                            double pivmin, double atol, double* eps, int nwarm = 0) {
+__device__ __forceinline__ void eigenvalues(const double* d, const double* esq, int N, int nneed, int nwarm, double gl,
+                                            double gu, double pivmin, double atol, double* eps, double* px, double* pc) {
+  const int tid = threadIdx.x;
   const int nlist = (nneed < N) ? nneed + 1 : N;
-  for (int slot = threadIdx.x; slot < nlist; slot += NT) {
-    const int k = (slot < nneed) ? slot : N - 1;
-    eps[k] = eigenvalue_k(d, esq, N, k, gl, gu, pivmin, atol, eps[k], nwarm > 0 && (k < nwarm || k == N - 1));
+  const int k = (tid < nneed) ? tid : N - 1;
+  const double dn = (double)N;
+  bool active = tid < nlist;
+  double lo = gl, hi = gu, x = gl + (gu - gl) * ((tid + 0.5) / nlist);
+  if (active && (k < nwarm || (nwarm > 0 && k == N - 1))) {
+    const double x0 = eps[k];
+    if (x0 > lo && x0 < hi) x = x0;
   }
+  for (int it = 0; it < 160; ++it) {
+    double p = 0.0, dp = 0.0, ddp = 0.0;
+    int c = 0;
+    if (active) {
+      c = sturm_poly(d, esq, N, x, pivmin, p, dp, ddp);
+      px[tid] = x;
+      pc[tid] = (double)c;
+    }
+    __syncthreads();
+    if (active) {
+      // the first round takes every point, later ones those next in line
+      const double kk = (double)(k + 1);
+      const int j0 = it == 0 ? 0 : max(tid - 4, 0), j1 = it == 0 ? nlist : min(tid + 5, nlist);
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        const double xj = px[j];
+        if (pc[j] >= kk)
+          hi = fmin(hi, xj);
+        else
+          lo = fmax(lo, xj);
+      }
+      const double tol = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + atol;
+      double xn = 0.5 * (lo + hi);
+      bool done = hi - lo <= tol;
+      if (!done && (c == k || c == k + 1)) {  // the Laguerre step of eigenvalue_k
+        const double u = p / dp;
+        const double w = (p * ddp) / (dp * dp);
+        const double sq = sqrt((dn - 1.0) * (dn * (1.0 - w) - 1.0));
+        const bool up = (c == k);
+        const double sigma = ((u > 0.0) == up) ? -1.0 : 1.0;
+        const double step = dn * u / (1.0 + sigma * sq);
+        const double xt = x - step;
+        const bool nearest = up ? (u < 0.0) : (u > 0.0);
+        if (nearest && fabs(step) <= 32.0 * tol) {
+          xn = fmin(fmax(xt, lo), hi);
+          done = true;
+        } else if (xt > lo && xt < hi && (nearest || fabs(step) >= 0.125 * (hi - lo))) {
+          xn = xt;
+        }
+      }
+      if (!done && (xn <= lo || xn >= hi)) {
+        xn = x;
+        done = true;
+      }
+      x = xn;
+      if (done) {
+        eps[k] = x;
+        active = false;
+      }
+    }
+    if (!__syncthreads_or(active)) break;
+  }
+  if (active) eps[k] = x;
   __syncthreads();
 }
 
@@ -956,64 +703,82 @@ __device__ void fermi_warp(const double* eps, int N, int nneed, double nelec, do
 // Finite-temperature occupations (kt > 0, 0 < nelec < 2N) by the whole CTA.
 // The reference bisects [eps_0 - 100 kT - 10, eps_N-1 + 100 kT + 10] on
 // "electron count < nelec" until the bracket stops shrinking
-// (src/electronic.rs:3853-3921); here each round places one trial mu per warp,
-// NW + 1 equal subintervals, and keeps the subinterval where the count crosses
-// nelec, so the bracket converges to the same crossing in log_(NW+1) rounds.
-// Eigenvalues beyond eps[nneed-1] are unknown (apart from eps[N-1]); they are
-// clamped at +80 kT like in fermi_warp, and a trial mu at which they would
-// matter makes the result ambiguous (the caller then computes all of them).
-// Shared scratch: sh.VtV rows 0 and 1.
+// (src/electronic.rs:3853-3921); here each round places one trial mu per thread,
+// NT + 1 equal subintervals, and keeps the subinterval where the count crosses
+// nelec, so the bracket converges to the same crossing in log_(NT+1) rounds, nine
+// for 128 threads.  (One trial per warp, its sum over the lanes, took 26 rounds
+// of a warp reduction and an exponential per orbital each.)  Orbitals more than
+// 40 kT outside the bracket are full or empty to the last bit of the count, so a
+// trial sums the few levels next to the gap.  Eigenvalues beyond
+// eps[nneed-1] are unknown (apart from eps[N-1]); they are clamped at +80 kT like
+// in fermi_warp, and a trial mu at which they would matter makes the result
+// ambiguous (the caller then computes all of them).  Shared scratch: sh.first.
 template <int NT, int CAP>
 __device__ void fermi_cta(const double* eps, int N, int nneed, double nelec, double kt, double* occ, SccShared& sh,
                           double& mu_out, double& ts_out, bool& ambiguous) {
   constexpr int NW = NT / 32;
   constexpr double cap = CAP;  // electrons per orbital: 2, or 1 in a spin channel
-  static_assert(NW <= 16, "one trial point per warp");
+  static_assert(NW <= 16, "one entry per warp");
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const double c80 = cap / (1.0 + exp(80.0));
   const double cm80 = cap / (1.0 + exp(-80.0));
   const int nunc = (nneed < N) ? (N - 1 - nneed) : 0;
-  const double etop = eps[nneed - 1];
-  const double ikt = 1.0 / kt;
+  const double etop = eps[nneed - 1], elast = eps[N - 1];
+  const double ikt = 1.0 / kt, w40 = 40.0 * kt;
   auto fo = [&](double ei, double m) {
     const double x = (ei - m) * ikt;
     if (x >= 80.0) return c80;
     if (x <= -80.0) return cm80;
     return cap / (1.0 + exp(x));
   };
-  double lo = eps[0] - 100.0 * kt - 10.0, hi = eps[N - 1] + 100.0 * kt + 10.0;
+  // The count crosses nelec within 40 kT of level k = ceil(nelec / cap) - 1: 40 kT
+  // below it the levels from k on hold less than 1e-17 electrons each and those
+  // before it cap k < nelec; 40 kT above it the first k + 1 levels are full to
+  // the last bit.
+  const int k = max(0, min(nneed - 1, (int)ceil(nelec / cap) - 1));
+  double lo = eps[nelec - cap * k > 1e-6 ? k : max(k - 1, 0)] - w40, hi = eps[k] + w40;
+  if ((nneed < N && k == nneed - 1) || !(hi > lo)) {
+    lo = eps[0] - 100.0 * kt - 10.0;
+    hi = elast + 100.0 * kt + 10.0;
+  }
   bool amb = false;
+  int i0 = k, i1 = k + 1;  // levels in reach of the bracket (eps ascends)
+  while (i0 > 0 && eps[i0 - 1] >= lo - w40) --i0;
+  while (i1 < nneed && eps[i1] <= hi + w40) ++i1;
   for (int round = 0; round < 64; ++round) {
-    const double h = (hi - lo) / (double)(NW + 1);
-    const double mid = fmin(lo + (double)(wid + 1) * h, hi);
-    double sm = 0.0;
-    for (int i = lane; i < nneed; i += 32) sm += fo(eps[i], mid);
-    if (lane == 0 && nneed < N) sm += fo(eps[N - 1], mid);
-    sm = warp_sum(sm);
-    double flag = 0.0;
+    const double h = (hi - lo) * (1.0 / (NT + 1));
+    const double mid = fmin(lo + (double)(tid + 1) * h, hi);
+    while (i0 < k && eps[i0] < lo - w40) ++i0;
+    while (i1 > k + 1 && eps[i1 - 1] > hi + w40) --i1;
+    double sm = (double)i0 * cm80 + (double)(nneed - i1) * c80;
+    for (int i = i0; i < i1; ++i) sm += fo(eps[i], mid);
+    if (nneed < N) sm += fo(elast, mid);
+    bool flag = false;
     if (nunc > 0) {
-      if ((etop - mid) / kt >= 80.0)
+      if ((etop - mid) * ikt >= 80.0)
         sm += nunc * c80;
       else if (sm < nelec)
-        flag = 1.0;
+        flag = true;
     }
-    if (lane == 0) {
-      sh.VtV[0][wid] = sm;
-      sh.VtV[1][wid] = flag;
-    }
+    const unsigned over = __ballot_sync(0xffffffffu, sm >= nelec);
+    const unsigned bad = __ballot_sync(0xffffffffu, flag);
+    int* first_at = sh.first[round & 1];  // two buffers: one barrier a round
+    if (lane == 0) first_at[wid] = (over ? 32 * wid + __ffs(over) - 1 : NT) | (bad ? 1 << 30 : 0);
     __syncthreads();
-    int j = NW;
-    for (int q = NW - 1; q >= 0; --q)
-      if (sh.VtV[0][q] >= nelec) j = q;
-    for (int q = 0; q < NW; ++q)
-      if (sh.VtV[1][q] != 0.0) amb = true;
+    int j = NT;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+      const int v = first_at[q];
+      j = min(j, v & ~(1 << 30));
+      amb = amb || (v >> 30);
+    }
     const double nlo = (j == 0) ? lo : fmin(lo + (double)j * h, hi);
-    const double nhi = (j == NW) ? hi : fmin(lo + (double)(j + 1) * h, hi);
-    __syncthreads();
+    const double nhi = (j == NT) ? hi : fmin(lo + (double)(j + 1) * h, hi);
     if (amb || (nlo == lo && nhi == hi)) break;
     lo = nlo;
     hi = nhi;
   }
+  __syncthreads();
   const double mu = 0.5 * (lo + hi);
   if (!amb && nunc > 0 && !((etop - mu) / kt >= 80.0)) amb = true;
   double ts = 0.0;
@@ -1077,128 +842,6 @@ __device__ __noinline__ void spin_channel_occupations(const double* eps, int N, 
     sh.iscal[2] = (aa || ab) ? 1 : 0;
   }
   __syncthreads();
-}
-
-// Z := Q Z for the first ncol columns, Q = H_0 ... H_{N-3}, applied in blocks of
-// kBackNB reflectors as Q_b = I - V T V^T (compact WY, forward direction).
-template <int NT>
-__device__ void back_transform(const double* A, int lda, const double* tau, int N, double* Z, int ldz, int ncol,
-                               double* W1, double* W2, SccShared& sh) {
-  constexpr int NW = NT / 32;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nref = N - 2;
-  if (nref <= 0 || ncol <= 0) return;
-  for (int kb = ((nref - 1) / kBackNB) * kBackNB; kb >= 0; kb -= kBackNB) {
-    const int nb = min(kBackNB, nref - kb);
-    // V^T V, one thread per pair i < j (rows >= kb + j + 1 hold both reflectors)
-    for (int p = tid; p < nb * (nb - 1) / 2; p += NT) {
-      int i = 0, rem = p;
-      while (rem >= nb - 1 - i) {
-        rem -= nb - 1 - i;
-        ++i;
-      }
-      const int j = i + 1 + rem;
-      const double* vi = A + (long long)(kb + i) * lda;
-      const double* vj = A + (long long)(kb + j) * lda;
-      double s0 = 0.0, s1 = 0.0;
-      int r = kb + j + 1;
-      for (; r + 1 < N; r += 2) {
-        s0 += vi[r] * vj[r];
-        s1 += vi[r + 1] * vj[r + 1];
-      }
-      if (r < N) s0 += vi[r] * vj[r];
-      sh.VtV[i][j] = s0 + s1;
-    }
-    __syncthreads();
-    if (wid == 0) {  // T upper triangular: T_jj = tau_j, T[0:j,j] = -tau_j T[0:j,0:j] V^T v_j
-      for (int j = 0; j < nb; ++j) {
-        const double tj = tau[kb + j];
-        if (lane < j) {
-          double s = 0.0;
-          for (int l = lane; l < j; ++l) s += sh.Tm[lane][l] * sh.VtV[l][j];
-          sh.Tm[lane][j] = -tj * s;
-        }
-        if (lane == j) sh.Tm[j][j] = tj;
-        __syncwarp();
-      }
-    }
-    // W1 = V^T Z on the FP64 tensor cores: pairs of 8x8 tiles of (reflector
-    // j, column c) sharing the reflector fragment, k over the rows r;
-    // reflector j has entries r > kb + j
-    {
-      const int g = lane >> 2, t4 = lane & 3;
-      const int TC = (ncol + 7) >> 3, TJ = (nb + 7) >> 3, TC2 = (TC + 1) >> 1;
-      for (int tile = wid; tile < TJ * TC2; tile += NW) {
-        const int JT = tile / TC2, CT = 2 * (tile - JT * TC2);
-        const int j = JT * 8 + g, cb0 = CT * 8 + g, cb1 = cb0 + 8;
-        const bool jok = j < nb, ok0 = cb0 < ncol, ok1 = cb1 < ncol;
-        const double* vj = A + (long long)(kb + (jok ? j : 0)) * lda;
-        double d00 = 0.0, d01 = 0.0, d10 = 0.0, d11 = 0.0;
-#pragma unroll 4
-        for (int r0 = kb + 1; r0 < N; r0 += 4) {
-          const int r = r0 + t4;
-          const bool rin = r < N;
-          const double* zr = Z + (long long)(rin ? r : 0) * ldz;
-          const double a = (jok && rin && r > kb + j) ? vj[r] : 0.0;
-          const double b0 = (rin && ok0) ? zr[cb0] : 0.0;
-          const double b1 = (rin && ok1) ? zr[cb1] : 0.0;
-          dmma_m8n8k4(d00, d01, a, b0);
-          dmma_m8n8k4(d10, d11, a, b1);
-        }
-        const int cc = CT * 8 + 2 * t4;
-        if (jok) {
-          double* w1 = W1 + j * ncol;
-          if (cc < ncol) w1[cc] = d00;
-          if (cc + 1 < ncol) w1[cc + 1] = d01;
-          if (cc + 8 < ncol) w1[cc + 8] = d10;
-          if (cc + 9 < ncol) w1[cc + 9] = d11;
-        }
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < nb * ncol; idx += NT) {
-      const int j = idx / ncol, c = idx - j * ncol;
-      double s = 0.0;
-      for (int l = j; l < nb; ++l) s += sh.Tm[j][l] * W1[l * ncol + c];
-      W2[j * ncol + c] = s;
-    }
-    __syncthreads();
-    // Z -= V W2 on the FP64 tensor cores: pairs of 8x8 tiles of (row r,
-    // column c) sharing the reflector fragment, starting from Z, k over the
-    // reflectors j
-    {
-      const int g = lane >> 2, t4 = lane & 3;
-      const int TC = (ncol + 7) >> 3, TR = (N - kb - 1 + 7) >> 3, TC2 = (TC + 1) >> 1;
-      for (int tile = wid; tile < TR * TC2; tile += NW) {
-        const int RT = tile / TC2, CT = 2 * (tile - RT * TC2);
-        const int r = kb + 1 + RT * 8 + g, cb0 = CT * 8 + g, cb1 = cb0 + 8, cc = CT * 8 + 2 * t4;
-        const bool rok = r < N, ok0 = cb0 < ncol, ok1 = cb1 < ncol;
-        double* zr = Z + (long long)(rok ? r : 0) * ldz;
-        double d00 = (rok && cc < ncol) ? zr[cc] : 0.0;
-        double d01 = (rok && cc + 1 < ncol) ? zr[cc + 1] : 0.0;
-        double d10 = (rok && cc + 8 < ncol) ? zr[cc + 8] : 0.0;
-        double d11 = (rok && cc + 9 < ncol) ? zr[cc + 9] : 0.0;
-#pragma unroll 4
-        for (int j0 = 0; j0 < nb; j0 += 4) {
-          const int j = j0 + t4;
-          const bool jok = j < nb;
-          const double a = (rok && jok && r > kb + j) ? -A[(long long)(kb + j) * lda + r] : 0.0;
-          const double* w2 = W2 + (jok ? j : 0) * ncol;
-          const double b0 = (jok && ok0) ? w2[cb0] : 0.0;
-          const double b1 = (jok && ok1) ? w2[cb1] : 0.0;
-          dmma_m8n8k4(d00, d01, a, b0);
-          dmma_m8n8k4(d10, d11, a, b1);
-        }
-        if (rok) {
-          if (cc < ncol) zr[cc] = d00;
-          if (cc + 1 < ncol) zr[cc + 1] = d01;
-          if (cc + 8 < ncol) zr[cc + 8] = d10;
-          if (cc + 9 < ncol) zr[cc + 9] = d11;
-        }
-      }
-    }
-    __syncthreads();
-  }
 }
 
 // Index tables of one molecule (one thread): shell -> atom, shell -> index
@@ -1511,236 +1154,741 @@ __device__ void stage_results(const Batch& B, const MolCtx& c, CtaWs& w, int ite
   for (int a = tid; a < nat; a += NT) B.atom_q[a0 + a] = w.qat[a];
 }
 
-template <int NT, bool Robust>
-__device__ void scc_molecule(const Batch& B, const Model& M, const SccOptions& opt, const SccLaunch& SL, int m,
-                             SccShared& sh, int* sh_atom, int* sh_k, int* ao_sh, int* atom_sh, int* sh_ao0,
-                             double* vec, double* As, long long as_cap) {
-  constexpr int NW = NT / 32;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int a0 = B.atom_off[m], nat = B.atom_off[m + 1] - a0;
-  const int sh0 = B.shell_off[m], nsh = B.shell_off[m + 1] - sh0;
-  const int N = B.ao_off[m + 1] - B.ao_off[m];
-  const long long mo = B.mat_off[m];
-  const double* S = B.S + mo;
-  const double* H0 = B.H0 + mo;
-  CtaWs w = cta_ws(SL.ws + (long long)blockIdx.x * SL.ws_stride, SL.maxn, SL.maxnsh, SL.cap);
-  double* L = w.L;
-  double* Li = w.Li;
-  double* Hp = w.Hp;
-  double* Z = w.Z;
-  double* C = w.C;
-  double* iw = w.iw;
-  const double* G = B.gam + B.gam_off[m];
-  const bool a_shared = (long long)N * work_lda(N) <= as_cap;  // shared memory when the launch gave room
-  const int lda = a_shared ? work_lda(N) : work_lda_global(N);
-  double* A = a_shared ? As : w.A;
-  double* d = vec;
-  double* e = vec + N;
-  double* tau = vec + 2 * N;
-  double* eps = vec + 3 * N;
-  double* occ = vec + 4 * N;
-  double* pop = vec + 5 * N;
-  double* vao = vec + 6 * N;
-  double* pvec = vec + 7 * N;
-  double* esq = vec + 8 * N;
-  const int cap = SL.cap;
+// ------------------------------------------------------------ one molecule per CTA
+// Everything a launch of the SCC kernel needs.
+struct SccArgs {
+  Batch B;
+  Model M;
+  SccOptions opt;
+  SccLaunch SL;
+};
 
-  // ---- index tables
-  if (tid == 0) {
-    build_index_tables(B, M, a0, nat, sh_atom, sh_k, sh_ao0, ao_sh, atom_sh);
-    sh.iscal[0] = kOk;
+// State of the molecule a CTA works on, at the start of the dynamic shared
+// memory.  The stages of the SCC are functions of their own that read it there:
+// inlined into one kernel they shared a register budget that the largest of
+// them needs alone, and each of them spilled.
+struct MolState {
+  int m, a0, nat, sh0, nsh, N, ld;  // molecule, first atom and shell, sizes, leading dimension
+  int vec_at, tri_at;               // offsets (doubles) of the N-vectors and of the reduction's scratch
+  int status, converged, iter, bro_iter, have_e, nneed, nneed0, nocc, spin;
+  long long mo, go;  // offsets of the molecule's matrices and of its Coulomb matrix
+  double nelec, nalpha, nbeta, kt, last_e, e_el, e2, e3, ts, mu, rms, onenrm;
+};
+struct alignas(16) SccCta {
+  SccShared sh;
+  MolState s;
+};
+__host__ __device__ constexpr size_t scc_cta_bytes() { return sizeof(SccCta); }
+
+struct CtaView {
+  SccShared& sh;
+  MolState& s;
+  MolCtx c;
+  CtaWs w;
+  double *d, *e, *tau, *eps, *occ, *pop, *vao, *esq;
+};
+__device__ __forceinline__ CtaView cta_view(const SccArgs& A) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  SccCta& cta = *reinterpret_cast<SccCta*>(smraw);
+  MolState& s = cta.s;
+  int* t = reinterpret_cast<int*>(smraw + scc_cta_bytes());
+  double* v = reinterpret_cast<double*>(smraw) + s.vec_at;
+  const int N = s.N, maxnsh = A.SL.maxnsh;
+  const MolCtx c{s.m, s.a0, s.nat, s.sh0, s.nsh, N,
+                 t, t + maxnsh, t + 2 * maxnsh, t + 3 * maxnsh, t + 3 * maxnsh + A.SL.maxn,
+                 A.B.gam + s.go};
+  return CtaView{cta.sh, s, c, cta_ws(A.SL.ws + (long long)blockIdx.x * A.SL.ws_stride, A.SL.maxn, maxnsh, A.SL.cap),
+                 v, v + N, v + 2 * N, v + 3 * N, v + 4 * N, v + 5 * N, v + 6 * N, v + 7 * N};
+}
+
+// Molecule m: sizes, index tables, electron counts.
+template <int KIND>
+__device__ __noinline__ void scc_begin(const SccArgs& A, int m) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  MolState& s = reinterpret_cast<SccCta*>(smraw)->s;
+  const Batch& B = A.B;
+  if (threadIdx.x == 0) {
+    s.m = m;
+    s.a0 = B.atom_off[m];
+    s.nat = B.atom_off[m + 1] - s.a0;
+    s.sh0 = B.shell_off[m];
+    s.nsh = B.shell_off[m + 1] - s.sh0;
+    s.N = B.ao_off[m + 1] - B.ao_off[m];
+    s.ld = work_ld(s.N);
+    s.vec_at = (int)(scc_vec_bytes(A.SL.maxnsh, A.SL.maxn, A.SL.maxnat) / 8);
+    s.tri_at = s.vec_at + ((kVecSlots * A.SL.maxn + 1) & ~1);
+    s.mo = B.mat_off[m];
+    s.go = B.gam_off[m];
+    s.status = kOk;
+    s.converged = 0;
+    s.iter = 0;
+    s.nocc = 0;
+    s.e_el = s.e2 = s.e3 = s.ts = s.mu = s.rms = 0.0;
+    const CtaView v = cta_view(A);
+    build_index_tables(B, A.M, s.a0, s.nat, const_cast<int*>(v.c.sh_atom), const_cast<int*>(v.c.sh_k),
+                       const_cast<int*>(v.c.sh_ao0), const_cast<int*>(v.c.ao_sh), const_cast<int*>(v.c.atom_sh));
+    double nref = 0.0;
+    for (int i = 0; i < s.nsh; ++i) nref += A.M.elem[B.z[s.a0 + v.c.sh_atom[i]]].refocc[v.c.sh_k[i]];
+    s.nelec = nref - B.charge[m];
+    // a requested spin multiplicity: alpha and beta electron counts (validated on the host)
+    s.spin = A.opt.spin_mult > 0;
+    s.nalpha = s.spin ? 0.5 * (rint(s.nelec) + (A.opt.spin_mult - 1)) : 0.0;
+    s.nbeta = s.spin ? 0.5 * (rint(s.nelec) - (A.opt.spin_mult - 1)) : 0.0;
+    s.nneed0 = min(s.N, max(1, (int)ceil(s.spin ? s.nalpha : 0.5 * s.nelec) + 8));
+    s.nneed = s.nneed0;
   }
   __syncthreads();
+}
 
-  StageClock clk(B.stage_cycles);
-  const MolCtx mc{m, a0, nat, sh0, nsh, N, sh_atom, sh_k, sh_ao0, ao_sh, atom_sh, G};
-  // ---- Cholesky S = L L^T, left-looking over panels of 8 columns: the
-  // panel minus (its rows of L) x (the panel's rows of L)^T over the finished
-  // columns on the FP64 tensor cores, the 8x8 diagonal block by one thread
-  // (registers; its factor and reciprocal pivots staged in shared memory),
-  // then the rows below by a triangular solve, one thread per row.
-  for (long long i = tid; i < (long long)N * N; i += NT) L[i] = S[i];
+// Cholesky S = L L^T, left-looking over panels of 8 columns: the panel minus
+// (its rows of L) x (the panel's rows of L)^T over the finished columns on the
+// FP64 tensor cores, the 8x8 diagonal block by one thread (registers; its
+// factor and reciprocal pivots staged in shared memory), then the rows below by
+// a triangular solve, one thread per row.
+template <int KIND>
+__device__ __noinline__ void scc_cholesky(const SccArgs& A) {
+  constexpr int NT = kSccKinds[KIND].nt, NW = NT / 32;
+  const CtaView v = cta_view(A);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int N = v.s.N, ld = v.s.ld;
+  const double* S = A.B.S + v.s.mo;
+  double* L = v.w.L;
+  double(*Ld)[9] = v.sh.Ld;
+  for (int idx = tid; idx < ld * ld; idx += NT) {  // zeros in the padding
+    const int i = idx / ld, j = idx - i * ld;
+    L[idx] = (i < N && j < N) ? S[(long long)i * N + j] : 0.0;
+  }
   __syncthreads();
-  {
-    const int g = lane >> 2, t4 = lane & 3;
-    double(*Ld)[kBackNB] = sh.Tm;  // free until the first back-transformation
-    for (int c0 = 0; c0 < N; c0 += 8) {
-      const int nbc = min(8, N - c0);
-      if (c0 > 0) {
-        const int TR = (N - c0 + 7) >> 3;
-        const bool jok = g < nbc;
-        const double* lj = L + (long long)(jok ? c0 + g : 0) * N;
-        for (int RT = wid; RT < TR; RT += NW) {
-          const int i = c0 + RT * 8 + g;
-          const bool iok = i < N;
-          const double* li = L + (long long)(iok ? i : 0) * N;
-          double d0 = 0.0, d1 = 0.0;
+  for (int c0 = 0; c0 < N; c0 += 8) {
+    const int nbc = min(8, N - c0);
+    if (c0 > 0) {
+      const int TR = (N - c0 + 7) >> 3;
+      const bool jok = g < nbc;
+      const double* lj = L + (long long)(jok ? c0 + g : 0) * ld;
+      for (int RT = wid; RT < TR; RT += NW) {
+        const int i = c0 + RT * 8 + g;
+        const bool iok = i < N;
+        const double* li = L + (long long)(iok ? i : 0) * ld;
+        double d0 = 0.0, d1 = 0.0;
 #pragma unroll 4
-          for (int k0 = 0; k0 < c0; k0 += 4) {
-            const int k = k0 + t4;
-            dmma_m8n8k4(d0, d1, iok ? li[k] : 0.0, jok ? lj[k] : 0.0);
-          }
-          if (iok) {
-            double* out = L + (long long)i * N + c0 + 2 * t4;
-            if (2 * t4 < nbc) out[0] -= d0;
-            if (2 * t4 + 1 < nbc) out[1] -= d1;
-          }
+        for (int k0 = 0; k0 < c0; k0 += 4) {
+          const int k = k0 + t4;
+          dmma_m8n8k4(d0, d1, iok ? li[k] : 0.0, jok ? lj[k] : 0.0);
         }
-        __syncthreads();
-      }
-      if (tid == 0) {
-        double D[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j <= i; ++j) D[i][j] = (i < nbc) ? L[(long long)(c0 + i) * N + c0 + j] : (i == j ? 1.0 : 0.0);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          // the reference rejects overlaps with an eigenvalue <= eigen_tolerance (1e-12)
-          if (j < nbc && !(D[j][j] > 1e-12)) sh.iscal[0] = kErrInvalidInput;
-          const double r = sqrt(fmax(D[j][j], 1e-300));
-          const double inv = 1.0 / r;
-          D[j][j] = r;
-          Ld[j][8] = inv;
-#pragma unroll
-          for (int i = j + 1; i < 8; ++i) D[i][j] *= inv;
-#pragma unroll
-          for (int k = j + 1; k < 8; ++k)
-#pragma unroll
-            for (int i = k; i < 8; ++i) D[i][k] -= D[i][j] * D[k][j];
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j <= i; ++j) {
-            Ld[i][j] = D[i][j];
-            if (i < nbc) L[(long long)(c0 + i) * N + c0 + j] = D[i][j];
-          }
-      }
-      __syncthreads();
-      for (int i = c0 + 8 + tid; i < N; i += NT) {  // rows below: x L_dd^T = row
-        double* row = L + (long long)i * N + c0;
-        double x[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = row[j];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-#pragma unroll
-          for (int k = 0; k < j; ++k) x[j] -= x[k] * Ld[j][k];
-          x[j] *= Ld[j][8];
-          row[j] = x[j];
+        if (iok) {
+          double* out = L + (long long)i * ld + c0 + 2 * t4;
+          if (2 * t4 < nbc) out[0] -= d0;
+          if (2 * t4 + 1 < nbc) out[1] -= d1;
         }
       }
       __syncthreads();
     }
-  }
-  if (sh.iscal[0] != kOk) {
     if (tid == 0) {
-      B.status[m] = sh.iscal[0];
-      B.iterations[m] = 0;
+      double D[8][8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) D[i][j] = (i < nbc) ? L[(long long)(c0 + i) * ld + c0 + j] : (i == j ? 1.0 : 0.0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        // the reference rejects overlaps with an eigenvalue <= eigen_tolerance (1e-12)
+        if (j < nbc && !(D[j][j] > 1e-12)) v.s.status = kErrInvalidInput;
+        const double r = sqrt(fmax(D[j][j], 1e-300));
+        const double inv = 1.0 / r;
+        D[j][j] = r;
+        Ld[j][8] = inv;
+#pragma unroll
+        for (int i = j + 1; i < 8; ++i) D[i][j] *= inv;
+#pragma unroll
+        for (int k = j + 1; k < 8; ++k)
+#pragma unroll
+          for (int i = k; i < 8; ++i) D[i][k] -= D[i][j] * D[k][j];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+          Ld[i][j] = D[i][j];
+          if (i < nbc) L[(long long)(c0 + i) * ld + c0 + j] = D[i][j];
+        }
+    }
+    __syncthreads();
+    for (int i = c0 + 8 + tid; i < N; i += NT) {  // rows below: x L_dd^T = row
+      double* row = L + (long long)i * ld + c0;
+      double x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = row[j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+#pragma unroll
+        for (int k = 0; k < j; ++k) x[j] -= x[k] * Ld[j][k];
+        x[j] *= Ld[j][8];
+        row[j] = x[j];
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = wid; i < N; i += NW)
+    for (int j = i + 1 + lane; j < N; j += 32) L[(long long)i * ld + j] = 0.0;
+  __syncthreads();
+}
+
+// L^-1, kept transposed, by 8 x 8 blocks: X = L^-1 has X_JJ = L_JJ^-1 and, down
+// block column J, X_IJ = -L_II^-1 sum_{J <= K < I} L_IK X_KJ.  The block columns
+// are independent, one warp each with the column (transposed) in tensor-core
+// accumulators, as the occupied orbitals are; the inverses of the diagonal
+// blocks go through the reduction's scratch.  (One thread per column of L^-1, a
+// chain of N multiply-adds with a load each, took 1M cycles at N = 128.)
+template <int KIND>
+__device__ __noinline__ void scc_inverse(const SccArgs& A) {
+  constexpr int NT = kSccKinds[KIND].nt, NW = NT / 32, P = kSccKinds[KIND].p, NB = P / 8;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const CtaView v = cta_view(A);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int N = v.s.N, ld = v.s.ld, nt = ld >> 3;
+  const double* __restrict__ L = v.w.L;
+  double* __restrict__ LiT = v.w.LiT;
+  double* inv = reinterpret_cast<double*>(smraw) + v.s.tri_at;  // [nt][8][8] row-major
+  for (int c = tid; c < ld; c += NT) {  // column c & 7 of the inverse of diagonal block c >> 3
+    const int b = c >> 3, j = c & 7;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 8 * b + i;
+      double t = i == j ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < i) t -= L[(long long)row * ld + 8 * b + k] * x[k];
+      x[i] = (row < N && c < N) ? t / L[(long long)row * ld + row] : 0.0;
+      inv[64 * b + 8 * i + j] = x[i];
+    }
+  }
+  __syncthreads();
+  for (int J = wid; J < nt; J += NW) {
+    double z[NB][2];
+#pragma unroll
+    for (int I = 0; I < NB; ++I) {
+      z[I][0] = z[I][1] = 0.0;
+      if (I < nt) {
+        if (I == J) {
+          z[I][0] = inv[64 * J + 8 * (2 * t4) + g];
+          z[I][1] = inv[64 * J + 8 * (2 * t4 + 1) + g];
+        } else if (I > J) {
+          const double* lrow = L + (long long)(8 * I + g) * ld + 2 * t4;
+          double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+#pragma unroll
+          for (int q = 0; q < (I + 3) / 4; ++q)
+            if (4 * q + 3 >= J) {
+              double2 l[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (4 * q + u < I) l[u] = *reinterpret_cast<const double2*>(lrow + 32 * q + 8 * u);
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (4 * q + u < I) {
+                  dmma_m8n8k4(s0[u & 1], s1[u & 1], z[4 * q + u][0], l[u].x);
+                  dmma_m8n8k4(s0[u & 1], s1[u & 1], z[4 * q + u][1], l[u].y);
+                }
+            }
+          const double2 r = *reinterpret_cast<const double2*>(inv + 64 * I + 8 * g + 2 * t4);
+          dmma_m8n8k4(z[I][0], z[I][1], -(s0[0] + s0[1]), r.x);
+          dmma_m8n8k4(z[I][0], z[I][1], -(s1[0] + s1[1]), r.y);
+        }
+        *reinterpret_cast<double2*>(LiT + (long long)(8 * J + g) * ld + 8 * I + 2 * t4) = make_double2(z[I][0], z[I][1]);
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// H0' = L^-1 H0 L^-T, one warp per block row: U = L^-1 H0 as tensor-core
+// accumulators for all columns, which are then the A operand of U L^-T (blocks on
+// and below the diagonal, written to both triangles so that H0' is exactly
+// symmetric).
+template <int KIND>
+__device__ __noinline__ void scc_h0(const SccArgs& A) {
+  constexpr int NT = kSccKinds[KIND].nt, NW = NT / 32, P = kSccKinds[KIND].p, NB = P / 8;
+  const CtaView v = cta_view(A);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const int N = v.s.N, ld = v.s.ld, nt = ld >> 3;
+  const double* __restrict__ H0 = A.B.H0 + v.s.mo;
+  const double* __restrict__ LiT = v.w.LiT;
+  double* __restrict__ Hp = v.w.Hp;
+  for (int I0 = wid; I0 < nt; I0 += NW) {
+    const int I = nt - 1 - I0;  // the longest rows first
+    double u[NB][2];
+#pragma unroll
+    for (int t = 0; t < NB; ++t) u[t][0] = u[t][1] = 0.0;
+#pragma unroll 2
+    for (int k0 = 0; k0 < 8 * I + 8; k0 += 4) {
+      const int k = k0 + t4;
+      const double a = LiT[(long long)k * ld + 8 * I + g];
+      const double* h = H0 + (long long)min(k, N - 1) * N;
+#pragma unroll
+      for (int t = 0; t < NB; ++t)
+        if (t < nt) {
+          const int j = 8 * t + g;
+          dmma_m8n8k4(u[t][0], u[t][1], a, (k < N && j < N) ? h[j] : 0.0);
+        }
+    }
+    for (int J = 0; J <= I; ++J) {
+      double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
+#pragma unroll
+      for (int t = 0; t < NB; ++t)
+        if (t <= J) {
+          const double* b = LiT + (long long)(8 * t + 2 * t4) * ld + 8 * J + g;
+          dmma_m8n8k4(d0[0], d1[0], u[t][0], b[0]);
+          dmma_m8n8k4(d0[1], d1[1], u[t][1], b[ld]);
+        }
+      const int i = 8 * I + g, j = 8 * J + 2 * t4;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (i < N && j + c <= i) {
+          const double h = c ? d1[0] + d1[1] : d0[0] + d0[1];
+          Hp[(long long)i * ld + j + c] = h;
+          Hp[(long long)(j + c) * ld + i] = h;
+        }
+    }
+  }
+  __syncthreads();
+}
+
+// (1) shell potential from the input charges.
+template <int KIND>
+__device__ __noinline__ void scc_potential(const SccArgs& A) {
+  CtaView v = cta_view(A);
+  stage_potential<kSccKinds[KIND].nt>(A.B, A.M, v.c, v.w, v.vao);
+}
+
+// Level shift F += b (S - S P_prev S / 2) (src/electronic.rs:2125-2137); in the
+// orthonormal basis F' += b (I - Z f Z^T / 2) with the previous iteration's
+// eigenvectors Z and occupations f.
+template <int KIND>
+__device__ __noinline__ void scc_level_shift(const SccArgs& A, double lshift) {
+  constexpr int NT = kSccKinds[KIND].nt;
+  const CtaView v = cta_view(A);
+  const int N = v.s.N, ld = v.s.ld, nocc = v.s.nocc;
+  const double *Z = v.w.Z, *occ = v.occ;
+  double* F = v.w.F;
+  for (long long idx = threadIdx.x; idx < (long long)N * N; idx += NT) {
+    const int i = (int)(idx / N), j = (int)(idx % N);
+    if (j > i) continue;
+    double sp = 0.0;
+    for (int k = 0; k < nocc; ++k) sp += occ[k] * Z[(long long)i * ld + k] * Z[(long long)j * ld + k];
+    const double val = lshift * ((i == j ? 1.0 : 0.0) - 0.5 * sp);
+    F[(long long)i * ld + j] += val;
+    if (i != j) F[(long long)j * ld + i] += val;
+  }
+  __syncthreads();
+}
+
+// (4) eigenvalues the occupations need and (5) the occupations
+// (src/electronic.rs:3815-3921); when the known eigenvalues do not decide them,
+// all eigenvalues and once more.  Also |T|_1 and the count of orbitals with
+// occupation above 1e-30 (beyond which they do not matter at FP64 resolution).
+// The marks: eigenvalues, occupations.
+template <int KIND>
+__device__ __noinline__ void scc_occupations(const SccArgs& A, StageClock* clk) {
+  constexpr int NT = kSccKinds[KIND].nt;
+  const CtaView v = cta_view(A);
+  SccShared& sh = v.sh;
+  MolState& s = v.s;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, N = s.N;
+  const double *d = v.d, *e = v.e;
+  double gl = INFINITY, gu = -INFINITY, onenrm = 0.0, emax2 = 0.0;
+  for (int i = tid; i < N; i += NT) {
+    const double off = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < N - 1 ? fabs(e[i]) : 0.0);
+    gl = fmin(gl, d[i] - off);
+    gu = fmax(gu, d[i] + off);
+    onenrm = fmax(onenrm, fabs(d[i]) + off);
+    if (i < N - 1) {
+      v.esq[i] = e[i] * e[i];
+      emax2 = fmax(emax2, v.esq[i]);
+    }
+  }
+  gl = -block_max(-gl, sh.red);
+  gu = block_max(gu, sh.red);
+  onenrm = block_max(onenrm, sh.red);
+  emax2 = block_max(emax2, sh.red);
+  const double pivmin = DBL_MIN * fmax(1.0, emax2);
+  {
+    const double span = gu - gl;
+    gl -= 2.1 * DBL_EPSILON * fabs(gl) + 4.0 * DBL_EPSILON * span + pivmin;
+    gu += 2.1 * DBL_EPSILON * fabs(gu) + 4.0 * DBL_EPSILON * span + pivmin;
+  }
+  const double nelec = s.nelec, kt = s.kt;
+  const int nwarm = s.iter > 1 ? s.nneed : 0;  // from the previous iteration's eigenvalues once this rung has one
+  int nneed = s.nneed0;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    eigenvalues<NT>(d, v.esq, N, nneed, attempt == 0 ? nwarm : 0, gl, gu, pivmin, 4.0 * DBL_EPSILON * onenrm, v.eps, v.occ,
+                    v.pop);
+    clk->mark(kStEigval);
+    if (s.spin) {
+      spin_channel_occupations<NT>(v.eps, N, nneed, s.nalpha, s.nbeta, kt, v.occ, v.pop, sh);
+    } else if (kt > 0.0 && nelec > 0.0 && nelec < 2.0 * N) {
+      double fm, ft;
+      bool amb;
+      fermi_cta<NT, 2>(v.eps, N, nneed, nelec, kt, v.occ, sh, fm, ft, amb);
+      if (tid == 0) {
+        sh.scal[1] = fm;
+        sh.scal[2] = ft;
+        sh.iscal[2] = amb ? 1 : 0;
+      }
+    } else if (wid == 0) {  // aufbau and the empty / full limits
+      double fm, ft;
+      bool amb;
+      fermi_warp<2>(v.eps, N, nneed, nelec, kt, v.occ, fm, ft, amb);
+      if (lane == 0) {
+        sh.scal[1] = fm;
+        sh.scal[2] = ft;
+        sh.iscal[2] = amb ? 1 : 0;
+      }
+    }
+    __syncthreads();
+    clk->mark(kStFermi);
+    if (!sh.iscal[2] || nneed == N) break;
+    nneed = N;
+  }
+  int nocc_loc = 0;
+  for (int i = tid; i < N; i += NT)
+    if ((i < nneed || i == N - 1) && v.occ[i] > 1e-30) nocc_loc = max(nocc_loc, i + 1);
+  const int nocc = (int)block_max((double)nocc_loc, sh.red);
+  if (tid == 0) {
+    s.mu = sh.scal[1];
+    s.ts = sh.scal[2];
+    s.nneed = nneed;
+    s.nocc = nocc;
+    s.onenrm = onenrm;
+  }
+  __syncthreads();
+}
+
+// Occupied eigenvectors of a cluster of eigenvalues j..jend-1, or of one that
+// the twisted factorisation did not settle: inverse iteration with partial
+// pivoting, modified Gram-Schmidt inside the cluster, one thread.
+__device__ __noinline__ void inverse_iteration(const double* d, const double* e, int N, int ld, const double* eps, int j,
+                                               int jend, double onenrm, double* iw, double* Z) {
+  const double tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
+  double* ws = iw + j;  // column j of the interleaved factor arrays
+  double lam_prev = -INFINITY;
+  for (int jj = j; jj < jend; ++jj) {
+    double lam = eps[jj];
+    const double pert = 10.0 * DBL_EPSILON * fmax(fabs(lam), onenrm);
+    if (jj > j && lam - lam_prev < pert) lam = lam_prev + pert;
+    lam_prev = lam;
+    double* x = Z + jj;  // column jj, stride ld
+    if (jend - j == 1) {
+      // the start vector's forward elimination runs with the factorisation, the
+      // two solves are not normalised in between (growth below 1e40), and the
+      // second one returns |x|^2
+      const double cur = tri_factor_rhs(d, e, N, lam, tiny, ws, ld, x, ld, (unsigned)jj);
+      tri_back(ws, N, ld, x, ld, cur);
+      const double nrm = tri_solve(ws, N, ld, x, ld);
+      const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
+      for (int i = 0; i < N; ++i) x[(long long)i * ld] *= inv;
+      continue;
+    }
+    tri_factor(d, e, N, lam, tiny, ws, ld);
+    for (int i = 0; i < N; ++i) x[(long long)i * ld] = hash_unit(i, jj) + 1e-3;
+    const int nit = 4;
+    for (int it = 0; it < nit; ++it) {
+      tri_solve(ws, N, ld, x, ld);
+      for (int q = j; q < jj; ++q) {
+        double dot = 0.0;
+        for (int i = 0; i < N; ++i) dot += Z[(long long)i * ld + q] * x[(long long)i * ld];
+        for (int i = 0; i < N; ++i) x[(long long)i * ld] -= dot * Z[(long long)i * ld + q];
+      }
+      double nrm = 0.0;
+      for (int i = 0; i < N; ++i) nrm += x[(long long)i * ld] * x[(long long)i * ld];
+      const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
+      for (int i = 0; i < N; ++i) x[(long long)i * ld] *= inv;
+    }
+  }
+}
+
+// (6) occupied eigenvectors of the tridiagonal, columns of Z up to the factors
+// scale[j] (in v.pop).  An isolated eigenvalue takes one twisted factorisation
+// (Parlett & Dhillon, "Fernando's solution to Wilkinson's problem", Linear
+// Algebra Appl. 267, 1997): T - lam = L D+ L^T from the top by one thread,
+// U D- U^T from the bottom by another, joined at the row r where
+// |gamma_r| = |D+_r + D-_r - (d_r - lam)| is smallest; z_r = 1 and
+// z_{i-1} = -(e_{i-1} / D+_{i-1}) z_i upward, z_{i+1} = -(e_i / D-_{i+1}) z_i
+// downward solve (T - lam) z = gamma_r e_r.  Both pivot chains are a divide per
+// row; inverse iteration needs a pivoted factorisation and two solves, five
+// dependent passes (147k cycles at N = 128 against 30k here).  Its residual
+// gamma_r / |z| is about the error of lam times |z|; a column where it is larger
+// than rounding explains, and clusters, fall back to inverse iteration.
+template <int KIND>
+__device__ __noinline__ void scc_vectors(const SccArgs& A) {
+  constexpr int NT = kSccKinds[KIND].nt, HALF = NT / 2;
+  const CtaView v = cta_view(A);
+  const int tid = threadIdx.x, N = v.s.N, ld = v.s.ld, nocc = v.s.nocc;
+  const double *d = v.d, *e = v.e, *eps = v.eps;
+  const double onenrm = v.s.onenrm, ortol = 1e-5 * onenrm, tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
+  double* __restrict__ Z = v.w.Z;
+  double *gam = v.pop, *twist = v.esq;  // per column: |gamma|, then the squared norm, then the scale; the row r
+  const long long n2 = (long long)ld * ld;
+  const bool top = tid < HALF;
+  for (int j0 = 0; j0 < nocc; j0 += HALF) {
+    const int j = j0 + (top ? tid : tid - HALF);
+    const bool col = j < nocc;
+    const bool first = col && (j == 0 || eps[j] - eps[j - 1] > ortol);
+    const bool single = first && (j + 1 >= nocc || eps[j + 1] - eps[j] > ortol);
+    const double lam = col ? eps[j] : 0.0;
+    double* dp = v.w.iw + (col ? j : 0);  // D+_i
+    double* lp = dp + n2;                 // e_i / D+_i
+    double* um = dp + 2 * n2;             // e_i / D-_{i+1}
+    if (single) {
+      if (top) {
+        double D = d[0] - lam;
+#pragma unroll 4
+        for (int i = 0; i < N - 1; ++i) {
+          const double ei = e[i], dn = d[i + 1] - lam;
+          if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
+          const double l = ei * (1.0 / D);
+          dp[(long long)i * ld] = D;
+          lp[(long long)i * ld] = l;
+          D = dn - ei * l;
+        }
+        dp[(long long)(N - 1) * ld] = D;
+      } else {
+        double D = d[N - 1] - lam;
+#pragma unroll 4
+        for (int i = N - 2; i >= 0; --i) {
+          const double ei = e[i], dn = d[i] - lam;
+          if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
+          const double u = ei * (1.0 / D);
+          um[(long long)i * ld] = u;
+          D = dn - ei * u;
+        }
+      }
+    }
+    __syncthreads();
+    double best = INFINITY;
+    int at = 0;
+    if (single) {  // smallest |gamma_i| = |D+_i - e_i u_i| over the thread's half of the rows
+      const int i0 = top ? 0 : N / 2, i1 = top ? N / 2 : N;
+#pragma unroll 4
+      for (int i = i0; i < i1; ++i) {
+        const double gi = fabs(dp[(long long)i * ld] - (i < N - 1 ? e[i] * um[(long long)i * ld] : 0.0));
+        if (gi < best) {
+          best = gi;
+          at = i;
+        }
+      }
+      if (!top) {
+        gam[j] = best;
+        twist[j] = (double)at;
+      }
+    }
+    __syncthreads();
+    if (single && top) {
+      if (!(gam[j] < best)) twist[j] = (double)at;
+      best = fmin(best, gam[j]);
+    }
+    __syncthreads();
+    double nrm = 0.0;
+    if (single) {
+      const int r = (int)twist[j];
+      double z = 1.0;
+      double* x = Z + j;
+      if (top) {
+        nrm = 1.0;
+        x[(long long)r * ld] = 1.0;
+#pragma unroll 8
+        for (int i = N - 2; i >= 0; --i) {
+          const double l = lp[(long long)i * ld];
+          if (i < r) {
+            z *= -l;
+            x[(long long)i * ld] = z;
+            nrm += z * z;
+          }
+        }
+      } else {
+#pragma unroll 8
+        for (int i = 0; i < N - 1; ++i) {
+          const double u = um[(long long)i * ld];
+          if (i >= r) {
+            z *= -u;
+            x[(long long)(i + 1) * ld] = z;
+            nrm += z * z;
+          }
+        }
+        gam[j] = nrm;
+      }
+    }
+    __syncthreads();
+    if (top && first) {
+      bool good = false;
+      if (single) {
+        nrm += gam[j];
+        good = best <= 64.0 * DBL_EPSILON * onenrm * nrm && nrm < 1e200;
+        if (good) gam[j] = 1.0 / sqrt(nrm);
+      }
+      if (!good) {
+        int jend = j + 1;
+        while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
+        inverse_iteration(d, e, N, ld, eps, j, jend, onenrm, v.w.iw, Z);
+        for (int q = j; q < jend; ++q) gam[q] = 1.0;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// (9) populations, output charges, energies and the convergence test.
+template <int KIND, bool Robust>
+__device__ __noinline__ void scc_energy(const SccArgs& A, double lshift) {
+  constexpr int NT = kSccKinds[KIND].nt, NW = NT / 32;
+  CtaView v = cta_view(A);
+  MolState& s = v.s;
+  const int tid = threadIdx.x, N = s.N, ld = s.ld;
+  for (int i = tid; i < N; i += NT) {
+    double p = 0.0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) p += v.w.popw[(long long)q * ld + i];
+    v.pop[i] = p;
+  }
+  __syncthreads();
+  double e_el, e2, e3, rms;
+  stage_charges_energy<NT>(A.B, A.M, v.c, v.w, v.pop, v.occ, v.eps, v.vao, s.nocc, v.sh, e_el, e2, e3, rms);
+  if (Robust && lshift != 0.0) {
+    // with a shifted Fock matrix sum(f eps) is not tr(F P): E_el = tr(H0 P) = sum_k f_k z_k^T H0' z_k
+    const double *Hp = v.w.Hp, *Z = v.w.Z;
+    const int nocc = s.nocc;
+    double part = 0.0;
+    for (long long idx = tid; idx < (long long)N * nocc; idx += NT) {
+      const int i = (int)(idx / nocc), k = (int)(idx % nocc);
+      double hz = 0.0;
+      for (int j = 0; j < N; ++j) hz += Hp[(long long)i * ld + j] * Z[(long long)j * ld + k];
+      part += v.occ[k] * Z[(long long)i * ld + k] * hz;
+    }
+    e_el = block_sum(part, v.sh.red);
+  }
+  if (tid == 0) {
+    const double escc = e_el + e2 + e3 + s.ts;
+    const double err = s.have_e ? fabs(escc - s.last_e) : INFINITY;
+    s.e_el = e_el;
+    s.e2 = e2;
+    s.e3 = e3;
+    s.rms = rms;
+    s.last_e = escc;
+    s.have_e = 1;
+    s.converged = err < A.opt.energy_tol && rms < A.opt.charge_tol;
+  }
+  __syncthreads();
+}
+
+// (10) charge mixing.
+template <int KIND>
+__device__ __noinline__ void scc_mix(const SccArgs& A, int broyden, double mixing) {
+  CtaView v = cta_view(A);
+  SccOptions ro = A.opt;
+  ro.broyden = broyden;
+  ro.mixing = mixing;
+  int bro = v.s.bro_iter;
+  __syncthreads();
+  stage_mix<kSccKinds[KIND].nt>(ro, v.c, v.w, A.SL.cap, bro, v.sh);
+  if (threadIdx.x == 0) v.s.bro_iter = bro;
+  __syncthreads();
+}
+
+// Results, and the density and energy-weighted density of the last
+// diagonalisation (src/linalg.rs:243-273), kept per molecule for the gradient
+// kernel: P = C f C^T and W = C f eps C^T on the FP64 tensor cores, 16 x 16 tiles
+// on and below the diagonal (eight accumulators share four operand loads)
+// written to both triangles.
+template <int KIND, bool Robust>
+__device__ __noinline__ void scc_finish(const SccArgs& A, int rung) {
+  constexpr int NT = kSccKinds[KIND].nt, NW = NT / 32;
+  CtaView v = cta_view(A);
+  const Batch& B = A.B;
+  MolState& s = v.s;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int m = s.m, N = s.N, ld = s.ld, nocc = s.nocc;
+  if (!Robust && !s.converged && B.failed && tid == 0) B.failed[atomicAdd(B.queue + 3, 1)] = m;
+  if constexpr (Robust) {  // rung-0 molecules keep the 0 the host wrote before the launches
+    if (B.rung && tid == 0) B.rung[m] = s.converged ? rung : -1;
+  }
+  stage_results<NT>(B, v.c, v.w, s.iter, s.converged != 0, s.e_el, s.e2, s.e3, s.ts, s.mu);
+  if (B.orb_eps) {  // orbital energies (NaN where the eigensolver did not need them) and occupations
+    const int ao0 = B.ao_off[m];
+    for (int i = tid; i < N; i += NT) {
+      B.orb_eps[ao0 + i] = (i < s.nneed || i == N - 1) ? v.eps[i] : __longlong_as_double(0x7ff8000000000000LL);
+      B.orb_occ[ao0 + i] = v.occ[i];
+    }
+  }
+  const double* __restrict__ Ct = v.w.Ct;
+  double* __restrict__ Pm = B.P + s.mo;
+  double* __restrict__ Wm = B.W + s.mo;
+  const int nt = ld >> 3, nt2 = (nt + 1) >> 1;
+  for (int tile = wid; tile < nt2 * (nt2 + 1) / 2; tile += NW) {
+    int I = 0;
+    while ((I + 1) * (I + 2) / 2 <= tile) ++I;
+    const int J = tile - I * (I + 1) / 2;
+    const bool i1 = 2 * I + 1 < nt, j1 = 2 * J + 1 < nt;
+    double p[2][2][2], q[2][2][2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) p[a][b][0] = p[a][b][1] = q[a][b][0] = q[a][b][1] = 0.0;
+#pragma unroll 2
+    for (int k0 = 0; k0 < nocc; k0 += 4) {
+      const int k = k0 + t4;
+      const bool kin = k < nocc;
+      const double f = kin ? v.occ[k] : 0.0, ek = kin ? v.eps[k] : 0.0;
+      const double* ck = Ct + (long long)(kin ? k : 0) * ld + g;
+      double a[2], b[2];
+      a[0] = f * ck[16 * I];
+      a[1] = i1 ? f * ck[16 * I + 8] : 0.0;
+      b[0] = ck[16 * J];
+      b[1] = j1 ? ck[16 * J + 8] : 0.0;
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          dmma_m8n8k4(p[x][y][0], p[x][y][1], a[x], b[y]);
+          dmma_m8n8k4(q[x][y][0], q[x][y][1], a[x] * ek, b[y]);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int i = 16 * I + 8 * x + g, j = 16 * J + 8 * y + 2 * t4 + c;
+          if (i < N && j <= i) {
+            Pm[(long long)i * N + j] = p[x][y][c];
+            Pm[(long long)j * N + i] = p[x][y][c];
+            Wm[(long long)i * N + j] = q[x][y][c];
+            Wm[(long long)j * N + i] = q[x][y][c];
+          }
+        }
+  }
+  __syncthreads();
+}
+
+template <int KIND, bool Robust>
+__device__ __forceinline__ void scc_molecule(const SccArgs& A, int m) {
+  constexpr int NT = kSccKinds[KIND].nt, P = kSccKinds[KIND].p, NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  MolState& s = reinterpret_cast<SccCta*>(smraw)->s;
+  const int tid = threadIdx.x;
+  StageClock clk(A.B.stage_cycles);
+  scc_begin<KIND>(A, m);
+  scc_cholesky<KIND>(A);
+  if (s.status != kOk) {
+    if (tid == 0) {
+      A.B.status[m] = s.status;
+      A.B.iterations[m] = 0;
     }
     return;
   }
-  for (int i = wid; i < N; i += NW)
-    for (int j = i + 1 + lane; j < N; j += 32) L[(long long)i * N + j] = 0.0;
-  __syncthreads();
   clk.mark(kStChol);
-  // L^-1 by forward substitution L X = I, one thread per column.  The lanes
-  // of a warp step through the rows together, so row i of L is a broadcast
-  // and the reads of X[k][c] coalesce; a warp starts at its first column
-  // (rows above it are zeros in all of its columns), four partial sums.
-  for (int c0 = 0; c0 < N; c0 += NT) {
-    const int c = c0 + tid;
-    const int cc = min(c, N - 1);
-    const int kw = min(N, c0 + (tid & ~31));  // the warp's first column
-    if (c < N)
-      for (int i = 0; i < kw; ++i) Li[(long long)i * N + c] = 0.0;
-    for (int i = kw; i < N; ++i) {
-      const double* li = L + (long long)i * N;
-      double s0 = (i == c) ? 1.0 : 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-      int k = kw;
-      for (; k + 3 < i; k += 4) {
-        s0 -= li[k] * Li[(long long)k * N + cc];
-        s1 -= li[k + 1] * Li[(long long)(k + 1) * N + cc];
-        s2 -= li[k + 2] * Li[(long long)(k + 2) * N + cc];
-        s3 -= li[k + 3] * Li[(long long)(k + 3) * N + cc];
-      }
-      for (; k < i; ++k) s0 -= li[k] * Li[(long long)k * N + cc];
-      if (c < N) Li[(long long)i * N + c] = ((s0 + s1) + (s2 + s3)) / li[i];
-    }
-  }
-  __syncthreads();
+  scc_inverse<KIND>(A);
   clk.mark(kStLinv);
-  // H0' = L^-1 H0 L^-T on the FP64 tensor cores: U = L^-1 H0 in 8x8 tiles
-  // (row i of L^-1 ends at the diagonal), then H0' = U (L^-1)^T for the tiles
-  // on and below the diagonal, each written to both triangles so that H0' is
-  // exactly symmetric.  U uses the global work matrix, free until the first
-  // iteration.  Each warp owns whole tiles; lanes beyond N load zeros.
-  {
-    double* U = w.A;
-    const int T = (N + 7) >> 3;
-    const int g = lane >> 2, t4 = lane & 3;
-    for (int tile = wid; tile < T * T; tile += NW) {
-      const int I = tile / T, J = tile - I * T;
-      const int i = I * 8 + g, jb = J * 8 + g;
-      const int kend = min(N, I * 8 + 8);
-      double d0 = 0.0, d1 = 0.0;
-#pragma unroll 4
-      for (int k0 = 0; k0 < kend; k0 += 4) {
-        const int k = k0 + t4;
-        const double a = (i < N && k < N) ? Li[(long long)i * N + k] : 0.0;
-        const double b = (k < N && jb < N) ? H0[(long long)k * N + jb] : 0.0;
-        dmma_m8n8k4(d0, d1, a, b);
-      }
-      const int jc = J * 8 + 2 * t4;
-      if (i < N && jc < N) U[(long long)i * N + jc] = d0;
-      if (i < N && jc + 1 < N) U[(long long)i * N + jc + 1] = d1;
-    }
-    __syncthreads();
-    for (int tile = wid; tile < T * (T + 1) / 2; tile += NW) {
-      int I = 0;
-      while ((I + 1) * (I + 2) / 2 <= tile) ++I;
-      const int J = tile - I * (I + 1) / 2;
-      const int i = I * 8 + g, jb = J * 8 + g;
-      const int kend = min(N, J * 8 + 8);
-      double d0 = 0.0, d1 = 0.0;
-#pragma unroll 4
-      for (int k0 = 0; k0 < kend; k0 += 4) {
-        const int k = k0 + t4;
-        const double a = (i < N && k < N) ? U[(long long)i * N + k] : 0.0;
-        const double b = (jb < N && k < N) ? Li[(long long)jb * N + k] : 0.0;
-        dmma_m8n8k4(d0, d1, a, b);
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int j = J * 8 + 2 * t4 + c;
-        if (i < N && j < N && (I != J || j <= i)) {
-          const double v = c ? d1 : d0;
-          Hp[(long long)i * N + j] = v;
-          Hp[(long long)j * N + i] = v;
-        }
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- SCC state
-  double nref = 0.0;
-  for (int s = 0; s < nsh; ++s) nref += M.elem[B.z[a0 + sh_atom[s]]].refocc[sh_k[s]];
-  const double nelec = nref - B.charge[m];
-  // a requested spin multiplicity: alpha and beta electron counts (validated on the host)
-  const bool spin = opt.spin_mult > 0;
-  const double nalpha = spin ? 0.5 * (rint(nelec) + (opt.spin_mult - 1)) : 0.0;
-  const double nbeta = spin ? 0.5 * (rint(nelec) - (opt.spin_mult - 1)) : 0.0;
-  const int nneed0 = min(N, max(1, (int)ceil(spin ? nalpha : 0.5 * nelec) + 8));
-  int bro_iter = 0;
-  double last_e = 0.0;
-  bool have_e = false;
-  bool converged = false;
-  int nneed_last = nneed0;  // eigenvalues 0..nneed_last-1 and N-1 of the last diagonalisation are known
-  int iter = 0;
-  int nocc = 0;
-  double e_el = 0.0, e2 = 0.0, e3 = 0.0, ts = 0.0, mu = 0.0, rms = 0.0;
+  scc_h0<KIND>(A);
   // The reference's fallback ladder (src/electronic.rs:1390-1447): rung 0 is
   // the requested options (the main kernel); rungs 1-3 (the Robust kernel,
   // for molecules rung 0 left unconverged) restart from the initial charges
@@ -1748,408 +1896,102 @@ __device__ void scc_molecule(const Batch& B, const Model& M, const SccOptions& o
   // 0.1 / max(requested, 0.1), then Broyden at T_el >= 3000 K without shift.
   // A requested level shift sends every molecule to the Robust kernel, which
   // then starts at rung 0 (the main kernel carries no level-shift code).
-  const int rung_first = Robust ? (opt.level_shift != 0.0 ? 0 : 1) : 0, rung_last = Robust ? 3 : 0;
-  [[maybe_unused]] int rung_used = rung_first;  // the rung whose SCC converged (reported by the ladder kernel)
-  for (int rung = rung_first; rung <= rung_last && !converged; ++rung) {
-  rung_used = rung;
-  SccOptions ro = opt;
-  double lshift = Robust ? opt.level_shift : 0.0;
-  if (rung == 1 || rung == 2) {
-    ro.broyden = 0;
-    ro.mixing = rung == 1 ? 0.20 : 0.10;
-    lshift = fmax(opt.level_shift, rung == 1 ? 0.20 : 0.10);
-    ro.max_scc = max(opt.max_scc, 800);
-  } else if (rung == 3) {
-    ro.etemp = fmax(opt.etemp, 3000.0);
-    ro.max_scc = max(opt.max_scc, 250);
-    lshift = 0.0;
-  }
-  const double kt = fmax(ro.etemp, 0.0) * kBoltzmann;
-  for (int s = tid; s < nsh; s += NT) w.qin[s] = B.init_q ? B.init_q[sh0 + s] : 0.0;
-  bro_iter = 0;
-  last_e = 0.0;
-  have_e = false;
-  bool have_prev = false;  // a previous density to shift against (rungs with a level shift)
-  __syncthreads();
-  clk.mark(kStPrologue);
-
-  for (iter = 1; iter <= ro.max_scc; ++iter) {
-    // (1) shell potential from the input charges
-    stage_potential<NT>(B, M, mc, w, vao);
-    // (2) F' = H0' - 1/2 (M + M^T) with M = L^-1 diag(v) L lower triangular,
-    //     so F'_ij = H0'_ij - M_ij / 2 below the diagonal and H0'_ii - M_ii on
-    //     it.  M on the FP64 tensor cores: pairs of 8x8 tiles (I, J), (I, J+1)
-    //     on and below the diagonal sharing the L^-1 fragment, k from the
-    //     pair's first column to its last row (the entries of L above the
-    //     diagonal are stored zeros, so the second tile's extra k add nothing).
-    {
-      const int T = (N + 7) >> 3;
-      const int g = lane >> 2, t4 = lane & 3;
-      int I = 0, base = 0;  // base: pairs of the rows of tiles before I
-      for (int task = wid;; task += NW) {
-        while (I < T && task >= base + (I >> 1) + 1) {
-          base += (I >> 1) + 1;
-          ++I;
-        }
-        if (I >= T) break;
-        const int J = 2 * (task - base);
-        const bool two = J + 1 <= I;
-        const int i = I * 8 + g, jb0 = J * 8 + g, jb1 = jb0 + 8;
-        const bool iok = i < N;
-        const double* lirow = Li + (long long)(iok ? i : 0) * N;
-        const int kend = min(N, I * 8 + 8);
-        double d00 = 0.0, d01 = 0.0, d10 = 0.0, d11 = 0.0;
-#pragma unroll 4
-        for (int k0 = J * 8; k0 < kend; k0 += 4) {
-          const int k = k0 + t4;
-          const bool kin = k < N;
-          const double* lk = L + (long long)(kin ? k : 0) * N;
-          const double vk = kin ? vao[k] : 0.0;
-          const double a = (iok && kin) ? lirow[k] : 0.0;
-          const double b0 = (kin && jb0 < N) ? lk[jb0] * vk : 0.0;
-          dmma_m8n8k4(d00, d01, a, b0);
-          if (two) {
-            const double b1 = (kin && jb1 < N) ? lk[jb1] * vk : 0.0;
-            dmma_m8n8k4(d10, d11, a, b1);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int j = J * 8 + 2 * t4 + (c & 1) + (c >> 1) * 8;
-          if (iok && j <= i && (c < 2 || two)) {
-            const double mv = c == 0 ? d00 : c == 1 ? d01 : c == 2 ? d10 : d11;
-            const double f = Hp[(long long)i * N + j] - (i == j ? mv : 0.5 * mv);
-            A[(long long)i * lda + j] = f;
-            A[(long long)j * lda + i] = f;
-          }
-        }
-      }
+  const int rung_first = Robust ? (A.opt.level_shift != 0.0 ? 0 : 1) : 0, rung_last = Robust ? 3 : 0;
+  int rung_used = rung_first;  // the rung whose SCC converged (reported by the ladder kernel)
+  for (int rung = rung_first; rung <= rung_last && !s.converged; ++rung) {
+    rung_used = rung;
+    int broyden = A.opt.broyden, max_scc = A.opt.max_scc;
+    double mixing = A.opt.mixing, etemp = A.opt.etemp, lshift = Robust ? A.opt.level_shift : 0.0;
+    if (rung == 1 || rung == 2) {
+      broyden = 0;
+      mixing = rung == 1 ? 0.20 : 0.10;
+      lshift = fmax(A.opt.level_shift, rung == 1 ? 0.20 : 0.10);
+      max_scc = max(A.opt.max_scc, 800);
+    } else if (rung == 3) {
+      etemp = fmax(A.opt.etemp, 3000.0);
+      max_scc = max(A.opt.max_scc, 250);
+      lshift = 0.0;
     }
     __syncthreads();
-    if (Robust && lshift != 0.0 && have_prev) {
-      // level shift F += lshift (S - S P_prev S / 2) (src/electronic.rs:2125-2137);
-      // in the orthonormal basis F' += lshift (I - Z f Z^T / 2) with the
-      // previous iteration's eigenvectors Z and occupations f
-      for (long long idx = tid; idx < (long long)N * N; idx += NT) {
-        const int i = (int)(idx / N), j = (int)(idx % N);
-        if (j > i) continue;
-        double sp = 0.0;
-        for (int k = 0; k < nocc; ++k) sp += occ[k] * Z[(long long)i * N + k] * Z[(long long)j * N + k];
-        const double val = lshift * ((i == j ? 1.0 : 0.0) - 0.5 * sp);
-        A[(long long)i * lda + j] += val;
-        if (i != j) A[(long long)j * lda + i] += val;
+    {
+      const CtaView v = cta_view(A);
+      for (int i = tid; i < s.nsh; i += NT) v.w.qin[i] = A.B.init_q ? A.B.init_q[s.sh0 + i] : 0.0;
+    }
+    if (tid == 0) {
+      s.kt = fmax(etemp, 0.0) * kBoltzmann;
+      s.bro_iter = 0;
+      s.have_e = 0;
+      s.last_e = 0.0;
+      s.iter = 1;
+    }
+    __syncthreads();
+    clk.mark(kStPrologue);
+    for (int iter = 1; iter <= max_scc; ++iter) {
+      scc_potential<KIND>(A);
+      {  // (2) F' = H0' - 1/2 (M + M^T), M = L^-1 diag(v) L
+        const CtaView v = cta_view(A);
+        fock_build<NW>(v.w.L, v.w.LiT, v.w.Hp, s.ld, s.vec_at + 6 * s.N, s.N, v.w.F, s.ld);
       }
       __syncthreads();
-    }
-    clk.mark(kStFock);
-    // (3) Householder tridiagonalisation
-    if constexpr (NT == 128) {
-      if (N <= 32 * 6 + 1 && !a_shared)  // e^2 is formed after the reduction, so its slot is the reduction's scratch
-        tridiagonalize_blocked<NT>(A, lda, N, d, e, tau, pvec, esq, w.W1, sh);
-      else
-        tridiagonalize<NT>(A, lda, N, d, e, tau, pvec, sh);
-    } else {
-      tridiagonalize<NT>(A, lda, N, d, e, tau, pvec, sh);
-    }
-    clk.mark(kStTridiag);
-    // (4) eigenvalues needed by the occupations
-    double gl = INFINITY, gu = -INFINITY, onenrm = 0.0, emax2 = 0.0;
-    for (int i = tid; i < N; i += NT) {
-      const double off = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < N - 1 ? fabs(e[i]) : 0.0);
-      gl = fmin(gl, d[i] - off);
-      gu = fmax(gu, d[i] + off);
-      onenrm = fmax(onenrm, fabs(d[i]) + off);
-      if (i < N - 1) {
-        esq[i] = e[i] * e[i];
-        emax2 = fmax(emax2, esq[i]);
+      if (Robust && lshift != 0.0 && iter > 1) scc_level_shift<KIND>(A, lshift);
+      clk.mark(kStFock);
+      {  // (3) Householder reduction: reflectors in the rows of w.V, their WY factors in its scratch
+        const CtaView v = cta_view(A);
+        const int N = s.N, ldv = refl_ld(N);
+        if (P == 128 && N <= 96)  // every slot in registers
+          tridiag_cta<NT, P == 128 ? 96 : P>(v.w.F, s.ld, N, s.vec_at, v.w.V, ldv, s.tri_at);
+        else
+          tridiag_cta<NT, P>(v.w.F, s.ld, N, s.vec_at, v.w.V, ldv, s.tri_at);
+        wy_factors<NW>(v.w.V, ldv, N, s.vec_at + 2 * N, s.tri_at);
       }
-    }
-    gl = -block_max(-gl, sh.red);
-    gu = block_max(gu, sh.red);
-    onenrm = block_max(onenrm, sh.red);
-    emax2 = block_max(emax2, sh.red);
-    const double pivmin = DBL_MIN * fmax(1.0, emax2);
-    {
-      const double span = gu - gl;
-      gl -= 2.1 * DBL_EPSILON * fabs(gl) + 4.0 * DBL_EPSILON * span + pivmin;
-      gu += 2.1 * DBL_EPSILON * fabs(gu) + 4.0 * DBL_EPSILON * span + pivmin;
-    }
-    int nneed = nneed0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      // from the previous iteration's eigenvalues once this rung has one
-      eigenvalues<NT>(d, esq, N, nneed, gl, gu, pivmin, 4.0 * DBL_EPSILON * onenrm, eps,
-                      (iter > 1 && attempt == 0) ? nneed_last : 0);
-      clk.mark(kStEigval);
-      // (5) occupations (src/electronic.rs:3815-3921)
-      if (spin) {
-        spin_channel_occupations<NT>(eps, N, nneed, nalpha, nbeta, kt, occ, pop, sh);
-      } else if (kt > 0.0 && nelec > 0.0 && nelec < 2.0 * N) {
-        double fm, ft;
-        bool amb;
-        fermi_cta<NT, 2>(eps, N, nneed, nelec, kt, occ, sh, fm, ft, amb);
-        if (tid == 0) {
-          sh.scal[1] = fm;
-          sh.scal[2] = ft;
-          sh.iscal[2] = amb ? 1 : 0;
-        }
-      } else if (wid == 0) {  // aufbau and the empty / full limits
-        double fm, ft;
-        bool amb;
-        fermi_warp<2>(eps, N, nneed, nelec, kt, occ, fm, ft, amb);
-        if (lane == 0) {
-          sh.scal[1] = fm;
-          sh.scal[2] = ft;
-          sh.iscal[2] = amb ? 1 : 0;
-        }
+      clk.mark(kStTridiag);
+      scc_occupations<KIND>(A, &clk);
+      scc_vectors<KIND>(A);
+      clk.mark(kStInvIter);
+      {  // (7) back-transformation, (8) C = L^-T Z and the AO populations
+        const CtaView v = cta_view(A);
+        const int N = s.N, ld = s.ld;
+        occupied_orbitals<NW, P>(v.w.V, refl_ld(N), s.tri_at, N, v.w.Z, ld, s.nocc, s.vec_at + 4 * N, s.vec_at + 5 * N,
+                                 v.w.L, v.w.LiT, ld, v.w.Ct, v.w.popw, Robust ? v.w.Z : nullptr);
       }
       __syncthreads();
-      clk.mark(kStFermi);
-      if (!sh.iscal[2] || nneed == N) break;
-      nneed = N;
-    }
-    mu = sh.scal[1];
-    ts = sh.scal[2];
-    nneed_last = nneed;
-    // number of orbitals whose occupation matters at FP64 resolution
-    int nocc_loc = 0;
-    for (int i = tid; i < N; i += NT)
-      if ((i < nneed || i == N - 1) && occ[i] > 1e-30) nocc_loc = max(nocc_loc, i + 1);
-    nocc = (int)block_max((double)nocc_loc, sh.red);
-    // (6) inverse iteration for the occupied eigenvectors (columns of Z)
-    const double ortol = 1e-5 * onenrm;
-    const double tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
-    for (int j = tid; j < nocc; j += NT) {
-      const bool start = (j == 0) || (eps[j] - eps[j - 1] > ortol);
-      if (!start) continue;
-      int jend = j + 1;
-      while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
-      double* ws = iw + j;  // column j of the interleaved factor arrays
-      double lam_prev = -INFINITY;
-      for (int jj = j; jj < jend; ++jj) {
-        double lam = eps[jj];
-        const double pert = 10.0 * DBL_EPSILON * fmax(fabs(lam), onenrm);
-        if (jj > j && lam - lam_prev < pert) lam = lam_prev + pert;
-        lam_prev = lam;
-        double* x = Z + jj;  // column jj, stride N
-        if (jend - j == 1) {
-          // isolated: the start vector's forward elimination runs with the
-          // factorisation, the two solves are not normalised in between
-          // (growth below 1e40), and the second one returns |x|^2
-          const double cur = tri_factor_rhs(d, e, N, lam, tiny, ws, N, x, N, (unsigned)jj);
-          tri_back(ws, N, N, x, N, cur);
-          const double nrm = tri_solve(ws, N, N, x, N);
-          const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
-#pragma unroll 8
-          for (int i = 0; i < N; ++i) x[(long long)i * N] *= inv;
-          continue;
-        }
-        tri_factor(d, e, N, lam, tiny, ws, N);
-#pragma unroll 4
-        for (int i = 0; i < N; ++i) x[(long long)i * N] = hash_unit(i, jj) + 1e-3;
-        const int nit = 4;
-        for (int it = 0; it < nit; ++it) {
-          tri_solve(ws, N, N, x, N);
-          for (int q = j; q < jj; ++q) {  // modified Gram-Schmidt inside the cluster
-            double dot = 0.0;
-            for (int i = 0; i < N; ++i) dot += Z[(long long)i * N + q] * x[(long long)i * N];
-            for (int i = 0; i < N; ++i) x[(long long)i * N] -= dot * Z[(long long)i * N + q];
-          }
-          double nrm = 0.0;
-#pragma unroll 8
-          for (int i = 0; i < N; ++i) nrm += x[(long long)i * N] * x[(long long)i * N];
-          const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
-#pragma unroll 8
-          for (int i = 0; i < N; ++i) x[(long long)i * N] *= inv;
-        }
-      }
-    }
-    __syncthreads();
-    clk.mark(kStInvIter);
-    // (7) back-transformation Z := Q Z
-    back_transform<NT>(A, lda, tau, N, Z, N, nocc, w.W1, w.W2, sh);
-    clk.mark(kStBackTr);
-    // (8) C = L^-T Z, D = L Z (= S C) and the AO populations
-    //     (S P)_mu,mu = sum_i f_i C_mu,i D_mu,i on the FP64 tensor cores: each
-    //     warp owns 8-row blocks of mu and runs over pairs of 8-column tiles
-    //     of the occupied eigenvectors (the rows of L and L^-T are shared by
-    //     the pair; four independent accumulator chains where the ranges of
-    //     k overlap).  Row mu of L ends and column mu of L^-1 starts at the
-    //     diagonal.  D only feeds the populations and is not stored.
-    {
-      const int T = (N + 7) >> 3, Ti = (nocc + 7) >> 3;
-      const int g = lane >> 2, t4 = lane & 3;
-      for (int MU = wid; MU < T; MU += NW) {
-        const int mu = MU * 8 + g;
-        const bool mu_ok = mu < N;
-        const double* lrow = L + (long long)(mu_ok ? mu : 0) * N;
-        const int kd = min(N, MU * 8 + 8), kc = MU * 8;  // D: k < kd; C: k >= kc
-        double pp = 0.0;
-        for (int IV = 0; IV < Ti; IV += 2) {
-          const int ib0 = IV * 8 + g, ib1 = ib0 + 8;
-          const bool ok0 = ib0 < nocc, ok1 = ib1 < nocc;
-          double c00 = 0.0, c01 = 0.0, c10 = 0.0, c11 = 0.0;
-          double d00 = 0.0, d01 = 0.0, d10 = 0.0, d11 = 0.0;
-#pragma unroll 4
-          for (int k0 = 0; k0 < N; k0 += 4) {
-            const int k = k0 + t4;
-            const bool kin = k < N;
-            const double* zk = Z + (long long)(kin ? k : 0) * N;
-            const double b0 = (kin && ok0) ? zk[ib0] : 0.0;
-            const double b1 = (kin && ok1) ? zk[ib1] : 0.0;
-            if (k0 < kd) {
-              const double a = (mu_ok && kin) ? lrow[k] : 0.0;
-              dmma_m8n8k4(d00, d01, a, b0);
-              dmma_m8n8k4(d10, d11, a, b1);
-            }
-            if (k0 >= kc) {
-              const double a = (mu_ok && kin) ? Li[(long long)k * N + mu] : 0.0;
-              dmma_m8n8k4(c00, c01, a, b0);
-              dmma_m8n8k4(c10, c11, a, b1);
-            }
-          }
-          const int ic = IV * 8 + 2 * t4;
-          if (mu_ok) {
-            if (ic < nocc) {
-              C[(long long)mu * N + ic] = c00;
-              pp += occ[ic] * c00 * d00;
-            }
-            if (ic + 1 < nocc) {
-              C[(long long)mu * N + ic + 1] = c01;
-              pp += occ[ic + 1] * c01 * d01;
-            }
-            if (ic + 8 < nocc) {
-              C[(long long)mu * N + ic + 8] = c10;
-              pp += occ[ic + 8] * c10 * d10;
-            }
-            if (ic + 9 < nocc) {
-              C[(long long)mu * N + ic + 9] = c11;
-              pp += occ[ic + 9] * c11 * d11;
-            }
-          }
-        }
-        pp += __shfl_xor_sync(0xffffffffu, pp, 1);
-        pp += __shfl_xor_sync(0xffffffffu, pp, 2);
-        if (t4 == 0 && mu < N) pop[mu] = pp;
-      }
-    }
-    __syncthreads();
-    clk.mark(kStPop);
-    // (9) output charges, energies
-    stage_charges_energy<NT>(B, M, mc, w, pop, occ, eps, vao, nocc, sh, e_el, e2, e3, rms);
-    if (Robust && lshift != 0.0) {
-      // with a shifted Fock matrix sum(f eps) is not tr(F P): E_el = tr(H0 P) = sum_k f_k z_k^T H0' z_k
-      double part = 0.0;
-      for (long long idx = tid; idx < (long long)N * nocc; idx += NT) {
-        const int i = (int)(idx / nocc), k = (int)(idx % nocc);
-        double hz = 0.0;
-        for (int j = 0; j < N; ++j) hz += Hp[(long long)i * N + j] * Z[(long long)j * N + k];
-        part += occ[k] * Z[(long long)i * N + k] * hz;
-      }
-      e_el = block_sum(part, sh.red);
-    }
-    const double escc = e_el + e2 + e3 + ts;
-    const double err = have_e ? fabs(escc - last_e) : INFINITY;
-    if (err < opt.energy_tol && rms < opt.charge_tol) {
-      converged = true;
-      break;
-    }
-    clk.mark(kStEnergy);
-    // (10) charge mixing
-    stage_mix<NT>(ro, mc, w, cap, bro_iter, sh);
-    last_e = escc;
-    have_e = true;
-    have_prev = lshift != 0.0;
-    __syncthreads();
-    clk.mark(kStMix);
-  }
-  if (iter > ro.max_scc) iter = ro.max_scc;
-  }  // rungs
-  if (!Robust && !converged && B.failed && tid == 0) B.failed[atomicAdd(B.queue + 3, 1)] = m;
-  if constexpr (Robust) {  // rung-0 molecules keep the 0 the host wrote before the launches
-    if (B.rung && tid == 0) B.rung[m] = converged ? rung_used : -1;
-  }
-
-  // ---- results
-  stage_results<NT>(B, mc, w, iter, converged, e_el, e2, e3, ts, mu);
-  if (B.orb_eps) {  // orbital energies (NaN where the eigensolver did not need them) and occupations
-    const int ao0 = B.ao_off[m];
-    for (int i = tid; i < N; i += NT) {
-      B.orb_eps[ao0 + i] = (i < nneed_last || i == N - 1) ? eps[i] : __longlong_as_double(0x7ff8000000000000LL);
-      B.orb_occ[ao0 + i] = occ[i];
+      clk.mark(kStPop);
+      scc_energy<KIND, Robust>(A, lshift);
+      clk.mark(kStEnergy);
+      if (s.converged || iter == max_scc) break;
+      scc_mix<KIND>(A, broyden, mixing);
+      if (tid == 0) s.iter = iter + 1;
+      __syncthreads();
+      clk.mark(kStMix);
     }
   }
-  // density and energy-weighted density of the last diagonalisation
-  // (src/linalg.rs:243-273), kept per molecule for the gradient kernel:
-  // P = C f C^T and W = C f eps C^T on the FP64 tensor cores, 8x8 tiles on
-  // and below the diagonal written to both triangles
-  {
-    const int T = (N + 7) >> 3;
-    const int g = lane >> 2, t4 = lane & 3;
-    for (int tile = wid; tile < T * (T + 1) / 2; tile += NW) {
-      int I = 0;
-      while ((I + 1) * (I + 2) / 2 <= tile) ++I;
-      const int J = tile - I * (I + 1) / 2;
-      const int i = I * 8 + g, jb = J * 8 + g;
-      double p0 = 0.0, p1 = 0.0, q0 = 0.0, q1 = 0.0;
-#pragma unroll 4
-      for (int k0 = 0; k0 < nocc; k0 += 4) {
-        const int k = k0 + t4;
-        const double ci = (i < N && k < nocc) ? C[(long long)i * N + k] * occ[k] : 0.0;
-        const double cj = (jb < N && k < nocc) ? C[(long long)jb * N + k] : 0.0;
-        dmma_m8n8k4(p0, p1, ci, cj);
-        dmma_m8n8k4(q0, q1, k < nocc ? ci * eps[k] : 0.0, cj);
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int j = J * 8 + 2 * t4 + c;
-        if (i < N && j <= i) {
-          const double pv = c ? p1 : p0, qv = c ? q1 : q0;
-          B.P[mo + (long long)i * N + j] = pv;
-          B.P[mo + (long long)j * N + i] = pv;
-          B.W[mo + (long long)i * N + j] = qv;
-          B.W[mo + (long long)j * N + i] = qv;
-        }
-      }
-    }
-  }
-  __syncthreads();
+  scc_finish<KIND, Robust>(A, rung_used);
   clk.mark(kStFinal);
 }
 
 // Persistent SCC kernel.  Robust = false: molecules q_begin..q_end of the
 // processing order (rung 0 of the fallback ladder); Robust = true: the
 // molecules the rung-0 launches left unconverged (rungs 1-3).
-template <int NT, bool Robust>
-__global__ void __launch_bounds__(NT, (kSccThreadsPerSm / NT) > 0 ? kSccThreadsPerSm / NT : 1)
-    scc_kernel(Batch B, Model M, SccOptions opt, SccLaunch SL) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ SccShared sh;
+template <int KIND, bool Robust>
+__global__ void __launch_bounds__(kSccKinds[KIND].nt, kSccKinds[KIND].ctas)
+    scc_kernel(const __grid_constant__ SccArgs A) {
   __shared__ int next;
-  int* sh_atom = (int*)smraw;
-  int* sh_k = sh_atom + SL.maxnsh;
-  int* sh_ao0 = sh_k + SL.maxnsh;
-  int* ao_sh = sh_ao0 + SL.maxnsh;
-  int* atom_sh = ao_sh + SL.maxn;  // maxnat + 1
-  const size_t ib = ((size_t)4 * scc_ints(SL.maxnsh, SL.maxn, SL.maxnat) + 15) & ~(size_t)15;
-  double* vec = (double*)(smraw + ib);
-  double* As = vec + (size_t)kVecSlots * SL.maxn;
-  const long long as_cap = ((long long)SL.smem_bytes - (long long)scc_smem_fixed(SL.maxnsh, SL.maxn, SL.maxnat)) / 8;
-  const int nfailed = Robust ? B.queue[3] : 0;  // written by the rung-0 launches before this one
+  const int nfailed = Robust ? A.B.queue[3] : 0;  // written by the rung-0 launches before this one
   for (;;) {
-    if (threadIdx.x == 0) next = Robust ? atomicAdd(B.queue + 2, 1) : SL.q_begin + atomicAdd(SL.counter, 1);
+    if (threadIdx.x == 0) next = Robust ? atomicAdd(A.B.queue + 2, 1) : A.SL.q_begin + atomicAdd(A.SL.counter, 1);
     __syncthreads();
     const int idx = next;
     __syncthreads();
     int m;
     if (Robust) {
       if (idx >= nfailed) break;
-      m = B.failed[idx];
+      m = A.B.failed[idx];
     } else {
-      if (idx >= SL.q_end) break;
-      m = B.order[idx];
-      if (B.status[m] != kOk) continue;  // rejected during setup
+      if (idx >= A.SL.q_end) break;
+      m = A.B.order[idx];
+      if (A.B.status[m] != kOk) continue;  // rejected during setup
     }
-    scc_molecule<NT, Robust>(B, M, opt, SL, m, sh, sh_atom, sh_k, ao_sh, atom_sh, sh_ao0, vec, As, as_cap);
+    scc_molecule<KIND, Robust>(A, m);
   }
 }
 
@@ -2178,53 +2020,44 @@ long long scc_workspace_doubles(int maxn, int maxnsh, int cap, int maxnat) {
   return cta_ws_size(maxn, maxnsh, cap, maxnat);
 }
 
-// Dynamic shared memory for a class: index tables, vectors and, when
-// `matrix_n` > 0, room for a matrix_n x work_lda(matrix_n) working matrix.
-size_t scc_smem_bytes(int maxnsh, int maxn, int maxnat, int matrix_n) {
-  const size_t fixed = scc_smem_fixed(maxnsh, maxn, maxnat);
-  return matrix_n > 0 ? fixed + sizeof(double) * (size_t)matrix_n * work_lda(matrix_n) : fixed;
+// The kernel a molecule of N AOs runs on: the first whose registers hold its
+// matrix (the last one takes what a raised large-molecule threshold leaves).
+int scc_kind(int N) { return N <= kSccKinds[0].p ? 0 : (N <= kSccKinds[1].p ? 1 : 2); }
+
+// Dynamic shared memory of a launch: index tables, N-vectors and the scratch of
+// the reduction.
+size_t scc_smem_bytes(int kind, int maxnsh, int maxn, int maxnat) {
+  const size_t tri = kind == 0   ? TriShape<kSccKinds[0].nt, kSccKinds[0].p>::kDoubles
+                     : kind == 1 ? TriShape<kSccKinds[1].nt, kSccKinds[1].p>::kDoubles
+                                 : TriShape<kSccKinds[2].nt, kSccKinds[2].p>::kDoubles;
+  return scc_smem_fixed(maxnsh, maxn, maxnat) + sizeof(double) * tri;
 }
 
-// Largest dynamic shared memory a CTA of the class may request: the SM's
-// 228 KB shared by its kSccThreadsPerSm / nt CTAs (1 KB of which each CTA reserves), less
-// the kernel's static shared memory.
-size_t scc_max_dynamic_smem(int nt) {
-  cudaFuncAttributes a;
-  const cudaError_t e = nt == 512   ? cudaFuncGetAttributes(&a, scc_kernel<512, false>)
-                        : nt == 256 ? cudaFuncGetAttributes(&a, scc_kernel<256, false>)
-                                    : cudaFuncGetAttributes(&a, scc_kernel<128, false>);
-  const size_t stat = e == cudaSuccess ? a.sharedSizeBytes : 8192;
-  const int ctas = std::max(1, kSccThreadsPerSm / nt);
-  const size_t per_cta = 233472 / ctas - 1024;  // the SM's 228 KB shared by its CTAs
-  return per_cta - stat - 256;
-}
-
-template <int NT, bool Robust>
-static cudaError_t launch_scc_nt(int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
-                                 const SccOptions& opt, const SccLaunch& SL) {
-  cudaError_t e = cudaFuncSetAttribute(scc_kernel<NT, Robust>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int KIND, bool Robust>
+static cudaError_t launch_scc_kind(int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
+                                   const SccOptions& opt, const SccLaunch& SL) {
+  cudaError_t e = cudaFuncSetAttribute(scc_kernel<KIND, Robust>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  scc_kernel<NT, Robust><<<grid, NT, smem, st>>>(B, M, opt, SL);
+  scc_kernel<KIND, Robust><<<grid, kSccKinds[KIND].nt, smem, st>>>(SccArgs{B, M, opt, SL});
   return cudaGetLastError();
 }
 
-// Host launcher of one size class (nt = 512, 256 or 128 threads per CTA;
-// 512 / nt CTAs share an SM).
-cudaError_t launch_scc(int nt, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
+// Host launcher of one size class.
+cudaError_t launch_scc(int kind, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
                        const SccOptions& opt, const SccLaunch& SL) {
-  if (nt == 512) return launch_scc_nt<512, false>(grid, smem, st, B, M, opt, SL);
-  if (nt == 256) return launch_scc_nt<256, false>(grid, smem, st, B, M, opt, SL);
-  if (nt == 128) return launch_scc_nt<128, false>(grid, smem, st, B, M, opt, SL);
+  if (kind == 0) return launch_scc_kind<0, false>(grid, smem, st, B, M, opt, SL);
+  if (kind == 1) return launch_scc_kind<1, false>(grid, smem, st, B, M, opt, SL);
+  if (kind == 2) return launch_scc_kind<2, false>(grid, smem, st, B, M, opt, SL);
   return cudaErrorInvalidValue;
 }
 
 // Host launcher of the fallback-ladder kernel (rungs 1-3 for the molecules
 // listed in B.failed; returns at once when the list is empty).
-cudaError_t launch_scc_robust(int nt, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
+cudaError_t launch_scc_robust(int kind, int grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
                               const SccOptions& opt, const SccLaunch& SL) {
-  if (nt == 512) return launch_scc_nt<512, true>(grid, smem, st, B, M, opt, SL);
-  if (nt == 256) return launch_scc_nt<256, true>(grid, smem, st, B, M, opt, SL);
-  if (nt == 128) return launch_scc_nt<128, true>(grid, smem, st, B, M, opt, SL);
+  if (kind == 0) return launch_scc_kind<0, true>(grid, smem, st, B, M, opt, SL);
+  if (kind == 1) return launch_scc_kind<1, true>(grid, smem, st, B, M, opt, SL);
+  if (kind == 2) return launch_scc_kind<2, true>(grid, smem, st, B, M, opt, SL);
   return cudaErrorInvalidValue;
 }
 
