@@ -25,10 +25,12 @@
 #include "model.cuh"
 
 namespace gfn1 {
-cudaError_t launch_setup(int max_l, dim3 grid, int nt, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
-                         int enable_dispersion, int max_nsh, const int* mols);
-cudaError_t launch_grad(int max_l, dim3 grid, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
-                        const int* mols, int phases);
+cudaError_t launch_setup(int max_l, int n, int max_nat, int max_nsh, bool halogens, int num_sms, cudaStream_t st,
+                         const Batch& B, const Model& M, int enable_dispersion, const int* mols);
+int setup_launches(int n, int max_nat, bool halogens, int num_sms);
+int grad_launches(int n, int max_nat, int num_sms);
+cudaError_t launch_grad(int max_l, int n, int max_nat, int num_sms, cudaStream_t st, const Batch& B, const Model& M,
+                        const int* mols);
 long long scc_workspace_doubles(int maxn, int maxnsh, int cap, int maxnat);
 int scc_kind(int N);
 size_t scc_smem_bytes(int kind, int maxnsh, int maxn, int maxnat);
@@ -289,6 +291,8 @@ struct gfn1_batch {
   int nmol = 0;
   long long natoms = 0, nshells = 0, naos = 0, mat_total = 0, gam_total = 0, pair_total = 0;
   int max_nat = 0, max_nsh = 0, max_n = 0, cap = 0;
+  int small_nat = 0, small_nsh = 0;  // largest of the molecules up to the large-molecule threshold
+  bool halogens = false;  // some atom is a halogen-bond donor
   int max_l = 0;  // highest shell angular momentum of the batch (selects the s/p setup and gradient kernels)
   // SCC size classes, largest molecules first: the molecules of each kernel
   struct SccClass {
@@ -333,7 +337,7 @@ struct gfn1_batch {
   BlobLayout lay;
   HostBuf h_in, h_out;               // pinned staging
   DevBuf<unsigned char> d_in, d_out; // device blobs
-  DevBuf<double> S, H0, P, W, ws, gam, pairbuf, cn, shell_pot, shell_pot_in, se, grad_classic, orb_eps, orb_occ;
+  DevBuf<double> S, H0, P, W, ws, gam, pairbuf, cn, shell_pot, shell_pot_in, se, grad_classic, atom_tmp, orb_eps, orb_occ;
   DevBuf<int> queue;
   // geometry optimisation on the device (gfn1_batch_optimize)
   const int* opt_skip = nullptr;  // molecules the engine kernels skip this round, or null
@@ -385,6 +389,7 @@ struct gfn1_batch {
     B.terms = dout<double>(lay.terms);
     B.grad = dout<double>(lay.grad);
     B.grad_classic = grad_classic.p;
+    B.atom_tmp = atom_tmp.p;
     B.dipole = dout<double>(lay.dipole);
     B.fermi = dout<double>(lay.fermi);
     B.iterations = dout<int>(lay.iterations);
@@ -402,7 +407,7 @@ struct gfn1_batch {
     h_out.release();
     d_in.release();
     d_out.release();
-    for (DevBuf<double>* d : {&S, &H0, &P, &W, &ws, &gam, &pairbuf, &cn, &shell_pot, &shell_pot_in, &se, &grad_classic, &orb_eps, &orb_occ})
+    for (DevBuf<double>* d : {&S, &H0, &P, &W, &ws, &gam, &pairbuf, &cn, &shell_pot, &shell_pot_in, &se, &grad_classic, &atom_tmp, &orb_eps, &orb_occ})
       d->release();
     queue.release();
     stage.release();
@@ -675,6 +680,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   b->natoms = natoms;
   b->max_nat = b->max_nsh = b->max_n = 0;
   b->max_l = 0;
+  b->halogens = false;
   // sizes first (for the blob layout)
   std::vector<int> nsh_m(nmol), n_m(nmol), st_m(nmol, GFN1_OK);
   std::vector<double> nref_m(nmol, 0.0);
@@ -702,6 +708,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
       n += eng->elem[zz].nao;
       s += eng->elem[zz].nsh;
       nref_m[m] += eng->refocc_total[zz];
+      b->halogens = b->halogens || eng->elem[zz].xb != 0.0;
       for (int k = 0; k < eng->elem[zz].nsh; ++k) b->max_l = std::max(b->max_l, eng->elem[zz].l[k]);
     }
     const double ch = charge ? charge[m] : 0.0;
@@ -886,6 +893,8 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
       R.maxnat = std::max(R.maxnat, atom_offsets[mm + 1] - atom_offsets[mm]);
     }
     const int count = nmol - n_dense;
+    b->small_nat = R.maxnat;
+    b->small_nsh = R.maxnsh;
     R.kind = scc_kind(R.maxn);
     // a requested level shift runs every molecule on this kernel: full width
     const int width = o.level_shift != 0.0 ? kSccKinds[R.kind].ctas * eng->num_sms : 64;
@@ -907,7 +916,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
             b->stage.ensure(kStages) && b->S.ensure(mat_total) && b->H0.ensure(mat_total) && b->P.ensure(mat_total) &&
             b->W.ensure(mat_total) && b->ws.ensure((size_t)std::max<long long>(ws_total, 1)) && b->gam.ensure(gam_total) &&
             b->pairbuf.ensure(8 * std::max<long long>(pair_total, 1)) && b->cn.ensure(natoms) &&
-            b->shell_pot.ensure(nshells) && b->shell_pot_in.ensure(nshells) && b->se.ensure(nshells) && b->grad_classic.ensure(3 * natoms) &&
+            b->shell_pot.ensure(nshells) && b->shell_pot_in.ensure(nshells) && b->se.ensure(nshells) && b->grad_classic.ensure(3 * natoms) && b->atom_tmp.ensure(4 * natoms) &&
             b->orb_eps.ensure(std::max<long long>(naos, 1)) && b->orb_occ.ensure(std::max<long long>(naos, 1));
   if (!ok) return fail(eng, GFN1_E_DEVICE, "device allocation failed for the batch workspace");
   if (!b->wide_ids.empty()) {
@@ -948,7 +957,6 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
   gfn1_engine* eng = b->eng;
   const Batch B = b->dev();
   const Model M = eng->model();
-  const int nt = 128;  // setup CTA: four per SM (measured 8.9 against 9.0 ms with 256 threads)
   cudaError_t e = cudaSuccess;
   if (stage == 0) {
     // reset status from the host-validated copy and the work counter
@@ -970,17 +978,13 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
               cudaSuccess)
         return cuda_fail(eng, e, "learned guess");
     }
-    const size_t smem = sizeof(double) * (16 * (size_t)b->max_nat + 32) +
-                        sizeof(int) * (3 * (size_t)b->max_nat + 2 + 2 * (size_t)b->max_nsh);
-    // one CTA per molecule; large molecules (the leading entries of the
-    // processing order) with their shell pairs split over many CTAs; the s/p
-    // instantiation unless the batch has a d shell
+    // the large molecules (the leading entries of the processing order) on their own
     const int nd = b->n_dense, ns = b->nmol - nd;
-    if (ns > 0 && (e = launch_setup(b->max_l, dim3(ns, 1), nt, smem, st, B, M, b->opt.enable_dispersion, b->max_nsh,
-                                    B.order + nd)) != cudaSuccess)
+    if (ns > 0 && (e = launch_setup(b->max_l, ns, b->small_nat, b->small_nsh, b->halogens, eng->num_sms, st, B, M,
+                                    b->opt.enable_dispersion, B.order + nd)) != cudaSuccess)
       return cuda_fail(eng, e, "setup launch");
-    if (nd > 0 && (e = launch_setup(b->max_l, dim3(nd, std::max(1, 4 * eng->num_sms / nd)), nt, smem, st, B, M,
-                                    b->opt.enable_dispersion, b->max_nsh, B.order)) != cudaSuccess)
+    if (nd > 0 && (e = launch_setup(b->max_l, nd, b->max_nat, b->max_nsh, b->halogens, eng->num_sms, st, B, M,
+                                    b->opt.enable_dispersion, B.order)) != cudaSuccess)
       return cuda_fail(eng, e, "setup launch");
   } else if (stage == 1) {
     SccOptions so;
@@ -1057,16 +1061,11 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
     }
   } else if (stage == 2) {
     if (!b->opt.compute_gradient) return GFN1_OK;
-    const size_t smem = sizeof(double) * 7 * (size_t)b->max_nat + sizeof(int) * (3 * (size_t)b->max_nat + 2);
     const int nd = b->n_dense, ns = b->nmol - nd;
-    if (ns > 0 && (e = launch_grad(b->max_l, dim3(ns, 1), smem, st, B, M, B.order + nd, 3)) != cudaSuccess)
+    if (ns > 0 && (e = launch_grad(b->max_l, ns, b->small_nat, eng->num_sms, st, B, M, B.order + nd)) != cudaSuccess)
       return cuda_fail(eng, e, "gradient launch");
-    if (nd > 0) {  // large molecules: atom pairs over many CTAs, then the per-atom sums
-      if ((e = launch_grad(b->max_l, dim3(nd, std::max(1, 4 * eng->num_sms / nd)), smem, st, B, M, B.order, 1)) !=
-              cudaSuccess ||
-          (e = launch_grad(b->max_l, dim3(nd, 1), smem, st, B, M, B.order, 2)) != cudaSuccess)
-        return cuda_fail(eng, e, "gradient launch");
-    }
+    if (nd > 0 && (e = launch_grad(b->max_l, nd, b->max_nat, eng->num_sms, st, B, M, B.order)) != cudaSuccess)
+      return cuda_fail(eng, e, "gradient launch");
   } else {
     return fail(eng, GFN1_E_INVALID_INPUT, "unknown stage");
   }
@@ -1357,8 +1356,11 @@ int gfn1_batch_info(const gfn1_batch* b, int64_t* natoms, int64_t* nshells, int6
   if (naos) *naos = b->naos;
   if (launches) {  // setup, one SCC launch per non-empty size class, the fallback ladder, gradient, learned guess
     const int nd = b->n_dense, ns = b->nmol - nd;  // (the large-molecule SCC launches vary with its iterations)
-    *launches = (ns > 0) + (nd > 0) + (b->cls[0].n_cta > 0) + (b->cls[1].n_cta > 0) + (b->cls[2].n_cta > 0) + (b->robust.n_cta > 0) +
-                (b->opt.compute_gradient ? (ns > 0) + 2 * (nd > 0) : 0) + (b->guess && !b->has_init_q ? 3 : 0);
+    const int sms = b->eng->num_sms;
+    *launches = setup_launches(ns, b->small_nat, b->halogens, sms) + setup_launches(nd, b->max_nat, b->halogens, sms) +
+                (b->cls[0].n_cta > 0) + (b->cls[1].n_cta > 0) + (b->cls[2].n_cta > 0) + (b->robust.n_cta > 0) +
+                (b->opt.compute_gradient ? grad_launches(ns, b->small_nat, sms) + grad_launches(nd, b->max_nat, sms) : 0) +
+                (b->guess && !b->has_init_q ? 3 : 0);
   }
   return GFN1_OK;
 }
@@ -1741,7 +1743,7 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   const size_t w_ws = take(sizeof(double) * ws_doubles), w_gam = take(sizeof(double) * (size_t)nsh * nsh),
                w_pair = take(sizeof(double) * 8 * std::max<long long>(npair, 1)), w_cn = take(sizeof(double) * nat),
                w_pot = take(sizeof(double) * nsh), w_se = take(sizeof(double) * nsh),
-               w_gcl = take(sizeof(double) * 3 * nat), w_queue = take(4 * sizeof(int));
+               w_gcl = take(sizeof(double) * 3 * nat), w_tmp = take(sizeof(double) * 4 * nat), w_queue = take(4 * sizeof(int));
   // the engine's learned guess (as gfn1_run uses it) when the caller gives no
   // initial charges: descriptors and network outputs of the molecule's atoms
   const bool use_guess = eng->guess != nullptr && init_shell_q == nullptr;
@@ -1806,6 +1808,7 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   B.terms = (double*)(base + o_terms);
   B.grad = (double*)(base + o_grad);
   B.grad_classic = (double*)(base + w_gcl);
+  B.atom_tmp = (double*)(base + w_tmp);
   B.dipole = (double*)(base + o_dip);
   B.fermi = (double*)(base + o_fermi);
   B.iterations = (int*)(base + o_iter);
@@ -1824,11 +1827,9 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   so.etemp = o.electronic_temperature;
   so.spin_mult = o.spin_multiplicity;
   so.level_shift = 0.0;
-  const size_t sm_setup = sizeof(double) * (16 * (size_t)nat + 32) + sizeof(int) * (3 * (size_t)nat + 2 + 2 * (size_t)nsh);
   constexpr int kNaKind = 1;  // 256 threads, up to 128 AOs in registers
   static_assert(kSccKinds[kNaKind].p >= kNaMaxAo, "the no-allocation path's largest molecule");
   const size_t sm_scc = scc_smem_bytes(kNaKind, nsh, n, nat);
-  const size_t sm_grad = sizeof(double) * 7 * (size_t)nat + sizeof(int) * (3 * (size_t)nat + 2);
   if (use_guess) {  // predicted shell charges into the initial-charge slot of the input region
     const GuessModel& g = eng->guess->model;
     float* gx = (float*)(base + w_gx);
@@ -1840,7 +1841,7 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
             cudaSuccess)
       return cuda_fail(eng, e, "learned guess");
   }
-  if ((e = launch_setup(2, dim3(1), 128, sm_setup, st, B, M, o.enable_dispersion, nsh, nullptr)) != cudaSuccess)
+  if ((e = launch_setup(2, 1, nat, nsh, true, eng->num_sms, st, B, M, o.enable_dispersion, nullptr)) != cudaSuccess)
     return cuda_fail(eng, e, "setup launch");
   SccLaunch SL;
   SL.q_begin = 0;
@@ -1855,7 +1856,7 @@ extern "C" int gfn1_run_noalloc(gfn1_engine* eng, int nat, const uint8_t* z, con
   SL.smem_bytes = (int)sm_scc;
   if ((e = launch_scc(kNaKind, 1, sm_scc, st, B, M, so, SL)) != cudaSuccess)
     return cuda_fail(eng, e, "scc launch");
-  if (o.compute_gradient && (e = launch_grad(2, dim3(1), sm_grad, st, B, M, nullptr, 3)) != cudaSuccess)
+  if (o.compute_gradient && (e = launch_grad(2, 1, nat, eng->num_sms, st, B, M, nullptr)) != cudaSuccess)
     return cuda_fail(eng, e, "gradient launch");
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(eng, e, "kernel launch");
   if ((e = cudaMemcpyAsync(hout, base + o_terms, out_end - o_terms, cudaMemcpyDeviceToHost, st)) != cudaSuccess)

@@ -32,14 +32,11 @@ constexpr int kMaxShAtom = 3;  // shells per atom on the device path
 constexpr int kMaxPrim = 8;    // H 2s after orthogonalisation to 1s has 7
 constexpr int kMaxRef = 5;     // D3 references per element for Z <= 86
 constexpr int kTerms = 15;     // EnergyTerms::named_values (src/electronic.rs:681-699)
-// Gradient kernel: threads per CTA (one CTA per molecule) and the CTAs per SM
-// its register budget is sized for.
+// Gradient kernel: threads per CTA and the CTAs per SM its register budget is
+// sized for; the s/p instantiation needs fewer registers.
 constexpr int kGradThreads = 128;
 constexpr int kGradMinBlocks = 4;
-// The s/p instantiation of the gradient kernel runs five CTAs per SM (96
-// registers; measured on the 4096-molecule batch: 3 CTAs 7.70 ms, 4: 7.00 ms,
-// 5: 6.63 ms, the spills staying in L1)
-constexpr int kGradMinBlocksSp = 5;
+constexpr int kGradMinBlocksSp = 4;
 
 // Per-element data, indexed by Z.  nsh == 0 marks an element the device path
 // does not support (f shells, more than three shells).  Values are already converted to the model
@@ -112,7 +109,8 @@ struct Batch {
   double* gam;              // Coulomb matrices (offset gam_off[m])
   double* pairbuf;          // gradient pair scratch (8 per atom pair)
   // per-atom / per-shell state
-  double *cn, *cn_disp_dedcn; // [natoms]
+  double* cn;               // [natoms]
+  double* atom_tmp;         // [natoms*4] setup and gradient of molecules whose phases are launches of their own
   double *shell_q, *shell_pot, *atom_q; // [nshells], [nshells], [natoms]
   double* shell_pot_in;     // [nshells] potential of the last diagonalised Fock matrix, or null
   double* se;               // [nshells] self energies

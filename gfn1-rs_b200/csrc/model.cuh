@@ -52,4 +52,45 @@ __device__ __forceinline__ void exp_count(double r, double rc, double& value, do
 // Klopman-Ohno effective kernel with exponent 2 (src/coulomb.rs:239-248)
 __device__ __forceinline__ double harmonic_avg(double a, double b) { return 2.0 / (1.0 / a + 1.0 / b); }
 
+// Exclusive prefix sums of the shell and AO counts of a molecule's atoms: the
+// first shell and AO of each atom, [nat] the totals.  All threads of the CTA.
+__device__ __forceinline__ void atom_offsets(const Model& M, const int* zs, int nat, int* atom_sh, int* atom_ao) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int s0 = 0, o0 = 0;
+    for (int a0 = 0; a0 < nat; a0 += 32) {
+      const int a = a0 + lane;
+      int s = a < nat ? M.elem[zs[a]].nsh : 0, o = a < nat ? M.elem[zs[a]].nao : 0;
+      const int ns = s, no = o;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int ts = __shfl_up_sync(0xffffffffu, s, d), to = __shfl_up_sync(0xffffffffu, o, d);
+        if (lane >= d) {
+          s += ts;
+          o += to;
+        }
+      }
+      if (a < nat) {
+        atom_sh[a] = s0 + s - ns;
+        atom_ao[a] = o0 + o - no;
+      }
+      s0 += __shfl_sync(0xffffffffu, s, 31);
+      o0 += __shfl_sync(0xffffffffu, o, 31);
+    }
+    if (lane == 0) {
+      atom_sh[nat] = s0;
+      atom_ao[nat] = o0;
+    }
+  }
+  __syncthreads();
+}
+
+// t-th unordered pair (i >= j) of a triangle with its diagonal.
+__device__ __forceinline__ void tri_inverse(int t, int& i, int& j) {
+  i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while ((long long)i * (i + 1) / 2 > t) --i;
+  while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
+  j = t - i * (i + 1) / 2;
+}
+
 }  // namespace gfn1

@@ -14,16 +14,7 @@
 
 namespace gfn1 {
 
-constexpr double kPi = 3.14159265358979323846;
 constexpr double kPrimScreen = 1.0e-13;
-
-// Cartesian component of AO k of a shell with angular momentum l (s: (0,0,0);
-// p: x, y, z in that order, src/basis.rs:390-405).
-__device__ __forceinline__ void ao_powers(int l, int k, int& px, int& py, int& pz) {
-  px = (l == 1 && k == 0);
-  py = (l == 1 && k == 1);
-  pz = (l == 1 && k == 2);
-}
 
 // 1D moments E[i][j], i,j <= 2 (normalised so E[0][0] = 1) along one axis.
 __device__ __forceinline__ void moments1d(double pa, double pb, double inv2p, double E[3][3]) {
@@ -44,11 +35,13 @@ __device__ __forceinline__ double ipow(double x, int n) {
   return r;
 }
 
-// Overlap block S[ka][kb] between shell (la, prims a) at A and shell (lb, prims b)
-// at B; nao = 2l+1 for l <= 1.  `order_extra` is the screening order offset
-// (+2 for the integral build, +3 for the gradient, src/integrals.rs:313-316, :498-501).
-// When `want_deriv`, dA[ka][kb][3] receives dS/dA (bra centre); dB, when not
-// null, the ket-centre derivative (equal to -dA for a two-centre overlap).
+// Overlap block S[ka][kb] between a shell (LA, prims a) at A and a shell (LB,
+// prims b) at B.  `order_extra` is the screening order offset (+2 for the
+// integral build, +3 for the gradient, src/integrals.rs:313-316, :498-501).  With
+// WantDeriv, dA[ka][kb][3] receives dS/dA (bra centre; the ket-centre derivative
+// is -dA for a two-centre overlap).  G lanes share a pair: lane `lane` of them
+// takes every G-th primitive pair and the caller adds up what they hold (S and dA
+// enter everything linearly).
 //
 // Screening: the reference evaluates bound = |c_a c_b| kab (pi/p)^3/2
 // (1 + r + p^-1/2)^order with kab = exp(-x), x = ab r^2 / p, and drops the pair
@@ -58,77 +51,27 @@ __device__ __forceinline__ double ipow(double x, int n) {
 constexpr double kSkipExpArg = 64.0;
 constexpr double kSkipPrefBound = 6.235149080811617e14;  // 1e-13 * e^64
 
-template <bool WantDeriv>
-__device__ void overlap_block(int la, int na, const double* alpha_a, const double* coef_a, const double* A, int lb,
-                              int nb, const double* alpha_b, const double* coef_b, const double* B, int order_extra,
-                              double S[3][3], double dA[3][3][3], double dB[3][3][3]) {
-  const int nao_a = 2 * la + 1, nao_b = 2 * lb + 1;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      S[i][j] = 0.0;
-      if (WantDeriv)
-        for (int k = 0; k < 3; ++k) {
-          dA[i][j][k] = 0.0;
-          if (dB) dB[i][j][k] = 0.0;
-        }
-    }
-  const double d[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-  const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-  const double r = sqrt(r2);
-  const int order = la + lb + order_extra;
-  for (int ia = 0; ia < na; ++ia) {
-    const double al = alpha_a[ia];
-    for (int ib = 0; ib < nb; ++ib) {
-      const double be = alpha_b[ib];
-      const double p = al + be;
-      const double ip = 1.0 / p;
-      const double xarg = al * be * ip * r2;
-      const double gpre = (kPi * ip) * sqrt(kPi * ip);
-      const double pref = coef_a[ia] * coef_b[ib];
-      // src/integrals.rs:30-45 (component scale is 1 for s and p AOs)
-      const double pbound = fabs(pref) * gpre * ipow(1.0 + r + sqrt(ip), order);
-      if (xarg > kSkipExpArg && pbound < kSkipPrefBound) continue;
-      const double kab = exp(-xarg);
-      if (pbound * kab < kPrimScreen) continue;
-      const double c = pref * kab * gpre;
-      const double inv2p = 0.5 * ip;
-      double E[3][3][3];
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        const double P = (al * A[x] + be * B[x]) * ip;
-        moments1d(P - A[x], P - B[x], inv2p, E[x]);
-      }
-      for (int ka = 0; ka < nao_a; ++ka) {
-        int a[3];
-        ao_powers(la, ka, a[0], a[1], a[2]);
-        for (int kb = 0; kb < nao_b; ++kb) {
-          int b[3];
-          ao_powers(lb, kb, b[0], b[1], b[2]);
-          const double ex = E[0][a[0]][b[0]], ey = E[1][a[1]][b[1]], ez = E[2][a[2]][b[2]];
-          S[ka][kb] += c * ex * ey * ez;
-          if (WantDeriv) {
-            const double e1[3] = {ex, ey, ez};
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              const double o = e1[(x + 1) % 3] * e1[(x + 2) % 3];
-              const double da = 2.0 * al * E[x][a[x] + 1][b[x]] - (a[x] ? E[x][a[x] - 1][b[x]] : 0.0);
-              dA[ka][kb][x] += c * da * o;
-              if (dB) {
-                const double db = 2.0 * be * E[x][a[x]][b[x] + 1] - (b[x] ? E[x][a[x]][b[x] - 1] : 0.0);
-                dB[ka][kb][x] += c * db * o;
-              }
-            }
-          }
-        }
-      }
+// 1/p, 1/sqrt(p) and (pi/p)^3/2 from one reciprocal square root (a divide and two
+// square roots were half of a primitive pair's latency).
+constexpr double kPi32 = 5.568327996831708;  // pi^(3/2)
+
+// Primitive pairs sub, sub + G, ... of na x nb.
+template <int G>
+struct PrimPairs {
+  int ia, ib, nb;
+  __device__ __forceinline__ PrimPairs(int sub, int nb_) : ia(sub / nb_), ib(sub - ia * nb_), nb(nb_) {}
+  __device__ __forceinline__ void next() {
+    ib += G;
+    while (ib >= nb) {
+      ib -= nb;
+      ++ia;
     }
   }
-}
+};
 
-// The same block with the angular momenta known at compile time (LA, LB in
-// {0, 1}): every loop is unrolled and the block lives in registers.
-template <int LA, int LB, bool WantDeriv>
-__device__ __forceinline__ void overlap_block_t(int na, const double* alpha_a, const double* coef_a, const double* A,
+// LA, LB in {0, 1}: every loop is unrolled and the block lives in registers.
+template <int LA, int LB, bool WantDeriv, int G>
+__device__ __forceinline__ void overlap_block_t(int lane, int na, const double* alpha_a, const double* coef_a, const double* A,
                                                 int nb, const double* alpha_b, const double* coef_b, const double* B,
                                                 int order_extra, double (&S)[2 * LA + 1][2 * LB + 1],
                                                 double (&dA)[2 * LA + 1][2 * LB + 1][3]) {
@@ -146,43 +89,40 @@ __device__ __forceinline__ void overlap_block_t(int na, const double* alpha_a, c
   const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
   const double r = sqrt(r2);
   const int order = LA + LB + order_extra;
-  for (int ia = 0; ia < na; ++ia) {
-    const double al = alpha_a[ia];
-    for (int ib = 0; ib < nb; ++ib) {
-      const double be = alpha_b[ib];
-      const double p = al + be;
-      const double ip = 1.0 / p;
-      const double xarg = al * be * ip * r2;
-      const double gpre = (kPi * ip) * sqrt(kPi * ip);
-      const double pref = coef_a[ia] * coef_b[ib];
-      const double pbound = fabs(pref) * gpre * ipow(1.0 + r + sqrt(ip), order);
-      if (xarg > kSkipExpArg && pbound < kSkipPrefBound) continue;
-      const double kab = exp(-xarg);
-      if (pbound * kab < kPrimScreen) continue;
-      const double c = pref * kab * gpre;
-      const double inv2p = 0.5 * ip;
-      double E[3][3][3];
+  for (PrimPairs<G> pp(lane, nb); pp.ia < na; pp.next()) {
+    const int ia = pp.ia, ib = pp.ib;
+    const double al = alpha_a[ia], be = alpha_b[ib];
+    const double rs = rsqrt(al + be);
+    const double ip = rs * rs;
+    const double xarg = al * be * ip * r2;
+    const double gpre = kPi32 * ip * rs;
+    const double pref = coef_a[ia] * coef_b[ib];
+    const double pbound = fabs(pref) * gpre * ipow(1.0 + r + rs, order);
+    if (xarg > kSkipExpArg && pbound < kSkipPrefBound) continue;
+    const double kab = exp(-xarg);
+    if (pbound * kab < kPrimScreen) continue;
+    const double c = pref * kab * gpre;
+    const double inv2p = 0.5 * ip;
+    double E[3][3][3];
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        const double P = (al * A[x] + be * B[x]) * ip;
-        moments1d(P - A[x], P - B[x], inv2p, E[x]);
-      }
+    for (int x = 0; x < 3; ++x) {
+      moments1d(-(be * ip) * d[x], (al * ip) * d[x], inv2p, E[x]);
+    }
 #pragma unroll
-      for (int ka = 0; ka < NA; ++ka) {
-        const int a[3] = {LA == 1 && ka == 0, LA == 1 && ka == 1, LA == 1 && ka == 2};
+    for (int ka = 0; ka < NA; ++ka) {
+      const int a[3] = {LA == 1 && ka == 0, LA == 1 && ka == 1, LA == 1 && ka == 2};
 #pragma unroll
-        for (int kb = 0; kb < NB; ++kb) {
-          const int b[3] = {LB == 1 && kb == 0, LB == 1 && kb == 1, LB == 1 && kb == 2};
-          const double ex = E[0][a[0]][b[0]], ey = E[1][a[1]][b[1]], ez = E[2][a[2]][b[2]];
-          S[ka][kb] += c * ex * ey * ez;
-          if (WantDeriv) {
-            const double e1[3] = {ex, ey, ez};
+      for (int kb = 0; kb < NB; ++kb) {
+        const int b[3] = {LB == 1 && kb == 0, LB == 1 && kb == 1, LB == 1 && kb == 2};
+        const double ex = E[0][a[0]][b[0]], ey = E[1][a[1]][b[1]], ez = E[2][a[2]][b[2]];
+        S[ka][kb] += c * ex * ey * ez;
+        if (WantDeriv) {
+          const double e1[3] = {ex, ey, ez};
 #pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              const double o = e1[(x + 1) % 3] * e1[(x + 2) % 3];
-              const double da = 2.0 * al * E[x][a[x] + 1][b[x]] - (a[x] ? E[x][a[x] - 1][b[x]] : 0.0);
-              dA[ka][kb][x] += c * da * o;
-            }
+          for (int x = 0; x < 3; ++x) {
+            const double o = e1[(x + 1) % 3] * e1[(x + 2) % 3];
+            const double da = 2.0 * al * E[x][a[x] + 1][b[x]] - (a[x] ? E[x][a[x] - 1][b[x]] : 0.0);
+            dA[ka][kb][x] += c * da * o;
           }
         }
       }
@@ -237,8 +177,8 @@ __device__ __forceinline__ void moments1d_t(double pa, double pb, double inv2p, 
 // Per primitive pair the Cartesian products are formed and added to each real
 // AO pair whose own screening bound, with the component scales of its two AOs,
 // reaches 1e-13, so the same primitive pairs are kept as in the reference.
-template <int LA, int LB, bool WantDeriv>
-__device__ __forceinline__ void overlap_block_d(int na, const double* alpha_a, const double* coef_a, const double* A,
+template <int LA, int LB, bool WantDeriv, int G>
+__device__ __forceinline__ void overlap_block_d(int lane, int na, const double* alpha_a, const double* coef_a, const double* A,
                                                 int nb, const double* alpha_b, const double* coef_b, const double* B,
                                                 int order_extra, double (&S)[2 * LA + 1][2 * LB + 1],
                                                 double (&dA)[2 * LA + 1][2 * LB + 1][3]) {
@@ -258,73 +198,70 @@ __device__ __forceinline__ void overlap_block_d(int na, const double* alpha_a, c
   const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
   const double r = sqrt(r2);
   const int order = LA + LB + order_extra;
-  for (int ia = 0; ia < na; ++ia) {
-    const double al = alpha_a[ia];
-    for (int ib = 0; ib < nb; ++ib) {
-      const double be = alpha_b[ib];
-      const double p = al + be;
-      const double ip = 1.0 / p;
-      const double xarg = al * be * ip * r2;
-      const double gpre = (kPi * ip) * sqrt(kPi * ip);
-      const double pref = coef_a[ia] * coef_b[ib];
-      const double pbound = fabs(pref) * gpre * ipow(1.0 + r + sqrt(ip), order);
-      if (xarg > kSkipExpArg && pbound * kMaxScale < kSkipPrefBound) continue;
-      const double kab = exp(-xarg);
-      const double bound = pbound * kab;
-      if (bound * kMaxScale < kPrimScreen) continue;
-      const double c = pref * kab * gpre;
-      const double inv2p = 0.5 * ip;
-      double E[3][IA + 1][LB + 1];
+  for (PrimPairs<G> pp(lane, nb); pp.ia < na; pp.next()) {
+    const int ia = pp.ia, ib = pp.ib;
+    const double al = alpha_a[ia], be = alpha_b[ib];
+    const double rs = rsqrt(al + be);
+    const double ip = rs * rs;
+    const double xarg = al * be * ip * r2;
+    const double gpre = kPi32 * ip * rs;
+    const double pref = coef_a[ia] * coef_b[ib];
+    const double pbound = fabs(pref) * gpre * ipow(1.0 + r + rs, order);
+    if (xarg > kSkipExpArg && pbound * kMaxScale < kSkipPrefBound) continue;
+    const double kab = exp(-xarg);
+    const double bound = pbound * kab;
+    if (bound * kMaxScale < kPrimScreen) continue;
+    const double c = pref * kab * gpre;
+    const double inv2p = 0.5 * ip;
+    double E[3][IA + 1][LB + 1];
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        const double P = (al * A[x] + be * B[x]) * ip;
-        moments1d_t<IA, LB>(P - A[x], P - B[x], inv2p, E[x]);
-      }
-#pragma unroll
-      for (int ca = 0; ca < CA; ++ca)
-#pragma unroll
-        for (int cb = 0; cb < CB; ++cb) {
-          const int a[3] = {cart_pow(LA, ca, 0), cart_pow(LA, ca, 1), cart_pow(LA, ca, 2)};
-          const int b[3] = {cart_pow(LB, cb, 0), cart_pow(LB, cb, 1), cart_pow(LB, cb, 2)};
-          const double e1[3] = {E[0][a[0]][b[0]], E[1][a[1]][b[1]], E[2][a[2]][b[2]]};
-          const double ov = c * e1[0] * e1[1] * e1[2];
-          double dv[3] = {0.0, 0.0, 0.0};
-          if constexpr (WantDeriv) {
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              const double o = e1[(x + 1) % 3] * e1[(x + 2) % 3];
-              const double da = 2.0 * al * E[x][a[x] + 1][b[x]] - (a[x] ? a[x] * E[x][a[x] - 1][b[x]] : 0.0);
-              dv[x] = c * da * o;
-            }
-          }
-#pragma unroll
-          for (int ka = 0; ka < NA; ++ka)
-#pragma unroll
-            for (int kb = 0; kb < NB; ++kb) {
-              const double t = sph_coef(LA, ka, ca) * sph_coef(LB, kb, cb);
-              if (t == 0.0) continue;
-              if (bound * (sph_abs_sum(LA, ka) * sph_abs_sum(LB, kb)) < kPrimScreen) continue;
-              S[ka][kb] += t * ov;
-              if (WantDeriv)
-#pragma unroll
-                for (int x = 0; x < 3; ++x) dA[ka][kb][x] += t * dv[x];
-            }
-        }
+    for (int x = 0; x < 3; ++x) {
+      moments1d_t<IA, LB>(-(be * ip) * d[x], (al * ip) * d[x], inv2p, E[x]);
     }
+#pragma unroll
+    for (int ca = 0; ca < CA; ++ca)
+#pragma unroll
+      for (int cb = 0; cb < CB; ++cb) {
+        const int a[3] = {cart_pow(LA, ca, 0), cart_pow(LA, ca, 1), cart_pow(LA, ca, 2)};
+        const int b[3] = {cart_pow(LB, cb, 0), cart_pow(LB, cb, 1), cart_pow(LB, cb, 2)};
+        const double e1[3] = {E[0][a[0]][b[0]], E[1][a[1]][b[1]], E[2][a[2]][b[2]]};
+        const double ov = c * e1[0] * e1[1] * e1[2];
+        double dv[3] = {0.0, 0.0, 0.0};
+        if constexpr (WantDeriv) {
+#pragma unroll
+          for (int x = 0; x < 3; ++x) {
+            const double o = e1[(x + 1) % 3] * e1[(x + 2) % 3];
+            const double da = 2.0 * al * E[x][a[x] + 1][b[x]] - (a[x] ? a[x] * E[x][a[x] - 1][b[x]] : 0.0);
+            dv[x] = c * da * o;
+          }
+        }
+#pragma unroll
+        for (int ka = 0; ka < NA; ++ka)
+#pragma unroll
+          for (int kb = 0; kb < NB; ++kb) {
+            const double t = sph_coef(LA, ka, ca) * sph_coef(LB, kb, cb);
+            if (t == 0.0) continue;
+            if (bound * (sph_abs_sum(LA, ka) * sph_abs_sum(LB, kb)) < kPrimScreen) continue;
+            S[ka][kb] += t * ov;
+            if (WantDeriv)
+#pragma unroll
+              for (int x = 0; x < 3; ++x) dA[ka][kb][x] += t * dv[x];
+          }
+      }
   }
 }
 
 // Dispatch: s/p pairs take the register block above, pairs with a d shell the
 // Cartesian-to-real one.
-template <int LA, int LB, bool WantDeriv>
-__device__ __forceinline__ void overlap_block_any(int na, const double* alpha_a, const double* coef_a, const double* A,
+template <int LA, int LB, bool WantDeriv, int G>
+__device__ __forceinline__ void overlap_block_any(int lane, int na, const double* alpha_a, const double* coef_a, const double* A,
                                                   int nb, const double* alpha_b, const double* coef_b, const double* B,
                                                   int order_extra, double (&S)[2 * LA + 1][2 * LB + 1],
                                                   double (&dA)[2 * LA + 1][2 * LB + 1][3]) {
   if constexpr (LA < 2 && LB < 2)
-    overlap_block_t<LA, LB, WantDeriv>(na, alpha_a, coef_a, A, nb, alpha_b, coef_b, B, order_extra, S, dA);
+    overlap_block_t<LA, LB, WantDeriv, G>(lane, na, alpha_a, coef_a, A, nb, alpha_b, coef_b, B, order_extra, S, dA);
   else
-    overlap_block_d<LA, LB, WantDeriv>(na, alpha_a, coef_a, A, nb, alpha_b, coef_b, B, order_extra, S, dA);
+    overlap_block_d<LA, LB, WantDeriv, G>(lane, na, alpha_a, coef_a, A, nb, alpha_b, coef_b, B, order_extra, S, dA);
 }
 
 }  // namespace gfn1

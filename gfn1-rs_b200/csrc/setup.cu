@@ -14,45 +14,97 @@
 //    (src/dispersion.rs:1232-1360, :1629-1692, :1753-1787);
 //  * the halogen-bond correction, energy and gradient (src/halogen.rs:64-160).
 //
-// Per-atom sums run one thread per atom over all partners in a fixed order, so
-// the results are bitwise reproducible (no floating-point atomics).
+// Per-atom sums run over all partners in a fixed order, so the results are bitwise
+// reproducible (no floating-point atomics).
 #include "common.cuh"
 #include "model.cuh"
 #include "overlap.cuh"
 
+#include <algorithm>
+
 namespace gfn1 {
 
-__device__ __forceinline__ void tri_inverse(long long w, int& i, int& j) {
-  long long ii = (long long)((sqrt(8.0 * (double)w + 1.0) - 1.0) * 0.5);
-  while (ii * (ii + 1) / 2 > w) --ii;
-  while ((ii + 1) * (ii + 2) / 2 <= w) ++ii;
-  i = (int)ii;
-  j = (int)(w - ii * (ii + 1) / 2);
-}
-
 // S and H0 entries of one shell pair (both triangles); LA, LB are the shells'
-// angular momenta, so the overlap block stays in registers.
-template <int LA, int LB>
-__device__ __forceinline__ void shell_pair_sh0(const ElemTable& ea, int ka, const double* xa, const ElemTable& eb, int kb,
-                                               const double* xb, bool zero, double hij, double* S, double* H0, int N,
-                                               int mu0, int nu0) {
+// angular momenta, so the overlap block stays in registers.  G lanes share the
+// pair (its primitive pairs, then its elements).
+template <int LA, int LB, int G>
+__device__ __forceinline__ void shell_pair_sh0(int sub, const ElemTable& ea, int ka, const double* xa,
+                                               const ElemTable& eb, int kb, const double* xb, bool zero, bool store,
+                                               double hij, double* S, double* H0, int N, int mu0, int nu0) {
   double Sb[2 * LA + 1][2 * LB + 1];
   double dummy[2 * LA + 1][2 * LB + 1][3];
-  if (!zero)
-    overlap_block_any<LA, LB, false>(ea.nprim[ka], ea.alpha[ka], ea.coef[ka], xa, eb.nprim[kb], eb.alpha[kb],
-                                     eb.coef[kb], xb, 2, Sb, dummy);
+  overlap_block_any<LA, LB, false, G>(sub, zero ? 0 : ea.nprim[ka], ea.alpha[ka], ea.coef[ka], xa, eb.nprim[kb],
+                                      eb.alpha[kb], eb.coef[kb], xb, 2, Sb, dummy);
 #pragma unroll
   for (int x = 0; x < 2 * LA + 1; ++x)
 #pragma unroll
     for (int y = 0; y < 2 * LB + 1; ++y) {
-      const double sv = zero ? 0.0 : Sb[x][y];
-      const long long i1 = (long long)(mu0 + x) * N + (nu0 + y);
-      const long long i2 = (long long)(nu0 + y) * N + (mu0 + x);
-      S[i1] = sv;
-      S[i2] = sv;
-      H0[i1] = sv * hij;
-      H0[i2] = sv * hij;
+      double sv = Sb[x][y];
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
+      if (store && (x * (2 * LB + 1) + y) % G == sub) {
+        const long long i1 = (long long)(mu0 + x) * N + (nu0 + y);
+        const long long i2 = (long long)(nu0 + y) * N + (mu0 + x);
+        S[i1] = sv;
+        S[i2] = sv;
+        H0[i1] = sv * hij;
+        H0[i2] = sv * hij;
+      }
     }
+}
+
+// What the shell pairs of a molecule need, in shared memory.
+struct PairCtx {
+  const int *zs, *atom_ao, *sh_atom, *sh_k, *ord;
+  const double *xyz, *se;
+  double *S, *H0;
+  int N;
+};
+
+// S and H0 for the pairs of one class: shells [a0, a0 + na) x [b0, b0 + nb) of the
+// order by angular momentum, or the unordered pairs of one range (same).
+template <int LA, int LB, int G>
+__device__ __forceinline__ void shell_pair_class(const Model& M, const PairCtx& P, int a0, int na, int b0, int nb,
+                                                 bool same, int split, int nsplit) {
+  const int n = same ? na * (na + 1) / 2 : na * nb;
+  constexpr int per = 32 / G;  // pairs of a warp
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, sub = lane % G;
+  for (int t0 = (split * nw + wid) * per; t0 < n; t0 += nsplit * nw * per) {
+    const int t = min(t0 + lane / G, n - 1);
+    const bool store = t0 + lane / G < n;
+    int i, j;
+    if (same) {
+      tri_inverse(t, i, j);
+    } else {
+      i = t / nb;
+      j = t - i * nb;
+    }
+    const int si = P.ord[a0 + i], sj = P.ord[b0 + j];
+    const int a = P.sh_atom[si], b = P.sh_atom[sj];
+    const int za = P.zs[a], zb = P.zs[b];
+    const int ka = P.sh_k[si], kb = P.sh_k[sj];
+    const ElemTable& ea = M.elem[za];
+    const ElemTable& eb = M.elem[zb];
+    const int mu0 = P.atom_ao[a] + ea.ao_first[ka], nu0 = P.atom_ao[b] + eb.ao_first[kb];
+    const double sei = P.se[si], sej = P.se[sj];
+    double hij = 0.0;
+    bool zero = false;
+    if (a == b) {
+      hij = 0.5 * (sei + sej);
+    } else {
+      const double dx = P.xyz[3 * a] - P.xyz[3 * b], dy = P.xyz[3 * a + 1] - P.xyz[3 * b + 1],
+                   dz = P.xyz[3 * a + 2] - P.xyz[3 * b + 2];
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      if (r2 <= 1e-24 || r2 > 900.0) {
+        zero = true;
+      } else {
+        const double rr = sqrt(sqrt(r2) / (ea.rad + eb.rad));
+        const double poly = (1.0 + ea.poly[ka] * rr) * (1.0 + eb.poly[kb] * rr);
+        hij = 0.5 * (sei + sej) * hscale(M, za, ka, zb, kb) * poly;
+      }
+    }
+    shell_pair_sh0<LA, LB, G>(sub, ea, ka, &P.xyz[3 * a], eb, kb, &P.xyz[3 * b], zero, store, hij, P.S, P.H0, P.N, mu0, nu0);
+  }
 }
 
 // Halogen-bond energy of one molecule; adds its gradient to gc [nat*3].  For
@@ -122,39 +174,63 @@ __device__ double halogen_term(const Model& M, const int* zs, const double* xyz,
   return e;
 }
 
-// 128-thread CTAs, four per SM (128 registers): the s/p pairs fit, pairs with
-// a d shell (rare) keep part of their blocks in local memory.
-// Molecule blockIdx.x of `mols` (or of the batch when null).  Large molecules
-// are launched with gridDim.y > 1: every CTA of a molecule computes the
-// coordination numbers and self energies (cheap, identical), then takes every
-// gridDim.y-th block of its shell pairs for S, H0 and the Coulomb matrix; the
-// classical terms (repulsion, D3, halogen bonds) stay with blockIdx.y == 0.
-// MaxL: the highest shell angular momentum of the batch; the s/p
-// instantiation (MaxL = 1) leaves out the d-shell blocks and their registers.
-template <int MaxL>
-__global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int enable_dispersion, int max_nsh,
-                                                        const int* mols) {
+// Phases of the setup of one molecule.  One CTA does them all for a molecule of
+// a large batch; for few molecules several CTAs (gridDim.y) share one.
+enum SetupPhase : int {
+  kSetupCn = 1,       // coordination numbers
+  kSetupPairs = 2,    // self energies, S, H0, Coulomb matrix (after the coordination numbers)
+  kSetupClassic = 4,  // repulsion and D3 pair terms (after the coordination numbers)
+  kSetupSums = 8,     // D3 coordination-number chain and energies (after the pair terms)
+  kSetupHalogen = 16, // halogen bonds (after the sums)
+  kSetupAll = 31
+};
+
+// Molecule blockIdx.x of `mols` (or of the batch when null).  Each unordered
+// shell pair is one work item; a warp takes pairs of one class of angular
+// momenta, so that its lanes run the same code (pairs in shell order put ss, sp
+// and pp pairs side by side, and every warp ran all of them: 8.6 ms for the
+// 4096-molecule batch).  G lanes share a pair where the pairs of the batch do not
+// fill the GPU.  Atoms with many partners are one warp each, lanes over partners.
+// CTAs 0..pair_parts-1 of a molecule take its shell pairs, the rest (or, without
+// any, the same) its classical terms; with all phases in one launch every CTA
+// forms the coordination numbers and at most one takes the classical terms.
+// MaxL: the highest shell angular momentum of the batch; the s/p instantiation
+// (MaxL = 1) leaves out the d-shell blocks and their registers.  128-thread CTAs,
+// four per SM (128 registers).
+template <int MaxL, int G>
+__global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int enable_dispersion, int max_nat,
+                                                        int max_nsh, const int* mols, int phases, int pair_parts) {
   extern __shared__ double smem[];
   const int m = mols ? mols[blockIdx.x] : blockIdx.x;
   if (B.status[m] != kOk) return;  // rejected by the host-side validation
   const int split = blockIdx.y, nsplit = gridDim.y;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
   const int a0 = B.atom_off[m], nat = B.atom_off[m + 1] - a0;
   const int sh0 = B.shell_off[m], nsh = B.shell_off[m + 1] - sh0;
   const int N = B.ao_off[m + 1] - B.ao_off[m];
-  const int maxn = B.max_nat;
-  double* xyz = smem;                 // 3*maxn
-  double* cn = xyz + 3 * maxn;        // maxn
-  double* cnd = cn + maxn;            // maxn
-  double* dedcn = cnd + maxn;         // maxn
-  double* gw = dedcn + maxn;          // kMaxRef*maxn
-  double* dgw = gw + kMaxRef * maxn;  // kMaxRef*maxn
-  double* red = dgw + kMaxRef * maxn; // 32
-  int* zs = (int*)(red + 32);         // maxn
-  int* atom_sh = zs + maxn;           // maxn+1
-  int* atom_ao = atom_sh + maxn + 1;  // maxn+1
-  int* sh_atom = atom_ao + maxn + 1;  // max_nsh
-  int* sh_k = sh_atom + max_nsh;      // max_nsh
+  const bool all = phases == kSetupAll;
+  const bool do_pairs = (phases & kSetupPairs) && split < pair_parts;
+  const bool classical = nsplit == pair_parts || split >= pair_parts;
+  const bool do_classic = (phases & kSetupClassic) && classical, do_sums = (phases & kSetupSums) && classical;
+  // the warp's atoms: all of them in one CTA, or shared by the CTAs of the phase
+  const int part = all ? 0 : (split >= pair_parts ? split - pair_parts : split);
+  const int at0 = part * nw + wid, atn = all ? nw : (nsplit > pair_parts ? nsplit - pair_parts : nsplit) * nw;
+  double* xyz = smem;                    // 3*max_nat
+  double* cn = xyz + 3 * max_nat;        // max_nat
+  double* cnd = cn + max_nat;            // max_nat
+  double* dedcn = cnd + max_nat;         // max_nat
+  double* eat = dedcn + max_nat;         // 2*max_nat: repulsion and dispersion energy of each atom
+  double* gw = eat + 2 * max_nat;        // kMaxRef*max_nat
+  double* dgw = gw + kMaxRef * max_nat;  // kMaxRef*max_nat
+  double* se = dgw + kMaxRef * max_nat;  // max_nsh
+  int* zs = (int*)(se + max_nsh);        // max_nat
+  int* atom_sh = zs + max_nat;           // max_nat+1
+  int* atom_ao = atom_sh + max_nat + 1;  // max_nat+1
+  int* sh_atom = atom_ao + max_nat + 1;  // max_nsh
+  int* sh_k = sh_atom + max_nsh;         // max_nsh
+  int* ord = sh_k + max_nsh;             // max_nsh
+  int* key = ord + max_nsh;              // max_nsh
+  int* lcount = key + max_nsh;           // 3
 
   for (int i = tid; i < nat; i += nt) {
     zs[i] = B.z[a0 + i];
@@ -162,271 +238,300 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
     xyz[3 * i + 1] = B.xyz[3 * (a0 + i) + 1];
     xyz[3 * i + 2] = B.xyz[3 * (a0 + i) + 2];
   }
+  if (tid < 3) lcount[tid] = 0;
   __syncthreads();
-  if (tid == 0) {
-    int s = 0, o = 0;
-    for (int a = 0; a < nat; ++a) {
-      const ElemTable& e = M.elem[zs[a]];
-      atom_sh[a] = s;
-      atom_ao[a] = o;
-      for (int k = 0; k < e.nsh; ++k) {
-        sh_atom[s + k] = a;
-        sh_k[s + k] = k;
+  atom_offsets(M, zs, nat, atom_sh, atom_ao);
+  if (phases & kSetupCn) {  // coordination numbers (both cutoffs)
+    for (int i = at0; i < nat; i += atn) {
+      const double ri = M.elem[zs[i]].rcov;
+      double c30 = 0.0, c25 = 0.0;
+      for (int j = lane; j < nat; j += 32) {
+        if (j == i) continue;
+        const double dx = xyz[3 * j] - xyz[3 * i], dy = xyz[3 * j + 1] - xyz[3 * i + 1], dz = xyz[3 * j + 2] - xyz[3 * i + 2];
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 <= 1e-24 || r2 > 900.0) continue;
+        const double rc = ri + M.elem[zs[j]].rcov;
+        double v, dv;
+        exp_count(sqrt(r2), rc, v, dv);
+        c30 += v;
+        if (r2 <= 625.0) c25 += v;
       }
-      s += e.nsh;
-      o += e.nao;
-    }
-    atom_sh[nat] = s;
-    atom_ao[nat] = o;
-  }
-  // coordination numbers (both cutoffs), one thread per atom
-  for (int i = tid; i < nat; i += nt) {
-    const double ri = M.elem[zs[i]].rcov;
-    double c30 = 0.0, c25 = 0.0;
-    for (int j = 0; j < nat; ++j) {
-      if (j == i) continue;
-      const double dx = xyz[3 * j] - xyz[3 * i], dy = xyz[3 * j + 1] - xyz[3 * i + 1], dz = xyz[3 * j + 2] - xyz[3 * i + 2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 <= 1e-24 || r2 > 900.0) continue;
-      const double rc = ri + M.elem[zs[j]].rcov;
-      double v, dv;
-      exp_count(sqrt(r2), rc, v, dv);
-      c30 += v;
-      if (r2 <= 625.0) c25 += v;
-    }
-    cn[i] = c30;
-    cnd[i] = c25;
-    B.cn[a0 + i] = c30;
-  }
-  __syncthreads();
-  for (int s = tid; s < nsh; s += nt) {
-    const int a = sh_atom[s], k = sh_k[s];
-    const ElemTable& e = M.elem[zs[a]];
-    B.se[sh0 + s] = e.hdiag[k] - e.kcn[k] * cn[a];
-  }
-  __syncthreads();
-
-  // ---- S and H0, one work item per unordered shell pair
-  double* S = B.S + B.mat_off[m];
-  double* H0 = B.H0 + B.mat_off[m];
-  const long long npairs = (long long)nsh * (nsh + 1) / 2;
-  for (long long w = tid + (long long)split * nt; w < npairs; w += (long long)nt * nsplit) {
-    int si, sj;
-    tri_inverse(w, si, sj);
-    const int a = sh_atom[si], b = sh_atom[sj];
-    const int za = zs[a], zb = zs[b];
-    const int ka = sh_k[si], kb = sh_k[sj];
-    const ElemTable& ea = M.elem[za];
-    const ElemTable& eb = M.elem[zb];
-    const int la = ea.l[ka], lb = eb.l[kb];
-    const int mu0 = atom_ao[a] + ea.ao_first[ka], nu0 = atom_ao[b] + eb.ao_first[kb];
-    const double sei = B.se[sh0 + si], sej = B.se[sh0 + sj];
-    double hij = 0.0;
-    bool zero = false;
-    if (a == b) {
-      hij = 0.5 * (sei + sej);
-    } else {
-      const double dx = xyz[3 * a] - xyz[3 * b], dy = xyz[3 * a + 1] - xyz[3 * b + 1], dz = xyz[3 * a + 2] - xyz[3 * b + 2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 <= 1e-24 || r2 > 900.0) {
-        zero = true;
-      } else {
-        const double rr = sqrt(sqrt(r2) / (ea.rad + eb.rad));
-        const double poly = (1.0 + ea.poly[ka] * rr) * (1.0 + eb.poly[kb] * rr);
-        hij = 0.5 * (sei + sej) * hscale(M, za, ka, zb, kb) * poly;
-      }
-    }
-    if constexpr (MaxL < 2) {
-      switch (la * 2 + lb) {
-        case 0: shell_pair_sh0<0, 0>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-        case 1: shell_pair_sh0<0, 1>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-        case 2: shell_pair_sh0<1, 0>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-        default: shell_pair_sh0<1, 1>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      }
-    } else
-    switch (la * 3 + lb) {
-      case 0: shell_pair_sh0<0, 0>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 1: shell_pair_sh0<0, 1>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 2: shell_pair_sh0<0, 2>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 3: shell_pair_sh0<1, 0>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 4: shell_pair_sh0<1, 1>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 5: shell_pair_sh0<1, 2>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 6: shell_pair_sh0<2, 0>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      case 7: shell_pair_sh0<2, 1>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-      default: shell_pair_sh0<2, 2>(ea, ka, &xyz[3 * a], eb, kb, &xyz[3 * b], zero, hij, S, H0, N, mu0, nu0); break;
-    }
-  }
-
-  // ---- Klopman-Ohno matrix (exactly symmetric: G_ij and G_ji come from the
-  // same commutative expression, which the SCC's column reads rely on)
-  double* G = B.gam + B.gam_off[m];
-  for (long long w = tid + (long long)split * nt; w < (long long)nsh * nsh; w += (long long)nt * nsplit) {
-    const int i = (int)(w / nsh), j = (int)(w % nsh);
-    const int a = sh_atom[i], b = sh_atom[j];
-    const double g = harmonic_avg(M.elem[zs[a]].hard[sh_k[i]], M.elem[zs[b]].hard[sh_k[j]]);
-    double v;
-    if (a == b) v = g;
-    else {
-      const double dx = xyz[3 * a] - xyz[3 * b], dy = xyz[3 * a + 1] - xyz[3 * b + 1], dz = xyz[3 * a + 2] - xyz[3 * b + 2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      v = 1.0 / sqrt(r2 + 1.0 / (g * g));
-    }
-    G[w] = v;
-  }
-
-  if (split != 0) return;  // the classical terms: one CTA per molecule
-  // ---- repulsion (pairs within 25 bohr), one thread per atom
-  double erep = 0.0;
-  for (int i = tid; i < nat; i += nt) {
-    const ElemTable& ei = M.elem[zs[i]];
-    double gx = 0, gy = 0, gz = 0, e = 0;
-    for (int j = 0; j < nat; ++j) {
-      if (j == i) continue;
-      const ElemTable& ej = M.elem[zs[j]];
-      const double dx = xyz[3 * j] - xyz[3 * i], dy = xyz[3 * j + 1] - xyz[3 * i + 1], dz = xyz[3 * j + 2] - xyz[3 * i + 2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 <= 1e-24 || r2 > 625.0) continue;
-      const double r = sqrt(r2);
-      const double alpha = sqrt(ei.repa * ej.repa);
-      const double zeff = ei.repb * ej.repb;
-      const double k = (zs[i] <= 2 && zs[j] <= 2) ? M.g.kexplight : M.g.kexp;
-      const double rk = pow(r, k);
-      const double en = zeff * exp(-alpha * rk) / r;
-      const double pref = (alpha * rk * k + 1.0) * en / r2;
-      e += 0.5 * en;
-      gx += dx * pref;
-      gy += dy * pref;
-      gz += dz * pref;
-    }
-    erep += e;
-    B.grad_classic[3 * (a0 + i)] = gx;
-    B.grad_classic[3 * (a0 + i) + 1] = gy;
-    B.grad_classic[3 * (a0 + i) + 2] = gz;
-  }
-  erep = block_sum(erep, red);
-
-  // ---- D3(BJ)
-  double edisp = 0.0;
-  if (enable_dispersion) {
-    for (int i = tid; i < nat; i += nt) {  // reference weights, src/dispersion.rs:1629-1692
-      const ElemTable& e = M.elem[zs[i]];
-      const int nr = e.d3_nref;
-      double logit[kMaxRef], mx = -INFINITY;
-      for (int k = 0; k < nr; ++k) {
-        const double d = cnd[i] - e.d3_cnref[k];
-        logit[k] = -4.0 * d * d;
-        mx = fmax(mx, logit[k]);
-      }
-      double raw[kMaxRef], norm = 0.0, dnorm = 0.0;
-      for (int k = 0; k < nr; ++k) {
-        raw[k] = exp(logit[k] - mx);
-        norm += raw[k];
-        dnorm += 8.0 * (e.d3_cnref[k] - cnd[i]) * raw[k];
-      }
-      const double ninv = 1.0 / norm;
-      for (int k = 0; k < kMaxRef; ++k) {
-        double gwk = 0.0, dgk = 0.0;
-        if (k < nr) {
-          const double expd = 8.0 * (e.d3_cnref[k] - cnd[i]) * raw[k];
-          gwk = raw[k] * ninv;
-          dgk = expd * ninv - raw[k] * dnorm * ninv * ninv;
-          if (!isfinite(gwk)) gwk = 0.0;
-          if (!isfinite(dgk)) dgk = 0.0;
+      c30 = warp_sum(c30);
+      c25 = warp_sum(c25);
+      if (lane == 0) {
+        cn[i] = c30;
+        cnd[i] = c25;
+        if (!all || split == 0) {
+          B.cn[a0 + i] = c30;
+          B.atom_tmp[4 * (a0 + i)] = c25;
         }
-        gw[k * maxn + i] = gwk;
-        dgw[k * maxn + i] = dgk;
+      }
+    }
+  } else {
+    for (int i = tid; i < nat; i += nt) {
+      cn[i] = B.cn[a0 + i];
+      cnd[i] = B.atom_tmp[4 * (a0 + i)];
+    }
+  }
+  __syncthreads();
+
+  if (do_pairs) {
+    for (int i = tid; i < nat; i += nt) {  // shells, self energies, shells per angular momentum
+      const ElemTable& e = M.elem[zs[i]];
+      for (int k = 0; k < e.nsh; ++k) {
+        const int s = atom_sh[i] + k;
+        const double v = e.hdiag[k] - e.kcn[k] * cn[i];
+        sh_atom[s] = i;
+        sh_k[s] = k;
+        se[s] = v;
+        key[s] = 16 * e.l[k] + e.nprim[k];
+        if (split == 0) B.se[sh0 + s] = v;
+        atomicAdd(lcount + e.l[k], 1);
+      }
+    }
+    __syncthreads();
+    // order of the shells by angular momentum, then primitives, then index
+    for (int s = tid; s < nsh; s += nt) {
+      const int ks = key[s];
+      int rank = 0;
+      for (int q = 0; q < nsh; ++q) rank += key[q] < ks || (key[q] == ks && q < s);
+      ord[rank] = s;
+    }
+    __syncthreads();
+    const PairCtx P{zs, atom_ao, sh_atom, sh_k, ord, xyz, se, B.S + B.mat_off[m], B.H0 + B.mat_off[m], N};
+    const int n0 = lcount[0], n1 = lcount[1], n2 = lcount[2], part = split, parts = pair_parts;
+    if constexpr (MaxL >= 2) {
+      shell_pair_class<2, 2, G>(M, P, n0 + n1, n2, n0 + n1, n2, true, part, parts);
+      shell_pair_class<1, 2, G>(M, P, n0, n1, n0 + n1, n2, false, part, parts);
+      shell_pair_class<0, 2, G>(M, P, 0, n0, n0 + n1, n2, false, part, parts);
+    }
+    shell_pair_class<1, 1, G>(M, P, n0, n1, n0, n1, true, part, parts);
+    shell_pair_class<0, 1, G>(M, P, 0, n0, n0, n1, false, part, parts);
+    shell_pair_class<0, 0, G>(M, P, 0, n0, 0, n0, true, part, parts);
+
+    // ---- Klopman-Ohno matrix (exactly symmetric: G_ij and G_ji come from the
+    // same commutative expression, which the SCC's column reads rely on)
+    double* Gm = B.gam + B.gam_off[m];
+    for (long long w = tid + (long long)part * nt; w < (long long)nsh * nsh; w += (long long)nt * parts) {
+      const int i = (int)(w / nsh), j = (int)(w - (long long)i * nsh);
+      const int a = sh_atom[i], b = sh_atom[j];
+      const double g = harmonic_avg(M.elem[zs[a]].hard[sh_k[i]], M.elem[zs[b]].hard[sh_k[j]]);
+      double v;
+      if (a == b) v = g;
+      else {
+        const double dx = xyz[3 * a] - xyz[3 * b], dy = xyz[3 * a + 1] - xyz[3 * b + 1], dz = xyz[3 * a + 2] - xyz[3 * b + 2];
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        v = rsqrt(r2 + 1.0 / (g * g));
+      }
+      Gm[w] = v;
+    }
+  }
+
+  if (do_classic) {
+    if (enable_dispersion) {
+      for (int i = tid; i < nat; i += nt) {  // reference weights, src/dispersion.rs:1629-1692
+        const ElemTable& e = M.elem[zs[i]];
+        const int nr = e.d3_nref;
+        double logit[kMaxRef], mx = -INFINITY;
+        for (int k = 0; k < nr; ++k) {
+          const double d = cnd[i] - e.d3_cnref[k];
+          logit[k] = -4.0 * d * d;
+          mx = fmax(mx, logit[k]);
+        }
+        double raw[kMaxRef], norm = 0.0, dnorm = 0.0;
+        for (int k = 0; k < nr; ++k) {
+          raw[k] = exp(logit[k] - mx);
+          norm += raw[k];
+          dnorm += 8.0 * (e.d3_cnref[k] - cnd[i]) * raw[k];
+        }
+        const double ninv = 1.0 / norm;
+        for (int k = 0; k < kMaxRef; ++k) {
+          double gwk = 0.0, dgk = 0.0;
+          if (k < nr) {
+            const double expd = 8.0 * (e.d3_cnref[k] - cnd[i]) * raw[k];
+            gwk = raw[k] * ninv;
+            dgk = expd * ninv - raw[k] * dnorm * ninv * ninv;
+            if (!isfinite(gwk)) gwk = 0.0;
+            if (!isfinite(dgk)) dgk = 0.0;
+          }
+          gw[k * max_nat + i] = gwk;
+          dgw[k * max_nat + i] = dgk;
+        }
       }
     }
     __syncthreads();
     const double s6 = M.g.s6, s8 = M.g.s8, a1 = M.g.a1, a2 = M.g.a2;
-    for (int i = tid; i < nat; i += nt) {  // pair terms, src/dispersion.rs:1260-1297
+    for (int i = at0; i < nat; i += atn) {
       const int zi = zs[i];
       const ElemTable& ei = M.elem[zi];
-      double gx = 0, gy = 0, gz = 0, e = 0, dc = 0;
-      for (int j = 0; j < nat; ++j) {
+      double gx = 0, gy = 0, gz = 0, er = 0, ed = 0, dc = 0;
+      for (int j = lane; j < nat; j += 32) {
         if (j == i) continue;
         const int zj = zs[j];
         const ElemTable& ej = M.elem[zj];
-        const double dx = xyz[3 * i] - xyz[3 * j], dy = xyz[3 * i + 1] - xyz[3 * j + 1], dz = xyz[3 * i + 2] - xyz[3 * j + 2];
+        const double dx = xyz[3 * j] - xyz[3 * i], dy = xyz[3 * j + 1] - xyz[3 * i + 1], dz = xyz[3 * j + 2] - xyz[3 * i + 2];
         const double r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 <= 1e-24 || r2 > 2500.0 || r2 <= 1e-14) continue;
-        const double* c6r = M.c6ref + (long long)(zi * kNZ + zj) * (kMaxRef * kMaxRef);
-        double c6 = 0.0, dc6 = 0.0;
-        for (int ra = 0; ra < ei.d3_nref; ++ra) {
-          double rowc = 0.0;
-          for (int rb = 0; rb < ej.d3_nref; ++rb) rowc += gw[rb * maxn + j] * c6r[ra * kMaxRef + rb];
-          c6 += gw[ra * maxn + i] * rowc;
-          dc6 += dgw[ra * maxn + i] * rowc;
+        double pref = 0.0;  // gradient along r_j - r_i
+        if (r2 > 1e-24 && r2 <= 625.0) {  // repulsion (pairs within 25 bohr)
+          const double r = sqrt(r2);
+          const double alpha = sqrt(ei.repa * ej.repa);
+          const double zeff = ei.repb * ej.repb;
+          const double k = (zi <= 2 && zj <= 2) ? M.g.kexplight : M.g.kexp;
+          const double rk = k == 1.5 ? r * sqrt(r) : pow(r, k);
+          const double en = zeff * exp(-alpha * rk) / r;
+          pref = (alpha * rk * k + 1.0) * en / r2;
+          er += 0.5 * en;
         }
-        const double r4r2ij = 3.0 * ei.r4r2 * ej.r4r2;
-        const double r0 = a1 * sqrt(r4r2ij) + a2;
-        const double r02 = r0 * r0, r06 = r02 * r02 * r02, r08 = r06 * r02;
-        const double r4 = r2 * r2;
-        const double t6 = 1.0 / (r4 * r2 + r06);
-        const double t8 = 1.0 / (r4 * r4 + r08);
-        const double d6 = -6.0 * r4 * t6 * t6;
-        const double d8 = -8.0 * r4 * r2 * t8 * t8;
-        const double ed = s6 * t6 + s8 * r4r2ij * t8;
-        const double gd = s6 * d6 + s8 * r4r2ij * d8;
-        e -= 0.5 * c6 * ed;
-        gx += dx * (-c6 * gd);
-        gy += dy * (-c6 * gd);
-        gz += dz * (-c6 * gd);
-        dc -= dc6 * ed;
-      }
-      edisp += e;
-      dedcn[i] = dc;
-      B.grad_classic[3 * (a0 + i)] += gx;
-      B.grad_classic[3 * (a0 + i) + 1] += gy;
-      B.grad_classic[3 * (a0 + i) + 2] += gz;
-    }
-    __syncthreads();
-    for (int i = tid; i < nat; i += nt) {  // CN chain, src/dispersion.rs:1330-1342
-      const double ri = M.elem[zs[i]].rcov;
-      double gx = 0, gy = 0, gz = 0;
-      for (int j = 0; j < nat; ++j) {
-        if (j == i) continue;
-        const double dx = xyz[3 * i] - xyz[3 * j], dy = xyz[3 * i + 1] - xyz[3 * j + 1], dz = xyz[3 * i + 2] - xyz[3 * j + 2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 <= 1e-24 || r2 > 625.0) continue;
-        const double r = sqrt(r2);
-        double v, dv;
-        exp_count(r, ri + M.elem[zs[j]].rcov, v, dv);
-        const double pref = (dedcn[i] + dedcn[j]) * dv / r;
+        if (enable_dispersion && r2 > 1e-14 && r2 <= 2500.0) {  // D3(BJ), src/dispersion.rs:1260-1297
+          const double* c6r = M.c6ref + (long long)(zi * kNZ + zj) * (kMaxRef * kMaxRef);
+          double c6 = 0.0, dc6 = 0.0;
+          for (int ra = 0; ra < ei.d3_nref; ++ra) {
+            double rowc = 0.0;
+            for (int rb = 0; rb < ej.d3_nref; ++rb) rowc += gw[rb * max_nat + j] * c6r[ra * kMaxRef + rb];
+            c6 += gw[ra * max_nat + i] * rowc;
+            dc6 += dgw[ra * max_nat + i] * rowc;
+          }
+          const double r4r2ij = 3.0 * ei.r4r2 * ej.r4r2;
+          const double r0 = a1 * sqrt(r4r2ij) + a2;
+          const double r02 = r0 * r0, r06 = r02 * r02 * r02, r08 = r06 * r02;
+          const double r4 = r2 * r2;
+          const double t6 = 1.0 / (r4 * r2 + r06);
+          const double t8 = 1.0 / (r4 * r4 + r08);
+          const double d6 = -6.0 * r4 * t6 * t6;
+          const double d8 = -8.0 * r4 * r2 * t8 * t8;
+          const double e6 = s6 * t6 + s8 * r4r2ij * t8;
+          ed -= 0.5 * c6 * e6;
+          pref += c6 * (s6 * d6 + s8 * r4r2ij * d8);
+          dc -= dc6 * e6;
+        }
         gx += dx * pref;
         gy += dy * pref;
         gz += dz * pref;
       }
-      B.grad_classic[3 * (a0 + i)] += gx;
-      B.grad_classic[3 * (a0 + i) + 1] += gy;
-      B.grad_classic[3 * (a0 + i) + 2] += gz;
+      gx = warp_sum(gx);
+      gy = warp_sum(gy);
+      gz = warp_sum(gz);
+      er = warp_sum(er);
+      ed = warp_sum(ed);
+      dc = warp_sum(dc);
+      if (lane == 0) {
+        B.grad_classic[3 * (a0 + i)] = gx;
+        B.grad_classic[3 * (a0 + i) + 1] = gy;
+        B.grad_classic[3 * (a0 + i) + 2] = gz;
+        dedcn[i] = dc;
+        eat[2 * i] = er;
+        eat[2 * i + 1] = ed;
+        if (!all) {
+          B.atom_tmp[4 * (a0 + i) + 1] = dc;
+          B.atom_tmp[4 * (a0 + i) + 2] = er;
+          B.atom_tmp[4 * (a0 + i) + 3] = ed;
+        }
+      }
     }
-    edisp = block_sum(edisp, red);
+    __syncthreads();
   }
-  // ---- halogen bonds (src/halogen.rs:64-160, triples :716-786).  Donors
-  // (Cl, Br, I, At with a CXB entry) are rare, so one thread sums every triple
-  // in atom order and adds the gradient after the per-atom terms above.
-  __syncthreads();
-  if (tid == 0) {
-    const double ehal = halogen_term(M, zs, xyz, nat, B.grad_classic + 3LL * a0);
-    double* t = B.terms + (long long)m * kTerms;
-    for (int k = 0; k < kTerms; ++k) t[k] = 0.0;
-    t[2] = erep;
-    t[7] = edisp;
-    t[8] = ehal;
+
+  if (do_sums) {
+    if (!all) {
+      for (int i = tid; i < nat; i += nt) {
+        dedcn[i] = B.atom_tmp[4 * (a0 + i) + 1];
+        eat[2 * i] = B.atom_tmp[4 * (a0 + i) + 2];
+        eat[2 * i + 1] = B.atom_tmp[4 * (a0 + i) + 3];
+      }
+      __syncthreads();
+    }
+    if (enable_dispersion)
+      for (int i = at0; i < nat; i += atn) {  // CN chain, src/dispersion.rs:1330-1342
+        const double ri = M.elem[zs[i]].rcov;
+        double gx = 0, gy = 0, gz = 0;
+        for (int j = lane; j < nat; j += 32) {
+          if (j == i) continue;
+          const double dx = xyz[3 * i] - xyz[3 * j], dy = xyz[3 * i + 1] - xyz[3 * j + 1], dz = xyz[3 * i + 2] - xyz[3 * j + 2];
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          if (r2 <= 1e-24 || r2 > 625.0) continue;
+          const double r = sqrt(r2);
+          double v, dv;
+          exp_count(r, ri + M.elem[zs[j]].rcov, v, dv);
+          const double pref = (dedcn[i] + dedcn[j]) * dv / r;
+          gx += dx * pref;
+          gy += dy * pref;
+          gz += dz * pref;
+        }
+        gx = warp_sum(gx);
+        gy = warp_sum(gy);
+        gz = warp_sum(gz);
+        if (lane == 0) {
+          B.grad_classic[3 * (a0 + i)] += gx;
+          B.grad_classic[3 * (a0 + i) + 1] += gy;
+          B.grad_classic[3 * (a0 + i) + 2] += gz;
+        }
+      }
+    __syncthreads();
+    if (part == 0 && wid == 0) {
+      double er = 0.0, ed = 0.0;
+      for (int i = lane; i < nat; i += 32) {
+        er += eat[2 * i];
+        ed += eat[2 * i + 1];
+      }
+      er = warp_sum(er);
+      ed = warp_sum(ed);
+      if (lane == 0) {
+        double* t = B.terms + (long long)m * kTerms;
+        for (int k = 0; k < kTerms; ++k) t[k] = 0.0;
+        t[2] = er;
+        t[7] = ed;
+      }
+    }
   }
+  // ---- halogen bonds (src/halogen.rs:64-160, triples :716-786).  Donors (Cl, Br,
+  // I, At with a CXB entry) are rare, so one thread sums every triple in atom
+  // order after the per-atom terms.
+  if ((phases & kSetupHalogen) && classical && tid == 0)
+    B.terms[(long long)m * kTerms + 8] = halogen_term(M, zs, xyz, nat, B.grad_classic + 3LL * a0);
 }
 
-// Launches the setup kernel for a batch whose highest shell angular momentum
-// is max_l (the s/p instantiation below 2).
-cudaError_t launch_setup(int max_l, dim3 grid, int nt, size_t smem, cudaStream_t st, const Batch& B, const Model& M,
-                         int enable_dispersion, int max_nsh, const int* mols) {
-  auto* k = max_l >= 2 ? setup_kernel<2> : setup_kernel<1>;
+size_t setup_smem_bytes(int max_nat, int max_nsh) {
+  return sizeof(double) * (18 * (size_t)max_nat + max_nsh) + sizeof(int) * (3 * (size_t)max_nat + 2 + 4 * (size_t)max_nsh + 4);
+}
+
+// Launches the setup of `n` molecules (`mols`, or the batch when null) whose
+// largest has max_nat atoms and max_nsh shells; max_l: the batch's highest shell
+// angular momentum (the s/p instantiation below 2); halogens: some atom is a
+// halogen-bond donor.
+//  * one CTA per molecule when they fill the GPU (four CTAs on each SM);
+//  * otherwise eight lanes per shell pair and as many CTAs per molecule as fill
+//    it: one launch for up to kSetupOneLaunch atoms (whose classical terms one CTA
+//    finishes while the others form the pairs), beyond that one launch each for
+//    the coordination numbers, the pair terms and the sums.
+constexpr int kSetupOneLaunch = 16;
+int setup_launches(int n, int max_nat, bool halogens, int num_sms) {
+  return n <= 0 ? 0 : (n >= 4 * num_sms || max_nat <= kSetupOneLaunch ? 1 : (halogens ? 4 : 3));
+}
+cudaError_t launch_setup(int max_l, int n, int max_nat, int max_nsh, bool halogens, int num_sms, cudaStream_t st,
+                         const Batch& B, const Model& M, int enable_dispersion, const int* mols) {
+  const size_t smem = setup_smem_bytes(max_nat, max_nsh);
+  const bool few = n < 4 * num_sms;
+  auto* k = max_l >= 2 ? (few ? setup_kernel<2, 8> : setup_kernel<2, 1>) : (few ? setup_kernel<1, 8> : setup_kernel<1, 1>);
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k<<<grid, nt, smem, st>>>(B, M, enable_dispersion, max_nsh, mols);
+  const int fill = std::max(1, 8 * num_sms / n);
+  const int yp = std::max(1, std::min(fill, (max_nsh * (max_nsh + 1) / 2 + 31) / 32));  // 16 pairs per CTA and step
+  const int ya = std::max(1, std::min(fill, (max_nat + 3) / 4));                        // four atoms per CTA and step
+  auto launch = [&](int y, int phases, int pair_parts) {
+    k<<<dim3(n, y), 128, smem, st>>>(B, M, enable_dispersion, max_nat, max_nsh, mols, phases, pair_parts);
+  };
+  if (!few) {
+    launch(1, kSetupAll, 1);
+  } else if (max_nat <= kSetupOneLaunch) {
+    launch(yp + 1, kSetupAll, yp);
+  } else {
+    launch(ya, kSetupCn, 0);
+    launch(yp + ya, kSetupPairs | kSetupClassic, yp);
+    launch(ya, kSetupSums, 0);
+    if (halogens) launch(1, kSetupHalogen, 0);
+  }
   return cudaGetLastError();
 }
 
