@@ -44,6 +44,7 @@
 #include "model.cuh"
 #include "orbitals.cuh"
 #include "tridiag.cuh"
+#include "tridiag_cluster.cuh"
 
 namespace gfn1 {
 

@@ -554,6 +554,39 @@ __host__ __device__ inline int tridiag_active(int nr, int G, int min_rows, int n
   return want < 1 ? 1 : (want < G ? want : G);
 }
 
+// Gerschgorin interval, 1-norm bound and e^2 of a finished reduction, by one CTA
+// of kRedNT threads.
+__device__ __forceinline__ void wide_spectrum_bounds(const WideMol& w, double* red) {
+  const int tid = threadIdx.x, N = w.N;
+  double gl = INFINITY, gu = -INFINITY, onenrm = 0.0, emax2 = 0.0;
+  for (int i = tid; i < N; i += kRedNT) {
+    const double ei = i < N - 1 ? ldcg(w.e + i) : 0.0;
+    const double em = i > 0 ? ldcg(w.e + i - 1) : 0.0;
+    const double di = ldcg(w.d + i);
+    const double off = fabs(em) + fabs(ei);
+    gl = fmin(gl, di - off);
+    gu = fmax(gu, di + off);
+    onenrm = fmax(onenrm, fabs(di) + off);
+    if (i < N - 1) {
+      w.esq[i] = ei * ei;
+      emax2 = fmax(emax2, ei * ei);
+    }
+  }
+  gl = -block_max(-gl, red);
+  gu = block_max(gu, red);
+  onenrm = block_max(onenrm, red);
+  emax2 = block_max(emax2, red);
+  if (tid == 0) {
+    const double pivmin = DBL_MIN * fmax(1.0, emax2);
+    const double span = gu - gl;
+    WideState* st = w.st;
+    st->gl = gl - (2.1 * DBL_EPSILON * fabs(gl) + 4.0 * DBL_EPSILON * span + pivmin);
+    st->gu = gu + (2.1 * DBL_EPSILON * fabs(gu) + 4.0 * DBL_EPSILON * span + pivmin);
+    st->pivmin = pivmin;
+    st->onenrm = onenrm;
+  }
+}
+
 __global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, int nb, int min_rows,
                                                                long long* prof, unsigned long long epoch) {
   extern __shared__ __align__(16) double sm[];
@@ -935,7 +968,7 @@ __global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, 
     return;
   }
   if (c != 0) return;
-  // ---- last 2 x 2 block, then the bounds of the eigenvalue search
+  // ---- last 2 x 2 block
   if (tid == 0) {
     if (N >= 2) {
       w.d[N - 2] = ldcg(A + (long long)(N - 2) * ld + N - 2);
@@ -947,38 +980,20 @@ __global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, 
     w.tau[N - 1] = 0.0;
   }
   __syncthreads();
-  double gl = INFINITY, gu = -INFINITY, onenrm = 0.0, emax2 = 0.0;
-  for (int i = tid; i < N; i += kRedNT) {
-    const double ei = i < N - 1 ? ldcg(w.e + i) : 0.0;
-    const double em = i > 0 ? ldcg(w.e + i - 1) : 0.0;
-    const double di = ldcg(w.d + i);
-    const double off = fabs(em) + fabs(ei);
-    gl = fmin(gl, di - off);
-    gu = fmax(gu, di + off);
-    onenrm = fmax(onenrm, fabs(di) + off);
-    if (i < N - 1) {
-      w.esq[i] = ei * ei;
-      emax2 = fmax(emax2, ei * ei);
-    }
-  }
-  gl = -block_max(-gl, ss.red);
-  gu = block_max(gu, ss.red);
-  onenrm = block_max(onenrm, ss.red);
-  emax2 = block_max(emax2, ss.red);
-  if (tid == 0) {
-    const double pivmin = DBL_MIN * fmax(1.0, emax2);
-    const double span = gu - gl;
-    WideState* st = w.st;
-    st->gl = gl - (2.1 * DBL_EPSILON * fabs(gl) + 4.0 * DBL_EPSILON * span + pivmin);
-    st->gu = gu + (2.1 * DBL_EPSILON * fabs(gu) + 4.0 * DBL_EPSILON * span + pivmin);
-    st->pivmin = pivmin;
-    st->onenrm = onenrm;
-  }
+  wide_spectrum_bounds(w, ss.red);
 }
 
-}  // namespace gfn1
-
-namespace gfn1 {
+// The reduction of molecules whose matrix a cluster of C CTAs holds on chip, one
+// cluster per molecule (tridiag_cluster.cuh).
+template <int C>
+__global__ void __launch_bounds__(ClusterShape<C>::NT, 1) wide_tridiag_cluster_kernel(WideCtx X) {
+  static_assert(ClusterShape<C>::NT == kRedNT, "wide_spectrum_bounds");
+  extern __shared__ __align__(16) double sm[];
+  const WideMol& w = X.mols[X.act[blockIdx.x / C]];
+  if (w.st->status != kOk) return;
+  cluster_tridiag<C>(ClusterOut{w.A, w.d, w.e, w.tau, w.N, w.ld}, sm);
+  if (blockIdx.x % C == 0) wide_spectrum_bounds(w, sm);
+}
 
 // ------------------------------------------------------------------ set-up and rung start
 // L = lower triangle of S (zeros above), L^-1 = 0, SCC state from the host-validated status.
@@ -1634,6 +1649,7 @@ __global__ void __launch_bounds__(kWideNT, 1) wide_results_kernel(Batch B, Model
 }  // namespace gfn1
 
 // ================================================================== host side
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -1738,8 +1754,42 @@ static cudaError_t wide_configure(int dev) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e != cudaSuccess) return e;
   }
+  cudaError_t e = cudaFuncSetAttribute((const void*)wide_tridiag_cluster_kernel<8>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ClusterShape<8>::kBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)wide_tridiag_cluster_kernel<16>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ClusterShape<16>::kBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)wide_tridiag_cluster_kernel<16>,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
   configured = dev;
   return cudaSuccess;
+}
+
+// Which reduction a molecule of N AOs takes: 0 and 1 the clusters of 8 and 16 CTAs
+// that hold its matrix on chip, 2 the blocked one.  Where a cluster fits it wins at
+// every size and count (a reduction at 320 AOs 0.47 against 3.6 ms, eight at 768 AOs
+// 3.9 against 10.1 ms).
+static int reduction_class(int N) {
+  return N <= ClusterShape<8>::P ? 0 : N <= ClusterShape<16>::P ? 1 : 2;
+}
+
+template <int C>
+static cudaError_t launch_tridiag_cluster(const WideCtx& X, int na, cudaStream_t st, int* max_clusters = nullptr) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(C * na);
+  cfg.blockDim = dim3(ClusterShape<C>::NT);
+  cfg.dynamicSmemBytes = ClusterShape<C>::kBytes;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (max_clusters) return cudaOccupancyMaxActiveClusters(max_clusters, wide_tridiag_cluster_kernel<C>, &cfg);
+  return cudaLaunchKernelEx(&cfg, wide_tridiag_cluster_kernel<C>, X);
 }
 
 static std::atomic<unsigned long long> g_tridiag_epoch{0};  // launches of the reduction (barrier flag generations)
@@ -1752,7 +1802,7 @@ static cudaError_t launch_tridiag(const WideCtx& X, int na, int G, int nb, int m
   return cudaLaunchCooperativeKernel((const void*)wide_tridiag_kernel, dim3(na * G), dim3(kRedNT), args, smem, st);
 }
 
-// The reduction of the na molecules of X.act: G CTAs per molecule, at least
+// The blocked reduction of the na molecules of X.act: G CTAs per molecule, at least
 // the group that fits the row cache, at most `gcap`; as many molecules per
 // cooperative launch as the resident CTAs allow.  Returns the group size of
 // the first launch in *group.
@@ -1773,6 +1823,25 @@ static cudaError_t tridiag_all(const WideCtx& X, int na, int maxn, int nb, int m
   return cudaSuccess;
 }
 
+// The reduction of molecules listed by class (ncls[] of each, in order).
+static cudaError_t reduce_all(const WideCtx& X, const int (&ncls)[3], int maxn, int nb, int min_rows, int capacity,
+                              int gcap, size_t smem, cudaStream_t st, int* group, long long* prof = nullptr) {
+  WideCtx x = X;
+  cudaError_t e = cudaSuccess;
+  if (ncls[0]) {
+    if (group) *group = 8;
+    if ((e = launch_tridiag_cluster<8>(x, ncls[0], st)) != cudaSuccess) return e;
+    x.act += ncls[0];
+  }
+  if (ncls[1]) {
+    if (group) *group = 16;
+    if ((e = launch_tridiag_cluster<16>(x, ncls[1], st)) != cudaSuccess) return e;
+    x.act += ncls[1];
+  }
+  if (ncls[2]) e = tridiag_all(x, ncls[2], maxn, nb, min_rows, capacity, gcap, smem, st, group, prof);
+  return e;
+}
+
 __global__ void wide_copy_hp_kernel(WideCtx X) {  // A = H0' (a realistic matrix for the autotuner)
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)w.N * w.ld;
@@ -1781,8 +1850,10 @@ __global__ void wide_copy_hp_kernel(WideCtx X) {  // A = H0' (a realistic matrix
 }
 
 // Times the reduction of the current H0' matrices for every candidate
-// (panel width x minimum rows per CTA) and keeps the fastest.
-static cudaError_t wide_autotune(const WideCtx& X, int na, int capacity, int gcap, size_t smem, int maxn,
+// (panel width x minimum rows per CTA) and keeps the fastest.  Without a molecule
+// that takes the blocked reduction there is nothing to choose: the default plan,
+// with the time of one reduction.
+static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[3], int capacity, int gcap, size_t smem, int maxn,
                                  cudaStream_t st, WidePlan& plan) {
   const int nbs[] = {8, 16, 32};
   const int mrs[] = {4, 8, 16, 32, 64, 128};
@@ -1796,10 +1867,10 @@ static cudaError_t wide_autotune(const WideCtx& X, int na, int capacity, int gca
   for (int warm = 1; warm >= 0 && e == cudaSuccess; --warm)
     for (int nb : nbs)
       for (int mr : mrs) {
-        if (warm && (nb != 16 || mr != 16)) continue;
+        if ((warm || !ncls[2]) && (nb != 16 || mr != 16)) continue;
         wide_copy_hp_kernel<<<cg, 256, 0, st>>>(X);
         if ((e = cudaEventRecord(e0, st)) != cudaSuccess) break;
-        if ((e = tridiag_all(X, na, maxn, nb, mr, capacity, gcap, smem, st, nullptr)) != cudaSuccess) break;
+        if ((e = reduce_all(X, ncls, maxn, nb, mr, capacity, gcap, smem, st, nullptr)) != cudaSuccess) break;
         if ((e = cudaEventRecord(e1, st)) != cudaSuccess) break;
         if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
         float ms = 0.f;
@@ -1900,9 +1971,31 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   };
   const int nblk = (maxn + 63) / 64;
   const long long mt = (long long)nblk * (nblk + 1) / 2;
+  // ---- the reduction of each slot: a cluster where its matrix fits on chip, unless a
+  // blocked plan is asked for or the device cannot place such a cluster
+  const char* env_nb = std::getenv("GFN1_WIDE_PANEL");
+  const bool fixed_plan = env_nb && *env_nb;
+  int nclusters[2] = {0, 0};
+  if (!fixed_plan) {
+    if ((e = launch_tridiag_cluster<8>(X, 1, st, &nclusters[0])) != cudaSuccess) return e;
+    if ((e = launch_tridiag_cluster<16>(X, 1, st, &nclusters[1])) != cudaSuccess) return e;
+  }
+  auto red_class = [&](int q) {
+    int c = reduction_class(R.mols[q].N);
+    while (c < 2 && nclusters[c] < 1) ++c;
+    return c;
+  };
+  // lists h_act by class of reduction
+  int ncls[3];
+  auto by_class = [&](int na) {
+    std::stable_sort(R.h_act, R.h_act + na, [&](int a, int b) { return red_class(a) < red_class(b); });
+    ncls[0] = ncls[1] = ncls[2] = 0;
+    for (int a = 0; a < na; ++a) ++ncls[red_class(R.h_act[a])];
+  };
   // ---- all slots: orthogonaliser and H0'
   int na = nslots;
   for (int q = 0; q < na; ++q) R.h_act[q] = q;
+  by_class(na);
   if ((e = upload_act(na)) != cudaSuccess) return e;
   wide_begin_kernel<<<dim3(gx(((long long)maxn * maxn + 255) / 256, na), na), 256, 0, st>>>(B, X);
   for (int k = 0; k < nblk; ++k) {
@@ -1926,8 +2019,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     const long long key = ((long long)dev << 40) | ((long long)((maxn + 127) / 128) << 16) | nab;
     std::lock_guard<std::mutex> lk(g_wide_tune_mu);
     auto it = g_wide_plans.find(key);
-    const char* env_nb = std::getenv("GFN1_WIDE_PANEL");
-    if (env_nb && *env_nb) {  // fixed plan (sweeps)
+    if (fixed_plan) {  // (sweeps)
       R.plan.nb = std::max(1, std::min(kMaxPanel, std::atoi(env_nb)));
       const char* env_mr = std::getenv("GFN1_WIDE_MIN_ROWS");
       R.plan.min_rows = env_mr && *env_mr ? std::max(1, std::atoi(env_mr)) : 16;
@@ -1935,7 +2027,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     } else if (it != g_wide_plans.end()) {
       R.plan = it->second;
     } else {
-      if ((e = wide_autotune(X, na, capacity, gcap, trsm, maxn, st, R.plan)) != cudaSuccess) return e;
+      if ((e = wide_autotune(X, na, ncls, capacity, gcap, trsm, maxn, st, R.plan)) != cudaSuccess) return e;
       g_wide_plans[key] = R.plan;
     }
   }
@@ -1950,6 +2042,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     for (int q = 0; q < nslots; ++q)
       if (!done[q]) R.h_act[na++] = q;
     if (na == 0) break;
+    by_class(na);
     SccOptions ro = opt;
     double lshift = opt.level_shift;
     if (rung == 1 || rung == 2) {
@@ -1971,8 +2064,8 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       wide_fock_kernel<<<dim3(gx(mt, na), na), kGemmNT, tsm, st>>>(X);
       if (lshift != 0.0) wide_shift_kernel<<<dim3(gx(mt, na), na), kGemmNT, tsm, st>>>(X, lshift);
       tm.mark("fock");
-      if ((e = tridiag_all(X, na, maxn, R.plan.nb, R.plan.min_rows, capacity, gcap, trsm, st, &R.group,
-                           tm.on ? (long long*)(R.d_stats + 32) : nullptr)) != cudaSuccess)
+      if ((e = reduce_all(X, ncls, maxn, R.plan.nb, R.plan.min_rows, capacity, gcap, trsm, st, &R.group,
+                          tm.on ? (long long*)(R.d_stats + 32) : nullptr)) != cudaSuccess)
         return e;
       tm.mark("tridiag");
       wide_eigval_kernel<<<dim3((maxn + kEigNT) / kEigNT, na), kEigNT, sizeof(double) * 2 * maxn, st>>>(X);
@@ -2006,6 +2099,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       }
       if (nn != na) {
         na = nn;
+        by_class(na);
         if (na > 0 && (e = upload_act(na)) != cudaSuccess) return e;
       }
     }

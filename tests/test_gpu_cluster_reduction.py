@@ -1,0 +1,51 @@
+"""Reductions of large molecules that a thread-block cluster holds on chip, at the
+sizes where the class changes (8 CTAs up to 384 AOs, 16 up to 768, the blocked
+reduction above) and where slot rows and columns fill up.
+
+Tolerance: both reductions are backward stable, so the eigenvalues of F' agree to
+about N eps |F'| (1e-12 Eh at 769 AOs) and a converged SCC of the same iterations
+amplifies that by at most about 1e4 (the charge response over the smallest orbital
+gaps): 1e-7 Eh, 1e-7 Eh/bohr and 1e-7 e hold with a margin; against the oracle, which
+converges to 1e-10 Eh and 1e-8 e, the same."""
+import os
+
+import numpy as np
+import pytest
+
+from test_gpu_scc_sizes import TIGHT, molecule
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (193, 255, 257, 320, 383, 384, 385, 513, 767, 768, 769)
+
+
+def _calculate(mols, panel):
+    from gfn1_rs import BatchCalculator
+    old = os.environ.pop("GFN1_WIDE_PANEL", None)
+    if panel:
+        os.environ["GFN1_WIDE_PANEL"] = panel
+    try:
+        off = np.concatenate([[0], np.cumsum([len(z) for z, _ in mols])]).astype(np.int32)
+        return off, BatchCalculator(**TIGHT).calculate_flat(off, np.concatenate([z for z, _ in mols]),
+                                                            np.concatenate([x for _, x in mols]))
+    finally:
+        os.environ.pop("GFN1_WIDE_PANEL", None)
+        if old is not None:
+            os.environ["GFN1_WIDE_PANEL"] = old
+
+
+@pytest.mark.parametrize("sizes", [SIZES, (384,) * 17, (768, 320, 769)])
+def test_cluster_and_blocked_reductions_agree(oracle_mod, sizes):
+    mols = [molecule(n) for n in sizes]
+    off, r = _calculate(mols, None)
+    _, b = _calculate(mols, "16")
+    assert (r.status == 0).all() and (b.status == 0).all()
+    assert np.array_equal(r.iterations, b.iterations)
+    assert np.abs(r.energy - b.energy).max() <= 1e-7
+    assert np.abs(r.gradient - b.gradient).max() <= 1e-7
+    assert np.abs(r.shell_charges - b.shell_charges).max() <= 1e-7
+    for m, n in enumerate(sizes):
+        if sizes is SIZES and n in (193, 385):
+            o = oracle_mod.run(*mols[m], options=oracle_mod.make_options(**TIGHT))
+            assert r.iterations[m] == o.iterations and abs(r.energy[m] - o.energy) <= 1e-7
+            assert np.abs(r.gradient[off[m]:off[m + 1]] - o.gradient).max() <= 1e-7
