@@ -45,6 +45,7 @@
 #include "orbitals.cuh"
 #include "tridiag.cuh"
 #include "tridiag_cluster.cuh"
+#include "tridiag_grid.cuh"
 
 namespace gfn1 {
 

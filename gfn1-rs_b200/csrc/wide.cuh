@@ -587,7 +587,14 @@ __device__ __forceinline__ void wide_spectrum_bounds(const WideMol& w, double* r
   }
 }
 
-__global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, int nb, int min_rows,
+// Columns the blocked reduction does (whole panels) before the rest of N AOs fits a
+// grid that holds `cap` rows on chip.
+__host__ __device__ inline int blocked_columns(int N, int cap, int nb) {
+  return N <= cap ? 0 : ((N - cap + nb - 1) / nb) * nb;
+}
+
+// cap > 0: only the columns before the trailing matrix has at most cap rows.
+__global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, int nb, int min_rows, int cap,
                                                                long long* prof, unsigned long long epoch) {
   extern __shared__ __align__(16) double sm[];
   __shared__ TridiagSmall ss;
@@ -627,7 +634,8 @@ __global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, 
     }
   }
   bool ok = true;
-  for (int k0 = 0; k0 < N - 2 && ok; k0 += nb) {
+  const int kstop = cap ? blocked_columns(N, cap, nb) : N - 2;
+  for (int k0 = 0; k0 < kstop && ok; k0 += nb) {
     const int nbc = min(nb, N - 2 - k0);
     const int nr = N - k0 - 1;
     const int Ga = tridiag_active(nr, G, min_rows, nb);
@@ -967,7 +975,7 @@ __global__ void __launch_bounds__(kRedNT) wide_tridiag_kernel(WideCtx X, int G, 
     if (tid == 0) w.st->status = kErrTimeout;
     return;
   }
-  if (c != 0) return;
+  if (c != 0 || cap) return;
   // ---- last 2 x 2 block
   if (tid == 0) {
     if (N >= 2) {
@@ -993,6 +1001,40 @@ __global__ void __launch_bounds__(ClusterShape<C>::NT, 1) wide_tridiag_cluster_k
   if (w.st->status != kOk) return;
   cluster_tridiag<C>(ClusterOut{w.A, w.d, w.e, w.tau, w.N, w.ld}, sm);
   if (blockIdx.x % C == 0) wide_spectrum_bounds(w, sm);
+}
+
+// The exchange ring of the reduction on a grid, in the panel buffer.
+__device__ __forceinline__ double2* wide_ring(const WideMol& w) {
+  return reinterpret_cast<double2*>((reinterpret_cast<unsigned long long>(w.VW) + 127) & ~127ULL);
+}
+
+// The reduction of molecules that the G CTAs of each hold on chip (tridiag_grid.cuh),
+// after the blocked reduction of the first columns where there are too many.
+__global__ void __launch_bounds__(GridShape::NT, 1) wide_tridiag_grid_kernel(WideCtx X, int G, int cap, int nb) {
+  static_assert(GridShape::NT == kRedNT, "wide_spectrum_bounds");
+  static_assert(4 * GridShape::kRing <= 2 * kMaxPanel, "the ring is in the panel buffer");
+  extern __shared__ __align__(16) double sm[];
+  const WideMol& w = X.mols[X.act[blockIdx.x / G]];
+  if (w.st->status != kOk) return;
+  const int k0 = blocked_columns(w.N, cap, nb);
+  const GridOut O{w.A + (long long)k0 * w.ld + k0, w.d + k0, w.e + k0, w.tau + k0, wide_ring(w),
+                  &w.sync->err, w.N - k0, w.ld, G, (int)(blockIdx.x % G)};
+  const bool ok = grid_tridiag(O, sm, kSpinCycles);
+  if (!ok && threadIdx.x == 0) w.st->status = kErrTimeout;
+}
+
+// Marks the ring unwritten.
+__global__ void wide_ring_kernel(WideCtx X) {
+  const WideMol& w = X.mols[X.act[blockIdx.y]];
+  unsigned long long* p = reinterpret_cast<unsigned long long*>(wide_ring(w));
+  const int n = 2 * GridShape::kRing * GridShape::ring_stride(w.N);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = kUnwritten;
+}
+
+__global__ void __launch_bounds__(kRedNT) wide_bounds_kernel(WideCtx X) {
+  __shared__ double red[32];
+  const WideMol& w = X.mols[X.act[blockIdx.x]];
+  if (w.st->status == kOk) wide_spectrum_bounds(w, red);
 }
 
 // ------------------------------------------------------------------ set-up and rung start
@@ -1762,17 +1804,55 @@ static cudaError_t wide_configure(int dev) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)wide_tridiag_cluster_kernel<16>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)wide_tridiag_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)GridShape::kBytes);
   if (e != cudaSuccess) return e;
   configured = dev;
   return cudaSuccess;
 }
 
 // Which reduction a molecule of N AOs takes: 0 and 1 the clusters of 8 and 16 CTAs
-// that hold its matrix on chip, 2 the blocked one.  Where a cluster fits it wins at
+// that hold its matrix on chip, 2 the grid that does, 3 the blocked one.  Where a cluster fits it wins at
 // every size and count (a reduction at 320 AOs 0.47 against 3.6 ms, eight at 768 AOs
 // 3.9 against 10.1 ms).
 static int reduction_class(int N) {
   return N <= ClusterShape<8>::P ? 0 : N <= ClusterShape<16>::P ? 1 : 2;
+}
+
+constexpr int kReductions = 4;
+
+static cudaError_t tridiag_all(const WideCtx& X, int na, int maxn, int nb, int min_rows, int capacity, int gcap,
+                               size_t smem, cudaStream_t st, int* group, long long* prof, int cap);
+
+// Rows a grid of G CTAs holds on chip.
+static int grid_rows(int G) { return std::min(GridShape::kRows * G, GridShape::P); }
+
+// The reduction on grids of the na molecules of X.act, as many at a time as the
+// resident CTAs hold; the blocked reduction of the columns that none can hold first.
+static cudaError_t grid_all(const WideCtx& X, int na, int maxn, int nb, int min_rows, int capacity, int gcap, size_t smem,
+                            int sms, cudaStream_t st, int* group, long long* prof) {
+  const int gmin = std::min((maxn + GridShape::kRows - 1) / GridShape::kRows, sms);
+  const int per = std::max(1, sms / gmin);
+  for (int a0 = 0; a0 < na; a0 += per) {
+    const int nn = std::min(per, na - a0);
+    int G = sms / nn, cap = grid_rows(G);
+    if (group && a0 == 0) *group = G;
+    WideCtx x = X;
+    x.act = X.act + a0;
+    cudaError_t e = cudaSuccess;
+    if (maxn > cap &&
+        (e = tridiag_all(x, nn, maxn, nb, min_rows, capacity, gcap, smem, st, nullptr, a0 == 0 ? prof : nullptr, cap)) !=
+            cudaSuccess)
+      return e;
+    wide_ring_kernel<<<dim3(16, nn), 256, 0, st>>>(x);
+    void* args[] = {(void*)&x, (void*)&G, (void*)&cap, (void*)&nb};
+    if ((e = cudaLaunchCooperativeKernel((const void*)wide_tridiag_grid_kernel, dim3(nn * G), dim3(GridShape::NT), args,
+                                         GridShape::kBytes, st)) != cudaSuccess)
+      return e;
+    wide_bounds_kernel<<<nn, kRedNT, 0, st>>>(x);
+  }
+  return cudaGetLastError();
 }
 
 template <int C>
@@ -1794,11 +1874,11 @@ static cudaError_t launch_tridiag_cluster(const WideCtx& X, int na, cudaStream_t
 
 static std::atomic<unsigned long long> g_tridiag_epoch{0};  // launches of the reduction (barrier flag generations)
 
-static cudaError_t launch_tridiag(const WideCtx& X, int na, int G, int nb, int min_rows, size_t smem, cudaStream_t st,
-                                  long long* prof) {
+static cudaError_t launch_tridiag(const WideCtx& X, int na, int G, int nb, int min_rows, int cap, size_t smem,
+                                  cudaStream_t st, long long* prof) {
   WideCtx x = X;
   unsigned long long epoch = g_tridiag_epoch.fetch_add(1) + 1;
-  void* args[] = {(void*)&x, (void*)&G, (void*)&nb, (void*)&min_rows, (void*)&prof, (void*)&epoch};
+  void* args[] = {(void*)&x, (void*)&G, (void*)&nb, (void*)&min_rows, (void*)&cap, (void*)&prof, (void*)&epoch};
   return cudaLaunchCooperativeKernel((const void*)wide_tridiag_kernel, dim3(na * G), dim3(kRedNT), args, smem, st);
 }
 
@@ -1807,7 +1887,7 @@ static cudaError_t launch_tridiag(const WideCtx& X, int na, int G, int nb, int m
 // cooperative launch as the resident CTAs allow.  Returns the group size of
 // the first launch in *group.
 static cudaError_t tridiag_all(const WideCtx& X, int na, int maxn, int nb, int min_rows, int capacity, int gcap,
-                               size_t smem, cudaStream_t st, int* group, long long* prof = nullptr) {
+                               size_t smem, cudaStream_t st, int* group, long long* prof, int cap) {
   const int gmin = tridiag_min_group(maxn, nb);
   if (gmin > capacity) return cudaErrorInvalidValue;
   const int per = std::max(1, capacity / gmin);
@@ -1817,15 +1897,16 @@ static cudaError_t tridiag_all(const WideCtx& X, int na, int maxn, int nb, int m
     if (group && a0 == 0) *group = G;
     WideCtx xs = X;
     xs.act = X.act + a0;
-    cudaError_t e = launch_tridiag(xs, nn, G, nb, min_rows, smem, st, a0 == 0 ? prof : nullptr);
+    cudaError_t e = launch_tridiag(xs, nn, G, nb, min_rows, cap, smem, st, a0 == 0 ? prof : nullptr);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
 // The reduction of molecules listed by class (ncls[] of each, in order).
-static cudaError_t reduce_all(const WideCtx& X, const int (&ncls)[3], int maxn, int nb, int min_rows, int capacity,
-                              int gcap, size_t smem, cudaStream_t st, int* group, long long* prof = nullptr) {
+static cudaError_t reduce_all(const WideCtx& X, const int (&ncls)[kReductions], int maxn, int nb, int min_rows,
+                              int capacity, int gcap, int grid_sms, size_t smem, cudaStream_t st, int* group,
+                              long long* prof = nullptr) {
   WideCtx x = X;
   cudaError_t e = cudaSuccess;
   if (ncls[0]) {
@@ -1838,7 +1919,12 @@ static cudaError_t reduce_all(const WideCtx& X, const int (&ncls)[3], int maxn, 
     if ((e = launch_tridiag_cluster<16>(x, ncls[1], st)) != cudaSuccess) return e;
     x.act += ncls[1];
   }
-  if (ncls[2]) e = tridiag_all(x, ncls[2], maxn, nb, min_rows, capacity, gcap, smem, st, group, prof);
+  if (ncls[2]) {
+    if ((e = grid_all(x, ncls[2], maxn, nb, min_rows, capacity, gcap, smem, grid_sms, st, group, prof)) != cudaSuccess)
+      return e;
+    x.act += ncls[2];
+  }
+  if (ncls[3]) e = tridiag_all(x, ncls[3], maxn, nb, min_rows, capacity, gcap, smem, st, group, prof, 0);
   return e;
 }
 
@@ -1853,7 +1939,7 @@ __global__ void wide_copy_hp_kernel(WideCtx X) {  // A = H0' (a realistic matrix
 // (panel width x minimum rows per CTA) and keeps the fastest.  Without a molecule
 // that takes the blocked reduction there is nothing to choose: the default plan,
 // with the time of one reduction.
-static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[3], int capacity, int gcap, size_t smem, int maxn,
+static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[kReductions], int capacity, int gcap, int grid_sms, size_t smem, int maxn,
                                  cudaStream_t st, WidePlan& plan) {
   const int nbs[] = {8, 16, 32};
   const int mrs[] = {4, 8, 16, 32, 64, 128};
@@ -1861,16 +1947,17 @@ static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[3],
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   if (e != cudaSuccess) return e;
+  const bool blocked = ncls[3] || (ncls[2] && maxn > grid_rows(grid_sms));
   float best = 1e30f;
   WidePlan bestp;
   const dim3 cg((unsigned)std::min<long long>(((long long)maxn * maxn + 255) / 256, 1024), na);
   for (int warm = 1; warm >= 0 && e == cudaSuccess; --warm)
     for (int nb : nbs)
       for (int mr : mrs) {
-        if ((warm || !ncls[2]) && (nb != 16 || mr != 16)) continue;
+        if ((warm || !blocked) && (nb != 16 || mr != 16)) continue;
         wide_copy_hp_kernel<<<cg, 256, 0, st>>>(X);
         if ((e = cudaEventRecord(e0, st)) != cudaSuccess) break;
-        if ((e = reduce_all(X, ncls, maxn, nb, mr, capacity, gcap, smem, st, nullptr)) != cudaSuccess) break;
+        if ((e = reduce_all(X, ncls, maxn, nb, mr, capacity, gcap, grid_sms, smem, st, nullptr)) != cudaSuccess) break;
         if ((e = cudaEventRecord(e1, st)) != cudaSuccess) break;
         if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
         float ms = 0.f;
@@ -1975,21 +2062,25 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   // blocked plan is asked for or the device cannot place such a cluster
   const char* env_nb = std::getenv("GFN1_WIDE_PANEL");
   const bool fixed_plan = env_nb && *env_nb;
-  int nclusters[2] = {0, 0};
+  int nclusters[2] = {0, 0}, grid_sms = 0;  // clusters that run at once; CTAs of a grid
   if (!fixed_plan) {
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid_sms, wide_tridiag_grid_kernel, GridShape::NT,
+                                                           GridShape::kBytes)) != cudaSuccess)
+      return e;
+    grid_sms = std::min(grid_sms * num_sms, GridShape::P / GridShape::kRows);
     if ((e = launch_tridiag_cluster<8>(X, 1, st, &nclusters[0])) != cudaSuccess) return e;
     if ((e = launch_tridiag_cluster<16>(X, 1, st, &nclusters[1])) != cudaSuccess) return e;
   }
   auto red_class = [&](int q) {
     int c = reduction_class(R.mols[q].N);
     while (c < 2 && nclusters[c] < 1) ++c;
-    return c;
+    return c == 2 && grid_sms < 1 ? 3 : c;
   };
   // lists h_act by class of reduction
-  int ncls[3];
+  int ncls[kReductions];
   auto by_class = [&](int na) {
     std::stable_sort(R.h_act, R.h_act + na, [&](int a, int b) { return red_class(a) < red_class(b); });
-    ncls[0] = ncls[1] = ncls[2] = 0;
+    std::fill(ncls, ncls + kReductions, 0);
     for (int a = 0; a < na; ++a) ++ncls[red_class(R.h_act[a])];
   };
   // ---- all slots: orthogonaliser and H0'
@@ -2027,7 +2118,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     } else if (it != g_wide_plans.end()) {
       R.plan = it->second;
     } else {
-      if ((e = wide_autotune(X, na, ncls, capacity, gcap, trsm, maxn, st, R.plan)) != cudaSuccess) return e;
+      if ((e = wide_autotune(X, na, ncls, capacity, gcap, grid_sms, trsm, maxn, st, R.plan)) != cudaSuccess) return e;
       g_wide_plans[key] = R.plan;
     }
   }
@@ -2064,7 +2155,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       wide_fock_kernel<<<dim3(gx(mt, na), na), kGemmNT, tsm, st>>>(X);
       if (lshift != 0.0) wide_shift_kernel<<<dim3(gx(mt, na), na), kGemmNT, tsm, st>>>(X, lshift);
       tm.mark("fock");
-      if ((e = reduce_all(X, ncls, maxn, R.plan.nb, R.plan.min_rows, capacity, gcap, trsm, st, &R.group,
+      if ((e = reduce_all(X, ncls, maxn, R.plan.nb, R.plan.min_rows, capacity, gcap, grid_sms, trsm, st, &R.group,
                           tm.on ? (long long*)(R.d_stats + 32) : nullptr)) != cudaSuccess)
         return e;
       tm.mark("tridiag");

@@ -1,6 +1,7 @@
-"""Reductions of large molecules that a thread-block cluster holds on chip, at the
-sizes where the class changes (8 CTAs up to 384 AOs, 16 up to 768, the blocked
-reduction above) and where slot rows and columns fill up.
+"""Reductions of large molecules that a thread-block cluster or a grid holds on chip,
+at the sizes where the class changes (8 CTAs up to 384 AOs, 16 up to 768, the SMs of
+the GPU above, the blocked reduction of the first columns above 2368) and where slot
+rows and columns fill up.
 
 Tolerance: both reductions are backward stable, so the eigenvalues of F' agree to
 about N eps |F'| (1e-12 Eh at 769 AOs) and a converged SCC of the same iterations
@@ -32,6 +33,33 @@ def _calculate(mols, panel):
         os.environ.pop("GFN1_WIDE_PANEL", None)
         if old is not None:
             os.environ["GFN1_WIDE_PANEL"] = old
+
+
+def spread(nao):
+    """Water clusters of 24 and one of the rest 40 A apart, so that the gap does not
+    close with size, and helium atoms for the remainder."""
+    z, x = [], []
+    left, k = nao, 0
+    while left:
+        zz, xx = molecule(min(left, 192))
+        z.append(zz)
+        x.append(xx + np.array([75.0 * (k % 4), 75.0 * (k // 4), 1.3 * k]))
+        left -= min(left, 192)
+        k += 1
+    return np.concatenate(z), np.concatenate(x)
+
+
+@pytest.mark.parametrize("sizes", [(777,), (1183, 1001, 801), (2368,), (2369,), (2401, 300)])
+def test_grid_and_blocked_reductions_agree(sizes):
+    """One molecule on all SMs, several that share them, and more rows than they hold."""
+    mols = [spread(n) for n in sizes]
+    _, r = _calculate(mols, None)
+    _, b = _calculate(mols, "16")
+    assert (r.status == 0).all() and (b.status == 0).all()
+    assert np.array_equal(r.iterations, b.iterations)
+    assert np.abs(r.energy - b.energy).max() <= 1e-7
+    assert np.abs(r.gradient - b.gradient).max() <= 1e-7
+    assert np.abs(r.shell_charges - b.shell_charges).max() <= 1e-7
 
 
 @pytest.mark.parametrize("sizes", [SIZES, (384,) * 17, (768, 320, 769)])
