@@ -552,13 +552,17 @@ __device__ __forceinline__ double eigenvalue_k(const double* d, const double* es
 // the Gerschgorin interval whenever its start was not next to its eigenvalue,
 // and the slowest of a warp's 32 decided: about 30 evaluations at N = 128, here
 // 4 to 8.)  warm: eps holds the previous SCC iteration's eigenvalues, the first
-// points.  px, pc: N doubles of shared scratch.
-template <int NT>
+// points.  px, pc: N doubles of shared scratch.  Part: the CTA finds only NT of them
+// from number `base` on; a cold start then takes two rounds of even points, the
+// second over the interval that the first leaves to the CTA's eigenvalues.
+template <int NT, bool Part = false>
 __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, int N, int nneed, int nwarm, double gl,
-                                            double gu, double pivmin, double atol, double* eps, double* px, double* pc) {
+                                            double gu, double pivmin, double atol, double* eps, double* px, double* pc,
+                                            int base = 0) {
   const int tid = threadIdx.x;
-  const int nlist = (nneed < N) ? nneed + 1 : N;
-  const int k = (tid < nneed) ? tid : N - 1;
+  const int nall = (nneed < N) ? nneed + 1 : N;
+  const int nlist = Part ? min(nall - base, NT) : nall;
+  const int k = (base + tid < nneed) ? base + tid : N - 1;
   const double dn = (double)N;
   bool active = tid < nlist;
   double lo = gl, hi = gu, x = gl + (gu - gl) * ((tid + 0.5) / nlist);
@@ -578,7 +582,8 @@ __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, 
     if (active) {
       // the first round takes every point, later ones those next in line
       const double kk = (double)(k + 1);
-      const int j0 = it == 0 ? 0 : max(tid - 4, 0), j1 = it == 0 ? nlist : min(tid + 5, nlist);
+      const bool every = it == 0 || (Part && it == 1);
+      const int j0 = every ? 0 : max(tid - 4, 0), j1 = every ? nlist : min(tid + 5, nlist);
 #pragma unroll 4
       for (int j = j0; j < j1; ++j) {
         const double xj = px[j];
@@ -617,6 +622,13 @@ __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, 
       }
     }
     if (!__syncthreads_or(active)) break;
+    if (Part && it == 0 && nwarm == 0) {
+      if (tid == 0) px[0] = lo;
+      if (tid == nlist - 1) pc[0] = hi;
+      __syncthreads();
+      if (active) x = px[0] + (pc[0] - px[0]) * ((tid + 0.5) / nlist);
+      __syncthreads();
+    }
   }
   if (active) eps[k] = x;
   __syncthreads();

@@ -281,7 +281,7 @@ struct WideMol {
   int nblk;     // 64-row blocks
   long long mo; // offset of the batch's S, H0, P, W (leading dimension N)
   double *L, *Li, *Hp, *A, *Z, *C, *iw, *VW;
-  double *xbuf, *d, *e, *tau, *esq, *eps, *occ, *pop, *vao, *part, *Tf, *Xp, *popp, *eshift;
+  double *xbuf, *d, *e, *tau, *esq, *eps, *occ, *pop, *vao, *part, *Tf, *popp, *eshift;
   double* ws;   // CtaWs layout with maxn = 1: SCC vectors and Broyden history
   WideState* st;
   GroupSync* sync;  // [2]: column barriers, panel barriers (error flags)
@@ -1230,11 +1230,13 @@ __global__ void __launch_bounds__(kGemmNT) wide_shift_kernel(WideCtx X, double l
   }
 }
 
-// (4) eigenvalues 0..nneed-1 and N-1 (one thread each), d and e^2 staged in
-// shared memory.
-constexpr int kEigNT = 32;  // one warp per CTA: the searches spread over the SMs
+// (4) eigenvalues 0..nneed-1 and N-1, one thread each, the points and counts shared in
+// the CTA (with a search each, up to 18 evaluations of 118k cycles at 2400 AOs were
+// in line, 1.15 ms); d and e^2 in shared memory.
+constexpr int kEigNT = 64;
 __global__ void __launch_bounds__(kEigNT) wide_eigval_kernel(WideCtx X) {
   extern __shared__ __align__(16) double dsm[];
+  __shared__ double px[kEigNT], pc[kEigNT];
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const WideState* st = w.st;
   if (st->status != kOk) return;
@@ -1248,12 +1250,8 @@ __global__ void __launch_bounds__(kEigNT) wide_eigval_kernel(WideCtx X) {
     esq[i] = i < N - 1 ? w.esq[i] : 0.0;
   }
   __syncthreads();
-  const int slot = blockIdx.x * kEigNT + threadIdx.x;
-  if (slot < nlist) {  // from the previous iteration's eigenvalue once the rung has one
-    const int k = slot < nneed ? slot : N - 1;
-    w.eps[k] = eigenvalue_k(d, esq, N, k, st->gl, st->gu, st->pivmin, 4.0 * DBL_EPSILON * st->onenrm, w.eps[k],
-                            st->iter > 0);
-  }
+  eigenvalues<kEigNT, true>(d, esq, N, nneed, st->iter > 0 ? nneed : 0, st->gl, st->gu, st->pivmin,
+                            4.0 * DBL_EPSILON * st->onenrm, w.eps, px, pc, blockIdx.x * kEigNT);
 }
 
 // (5) occupations (src/electronic.rs:3815-3921, spin channels :3930-4045); when
@@ -1310,204 +1308,440 @@ __global__ void __launch_bounds__(kWideNT, 1) wide_fermi_kernel(WideCtx X) {
   }
 }
 
-// (6) inverse iteration for the occupied eigenvectors of the tridiagonal (one
-// thread per cluster of eigenvalues closer than ortol_rel |T|_1, modified
-// Gram-Schmidt inside a cluster), columns of Z with stride ld.
-__global__ void __launch_bounds__(64) wide_inviter_kernel(WideCtx X, double ortol_rel, int* stats) {
+// (6) occupied eigenvectors of the tridiagonal, columns of Z up to the factors in
+// w.esq: the twisted factorisation of scc_vectors for the eigenvalues farther than
+// kTwistGap |T|_1 from their neighbours, 32 a CTA, one warp's lanes from the top and
+// the other's from the bottom; inverse iteration for the rest.  The error of lam over
+// the gap is that of the vector: where it would exceed 1e-12, lam takes its Rayleigh
+// quotient gamma_r / |z|^2 and the factorisation runs once more.  The chain of divides
+// is the time (110 cycles a row); the pivoted factorisation and two solves that it
+// replaces took 3.7 ms at 2400 AOs.
+constexpr double kTwistGap = 1e-9;
+__global__ void __launch_bounds__(64) wide_vectors_kernel(WideCtx X, int* stats) {
+  __shared__ double gam[32], other[32], lams[32];
+  __shared__ int twist[32];
+  constexpr int U = 8;  // rows whose operands are loaded together
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const WideState* st = w.st;
   if (st->status != kOk) return;
-  const int N = w.N, ld = w.ld, nocc = st->nocc;
-  const int j = blockIdx.x * 64 + threadIdx.x;
-  if (j >= nocc) return;
-  const double* eps = w.eps;
-  const double onenrm = st->onenrm;
-  const double ortol = ortol_rel * onenrm;
-  const double tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
-  if (!(j == 0 || eps[j] - eps[j - 1] > ortol)) return;
-  int jend = j + 1;
-  while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
-  if (stats) {
-    atomicMax(stats, jend - j);
-    if (jend - j > 1) atomicAdd(stats + 1, 1);
-  }
-  double* Z = w.Z;
-  double* wsv = w.iw + j;
-  double lam_prev = -INFINITY;
-  for (int jj = j; jj < jend; ++jj) {
-    double lam = eps[jj];
-    const double pert = 10.0 * DBL_EPSILON * fmax(fabs(lam), onenrm);
-    if (jj > j && lam - lam_prev < pert) lam = lam_prev + pert;
-    lam_prev = lam;
-    double* x = Z + jj;
-    if (jend - j == 1) {
-      // isolated: the start vector's forward elimination runs with the
-      // factorisation, the two solves are not normalised in between (growth
-      // below 1e40), and the second one returns |x|^2
-      const double cur = tri_factor_rhs(w.d, w.e, N, lam, tiny, wsv, ld, x, ld, (unsigned)jj);
-      tri_back(wsv, N, ld, x, ld, cur);
-      const double nrm = tri_solve(wsv, N, ld, x, ld);
-      const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
-#pragma unroll 8
-      for (int i = 0; i < N; ++i) x[(long long)i * ld] *= inv;
-      continue;
+  const int N = w.N, nocc = st->nocc, lane = threadIdx.x & 31;
+  if (32 * (int)blockIdx.x >= nocc) return;
+  const long long ld = w.ld, n2 = ld * N;
+  const bool top = threadIdx.x < 32;
+  const int j = blockIdx.x * 32 + lane;
+  const bool col = j < nocc;
+  const double *__restrict__ d = w.d, *__restrict__ e = w.e, *eps = w.eps;
+  const double onenrm = st->onenrm, ortol = kTwistGap * onenrm, tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
+  const double below = col && j > 0 ? eps[j] - eps[j - 1] : INFINITY;
+  const double above = col && j + 1 < nocc ? eps[j + 1] - eps[j] : INFINITY;
+  const bool first = col && below > ortol;
+  const bool single = first && above > ortol;
+  double lam = col ? eps[j] : 0.0, best = INFINITY, nrm = 0.0;
+  double* __restrict__ dp = w.iw + (col ? j : 0);  // D+_i
+  double* __restrict__ lp = dp + n2;               // e_i / D+_i
+  double* __restrict__ um = dp + 2 * n2;           // e_i / D-_{i+1}
+  bool again = single;
+  for (int pass = 0;; ++pass) {
+    if (again) {
+      double D = (top ? d[0] : d[N - 1]) - lam;
+      for (int k0 = 0; k0 < N - 1; k0 += U) {  // step k: row k from the top, N - 2 - k from the bottom
+        double ev[U], dn[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int k = min(k0 + q, N - 2), i = top ? k : N - 2 - k;
+          ev[q] = e[i];
+          dn[q] = d[top ? i + 1 : i] - lam;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const int k = k0 + q;
+          if (k < N - 1) {
+            if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
+            const double l = ev[q] * (1.0 / D);
+            if (top) {
+              dp[k * ld] = D;
+              lp[k * ld] = l;
+            } else {
+              um[(N - 2 - k) * ld] = l;
+            }
+            D = dn[q] - ev[q] * l;
+          }
+        }
+      }
+      if (top) dp[(N - 1) * ld] = D;
     }
-    tri_factor(w.d, w.e, N, lam, tiny, wsv, ld);
-#pragma unroll 8
-    for (int i = 0; i < N; ++i) x[(long long)i * ld] = hash_unit(i, jj) + 1e-3;
-    const int nit = 4;
-    for (int it = 0; it < nit; ++it) {
-      tri_solve(wsv, N, ld, x, ld);
-      for (int q = j; q < jj; ++q) {
+    __syncthreads();
+    int at = 0;
+    double mine = INFINITY;  // the smallest gamma_i = D+_i - e_i u_i of the thread's half of the rows
+    if (again) {
+      const int i0 = top ? 0 : N / 2, i1 = top ? N / 2 : N;
+      for (int b = i0; b < i1; b += 2 * U) {
+        double g[2 * U];
+#pragma unroll
+        for (int q = 0; q < 2 * U; ++q) {
+          const int i = min(b + q, i1 - 1), u = min(i, N - 2);
+          g[q] = dp[i * ld] - (i < N - 1 ? e[u] * um[u * ld] : 0.0);
+        }
+#pragma unroll
+        for (int q = 0; q < 2 * U; ++q)
+          if (b + q < i1 && fabs(g[q]) < fabs(mine)) {
+            mine = g[q];
+            at = b + q;
+          }
+      }
+      if (!top) {
+        gam[lane] = mine;
+        twist[lane] = at;
+      }
+    }
+    __syncthreads();
+    if (again && top) {
+      if (fabs(gam[lane]) < fabs(mine))
+        mine = gam[lane];
+      else
+        twist[lane] = at;
+      best = mine;
+    }
+    __syncthreads();
+    if (again) {
+      const int r = twist[lane];
+      double z = 1.0;
+      double* __restrict__ x = w.Z + j;
+      nrm = 0.0;
+      if (top) {
+        nrm = 1.0;
+        x[r * ld] = 1.0;
+        for (int b = N - 2; b >= 0; b -= 2 * U) {
+          double l[2 * U];
+#pragma unroll
+          for (int q = 0; q < 2 * U; ++q) l[q] = lp[max(b - q, 0) * ld];
+#pragma unroll
+          for (int q = 0; q < 2 * U; ++q)
+            if (b - q >= 0 && b - q < r) {
+              z *= -l[q];
+              x[(b - q) * ld] = z;
+              nrm += z * z;
+            }
+        }
+      } else {
+        for (int b = 0; b < N - 1; b += 2 * U) {
+          double u[2 * U];
+#pragma unroll
+          for (int q = 0; q < 2 * U; ++q) u[q] = um[min(b + q, N - 2) * ld];
+#pragma unroll
+          for (int q = 0; q < 2 * U; ++q)
+            if (b + q < N - 1 && b + q >= r) {
+              z *= -u[q];
+              x[(b + q + 1) * ld] = z;
+              nrm += z * z;
+            }
+        }
+        other[lane] = nrm;
+      }
+    }
+    __syncthreads();
+    if (again && top) {
+      nrm += other[lane];
+      const double shift = best / nrm;  // of lam to its Rayleigh quotient
+      again = fabs(shift) > 1e-12 * fmin(below, above) && fabs(shift) < 0.5 * fmin(below, above);
+      lam += again ? shift : 0.0;
+      lams[lane] = again ? lam : INFINITY;
+    } else if (top) {
+      lams[lane] = INFINITY;
+    }
+    __syncthreads();
+    if (!top) again = lams[lane] < INFINITY;
+    if (!top && again) lam = lams[lane];
+    if (pass == 1 || !__syncthreads_or(again)) break;
+  }
+  if (top && first) {
+    double* scale = w.esq;
+    const bool good = single && fabs(best) <= 64.0 * DBL_EPSILON * onenrm * nrm && nrm < 1e200;
+    if (good) scale[j] = 1.0 / sqrt(nrm);
+    if (!good) {
+      int jend = j + 1;
+      while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
+      if (stats) {
+        atomicMax(stats, jend - j);
+        if (jend - j > 1) atomicAdd(stats + 1, 1);
+      }
+      inverse_iteration(d, e, N, (int)ld, eps, j, jend, onenrm, w.iw, w.Z);
+      for (int q = j; q < jend; ++q) scale[q] = 1.0;
+    }
+  }
+}
+
+// Modified Gram-Schmidt of the vectors whose eigenvalues are closer than ortol: those
+// of wide_vectors_kernel span the right space (they may overlap by the error of lam
+// over the gap).  The warp's lanes look for the first of a chain, then share its rows.
+__device__ __forceinline__ void orthogonalise_chains(const WideMol& w, int j0, double ortol) {
+  const int N = w.N, nocc = w.st->nocc, lane = threadIdx.x & 31;
+  const long long ld = w.ld;
+  const double* eps = w.eps;
+  const int j = j0 + lane;
+  const bool head = j + 1 < nocc && eps[j + 1] - eps[j] <= ortol && (j == 0 || eps[j] - eps[j - 1] > ortol);
+  for (unsigned todo = __ballot_sync(0xffffffffu, head); todo; todo &= todo - 1) {
+    const int a = j0 + __ffs(todo) - 1;
+    for (int q = a + 1; q < nocc && eps[q] - eps[q - 1] <= ortol; ++q) {
+      for (int p = a; p < q; ++p) {
         double dot = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < N; ++i) dot += Z[(long long)i * ld + q] * x[(long long)i * ld];
-#pragma unroll 8
-        for (int i = 0; i < N; ++i) x[(long long)i * ld] -= dot * Z[(long long)i * ld + q];
+        for (int i = lane; i < N; i += 32) dot += w.Z[i * ld + p] * w.Z[i * ld + q];
+        const double f = warp_sum(dot) * w.esq[p] * w.esq[p];
+        for (int i = lane; i < N; i += 32) w.Z[i * ld + q] -= f * w.Z[i * ld + p];
       }
       double nrm = 0.0;
-#pragma unroll 8
-      for (int i = 0; i < N; ++i) nrm += x[(long long)i * ld] * x[(long long)i * ld];
-      const double inv = 1.0 / sqrt(fmax(nrm, 1e-300));
-#pragma unroll 8
-      for (int i = 0; i < N; ++i) x[(long long)i * ld] *= inv;
+      for (int i = lane; i < N; i += 32) nrm += w.Z[i * ld + q] * w.Z[i * ld + q];
+      nrm = warp_sum(nrm);
+      if (lane == 0) w.esq[q] = 1.0 / sqrt(fmax(nrm, 1e-300));
+      __syncwarp();
     }
   }
 }
 
-// (7) back-transformation Z := Q Z, Q = H_0 ... H_{N-3}, in blocks of 64
-// reflectors applied last block first as Q_b = I - V T V^T (compact WY,
-// LAPACK dlarft forward/columnwise).  V(i, a) of block b: reflector kb + a,
-// 1 at row kb + a + 1, A[i][kb + a] below, 0 above.
-__device__ __forceinline__ double refl(const double* A, int ld, int N, int kb, int a, int i) {
+// (7) back-transformation Z := Q Z, Q = H_0 ... H_{N-3}, in blocks of kWyK
+// reflectors applied last block first as Q_b = I - V T V^T (compact WY).  V(i, a) of
+// block b: reflector kb + a, 1 at row kb + a + 1, A[i][kb + a] below, 0 above.
+constexpr int kWyK = 32;
+__device__ __forceinline__ double refl(const double* A, long long ld, int N, int kb, int a, int i) {
   const int r = kb + a + 1;
-  return (i == r && r < N) ? 1.0 : ((i > r && i < N) ? A[(long long)i * ld + kb + a] : 0.0);
+  return i < N && r < N - 1 ? (i > r ? A[i * ld + kb + a] : i == r ? 1.0 : 0.0) : 0.0;
 }
 
-// T factors of every block: V^T V on the tensor cores, then the triangular
-// recurrence T[0:j, j] = -tau_j T[0:j, 0:j] (V^T V)[0:j, j], T_jj = tau_j.
-__global__ void __launch_bounds__(kGemmNT) wide_bt_t_kernel(WideCtx X) {
-  extern __shared__ __align__(16) double tsm[];
-  double* G = tsm + kTileSmemBytes / sizeof(double);  // 64 x 65
-  double* T = G + 64 * 65;                           // 64 x 65
+// T of every block: V^T V on the tensor cores (one load per tile of both operands),
+// then T[0:j, j] = -tau_j T[0:j, 0:j] (V^T V)[0:j, j], T_jj = tau_j, a row a lane.
+// The CTAs after those of the blocks take 128 columns of Z each (orthogonalise_chains).
+__global__ void __launch_bounds__(128) wide_wy_kernel(WideCtx X, int nblk, double ortol_rel) {
+  constexpr int K = kWyK, M = K / 8;
+  __shared__ double G[4][K * (K + 1)];
   const WideMol& w = X.mols[X.act[blockIdx.y]];
+  const int N = w.N, nref = N - 2, b = blockIdx.x, kb = K * b;
   if (w.st->status != kOk) return;
-  const int N = w.N, ld = w.ld;
-  const int nref = N - 2, nblk = (nref + 63) / 64;
-  const int b = blockIdx.x;
-  if (b >= nblk) return;
-  const int kb = 64 * b, nbk = min(64, nref - kb);
+  if (b >= nblk) orthogonalise_chains(w, 128 * (b - nblk) + (threadIdx.x & ~31), ortol_rel * w.st->onenrm);
+  if (b >= nblk || kb >= nref) return;
   const double* A = w.A;
-  double acc[4][TileShape<kGemmNT>::kNJ][2];
-  tile_zero<kGemmNT>(acc);
-  auto la = [&](int a, int i) { return a < nbk ? refl(A, ld, N, kb, a, i) : 0.0; };
-  auto lb = [&](int i, int bb) { return bb < nbk ? refl(A, ld, N, kb, bb, i) : 0.0; };
-  tile_mma<kGemmNT, true, true>(la, lb, 0, 0, kb + 1, N, acc, tsm);
-  tile_for_each<kGemmNT>(acc, 0, 0, [&](int a, int bb, double v) { G[a * 65 + bb] = v; });
-  for (int idx = threadIdx.x; idx < 64 * 65; idx += kGemmNT) T[idx] = 0.0;
+  const long long ld = w.ld;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  double acc[M][M][2];
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+#pragma unroll
+    for (int q = 0; q < M; ++q) acc[m][q][0] = acc[m][q][1] = 0.0;
+  double next[M];
+  auto load = [&](int r0) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) next[m] = refl(A, ld, N, kb, 8 * m + g, r0 + t4);
+  };
+  int r0 = kb + 4 * wid;
+  load(r0);
+  for (; r0 < N; r0 += 16) {
+    double v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = next[m];
+    load(r0 + 16);
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int q = m; q < M; ++q) dmma_m8n8k4(acc[m][q][0], acc[m][q][1], v[m], v[q]);
+  }
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+#pragma unroll
+    for (int q = m; q < M; ++q)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) G[wid][(8 * m + g) * (K + 1) + 8 * q + 2 * t4 + c] = acc[m][q][c];
   __syncthreads();
-  for (int j = 0; j < nbk; ++j) {
-    const double tj = w.tau[kb + j];
-    double s = 0.0;
-    if (threadIdx.x < j)
-      for (int q = threadIdx.x; q < j; ++q) s += T[threadIdx.x * 65 + q] * G[q * 65 + j];
-    __syncthreads();
-    if (threadIdx.x < j) T[threadIdx.x * 65 + j] = -tj * s;
-    if (threadIdx.x == j) T[j * 65 + j] = tj;
-    __syncthreads();
+  for (int i = threadIdx.x; i < K * (K + 1); i += 128) {
+    const int row = i / (K + 1), cl = i - row * (K + 1);
+    if (cl < K && cl / 8 >= row / 8) G[0][i] = (G[0][i] + G[1][i]) + (G[2][i] + G[3][i]);
   }
-  double* Tf = w.Tf + (long long)b * 64 * 64;
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += kGemmNT) Tf[idx] = T[(idx >> 6) * 65 + (idx & 63)];
-}
-
-// Xp[s] = V_b^T Z for the rows of split s (tiles of 64 columns of Z).
-__global__ void __launch_bounds__(kGemmNT) wide_bt_x_kernel(WideCtx X, int b, int ksplit) {
-  extern __shared__ __align__(16) double tsm[];
-  const WideMol& w = X.mols[X.act[blockIdx.y]];
-  const WideState* st = w.st;
-  if (st->status != kOk) return;
-  const int N = w.N, ld = w.ld, nocc = st->nocc;
-  const int nref = N - 2;
-  const int kb = 64 * b;
-  if (kb >= nref || nocc <= 0) return;
-  const int nbk = min(64, nref - kb);
-  const int nct = (nocc + 63) / 64;
-  const int rows = N - kb - 1, chunk = (rows + ksplit - 1) / ksplit;
-  const double *A = w.A, *Z = w.Z;
-  for (int t = blockIdx.x; t < nct * ksplit; t += gridDim.x) {
-    const int ct = t / ksplit, s = t - ct * ksplit;
-    const int r0 = kb + 1 + s * chunk, r1 = min(N, r0 + chunk);
-    double acc[4][TileShape<kGemmNT>::kNJ][2];
-    tile_zero<kGemmNT>(acc);
-    auto la = [&](int a, int i) { return a < nbk ? refl(A, ld, N, kb, a, i) : 0.0; };
-    auto lb = [&](int i, int col) { return col < nocc ? Z[(long long)i * ld + col] : 0.0; };
-    if (r0 < r1) tile_mma<kGemmNT, true, true>(la, lb, 0, 64 * ct, r0, r1, acc, tsm);
-    tile_for_each<kGemmNT>(acc, 0, 64 * ct, [&](int a, int col, double v) {
-      if (col < nocc) w.Xp[((long long)s * 64 + a) * ld + col] = v;
-    });
-  }
-}
-
-// Y = T (sum_s Xp[s]) into Xp[0] (tiles of 64 columns).
-__global__ void __launch_bounds__(kGemmNT) wide_bt_y_kernel(WideCtx X, int b, int ksplit) {
-  extern __shared__ __align__(16) double tsm[];
-  double* Xs = tsm + kTileSmemBytes / sizeof(double);  // 64 x 65
-  const WideMol& w = X.mols[X.act[blockIdx.y]];
-  const WideState* st = w.st;
-  if (st->status != kOk) return;
-  const int N = w.N, ld = w.ld, nocc = st->nocc;
-  if (64 * b >= N - 2 || nocc <= 0) return;
-  const int nct = (nocc + 63) / 64;
-  const double* Tf = w.Tf + (long long)b * 64 * 64;
-  for (int ct = blockIdx.x; ct < nct; ct += gridDim.x) {
-    for (int idx = threadIdx.x; idx < 64 * 64; idx += kGemmNT) {
-      const int a = idx >> 6, col = 64 * ct + (idx & 63);
-      double s = 0.0;
-      if (col < nocc)
-        for (int q = 0; q < ksplit; ++q) s += w.Xp[((long long)q * 64 + a) * ld + col];
-      Xs[a * 65 + (idx & 63)] = s;
+  __syncthreads();
+  if (wid == 0) {
+    double t[K];
+#pragma unroll
+    for (int q = 0; q < K; ++q) t[q] = 0.0;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const double tq = kb + q < nref ? w.tau[kb + q] : 0.0;
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int l = 0; l < q; ++l) {  // zero left of the diagonal
+        if (l & 1)
+          s1 += t[l] * G[0][l * (K + 1) + q];
+        else
+          s0 += t[l] * G[0][l * (K + 1) + q];
+      }
+      t[q] = q == lane ? tq : q > lane ? -tq * (s0 + s1) : 0.0;
     }
-    __syncthreads();
-    double acc[4][TileShape<kGemmNT>::kNJ][2];
-    tile_zero<kGemmNT>(acc);
-    auto la = [&](int a, int q) { return Tf[a * 64 + q]; };
-    auto lb = [&](int q, int cl) { return Xs[q * 65 + cl]; };
-    tile_mma<kGemmNT, false, true>(la, lb, 0, 0, 0, 64, acc, tsm);
-    tile_for_each<kGemmNT>(acc, 0, 0, [&](int a, int cl, double v) {
-      const int col = 64 * ct + cl;
-      if (col < nocc) w.Xp[(long long)a * ld + col] = v;
-    });
-    __syncthreads();
+    double* Tf = w.Tf + (long long)b * K * K + lane * K;
+#pragma unroll
+    for (int q = 0; q < K; ++q) Tf[q] = t[q];
   }
 }
 
-// Z[kb+1:, :] -= V_b Y (tiles of 64 rows x 64 columns).
-__global__ void __launch_bounds__(kGemmNT) wide_bt_upd_kernel(WideCtx X, int b) {
-  extern __shared__ __align__(16) double tsm[];
+// A CTA transforms eight columns of Z from the first block to the last, without a
+// word to the others.  Its columns stay in shared memory (Shared) as FP64 tensor-core
+// accumulators of Z^T, a tile of eight rows always with the same warp, so that the
+// passes over them need no barrier; see occupied_orbitals for the layout.  One pass a
+// block: every tile takes the update with block b and then contributes to V^T Z of
+// block b - 1; the warps' sums are added and multiplied by T at its end.  Per column
+// of Q both reads of the reflectors come from L2, 46 MB a CTA at 2400 AOs, which
+// bounds it.  Before (three kernels a block of 64, Z through L2): 4.3 ms at 2400 AOs
+// and 1200 orbitals, 0.34 ms at 320 and 160.
+constexpr int kBtNT = 512, kBtW = 8;
+struct BackTransform {
+  static constexpr int NW = kBtNT / 32, XP = kWyK + 1;
+  static constexpr int kSmall = NW * kBtW * XP + 2 * kBtW * XP + kWyK * (kWyK + 1);
+  static size_t bytes(int N, bool shared) {
+    return sizeof(double) * (kSmall + (shared ? (size_t)64 * ((N + 7) / 8) : 0));
+  }
+};
+
+template <bool Shared>
+__global__ void __launch_bounds__(kBtNT, 1) wide_backtr_kernel(WideCtx X) {
+  using BT = BackTransform;
+  constexpr int K = kWyK, M = K / 8, NW = BT::NW, XP = BT::XP;
+  extern __shared__ __align__(16) double sm[];
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const WideState* st = w.st;
-  if (st->status != kOk) return;
-  const int N = w.N, ld = w.ld, nocc = st->nocc;
-  const int nref = N - 2, kb = 64 * b;
-  if (kb >= nref || nocc <= 0) return;
-  const int nbk = min(64, nref - kb);
-  const int r0 = kb + 1;
-  const int nrt = (N - r0 + 63) / 64, nct = (nocc + 63) / 64;
-  const double* A = w.A;
-  double* Z = w.Z;
-  const double* Y = w.Xp;
-  for (int t = blockIdx.x; t < nrt * nct; t += gridDim.x) {
-    const int rt = t / nct, ct = t - rt * nct;
-    const int i0 = r0 + 64 * rt, c0 = 64 * ct;
-    double acc[4][TileShape<kGemmNT>::kNJ][2];
-    tile_zero<kGemmNT>(acc);
-    auto la = [&](int i, int a) { return a < nbk ? refl(A, ld, N, kb, a, i) : 0.0; };
-    auto lb = [&](int a, int col) { return col < nocc ? Y[(long long)a * ld + col] : 0.0; };
-    tile_mma<kGemmNT, false, true>(la, lb, i0, c0, 0, nbk, acc, tsm);
-    tile_for_each<kGemmNT>(acc, i0, c0, [&](int i, int col, double v) {
-      if (i < N && col < nocc) Z[(long long)i * ld + col] -= v;
-    });
+  const int N = w.N, nocc = st->nocc, j0 = kBtW * blockIdx.x;
+  if (st->status != kOk || j0 >= nocc) return;
+  double* Xw = sm;                    // [NW][8][XP] V^T Z of the warps
+  double* Xs = Xw + NW * kBtW * XP;   // [8][XP] their sum
+  double* Ys = Xs + kBtW * XP;        // [8][XP] -T X
+  double* Ts = Ys + kBtW * XP;        // [K][K + 1]
+  double2* Zs = reinterpret_cast<double2*>(sm + BT::kSmall);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const double* __restrict__ A = w.A;
+  const long long ld = w.ld;
+  const int nref = N - 2, nblk = (nref + K - 1) / K, ntile = (N + 7) / 8;
+  const bool col = j0 + g < nocc;
+  double* Zg = w.Z + j0 + g;
+  auto z_get = [&](int T) {
+    if (Shared) return Zs[32 * T + lane];
+    const int i = 8 * T + 2 * t4;
+    return make_double2(col && i < N ? Zg[i * ld] : 0.0, col && i + 1 < N ? Zg[(i + 1) * ld] : 0.0);
+  };
+  auto z_out = [&](int T, const double2& z) {
+    const int i = 8 * T + 2 * t4;
+    if (col && i < N) Zg[i * ld] = z.x;
+    if (col && i + 1 < N) Zg[(i + 1) * ld] = z.y;
+  };
+  auto z_put = [&](int T, const double2& z) {
+    if (Shared)
+      Zs[32 * T + lane] = z;
+    else
+      z_out(T, z);
+  };
+  {
+    const double sc = col ? w.esq[j0 + g] : 0.0;
+    for (int T = wid; T < ntile; T += NW) {
+      const int i = 8 * T + 2 * t4;
+      z_put(T, make_double2(col && i < N ? Zg[i * ld] * sc : 0.0, col && i + 1 < N ? Zg[(i + 1) * ld] * sc : 0.0));
+    }
   }
+  for (int b = nblk; b >= 0; --b) {
+    const bool upd = b < nblk, dot = b > 0;
+    const int ku = K * b, kd = K * (b - 1);
+    double y[2 * M], xt[M][2], vu[2 * M], vd[2 * M];
+#pragma unroll
+    for (int q = 0; q < 2 * M; ++q) {
+      y[q] = upd ? Ys[g * XP + 4 * q + t4] : 0.0;
+      vu[q] = vd[q] = 0.0;
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) xt[m][0] = xt[m][1] = 0.0;
+    if (dot)
+      for (int i = tid; i < K * K; i += kBtNT) Ts[(i / K) * (K + 1) + i % K] = __ldg(w.Tf + (long long)(b - 1) * K * K + i);
+    auto load = [&](int T) {
+      if (T >= ntile) return;
+      // whole tiles below the diagonal need no masks
+      if (8 * T > (upd ? ku : kd) + K && 8 * T + 8 <= N) {
+        const double* pu = A + (8 * T + g) * ld + ku + t4;
+        const double* pd = A + (8 * T + 2 * t4) * ld + kd + g;
+        if (upd) {
+#pragma unroll
+          for (int q = 0; q < 2 * M; ++q) vu[q] = __ldg(pu + 4 * q);
+        }
+        if (dot) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            vd[2 * m] = __ldg(pd + 8 * m);
+            vd[2 * m + 1] = __ldg(pd + ld + 8 * m);
+          }
+        }
+      } else {
+        if (upd) {
+#pragma unroll
+          for (int q = 0; q < 2 * M; ++q) vu[q] = refl(A, ld, N, ku, 4 * q + t4, 8 * T + g);
+        }
+        if (dot) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            vd[2 * m] = refl(A, ld, N, kd, 8 * m + g, 8 * T + 2 * t4);
+            vd[2 * m + 1] = refl(A, ld, N, kd, 8 * m + g, 8 * T + 2 * t4 + 1);
+          }
+        }
+      }
+    };
+    const int T0 = (dot ? kd : ku) / 8;  // rows from the first reflector's 1
+    int T = T0 + ((wid - T0) & (NW - 1));
+    load(T);
+    for (; T < ntile; T += NW) {
+      double cu[2 * M], cd[2 * M];
+#pragma unroll
+      for (int q = 0; q < 2 * M; ++q) {
+        cu[q] = vu[q];
+        cd[q] = vd[q];
+      }
+      double2 z = z_get(T);
+      load(T + NW);
+      if (upd) {
+        double e0 = 0.0, e1 = 0.0;  // two chains
+#pragma unroll
+        for (int q = 0; q < 2 * M; q += 2) {
+          dmma_m8n8k4(z.x, z.y, y[q], cu[q]);
+          dmma_m8n8k4(e0, e1, y[q + 1], cu[q + 1]);
+        }
+        z.x += e0;
+        z.y += e1;
+        z_put(T, z);
+      }
+      if (dot) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) dmma_m8n8k4(xt[m][0], xt[m][1], z.x, cd[2 * m]);
+#pragma unroll
+        for (int m = 0; m < M; ++m) dmma_m8n8k4(xt[m][0], xt[m][1], z.y, cd[2 * m + 1]);
+      }
+    }
+    if (dot) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        Xw[(wid * kBtW + g) * XP + 8 * m + 2 * t4] = xt[m][0];
+        Xw[(wid * kBtW + g) * XP + 8 * m + 2 * t4 + 1] = xt[m][1];
+      }
+      __syncthreads();
+      const int c = tid / K, a = tid % K;
+      if (c < kBtW) {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < NW; q += 2) {
+          s0 += Xw[(q * kBtW + c) * XP + a];
+          s1 += Xw[((q + 1) * kBtW + c) * XP + a];
+        }
+        Xs[c * XP + a] = s0 + s1;
+      }
+      __syncthreads();
+      if (c < kBtW) {
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int q = 0; q < K; ++q) s[q & 3] += Ts[a * (K + 1) + q] * Xs[c * XP + q];
+        Ys[c * XP + a] = -((s[0] + s[1]) + (s[2] + s[3]));
+      }
+      __syncthreads();
+    }
+  }
+  if (Shared)
+    for (int T = wid; T < ntile; T += NW) z_out(T, Zs[32 * T + lane]);
 }
 
 // (8) C = L^-T Z, D = L Z and the partial AO populations
@@ -1703,11 +1937,11 @@ __global__ void __launch_bounds__(kWideNT, 1) wide_results_kernel(Batch B, Model
 namespace gfn1 {
 
 constexpr int kWideMaxG = 1024;   // CTAs per molecule (partial-sum slots)
-constexpr int kWideMaxSplit = 8;  // row splits of the back-transformation's V^T Z
+constexpr size_t kBtMaxSmem = 227 * 1024;  // columns of the back-transformation in shared memory up to this
 
 struct WideSlotLayout {
   int ld;
-  long long L, Li, Hp, A, Z, C, iw, VW, xbuf, d, e, tau, esq, eps, occ, pop, vao, part, Tf, Xp, popp, eshift, ws;
+  long long L, Li, Hp, A, Z, C, iw, VW, xbuf, d, e, tau, esq, eps, occ, pop, vao, part, Tf, popp, eshift, ws;
   long long total;
 };
 
@@ -1743,7 +1977,6 @@ inline WideSlotLayout wide_slot_layout(int N, int nsh, int nat, int cap) {
   s.vao = take(nv);
   s.part = take((long long)kWideMaxG * (2 * kMaxPanel + 2));
   s.Tf = take(nblk * 64 * 64);
-  s.Xp = take((long long)kWideMaxSplit * 64 * s.ld);
   s.popp = take(nblk * s.ld);
   s.eshift = take(nblk * nblk);
   s.ws = take(cta_ws_size(1, std::max(nsh, 1), cap, std::max(nat, 1)));
@@ -1786,9 +2019,7 @@ static cudaError_t wide_configure(int dev) {
                       (const void*)wide_inv_row_kernel,    (const void*)wide_hp1_kernel,
                       (const void*)wide_hp2_kernel,        (const void*)wide_fock_kernel,
                       (const void*)wide_shift_kernel,      (const void*)wide_tridiag_kernel,
-                      (const void*)wide_eigval_kernel,     (const void*)wide_bt_t_kernel,
-                      (const void*)wide_bt_x_kernel,       (const void*)wide_bt_y_kernel,
-                      (const void*)wide_bt_upd_kernel,     (const void*)wide_cd_kernel,
+                      (const void*)wide_eigval_kernel,     (const void*)wide_cd_kernel,
                       (const void*)wide_eshift_kernel,     (const void*)wide_pw_kernel,
                       (const void*)wide_rung_kernel,       (const void*)wide_potential_kernel,
                       (const void*)wide_energy_mix_kernel, (const void*)wide_results_kernel};
@@ -1804,6 +2035,12 @@ static cudaError_t wide_configure(int dev) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)wide_tridiag_cluster_kernel<16>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)wide_backtr_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBtMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)wide_backtr_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)BackTransform::bytes(0, false));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)wide_tridiag_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)GridShape::kBytes);
@@ -2049,6 +2286,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   const size_t tsm2 = kTileSmemBytes + 2 * sizeof(double) * 64 * 65;
   const size_t rsm = dense_table_bytes(maxnsh, maxn, maxnat);
   const size_t trsm = tridiag_smem_bytes(maxn);
+  const size_t btsm = BackTransform::bytes(maxn, true);
   if (rsm > 200 * 1024 || trsm > 200 * 1024) return cudaErrorInvalidValue;
   auto upload_act = [&](int na) {
     return cudaMemcpyAsync(R.d_act, R.h_act, sizeof(int) * na, cudaMemcpyHostToDevice, st);
@@ -2163,20 +2401,20 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       tm.mark("eigval");
       wide_fermi_kernel<<<na, kWideNT, 0, st>>>(X);
       tm.mark("fermi");
-      wide_inviter_kernel<<<dim3((maxn + 63) / 64, na), 64, 0, st>>>(X, ortol_rel, tm.on ? R.d_stats : nullptr);
+      wide_vectors_kernel<<<dim3((maxn + 31) / 32, na), 64, 0, st>>>(X, tm.on ? R.d_stats : nullptr);
       tm.mark("inviter");
-      const int nref_blk = (std::max(maxn - 2, 0) + 63) / 64;
-      wide_bt_t_kernel<<<dim3(std::max(nref_blk, 1), na), kGemmNT, tsm + 2 * sizeof(double) * 64 * 65, st>>>(X);
-      const int nct = nblk;
-      const int ksplit = std::max(1, std::min(kWideMaxSplit, num_sms / std::max(1, na * nct)));
-      for (int b = nref_blk - 1; b >= 0; --b) {
-        wide_bt_x_kernel<<<dim3(gx((long long)nct * ksplit, na), na), kGemmNT, tsm, st>>>(X, b, ksplit);
-        wide_bt_y_kernel<<<dim3(gx(nct, na), na), kGemmNT, tsm1, st>>>(X, b, ksplit);
-        wide_bt_upd_kernel<<<dim3(gx((long long)nblk * nct, na), na), kGemmNT, tsm, st>>>(X, b);
+      const int nwy = (maxn - 2 + kWyK - 1) / kWyK;
+      wide_wy_kernel<<<dim3(nwy + (maxn + 127) / 128, na), 128, 0, st>>>(X, nwy, ortol_rel);
+      {
+        const dim3 grid((maxn + kBtW - 1) / kBtW, na);
+        if (btsm <= kBtMaxSmem)
+          wide_backtr_kernel<true><<<grid, kBtNT, btsm, st>>>(X);
+        else
+          wide_backtr_kernel<false><<<grid, kBtNT, BackTransform::bytes(maxn, false), st>>>(X);
       }
       tm.mark("backtr");
-      wide_cd_kernel<<<dim3(gx((long long)nblk * nct, na), na), kGemmNT, tsm2, st>>>(X);
-      if (lshift != 0.0) wide_eshift_kernel<<<dim3(gx((long long)nblk * nct, na), na), kGemmNT, tsm, st>>>(X);
+      wide_cd_kernel<<<dim3(gx((long long)nblk * nblk, na), na), kGemmNT, tsm2, st>>>(X);
+      if (lshift != 0.0) wide_eshift_kernel<<<dim3(gx((long long)nblk * nblk, na), na), kGemmNT, tsm, st>>>(X);
       tm.mark("cd");
       wide_energy_mix_kernel<<<na, kWideNT, rsm, st>>>(B, M, X, ro, lshift);
       tm.mark("energy");
@@ -2277,7 +2515,6 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
     w.vao = p + s.vao;
     w.part = p + s.part;
     w.Tf = p + s.Tf;
-    w.Xp = p + s.Xp;
     w.popp = p + s.popp;
     w.eshift = p + s.eshift;
     w.ws = p + s.ws;

@@ -77,3 +77,34 @@ def test_cluster_and_blocked_reductions_agree(oracle_mod, sizes):
             o = oracle_mod.run(*mols[m], options=oracle_mod.make_options(**TIGHT))
             assert r.iterations[m] == o.iterations and abs(r.energy[m] - o.energy) <= 1e-7
             assert np.abs(r.gradient[off[m]:off[m + 1]] - o.gradient).max() <= 1e-7
+
+
+@pytest.mark.parametrize("copies, distance", [(25, 90.0), (25, 16.0)])
+def test_degenerate_and_close_eigenvalues(oracle_mod, copies, distance):
+    """Copies of one water on a lattice: orbitals degenerate to rounding far apart
+    (inverse iteration in a cluster), split by 1e-9 to 1e-4 Eh closer (twisted
+    factorisation, then orthogonalised chains).  Energies are invariant under the
+    mixing of degenerate orbitals, so the tolerance is the one above."""
+    z1, x1 = molecule(8)
+    at = np.array([[i % 3, (i // 3) % 3, i // 9] for i in range(copies)], dtype=float) * distance
+    z = np.tile(z1, copies)
+    x = (x1[None, :, :] + at[:, None, :]).reshape(-1, 3)
+    _, r = _calculate([(z, x)], None)
+    o = oracle_mod.run(z, x, options=oracle_mod.make_options(**TIGHT))
+    assert r.status[0] == 0 and r.iterations[0] == o.iterations
+    assert abs(r.energy[0] - o.energy) <= 1e-7
+    assert np.abs(r.gradient - o.gradient).max() <= 1e-7
+    assert np.abs(r.shell_charges - o.shell_charges).max() <= 1e-7
+
+
+def test_back_transformation_beyond_shared_memory():
+    """At 2920 AOs the columns of the back-transformation stay in global memory, at 2880
+    in shared memory; the difference here is 40 helium atoms too far away to interact."""
+    z, x = spread(2880)
+    he = np.array([[-200.0 - 60.0 * k, 40.0, 10.0] for k in range(40)])
+    more = (np.concatenate([z, np.full(40, 2, np.uint8)]), np.concatenate([x, he]))
+    _, r = _calculate([(z, x), more, (np.array([2], np.uint8), np.zeros((1, 3)))], None)
+    assert (r.status == 0).all() and r.iterations[0] == r.iterations[1]
+    assert abs(r.energy[1] - r.energy[0] - 40 * r.energy[2]) <= 1e-7
+    n = len(z)
+    assert np.abs(r.gradient[n:2 * n] - r.gradient[:n]).max() <= 1e-7
