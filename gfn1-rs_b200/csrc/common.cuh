@@ -184,6 +184,44 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int i = 0; i < nw; ++i) s += red[i];
   return s;
 }
+// K block-wide sums at once, as block_sum one by one: one pair of barriers and the
+// latencies overlapped.  `red` needs K blockDim/32 doubles.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double* red) {
+  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < K; ++k) red[k * nw + wid] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = 0.0;
+#pragma unroll 4
+  for (int i = 0; i < nw; ++i)
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] += red[k * nw + i];
+}
+template <int K>
+__device__ __forceinline__ void block_maxs(double (&v)[K], double* red) {
+  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < K; ++k) red[k * nw + wid] = v[k];
+  __syncthreads();
+#pragma unroll 1
+  for (int i = 0; i < nw; ++i)
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = fmax(v[k], red[k * nw + i]);
+}
 __device__ __forceinline__ double block_max(double v, double* red) {
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   v = warp_max(v);

@@ -640,7 +640,7 @@ __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, 
 // +80 kT clamp each contributes exactly 2/(1+e^80).  When a decision would need
 // them, `ambiguous` is set and the caller computes every eigenvalue.
 template <int CAP>
-__device__ void fermi_warp(const double* eps, int N, int nneed, double nelec, double kt, double* occ, double& mu_out,
+__device__ __noinline__ void fermi_warp(const double* eps, int N, int nneed, double nelec, double kt, double* occ, double& mu_out,
                            double& ts_out, bool& ambiguous) {
   constexpr double cap = CAP;  // electrons per orbital: 2, or 1 in a spin channel
   const int lane = threadIdx.x & 31;
@@ -757,14 +757,19 @@ __device__ void fermi_cta(const double* eps, int N, int nneed, double nelec, dou
   }
   bool amb = false;
   int i0 = k, i1 = k + 1;  // levels in reach of the bracket (eps ascends)
+#pragma unroll 1
   while (i0 > 0 && eps[i0 - 1] >= lo - w40) --i0;
+#pragma unroll 1
   while (i1 < nneed && eps[i1] <= hi + w40) ++i1;
   for (int round = 0; round < 64; ++round) {
     const double h = (hi - lo) * (1.0 / (NT + 1));
     const double mid = fmin(lo + (double)(tid + 1) * h, hi);
+#pragma unroll 1
     while (i0 < k && eps[i0] < lo - w40) ++i0;
+#pragma unroll 1
     while (i1 > k + 1 && eps[i1 - 1] > hi + w40) --i1;
     double sm = (double)i0 * cm80 + (double)(nneed - i1) * c80;
+#pragma unroll 1
     for (int i = i0; i < i1; ++i) sm += fo(eps[i], mid);
     if (nneed < N) sm += fo(elast, mid);
     bool flag = false;
@@ -798,6 +803,7 @@ __device__ void fermi_cta(const double* eps, int N, int nneed, double nelec, dou
   double ts = 0.0;
   if (!amb) {
     double t = 0.0;
+#pragma unroll 1
     for (int i = tid; i < N; i += NT) {
       const bool known = i < nneed || i == N - 1;
       const double f = known ? fo(eps[i], mu) : c80;
@@ -849,6 +855,7 @@ __device__ __noinline__ void spin_channel_occupations(const double* eps, int N, 
   bool aa, ab;
   channel(nalpha, occ, fa, ta, aa);
   channel(nbeta, tmp, fb, tb, ab);
+#pragma unroll 1
   for (int i = tid; i < N; i += NT) occ[i] += tmp[i];
   if (tid == 0) {
     sh.scal[1] = 0.5 * (fa + fb);
@@ -895,12 +902,14 @@ __device__ void stage_potential(const Batch& B, const Model& M, const MolCtx& c,
   const int a0 = c.a0, nat = c.nat, nsh = c.nsh, N = c.N;
   const int *sh_atom = c.sh_atom, *ao_sh = c.ao_sh, *atom_sh = c.atom_sh;
   const double* G = c.G;
+#pragma unroll 1
   for (int a = tid; a < nat; a += NT) {
     double q = 0.0;
     for (int s = atom_sh[a]; s < atom_sh[a + 1]; ++s) q += w.qin[s];
     w.qat[a] = q;
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < nsh; i += NT) {
     double v = 0.0;
     for (int j = 0; j < nsh; ++j) v += G[(long long)j * nsh + i] * w.qin[j];  // G symmetric: coalesced column
@@ -910,6 +919,7 @@ __device__ void stage_potential(const Batch& B, const Model& M, const MolCtx& c,
     w.vsh[i] = v;
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < N; i += NT) vao[i] = w.vsh[ao_sh[i]];
   __syncthreads();
 }
@@ -925,6 +935,7 @@ __device__ void stage_charges_energy(const Batch& B, const Model& M, const MolCt
   const int a0 = c.a0, nat = c.nat, nsh = c.nsh, N = c.N;
   const int *sh_atom = c.sh_atom, *sh_k = c.sh_k, *sh_ao0 = c.sh_ao0, *atom_sh = c.atom_sh;
   const double* G = c.G;
+#pragma unroll 1
   for (int s = tid; s < nsh; s += NT) {
     const ElemTable& el = M.elem[B.z[a0 + sh_atom[s]]];
     const int k = sh_k[s];
@@ -933,8 +944,10 @@ __device__ void stage_charges_energy(const Batch& B, const Model& M, const MolCt
     w.qout[s] = el.refocc[k] - p;
   }
   double part = 0.0;
+#pragma unroll 1
   for (int i = tid; i < N; i += NT) part += (i < nocc ? occ[i] * eps[i] : 0.0) + vao[i] * pop[i];
-  e_el = block_sum(part, sh.red);
+  __syncthreads();
+#pragma unroll 1
   for (int a = tid; a < nat; a += NT) {
     double q = 0.0;
     for (int s = atom_sh[a]; s < atom_sh[a + 1]; ++s) q += w.qout[s];
@@ -942,6 +955,7 @@ __device__ void stage_charges_energy(const Batch& B, const Model& M, const MolCt
   }
   __syncthreads();
   double p2 = 0.0, p3 = 0.0, pr = 0.0;
+#pragma unroll 1
   for (int i = tid; i < nsh; i += NT) {
     double v = 0.0;
     for (int j = 0; j < nsh; ++j) v += G[(long long)j * nsh + i] * w.qout[j];  // G symmetric: coalesced column
@@ -953,13 +967,17 @@ __device__ void stage_charges_energy(const Batch& B, const Model& M, const MolCt
     const double r = w.qout[i] - w.qin[i];
     pr += r * r;
   }
+#pragma unroll 1
   for (int a = tid; a < nat; a += NT) {
     const double qa = w.qat[a];
     p3 += qa * qa * qa * M.elem[B.z[a0 + a]].gam3 / 3.0;
   }
-  e2 = 0.5 * block_sum(p2, sh.red);
-  e3 = block_sum(p3, sh.red);
-  rms = nsh ? sqrt(block_sum(pr, sh.red) / nsh) : 0.0;
+  double sums[4] = {part, p2, p3, pr};
+  block_sums<4>(sums, sh.red);
+  e_el = sums[0];
+  e2 = 0.5 * sums[1];
+  e3 = sums[2];
+  rms = nsh ? sqrt(sums[3] / nsh) : 0.0;
 }
 
 // (10) Charge mixing: modified Broyden (src/electronic.rs:3203-3309), linear
@@ -976,6 +994,7 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
   if (opt.broyden) {
     bro_iter += 1;
     if (bro_iter == 1) {
+#pragma unroll 1
       for (int s = tid; s < nsh; s += NT) {
         const double r = w.qout[s] - w.qin[s];
         w.dqlast[s] = r;
@@ -989,17 +1008,20 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
       const int it1 = (itn - 1) % memory;
       const int slot = it1 % cap;
       double pn = 0.0, pd = 0.0;
+#pragma unroll 1
       for (int s = tid; s < nsh; s += NT) {
         const double r = w.qout[s] - w.qin[s];
         pn += r * r;
         const double dfv = r - w.dqlast[s];
         pd += dfv * dfv;
       }
-      const double dqn = sqrt(block_sum(pn, sh.red));
-      const double dfn = sqrt(block_sum(pd, sh.red));
+      double sums[2] = {pn, pd};
+      block_sums<2>(sums, sh.red);
+      const double dqn = sqrt(sums[0]), dfn = sqrt(sums[1]);
       const double inv = 1.0 / fmax(dfn, DBL_EPSILON);
       double* dfs = w.df + (long long)slot * nsh;
       double* us = w.u + (long long)slot * nsh;
+#pragma unroll 1
       for (int s = tid; s < nsh; s += NT) {
         const double r = w.qout[s] - w.qin[s];
         const double dfv = (r - w.dqlast[s]) * inv;
@@ -1015,6 +1037,7 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
       const int start = itn > memory ? itn - memory + 1 : 1;
       const int mact = itn - start + 1;
       // dot products df_new . df_j for every active slot, and c_j = omega_j df_j . dq
+#pragma unroll 1
       for (int r = wid; r < mact; r += NW) {
         const int sj = ((start + r - 1) % memory) % cap;
         const double* dj = w.df + (long long)sj * nsh;
@@ -1032,6 +1055,7 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
         }
       }
       __syncthreads();
+#pragma unroll 1
       for (int idx = tid; idx < mact * mact; idx += NT) {
         const int r = idx / mact, c = idx % mact;
         const int si = ((start + r - 1) % memory) % cap, sj = ((start + c - 1) % memory) % cap;
@@ -1039,71 +1063,111 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
         if (r == c) b += 0.01 * 0.01;
         w.beta[(long long)r * mact + c] = b;
       }
+#pragma unroll 1
       for (int r = tid; r < mact; r += NT) {
         const int si = ((start + r - 1) % memory) % cap;
         w.cvec[r] *= w.omega[si];
       }
       __syncthreads();
-      // Gauss-Jordan with partial pivoting (src/electronic.rs:3767-3806)
+      // Gauss-Jordan with partial pivoting (src/electronic.rs:3767-3806); up to 16
+      // vectors by one warp, whose steps need no block barrier (six a column: most of the
+      // mixing of a small molecule)
+      const bool one = mact <= 16;
+      const int t = one ? lane : tid, nt = one ? 32 : NT;
+      auto sync = [&]() {
+        if (one)
+          __syncwarp();
+        else
+          __syncthreads();
+      };
       bool ok = true;
-      for (int col = 0; col < mact; ++col) {
-        if (tid == 0) {
+      if (!one || wid == 0) {
+#pragma unroll 1
+        for (int col = 0; col < mact; ++col) {
           int piv = col;
-          double pabs = fabs(w.beta[(long long)col * mact + col]);
-          for (int r = col + 1; r < mact; ++r) {
-            const double v = fabs(w.beta[(long long)r * mact + col]);
-            if (v > pabs) {
-              piv = r;
-              pabs = v;
+          if (one) {  // the first of the largest
+            double pabs = lane >= col && lane < mact ? fabs(w.beta[(long long)lane * mact + col]) : -1.0;
+            piv = lane;
+#pragma unroll 1
+            for (int o = 8; o > 0; o >>= 1) {
+              const double v = __shfl_xor_sync(0xffffffffu, pabs, o);
+              const int at = __shfl_xor_sync(0xffffffffu, piv, o);
+              if (v > pabs || (v == pabs && at < piv)) {
+                pabs = v;
+                piv = at;
+              }
+            }
+            piv = __shfl_sync(0xffffffffu, pabs < 1e-18 ? -1 : piv, 0);
+          } else {
+            if (tid == 0) {
+              double pabs = fabs(w.beta[(long long)col * mact + col]);
+#pragma unroll 1
+              for (int r = col + 1; r < mact; ++r) {
+                const double v = fabs(w.beta[(long long)r * mact + col]);
+                if (v > pabs) {
+                  piv = r;
+                  pabs = v;
+                }
+              }
+              sh.iscal[1] = (pabs < 1e-18) ? -1 : piv;
+            }
+            __syncthreads();
+            piv = sh.iscal[1];
+          }
+          if (piv < 0) {
+            ok = false;
+            break;
+          }
+          if (piv != col) {
+#pragma unroll 1
+            for (int j = t; j < mact; j += nt) {
+              const double v = w.beta[(long long)piv * mact + j];
+              w.beta[(long long)piv * mact + j] = w.beta[(long long)col * mact + j];
+              w.beta[(long long)col * mact + j] = v;
+            }
+            if (t == 0) {
+              const double v = w.cvec[piv];
+              w.cvec[piv] = w.cvec[col];
+              w.cvec[col] = v;
+            }
+            sync();
+          }
+          const double dg = w.beta[(long long)col * mact + col];
+          sync();
+#pragma unroll 1
+          for (int j = col + t; j <= mact; j += nt) {  // the last one is the right-hand side
+            double* at = j < mact ? w.beta + (long long)col * mact + j : w.cvec + col;
+            *at /= dg;
+          }
+          sync();
+#pragma unroll 1
+          for (int r = t >> 4; r < mact; r += nt >> 4) {  // 16 threads a row; column `col` is zeroed below
+            const double f = w.beta[(long long)r * mact + col];
+            if (r == col || f == 0.0) continue;
+#pragma unroll 1
+            for (int j = col + 1 + (t & 15); j <= mact; j += 16) {
+              if (j < mact)
+                w.beta[(long long)r * mact + j] -= f * w.beta[(long long)col * mact + j];
+              else
+                w.cvec[r] -= f * w.cvec[col];
             }
           }
-          sh.iscal[1] = (pabs < 1e-18) ? -1 : piv;
+          sync();
+#pragma unroll 1
+          for (int r = t; r < mact; r += nt)
+            if (r != col) w.beta[(long long)r * mact + col] = 0.0;
+          sync();
         }
-        __syncthreads();
-        const int piv = sh.iscal[1];
-        if (piv < 0) {
-          ok = false;
-          break;
-        }
-        if (piv != col) {
-          for (int j = tid; j < mact; j += NT) {
-            const double t = w.beta[(long long)piv * mact + j];
-            w.beta[(long long)piv * mact + j] = w.beta[(long long)col * mact + j];
-            w.beta[(long long)col * mact + j] = t;
-          }
-          if (tid == 0) {
-            const double t = w.cvec[piv];
-            w.cvec[piv] = w.cvec[col];
-            w.cvec[col] = t;
-          }
-          __syncthreads();
-        }
-        const double dg = w.beta[(long long)col * mact + col];
-        __syncthreads();
-        for (int j = col + tid; j < mact; j += NT) w.beta[(long long)col * mact + j] /= dg;
-        if (tid == 0) w.cvec[col] /= dg;
-        __syncthreads();
-        for (int idx = tid; idx < mact * (mact - col); idx += NT) {
-          const int r = idx / (mact - col), j = col + idx % (mact - col);
-          if (r == col) continue;
-          const double f = w.beta[(long long)r * mact + col];
-          if (f == 0.0 || j == col) continue;
-          w.beta[(long long)r * mact + j] -= f * w.beta[(long long)col * mact + j];
-        }
-        for (int r = tid; r < mact; r += NT) {
-          if (r == col) continue;
-          const double f = w.beta[(long long)r * mact + col];
-          if (f != 0.0) w.cvec[r] -= f * w.cvec[col];
-        }
-        __syncthreads();
-        for (int r = tid; r < mact; r += NT)
-          if (r != col) w.beta[(long long)r * mact + col] = 0.0;
-        __syncthreads();
+        if (one && lane == 0) sh.iscal[1] = ok ? 1 : -1;
       }
+      __syncthreads();
+      if (one) ok = sh.iscal[1] > 0;
       if (ok) {
+#pragma unroll 1
         for (int s = tid; s < nsh; s += NT) {
           const double r = w.qout[s] - w.qin[s];
           double qn = w.qin[s] + mixing * r;
+#pragma unroll 2
           for (int rr = 0; rr < mact; ++rr) {
             const int si = ((start + rr - 1) % memory) % cap;
             qn -= w.omega[si] * w.cvec[rr] * w.u[(long long)si * nsh + s];
@@ -1118,14 +1182,17 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
     }
     if (have_next) {  // trusted_charge_vector (src/electronic.rs:3759-3761)
       int bad = 0;
+#pragma unroll 1
       for (int s = tid; s < nsh; s += NT)
         if (!isfinite(w.qnext[s]) || fabs(w.qnext[s]) >= 10.0) bad = 1;
-      if (block_max((double)bad, sh.red) > 0.0) have_next = false;
+      if (__syncthreads_or(bad)) have_next = false;
     }
   }
   if (!have_next)
+#pragma unroll 1
     for (int s = tid; s < nsh; s += NT) w.qnext[s] = w.qin[s] + mixing * (w.qout[s] - w.qin[s]);
   __syncthreads();
+#pragma unroll 1
   for (int s = tid; s < nsh; s += NT) w.qin[s] = w.qnext[s];
 }
 
@@ -1160,11 +1227,13 @@ __device__ void stage_results(const Batch& B, const MolCtx& c, CtaWs& w, int ite
     B.dipole[3 * m + 1] = dy;
     B.dipole[3 * m + 2] = dz;
   }
+#pragma unroll 1
   for (int s = tid; s < nsh; s += NT) {
     B.shell_q[sh0 + s] = w.qout[s];
     B.shell_pot[sh0 + s] = w.vout[s];
     if (B.shell_pot_in) B.shell_pot_in[sh0 + s] = w.vsh[s];
   }
+#pragma unroll 1
   for (int a = tid; a < nat; a += NT) B.atom_q[a0 + a] = w.qat[a];
 }
 
@@ -1268,6 +1337,7 @@ __device__ __noinline__ void scc_cholesky(const SccArgs& A) {
   const double* S = A.B.S + v.s.mo;
   double* L = v.w.L;
   double(*Ld)[9] = v.sh.Ld;
+#pragma unroll 1
   for (int idx = tid; idx < ld * ld; idx += NT) {  // zeros in the padding
     const int i = idx / ld, j = idx - i * ld;
     L[idx] = (i < N && j < N) ? S[(long long)i * N + j] : 0.0;
@@ -1363,6 +1433,7 @@ __device__ __noinline__ void scc_inverse(const SccArgs& A) {
   const double* __restrict__ L = v.w.L;
   double* __restrict__ LiT = v.w.LiT;
   double* inv = reinterpret_cast<double*>(smraw) + v.s.tri_at;  // [nt][8][8] row-major
+#pragma unroll 1
   for (int c = tid; c < ld; c += NT) {  // column c & 7 of the inverse of diagonal block c >> 3
     const int b = c >> 3, j = c & 7;
     double x[8];
@@ -1510,6 +1581,7 @@ __device__ __noinline__ void scc_occupations(const SccArgs& A, StageClock* clk) 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, N = s.N;
   const double *d = v.d, *e = v.e;
   double gl = INFINITY, gu = -INFINITY, onenrm = 0.0, emax2 = 0.0;
+#pragma unroll 1
   for (int i = tid; i < N; i += NT) {
     const double off = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < N - 1 ? fabs(e[i]) : 0.0);
     gl = fmin(gl, d[i] - off);
@@ -1520,10 +1592,14 @@ __device__ __noinline__ void scc_occupations(const SccArgs& A, StageClock* clk) 
       emax2 = fmax(emax2, v.esq[i]);
     }
   }
-  gl = -block_max(-gl, sh.red);
-  gu = block_max(gu, sh.red);
-  onenrm = block_max(onenrm, sh.red);
-  emax2 = block_max(emax2, sh.red);
+  {
+    double v4[4] = {-gl, gu, onenrm, emax2};
+    block_maxs<4>(v4, sh.red);
+    gl = -v4[0];
+    gu = v4[1];
+    onenrm = v4[2];
+    emax2 = v4[3];
+  }
   const double pivmin = DBL_MIN * fmax(1.0, emax2);
   {
     const double span = gu - gl;
@@ -1564,9 +1640,15 @@ __device__ __noinline__ void scc_occupations(const SccArgs& A, StageClock* clk) 
     nneed = N;
   }
   int nocc_loc = 0;
+#pragma unroll 1
   for (int i = tid; i < N; i += NT)
     if ((i < nneed || i == N - 1) && v.occ[i] > 1e-30) nocc_loc = max(nocc_loc, i + 1);
-  const int nocc = (int)block_max((double)nocc_loc, sh.red);
+  nocc_loc = __reduce_max_sync(0xffffffffu, nocc_loc);
+  if (lane == 0) sh.first[0][wid] = nocc_loc;
+  __syncthreads();
+  int nocc = 0;
+#pragma unroll
+  for (int q = 0; q < NT / 32; ++q) nocc = max(nocc, sh.first[0][q]);
   if (tid == 0) {
     s.mu = sh.scal[1];
     s.ts = sh.scal[2];
@@ -1757,6 +1839,7 @@ __device__ __noinline__ void scc_energy(const SccArgs& A, double lshift) {
   CtaView v = cta_view(A);
   MolState& s = v.s;
   const int tid = threadIdx.x, N = s.N, ld = s.ld;
+#pragma unroll 1
   for (int i = tid; i < N; i += NT) {
     double p = 0.0;
 #pragma unroll
@@ -1771,6 +1854,7 @@ __device__ __noinline__ void scc_energy(const SccArgs& A, double lshift) {
     const double *Hp = v.w.Hp, *Z = v.w.Z;
     const int nocc = s.nocc;
     double part = 0.0;
+#pragma unroll 1
     for (long long idx = tid; idx < (long long)N * nocc; idx += NT) {
       const int i = (int)(idx / nocc), k = (int)(idx % nocc);
       double hz = 0.0;
@@ -1827,6 +1911,7 @@ __device__ __noinline__ void scc_finish(const SccArgs& A, int rung) {
   stage_results<NT>(B, v.c, v.w, s.iter, s.converged != 0, s.e_el, s.e2, s.e3, s.ts, s.mu);
   if (B.orb_eps) {  // orbital energies (NaN where the eigensolver did not need them) and occupations
     const int ao0 = B.ao_off[m];
+#pragma unroll 1
     for (int i = tid; i < N; i += NT) {
       B.orb_eps[ao0 + i] = (i < s.nneed || i == N - 1) ? v.eps[i] : __longlong_as_double(0x7ff8000000000000LL);
       B.orb_occ[ao0 + i] = v.occ[i];
@@ -1929,6 +2014,7 @@ __device__ __forceinline__ void scc_molecule(const SccArgs& A, int m) {
     __syncthreads();
     {
       const CtaView v = cta_view(A);
+#pragma unroll 1
       for (int i = tid; i < s.nsh; i += NT) v.w.qin[i] = A.B.init_q ? A.B.init_q[s.sh0 + i] : 0.0;
     }
     if (tid == 0) {
