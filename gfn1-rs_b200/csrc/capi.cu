@@ -905,9 +905,11 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
     ws_total += R.ws_stride * R.n_cta;
     R.smem = scc_smem_bytes(R.kind, R.maxnsh, R.maxn, R.maxnat);
   }
-  if (!b->ev_fork && cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess)
+  int classes = 0;  // the first one runs on the caller's stream
+  for (const gfn1_batch::SccClass& K : b->cls) classes += K.n_cta > 0;
+  if (classes > 1 && !b->ev_fork && cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess)
     return fail(eng, GFN1_E_DEVICE, "event creation failed");
-  for (int c = 0; c < 2; ++c)
+  for (int c = 0; c < classes - 1; ++c)
     if ((!b->side[c] && cudaStreamCreateWithFlags(&b->side[c], cudaStreamNonBlocking) != cudaSuccess) ||
         (!b->ev_join[c] && cudaEventCreateWithFlags(&b->ev_join[c], cudaEventDisableTiming) != cudaSuccess))
       return fail(eng, GFN1_E_DEVICE, "stream creation failed");
