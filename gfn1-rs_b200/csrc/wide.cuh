@@ -19,11 +19,13 @@
 //   A    working matrix: F' = L^-1 F L^-T, then the Householder reflectors in
 //        its strictly lower triangle (column j holds reflector j below the
 //        subdiagonal; its first entry is an implicit 1)
-//   Z    eigenvectors of F' (columns 0..nocc-1): tridiagonal basis after
-//        inverse iteration, orthonormal basis after the back-transformation
+//   Z    eigenvectors of F' (columns 0..nocc-1): tridiagonal basis, up to the
+//        factors in esq, after wide_vectors_kernel, orthonormal basis after the
+//        back-transformation
 //   C    MO coefficients L^-T Z (columns 0..nocc-1)
-// plus the factor arrays of inverse iteration (5 N x N, interleaved per
-// eigenvector), the panel buffer of the reduction, N-vectors and the SCC
+// plus the factor arrays of the eigenvectors (5 N x N, interleaved per
+// eigenvector), the panel buffer of the reduction (the exchange ring where the
+// matrix is on chip), N-vectors and the SCC
 // vectors and Broyden history in the CtaWs layout.
 #pragma once
 
@@ -2270,9 +2272,9 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   if (e != cudaSuccess) return e;
   WideCtx X{R.d_mols, R.d_act, maxnsh, maxn, maxnat, cap};
   WideTimer tm(st);
-  // Eigenvalues closer than ortol_rel |T|_1 form a cluster whose vectors are
-  // re-orthogonalised (modified Gram-Schmidt).  Inverse iteration alone leaves
-  // an overlap of about eps |T| / gap between two vectors, at most 2e-9 here;
+  // Eigenvalues closer than ortol_rel |T|_1 form a chain whose vectors are
+  // re-orthogonalised (modified Gram-Schmidt).  Each vector alone leaves an
+  // overlap of about eps |T| / gap between two of them, at most 2e-9 here;
   // a wider threshold (LAPACK dstein: 1e-3) chains hundreds of the dense
   // levels of a large molecule into clusters one thread would orthogonalise.
   double ortol_rel = 1e-7;

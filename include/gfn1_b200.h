@@ -154,17 +154,19 @@ int gfn1_batch_launch(gfn1_batch* b, void* stream);
 int gfn1_batch_launch_stage(gfn1_batch* b, int stage, void* stream);
 /* Per-stage SCC clock totals (GFN1_PROFILE=1 at batch creation), n <= 13:
  * prologue (H0' and the SCC state), Fock, tridiagonalisation, eigenvalues,
- * occupations, inverse iteration, back-transformation, populations, energy,
- * mixing, final, Cholesky, L^-1. */
+ * occupations, eigenvectors, back-transformation (0: counted with the
+ * populations), back-transformation and populations, energy, mixing, final,
+ * Cholesky, L^-1. */
 int gfn1_batch_stage_cycles(const gfn1_batch* b, uint64_t* cycles, int n);
 /* Bytes of the input blob (one host->device copy per call) and of the output
  * blob (one device->host copy per call). */
 int gfn1_batch_io_bytes(const gfn1_batch* b, int64_t* h2d, int64_t* d2h);
-/* Plan of the large-molecule path (molecules above 256 AOs) in the last
- * gfn1_batch_energy_gradient / gfn1_run call on this engine: the Householder
- * reduction's panel width, its minimum rows per CTA, the CTAs per molecule,
- * the reduction time the autotuner measured for that plan (ms) and whether the
- * autotuner chose it (1) or GFN1_WIDE_PANEL fixed it (0).  All zero when that
+/* Plan of the large-molecule path (molecules above 192 AOs) in the last
+ * gfn1_batch_energy_gradient / gfn1_run call on this engine: the blocked
+ * Householder reduction's panel width and minimum rows per CTA (its defaults
+ * where every matrix fits on chip, up to 2368 AOs), the CTAs per molecule, the
+ * time of one reduction with that plan (ms) and whether the autotuner measured
+ * it (1) or GFN1_WIDE_PANEL fixed it (0).  All zero when that
  * call had no large molecule.  No counterpart in the reference (faer chooses
  * its own blocking inside self_adjoint_eigen, src/linalg.rs:176). */
 int gfn1_last_wide_plan(gfn1_engine* eng, int32_t* panel, int32_t* min_rows, int32_t* ctas_per_molecule,
