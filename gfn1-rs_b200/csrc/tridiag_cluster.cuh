@@ -43,9 +43,9 @@ struct ClusterShape {
   static constexpr int kKeep = 16;             // columns kept in shared memory before they are written out
   static constexpr int kOut = TR * NA * (kKeep + 1) + 3 * kKeep;  // the CTA's rows of the reflectors; d, e, tau
   // x (two buffers), (v, w), gathered (y, next column) (two buffers), partial sums,
-  // next column's entries, warp sums, x.y of the CTAs (two buffers); then what waits to be written
-  // out, then the slots
-  static constexpr int kVec = 8 * P + WC * TR * NA + TR * NA + 2 * NW + 2 * C + kOut;
+  // next column's entries, warp sums of |x|^2 (two buffers) and of x.y, x.y of the CTAs (two buffers);
+  // then what waits to be written out, then the slots
+  static constexpr int kVec = 8 * P + WC * TR * NA + TR * NA + 3 * NW + 2 * C + kOut;
   static constexpr size_t kBytes = sizeof(double) * (kVec + NA * BS * NT);
 };
 
@@ -105,8 +105,9 @@ __device__ __forceinline__ void cluster_phase(ClusterReg<C>& R, const ClusterOut
   double2* gat = reinterpret_cast<double2*>(sm + 4 * P);       // [2][P]
   double* part = sm + 8 * P;                                   // [WC][TR NA]
   double* xnl = part + WC * TR * NA;                           // [TR NA]
-  double* red = xnl + TR * NA;                                 // [NW] |x|^2, [NW] x.y
-  double* xyc = red + 2 * NW;                                  // [2][C]
+  double* red = xnl + TR * NA;                                 // [2][NW] |x|^2, by the column's parity
+  double* redxy = red + 2 * NW;                                // [NW] x.y
+  double* xyc = redxy + NW;                                    // [2][C]
   double* vk = xyc + 2 * C;                                    // [TR NA][kKeep + 1]
   double* det = vk + TR * NA * (CS::kKeep + 1);                // [3][kKeep] d of column k + 1, e, tau
   double2* priv = reinterpret_cast<double2*>(sm + CS::kVec) + tid;
@@ -208,7 +209,7 @@ __device__ __forceinline__ void cluster_phase(ClusterReg<C>& R, const ClusterOut
       const int q = 2 * u + 1 < n1 ? 2 * u + ((lc >> 1) & 1) : 2 * u;
       const int a = 2 * q + 1 < n ? 2 * q + (lc & 1) : 2 * q;
       part[wc * TR * NA + TR * (A0 + a) + tr] = s3;
-      if (lane == 0) red[NW + wid] = xy;
+      if (lane == 0) redxy[wid] = xy;
     }
     __syncthreads();
     // the CTA's rows to every CTA
@@ -222,10 +223,11 @@ __device__ __forceinline__ void cluster_phase(ClusterReg<C>& R, const ClusterOut
       double2* at = gat + (k & 1) * P + TR * (C * (l / TR) + rank) + l % TR;
       for (int q = g; q < C; q += groups) *cl.map_shared_rank(at, q) = v;
     }
-    if (wid == NW - 1 && lane < C) *cl.map_shared_rank(xyc + (k & 1) * C + rank, lane) = tree_sum<NW>(red + NW);
+    if (wid == NW - 1 && lane < C) *cl.map_shared_rank(xyc + (k & 1) * C + rank, lane) = tree_sum<NW>(redxy);
     cl.barrier_arrive();
-    // the reflector's scalars, in every thread while the barrier completes
-    const double xx = tree_sum<NW>(red), x0 = x[k1];
+    // the reflector's scalars, in every thread while the barrier completes (a warp may read them after
+    // the others are through it and have written the next column's |x|^2: hence the two buffers)
+    const double xx = tree_sum<NW>(red + (k & 1) * NW), x0 = x[k1];
     double alpha = 0.0, beta = 0.0, iv = 0.0;
     if (xx > 1e-280) {  // below: the column is zero next to any entry that matters
       const double nrm = sqrt(xx);
@@ -272,7 +274,7 @@ __device__ __forceinline__ void cluster_phase(ClusterReg<C>& R, const ClusterOut
       sq += xnext * xnext;
     }
     sq = warp_sum(sq);
-    if (lane == 0) red[wid] = sq;
+    if (lane == 0) red[((k + 1) & 1) * NW + wid] = sq;
     __syncthreads();
     if (kq == CS::kKeep - 1 || k == P - 3) cluster_write_out<C>(O, k, sm);
   }
@@ -320,7 +322,7 @@ __device__ __forceinline__ void cluster_tridiag(const ClusterOut& O, double* sm)
   }
   sq = warp_sum(sq);
   double* red = sm + 8 * P + CS::WC * TR * NA + TR * NA;
-  if (lane == 0) red[wid] = sq;
+  if (lane == 0) red[(off & 1) * CS::NW + wid] = sq;
   cl.sync();  // the matrix is read before the reflectors overwrite it
   cluster_phase<C, 0>(R, O, sm);
   // the last 2 x 2 block: its corner belongs to the last row's CTA

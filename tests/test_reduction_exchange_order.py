@@ -1,0 +1,47 @@
+"""Order of the shared and global exchanges of the on-chip Householder reductions, read from their
+source (CPU only: a race shows on a GPU as a rare wrong column, not as a failing run).
+
+A column of the cluster reduction is: products, sums, remote stores, barrier_arrive, the reflector's
+scalars, barrier_wait, vectors, block barrier.  The barrier's wait returns once every warp has
+arrived, so whatever a warp reads between its arrive and its wait may already be overwritten by
+another warp's code after the wait."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gfn1-rs_b200", "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as fh:
+        return re.sub(r"//[^\n]*", "", fh.read())
+
+
+def _index(expression, k):
+    """Buffer number of `base + (...) * NW` or `[(...) * NW + wid]` at column k; 0 without one."""
+    m = re.search(r"\(\(?k(?: \+ (\d))?\)? & 1\) \* NW", expression)
+    return None if not m else (k + int(m.group(1) or 0)) & 1
+
+
+def test_cluster_scalars_are_not_overwritten_before_they_are_read():
+    text = _source("tridiag_cluster.cuh")
+    body = text[text.index("cl.barrier_arrive();"):]
+    split = body.index("cl.barrier_wait();")
+    overlapped, after = body[:split], body[split:body.index("cluster_write_out<C>(O, k, sm);")]
+    reads = re.findall(r"tree_sum<NW>\((red\w*[^;,]*?)\)[,;]", overlapped)
+    writes = re.findall(r"(red\w*\[[^\]]*\]) =", after)
+    assert reads and writes
+    for r in reads:
+        for w in writes:
+            if re.match(r"\w+", r).group() != re.match(r"\w+", w).group():
+                continue
+            for k in (0, 1):
+                assert _index(r, k) is not None and _index(w, k) is not None, (r, w)
+                assert _index(r, k) != _index(w, k), (r, w)  # read at column k, written for column k + 1
+                assert _index(r, k + 1) == _index(w, k)
+
+
+def test_cluster_shared_memory_holds_its_buffers():
+    text = _source("tridiag_cluster.cuh")
+    body = text[text.index("cluster_phase("):]
+    assert "xyc = redxy + NW" in body and "redxy = red + 2 * NW" in body
+    assert "3 * NW + 2 * C + kOut" in text
