@@ -15,9 +15,13 @@
 // barrier and a load after it are two round trips to L2, this is one.  Sixteen slots:
 // once every CTA's values of column k, a multiple of eight, are there, all of them
 // have read columns k - 8 .. k - 1; their owners mark those slots unwritten again and
-// fence that before their values of column k + 2, which a reader has seen before it
-// looks for those of column k + 8, the first to use these slots.  Every wait is bounded: after kSpinCycles, or when
-// another CTA has raised the molecule's error flag, the CTA raises it and leaves.
+// fence that before their values of column k + 2.  Every thread of a reader has its values
+// of column k + 2 and fences in turn before it looks for those of column k + 8, the first to
+// use these slots: with the two fences the marks happen before that look, so it finds the
+// mark or a new value, never the number of sixteen columns ago.  (The loads and stores of the
+// ring are relaxed; one fence by the readers in eight columns is all the order they need.)
+// Every wait is bounded: after kSpinCycles, or when another CTA has raised the molecule's
+// error flag, the CTA raises it and leaves.
 //
 // Measured on B200 (the blocked reduction before): 2368 AOs 42 -> 8.9 ms, 1300 -> 3.7 ms,
 // 769 -> 1.9 ms.  Of the 7,250 cycles a column at 2368 AOs 1,840 are the products (660
@@ -49,6 +53,7 @@ struct GridShape {
   // A ring slot has N values, rounded up so that the rows of a block start on 64 bytes.
   static __host__ __device__ constexpr int ring_stride(int N) { return (N + 2 * kBlock - 1) & ~(kBlock - 1); }
   static constexpr int kRing = 16, kMark = 8;    // ring slots; slots marked unwritten at a time
+  static constexpr int kRelease = 1, kAcquire = 2;  // columns after the marks: the owner's fence, the readers'
   // (v, w), x, partial sums, next column's entries, warp sums, scalars; then the slots
   static constexpr int kVec = 3 * P + WC * kRows + kRows + 2 * NW + 8;
   static constexpr size_t kBytes = sizeof(double) * (kVec + NA * BS * NT);
@@ -84,6 +89,7 @@ __device__ __forceinline__ double2 ring_load(const double2* p) {
   asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void ring_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ bool unwritten(const double2& v) {
   return (unsigned long long)__double_as_longlong(v.x) == kUnwritten ||
          (unsigned long long)__double_as_longlong(v.y) == kUnwritten;
@@ -291,7 +297,7 @@ __device__ __forceinline__ bool grid_phase(GridReg& R, const GridOut& O, double*
       if (i >= k1 && i < N) g[q] = ring_load(ring + i);
     }
     // what was marked at the previous column, before the next column's values
-    if (wid == 0 && (k & (GS::kMark - 1)) == 1) __threadfence();
+    if (wid == 0 && (k & (GS::kMark - 1)) == GS::kRelease) ring_fence();
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
       if (q >= q0) wait |= unwritten(g[q]);
@@ -312,6 +318,9 @@ __device__ __forceinline__ bool grid_phase(GridReg& R, const GridOut& O, double*
         }
       }
     }
+    // the owners' marks before the next look at those slots (each row's owner marks its slots, and
+    // the thread that reads the row here is the one that will look there)
+    if ((k & (GS::kMark - 1)) == GS::kAcquire) ring_fence();
     double xy = 0.0;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {

@@ -45,3 +45,25 @@ def test_cluster_shared_memory_holds_its_buffers():
     body = text[text.index("cluster_phase("):]
     assert "xyc = redxy + NW" in body and "redxy = red + 2 * NW" in body
     assert "3 * NW + 2 * C + kOut" in text
+
+
+def test_grid_readers_fence_between_the_marks_and_the_reuse_of_their_slots():
+    """Marks are made in phase C of column 0 (modulo kMark), published by the owner's fence before its
+    values of a later column p, seen by a reader with that column's values, and needed before the
+    look at column kMark.  So a reader fences in every thread after its wait of a column in
+    p .. kMark - 1, at least once per kMark columns."""
+    text = _source("tridiag_grid.cuh")
+    const = {m.group(1): int(m.group(2)) for m in re.finditer(r"(k\w+) = (\d+)\b", text)}
+    mark, ring = const["kMark"], const["kRing"]
+    assert ring == 2 * mark
+    body = text[text.index("__forceinline__ bool grid_phase("):text.index("__forceinline__ bool grid_tridiag(")]
+    fences = re.findall(r"if \((wid == 0 && )?\(k & \(GS::kMark - 1\)\) == (?:GS::)?(\w+)\) (?:ring_fence|__threadfence)\(\);",
+                        body)
+    column = {bool(owner): int(const.get(c, c)) for owner, c in fences}
+    assert set(column) == {True, False}, "one fence by the owner's publishing warp, one by every reading thread"
+    published = column[True] + 1  # the first values stored after the owner's fence
+    assert 1 <= column[True] and published <= column[False] < mark
+    at = body.index("ring_fence();", body.index("double2 g[NQ];"))
+    wait, reader = body.index("if (wait) {"), body.rindex("ring_fence();")
+    assert at < wait < reader < body.index("double xy = 0.0;")
+    assert re.search(r"fence\.acq_rel\.gpu", text)
