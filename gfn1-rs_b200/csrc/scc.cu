@@ -554,7 +554,9 @@ __device__ __forceinline__ double eigenvalue_k(const double* d, const double* es
 // 4 to 8.)  warm: eps holds the previous SCC iteration's eigenvalues, the first
 // points.  px, pc: N doubles of shared scratch.  Part: the CTA finds only NT of them
 // from number `base` on; a cold start then takes two rounds of even points, the
-// second over the interval that the first leaves to the CTA's eigenvalues.
+// second over the interval that the first leaves to the CTA's eigenvalues, in two
+// words of its own behind the NT of px (a thread that found its eigenvalue in the first
+// round still has its point and count in px and pc for the others).
 template <int NT, bool Part = false>
 __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, int N, int nneed, int nwarm, double gl,
                                             double gu, double pivmin, double atol, double* eps, double* px, double* pc,
@@ -623,11 +625,10 @@ __device__ __forceinline__ void eigenvalues(const double* d, const double* esq, 
     }
     if (!__syncthreads_or(active)) break;
     if (Part && it == 0 && nwarm == 0) {
-      if (tid == 0) px[0] = lo;
-      if (tid == nlist - 1) pc[0] = hi;
+      if (tid == 0) px[NT] = lo;
+      if (tid == nlist - 1) px[NT + 1] = hi;
       __syncthreads();
-      if (active) x = px[0] + (pc[0] - px[0]) * ((tid + 0.5) / nlist);
-      __syncthreads();
+      if (active) x = px[NT] + (px[NT + 1] - px[NT]) * ((tid + 0.5) / nlist);
     }
   }
   if (active) eps[k] = x;

@@ -1238,7 +1238,7 @@ __global__ void __launch_bounds__(kGemmNT) wide_shift_kernel(WideCtx X, double l
 constexpr int kEigNT = 64;
 __global__ void __launch_bounds__(kEigNT) wide_eigval_kernel(WideCtx X) {
   extern __shared__ __align__(16) double dsm[];
-  __shared__ double px[kEigNT], pc[kEigNT];
+  __shared__ double px[kEigNT + 2], pc[kEigNT];
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const WideState* st = w.st;
   if (st->status != kOk) return;
