@@ -1040,7 +1040,9 @@ __global__ void __launch_bounds__(kRedNT) wide_bounds_kernel(WideCtx X) {
 }
 
 // ------------------------------------------------------------------ set-up and rung start
-// L = lower triangle of S (zeros above), L^-1 = 0, SCC state from the host-validated status.
+// L = lower triangle of S (zeros above), L^-1 = 0, SCC state from the host-validated status, and
+// the group's barriers as new: a wait that gave up in an earlier run of the same slots (a resident
+// batch, a repeated topology) has left its error flag and, in a counter, its arrivals.
 __global__ void wide_begin_kernel(Batch B, WideCtx X) {
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const int N = w.N, ld = w.ld;
@@ -1057,6 +1059,7 @@ __global__ void wide_begin_kernel(Batch B, WideCtx X) {
     st->converged = 0;
     st->iter = 0;
     st->nocc = 0;
+    w.sync[0] = w.sync[1] = GroupSync{0u, 0u, 0, 0};  // column and panel barriers
   }
 }
 

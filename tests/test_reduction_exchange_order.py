@@ -67,3 +67,14 @@ def test_grid_readers_fence_between_the_marks_and_the_reuse_of_their_slots():
     wait, reader = body.index("if (wait) {"), body.rindex("ring_fence();")
     assert at < wait < reader < body.index("double xy = 0.0;")
     assert re.search(r"fence\.acq_rel\.gpu", text)
+
+
+def test_every_run_starts_with_clear_error_flags():
+    """A wait that gave up raises the flag of its slot for the run it belongs to: the kernel that begins
+    a run clears both barriers of every slot, before the reductions poll them."""
+    text = _source("wide.cuh")
+    body = text[text.index("__global__ void wide_begin_kernel("):]
+    body = body[:body.index("\n}\n")]
+    assert re.search(r"w\.sync\[0\] = w\.sync\[1\] = GroupSync\{0u, 0u, 0, 0\};", body)
+    run = text[text.index("cudaError_t run_wide("):]
+    assert run.index("wide_begin_kernel<<<") < run.index("wide_autotune(") < run.index("reduce_all(")
