@@ -1703,18 +1703,189 @@ __device__ __noinline__ void inverse_iteration(const double* d, const double* e,
   }
 }
 
+// Eigenvector of an isolated eigenvalue lam of the tridiagonal (d, e) by one twisted
+// factorisation (Parlett & Dhillon, "Fernando's solution to Wilkinson's problem", Linear
+// Algebra Appl. 267, 1997) and one step of inverse iteration with its factors, by a pair
+// of threads: T - lam = N_r D_r N_r^T with the pivots D+ from the top (thread `top`), D-
+// from the bottom (the other) and gamma_r = D+_r + D-_r - (d_r - lam) in the row r where
+// |gamma| is smallest.  N_r^T z = e_r (z_r = 1, z_{i-1} = -(e_{i-1} / D+_{i-1}) z_i upward
+// and z_{i+1} = -(e_i / D-_{i+1}) z_i downward) solves (T - lam) z = gamma_r e_r, which
+// leaves in z a part (error of lam) / gap of the neighbouring vectors, and so that much
+// overlap of two vectors: 5e-12 at 128 AOs, 4e-11 at 2400.  The second solve squares it:
+//   N_r y = z                 from both ends to r, where y_r = |z|^2,
+//   N_r^T x = gamma_r D_r^-1 y from r to both ends, x_r = y_r / |z|^2 (scaled to 1),
+// multiplied through by gamma_r, so that a gamma_r of zero needs no guard (x is z then).
+// With the reciprocals of the pivots kept, both sweeps are multiply-adds; the chain of
+// divides of the factorisation is the time.  (A Rayleigh quotient for lam and a second
+// factorisation instead made lam better but squared nothing: 4e-11 at 2400 AOs.)
+//   fac  five arrays `plane` apart: D+, then 1 / D and e / D (what couples a row to the next one
+//        towards r) from the top and from the bottom; x the vector, up to the factor returned;
+//        row i of each at [i * ld]
+//   pa, pb, pc  a word each that the pair shares
+// on: the pair has a column; every thread of the CTA calls (seven barriers).  Returns
+// 1 / |x| in the top thread, or 0 where gamma_r is larger than the rounding of lam
+// (limit) explains.  The lanes of a warp are at the same row in every sweep (their columns are
+// side by side), U rows at a time loaded before the first of them is worked on.
+template <int U>
+__device__ __forceinline__ double twisted_vector(const double* d, const double* e, int N, double lam, double tiny,
+                                                 double limit, bool on, bool top, double* __restrict__ fac,
+                                                 long long plane, double* __restrict__ x, int ld, double* pa, double* pb,
+                                                 double* pc) {
+  double* __restrict__ dp = fac;
+  double* __restrict__ rc = fac + (top ? 1 : 3) * plane;  // the thread's 1 / D and e / D
+  double* __restrict__ cl = rc + plane;
+  if (on) {
+    // step s: row s from the top, N - 1 - s from the bottom
+    const double* ep = top ? e : e + N - 2;
+    const double* np = top ? d + 1 : d + N - 2;
+    const int inc = top ? 1 : -1, step = inc * ld;
+    double D = (top ? d[0] : d[N - 1]) - lam;
+    int o = top ? 0 : (N - 1) * ld;
+#pragma unroll 4
+    for (int s = 0; s < N - 1; ++s, o += step, ep += inc, np += inc) {
+      const double ei = *ep, dn = *np - lam;
+      if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
+      const double q = 1.0 / D, l = ei * q;
+      if (top) dp[o] = D;
+      rc[o] = q;
+      cl[o] = l;
+      D = dn - ei * l;
+    }
+    if (top) dp[o] = D;
+  }
+  __syncthreads();
+  double best = INFINITY;  // the smallest gamma_i = D+_i - e_i (e_i / D-_{i+1}) of the thread's half of the rows
+  int at = 0;
+  if (on) {
+    const double* cb = fac + 4 * plane;
+    const int i0 = top ? 0 : N / 2, i1 = top ? N / 2 : N;
+#pragma unroll 8
+    for (int i = i0; i < i1; ++i) {
+      double g = dp[i * ld];
+      if (i < N - 1) g -= e[i] * cb[(i + 1) * ld];
+      if (fabs(g) < fabs(best)) {
+        best = g;
+        at = i;
+      }
+    }
+    if (!top) {
+      *pa = best;
+      *pb = (double)at;
+    }
+  }
+  __syncthreads();
+  if (on && top) {
+    if (fabs(*pa) < fabs(best))
+      best = *pa;
+    else
+      *pb = (double)at;
+  }
+  __syncthreads();
+  const int r = on ? (int)*pb : 0;
+  // Outward sweeps (from r to the thread's end) visit row N - 2 - s or s + 1 at step s and work from
+  // step s_out on, inward ones row s or N - 1 - s before step s_in.
+  const int s_out = top ? N - 1 - r : r, s_in = top ? r : N - 1 - r;
+  const int o_out = top ? (N - 2) * ld : ld, o_in = top ? 0 : (N - 1) * ld, away = top ? -ld : ld;
+  double nrm = top ? 1.0 : 0.0;
+  if (on) {
+    double z = 1.0;
+    if (top) x[r * ld] = 1.0;
+    auto row = [&](bool act, int o, double l) {
+      if (act) {
+        z *= -l;
+        x[o] = z;
+        nrm = fma(z, z, nrm);
+      }
+    };
+    int s = 0, o = o_out;
+    for (; s + U <= N - 1; s += U, o += U * away) {
+      double lv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) lv[q] = cl[o + q * away];
+#pragma unroll
+      for (int q = 0; q < U; ++q) row(s + q >= s_out, o + q * away, lv[q]);
+    }
+    for (; s < N - 1; ++s, o += away) row(s >= s_out, o, cl[o]);
+    if (!top) *pc = nrm;
+  }
+  __syncthreads();
+  bool good = false;
+  double w = 0.0, g = 0.0;
+  if (on && top) {
+    nrm += *pc;
+    good = fabs(best) <= limit * nrm && nrm < 1e200;
+    w = 1.0 / nrm;
+    g = best * w;
+    *pa = g;
+    *pb = w;
+  }
+  __syncthreads();
+  if (on) {
+    if (!top) {  // (the top thread does not look at pa again before its partner writes it)
+      g = *pa;
+      w = *pb;
+    }
+    double y = 0.0, l = 0.0;  // of the row before, and what couples it to this one
+    auto row = [&](bool act, int o, double zi, double li, double ri) {
+      if (act) {
+        y = fma(-l, y, zi);
+        l = li;
+        x[o] = (g * ri) * y;
+      }
+    };
+    int s = 0, o = o_in;
+    for (; s + U <= N - 1; s += U, o -= U * away) {
+      double xv[U], lv[U], rv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        xv[q] = x[o - q * away];
+        lv[q] = cl[o - q * away];
+        rv[q] = rc[o - q * away];
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q) row(s + q < s_in, o - q * away, xv[q], lv[q], rv[q]);
+    }
+    for (; s < N - 1; ++s, o -= away) row(s < s_in, o, x[o], cl[o], rc[o]);
+    *(top ? pc : pa) = l * y;
+  }
+  __syncthreads();
+  if (on) {
+    double v = w * ((1.0 - *pc) - *pa);
+    nrm = top ? v * v : 0.0;
+    if (top) x[r * ld] = v;
+    auto row = [&](bool act, int o, double wi, double li) {
+      if (act) {
+        v = fma(-li, v, wi);
+        x[o] = v;
+        nrm = fma(v, v, nrm);
+      }
+    };
+    int s = 0, o = o_out;
+    for (; s + U <= N - 1; s += U, o += U * away) {
+      double xv[U], lv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        xv[q] = x[o + q * away];
+        lv[q] = cl[o + q * away];
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q) row(s + q >= s_out, o + q * away, xv[q], lv[q]);
+    }
+    for (; s < N - 1; ++s, o += away) row(s >= s_out, o, x[o], cl[o]);
+    if (!top) *pb = nrm;
+  }
+  __syncthreads();
+  if (!on || !top || !good) return 0.0;
+  nrm += *pb;
+  return nrm > 0.0 && nrm < 1e300 ? 1.0 / sqrt(nrm) : 0.0;
+}
+
 // (6) occupied eigenvectors of the tridiagonal, columns of Z up to the factors
-// scale[j] (in v.pop).  An isolated eigenvalue takes one twisted factorisation
-// (Parlett & Dhillon, "Fernando's solution to Wilkinson's problem", Linear
-// Algebra Appl. 267, 1997): T - lam = L D+ L^T from the top by one thread,
-// U D- U^T from the bottom by another, joined at the row r where
-// |gamma_r| = |D+_r + D-_r - (d_r - lam)| is smallest; z_r = 1 and
-// z_{i-1} = -(e_{i-1} / D+_{i-1}) z_i upward, z_{i+1} = -(e_i / D-_{i+1}) z_i
-// downward solve (T - lam) z = gamma_r e_r.  Both pivot chains are a divide per
-// row; inverse iteration needs a pivoted factorisation and two solves, five
-// dependent passes (147k cycles at N = 128 against 30k here).  Its residual
-// gamma_r / |z| is about the error of lam times |z|; a column where it is larger
-// than rounding explains, and clusters, fall back to inverse iteration.
+// scale[j] (in v.pop): twisted_vector for the eigenvalues farther than 1e-5 |T|_1 from
+// their neighbours, a pair of threads each; clusters, and a column that it does not
+// settle, by inverse iteration (a pivoted factorisation and two solves, five dependent
+// passes over global memory, 147k cycles at N = 128, against 30k for the twisted
+// factorisation with its first solve; the second solve adds 1% to the SCC at 128 AOs).
 template <int KIND>
 __device__ __noinline__ void scc_vectors(const SccArgs& A) {
   constexpr int NT = kSccKinds[KIND].nt, HALF = NT / 2;
@@ -1722,8 +1893,7 @@ __device__ __noinline__ void scc_vectors(const SccArgs& A) {
   const int tid = threadIdx.x, N = v.s.N, ld = v.s.ld, nocc = v.s.nocc;
   const double *d = v.d, *e = v.e, *eps = v.eps;
   const double onenrm = v.s.onenrm, ortol = 1e-5 * onenrm, tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
-  double* __restrict__ Z = v.w.Z;
-  double *gam = v.pop, *twist = v.esq;  // per column: |gamma|, then the squared norm, then the scale; the row r
+  double* Z = v.w.Z;
   const long long n2 = (long long)ld * ld;
   const bool top = tid < HALF;
   for (int j0 = 0; j0 < nocc; j0 += HALF) {
@@ -1731,102 +1901,18 @@ __device__ __noinline__ void scc_vectors(const SccArgs& A) {
     const bool col = j < nocc;
     const bool first = col && (j == 0 || eps[j] - eps[j - 1] > ortol);
     const bool single = first && (j + 1 >= nocc || eps[j + 1] - eps[j] > ortol);
-    const double lam = col ? eps[j] : 0.0;
-    double* dp = v.w.iw + (col ? j : 0);  // D+_i
-    double* lp = dp + n2;                 // e_i / D+_i
-    double* um = dp + 2 * n2;             // e_i / D-_{i+1}
-    if (single) {
-      if (top) {
-        double D = d[0] - lam;
-#pragma unroll 4
-        for (int i = 0; i < N - 1; ++i) {
-          const double ei = e[i], dn = d[i + 1] - lam;
-          if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
-          const double l = ei * (1.0 / D);
-          dp[(long long)i * ld] = D;
-          lp[(long long)i * ld] = l;
-          D = dn - ei * l;
-        }
-        dp[(long long)(N - 1) * ld] = D;
-      } else {
-        double D = d[N - 1] - lam;
-#pragma unroll 4
-        for (int i = N - 2; i >= 0; --i) {
-          const double ei = e[i], dn = d[i] - lam;
-          if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
-          const double u = ei * (1.0 / D);
-          um[(long long)i * ld] = u;
-          D = dn - ei * u;
-        }
-      }
-    }
-    __syncthreads();
-    double best = INFINITY;
-    int at = 0;
-    if (single) {  // smallest |gamma_i| = |D+_i - e_i u_i| over the thread's half of the rows
-      const int i0 = top ? 0 : N / 2, i1 = top ? N / 2 : N;
-#pragma unroll 4
-      for (int i = i0; i < i1; ++i) {
-        const double gi = fabs(dp[(long long)i * ld] - (i < N - 1 ? e[i] * um[(long long)i * ld] : 0.0));
-        if (gi < best) {
-          best = gi;
-          at = i;
-        }
-      }
-      if (!top) {
-        gam[j] = best;
-        twist[j] = (double)at;
-      }
-    }
-    __syncthreads();
-    if (single && top) {
-      if (!(gam[j] < best)) twist[j] = (double)at;
-      best = fmin(best, gam[j]);
-    }
-    __syncthreads();
-    double nrm = 0.0;
-    if (single) {
-      const int r = (int)twist[j];
-      double z = 1.0;
-      double* x = Z + j;
-      if (top) {
-        nrm = 1.0;
-        x[(long long)r * ld] = 1.0;
-#pragma unroll 8
-        for (int i = N - 2; i >= 0; --i) {
-          const double l = lp[(long long)i * ld];
-          if (i < r) {
-            z *= -l;
-            x[(long long)i * ld] = z;
-            nrm += z * z;
-          }
-        }
-      } else {
-#pragma unroll 8
-        for (int i = 0; i < N - 1; ++i) {
-          const double u = um[(long long)i * ld];
-          if (i >= r) {
-            z *= -u;
-            x[(long long)(i + 1) * ld] = z;
-            nrm += z * z;
-          }
-        }
-        gam[j] = nrm;
-      }
-    }
-    __syncthreads();
+    const int jc = col ? j : 0;
+    // (tau and e^2 have served; the words are the pair's)
+    const double scale = twisted_vector<8>(d, e, N, eps[jc], tiny, 64.0 * DBL_EPSILON * onenrm, single, top, v.w.iw + jc,
+                                           n2, Z + jc, ld, v.pop + jc, v.esq + jc, v.tau + jc);
     if (top && first) {
-      bool good = false;
-      if (single) {
-        nrm += gam[j];
-        good = best <= 64.0 * DBL_EPSILON * onenrm * nrm && nrm < 1e200;
-        if (good) gam[j] = 1.0 / sqrt(nrm);
-      }
-      if (!good) {
+      if (scale > 0.0) {
+        v.pop[j] = scale;
+      } else {
         int jend = j + 1;
         while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
         inverse_iteration(d, e, N, ld, eps, j, jend, onenrm, v.w.iw, Z);
-        for (int q = j; q < jend; ++q) gam[q] = 1.0;
+        for (int q = j; q < jend; ++q) v.pop[q] = 1.0;
       }
     }
     __syncthreads();
