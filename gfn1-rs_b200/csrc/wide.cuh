@@ -1314,171 +1314,51 @@ __global__ void __launch_bounds__(kWideNT, 1) wide_fermi_kernel(WideCtx X) {
 }
 
 // (6) occupied eigenvectors of the tridiagonal, columns of Z up to the factors in
-// w.esq: the twisted factorisation of scc_vectors for the eigenvalues farther than
-// kTwistGap |T|_1 from their neighbours, 32 a CTA, one warp's lanes from the top and
-// the other's from the bottom; inverse iteration for the rest.  The error of lam over
-// the gap is that of the vector: where it would exceed 1e-12, lam takes its Rayleigh
-// quotient gamma_r / |z|^2 and the factorisation runs once more.  The chain of divides
-// is the time (110 cycles a row); the pivoted factorisation and two solves that it
-// replaces took 3.7 ms at 2400 AOs.
+// w.esq: twisted_vector for the eigenvalues farther than kTwistGap |T|_1 from their
+// neighbours, 32 a CTA, one warp's lanes from the top and the other's from the bottom;
+// inverse iteration for the rest.  The chain of divides is the time (110 cycles a row); a
+// Rayleigh quotient and a second factorisation in the place of the second solve took 10.7 ms
+// for the nine iterations at 2400 AOs, this 8.0 (16 rows loaded at a time; 10.1 with 8), and two
+// pivoted inverse iterations 40.3.
 constexpr double kTwistGap = 1e-9;
 __global__ void __launch_bounds__(64) wide_vectors_kernel(WideCtx X, int* stats) {
-  __shared__ double gam[32], other[32], lams[32];
-  __shared__ int twist[32];
-  constexpr int U = 8;  // rows whose operands are loaded together
+  __shared__ double pair[3][32];
   const WideMol& w = X.mols[X.act[blockIdx.y]];
   const WideState* st = w.st;
   if (st->status != kOk) return;
   const int N = w.N, nocc = st->nocc, lane = threadIdx.x & 31;
   if (32 * (int)blockIdx.x >= nocc) return;
-  const long long ld = w.ld, n2 = ld * N;
+  const int ld = w.ld;
   const bool top = threadIdx.x < 32;
   const int j = blockIdx.x * 32 + lane;
   const bool col = j < nocc;
   const double *__restrict__ d = w.d, *__restrict__ e = w.e, *eps = w.eps;
   const double onenrm = st->onenrm, ortol = kTwistGap * onenrm, tiny = DBL_EPSILON * fmax(onenrm, 1e-300);
-  const double below = col && j > 0 ? eps[j] - eps[j - 1] : INFINITY;
-  const double above = col && j + 1 < nocc ? eps[j + 1] - eps[j] : INFINITY;
-  const bool first = col && below > ortol;
-  const bool single = first && above > ortol;
-  double lam = col ? eps[j] : 0.0, best = INFINITY, nrm = 0.0;
-  double* __restrict__ dp = w.iw + (col ? j : 0);  // D+_i
-  double* __restrict__ lp = dp + n2;               // e_i / D+_i
-  double* __restrict__ um = dp + 2 * n2;           // e_i / D-_{i+1}
-  bool again = single;
-  for (int pass = 0;; ++pass) {
-    if (again) {
-      double D = (top ? d[0] : d[N - 1]) - lam;
-      for (int k0 = 0; k0 < N - 1; k0 += U) {  // step k: row k from the top, N - 2 - k from the bottom
-        double ev[U], dn[U];
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-          const int k = min(k0 + q, N - 2), i = top ? k : N - 2 - k;
-          ev[q] = e[i];
-          dn[q] = d[top ? i + 1 : i] - lam;
-        }
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-          const int k = k0 + q;
-          if (k < N - 1) {
-            if (fabs(D) < tiny) D = D >= 0.0 ? tiny : -tiny;
-            const double l = ev[q] * (1.0 / D);
-            if (top) {
-              dp[k * ld] = D;
-              lp[k * ld] = l;
-            } else {
-              um[(N - 2 - k) * ld] = l;
-            }
-            D = dn[q] - ev[q] * l;
-          }
-        }
-      }
-      if (top) dp[(N - 1) * ld] = D;
-    }
-    __syncthreads();
-    int at = 0;
-    double mine = INFINITY;  // the smallest gamma_i = D+_i - e_i u_i of the thread's half of the rows
-    if (again) {
-      const int i0 = top ? 0 : N / 2, i1 = top ? N / 2 : N;
-      for (int b = i0; b < i1; b += 2 * U) {
-        double g[2 * U];
-#pragma unroll
-        for (int q = 0; q < 2 * U; ++q) {
-          const int i = min(b + q, i1 - 1), u = min(i, N - 2);
-          g[q] = dp[i * ld] - (i < N - 1 ? e[u] * um[u * ld] : 0.0);
-        }
-#pragma unroll
-        for (int q = 0; q < 2 * U; ++q)
-          if (b + q < i1 && fabs(g[q]) < fabs(mine)) {
-            mine = g[q];
-            at = b + q;
-          }
-      }
-      if (!top) {
-        gam[lane] = mine;
-        twist[lane] = at;
-      }
-    }
-    __syncthreads();
-    if (again && top) {
-      if (fabs(gam[lane]) < fabs(mine))
-        mine = gam[lane];
-      else
-        twist[lane] = at;
-      best = mine;
-    }
-    __syncthreads();
-    if (again) {
-      const int r = twist[lane];
-      double z = 1.0;
-      double* __restrict__ x = w.Z + j;
-      nrm = 0.0;
-      if (top) {
-        nrm = 1.0;
-        x[r * ld] = 1.0;
-        for (int b = N - 2; b >= 0; b -= 2 * U) {
-          double l[2 * U];
-#pragma unroll
-          for (int q = 0; q < 2 * U; ++q) l[q] = lp[max(b - q, 0) * ld];
-#pragma unroll
-          for (int q = 0; q < 2 * U; ++q)
-            if (b - q >= 0 && b - q < r) {
-              z *= -l[q];
-              x[(b - q) * ld] = z;
-              nrm += z * z;
-            }
-        }
-      } else {
-        for (int b = 0; b < N - 1; b += 2 * U) {
-          double u[2 * U];
-#pragma unroll
-          for (int q = 0; q < 2 * U; ++q) u[q] = um[min(b + q, N - 2) * ld];
-#pragma unroll
-          for (int q = 0; q < 2 * U; ++q)
-            if (b + q < N - 1 && b + q >= r) {
-              z *= -u[q];
-              x[(b + q + 1) * ld] = z;
-              nrm += z * z;
-            }
-        }
-        other[lane] = nrm;
-      }
-    }
-    __syncthreads();
-    if (again && top) {
-      nrm += other[lane];
-      const double shift = best / nrm;  // of lam to its Rayleigh quotient
-      again = fabs(shift) > 1e-12 * fmin(below, above) && fabs(shift) < 0.5 * fmin(below, above);
-      lam += again ? shift : 0.0;
-      lams[lane] = again ? lam : INFINITY;
-    } else if (top) {
-      lams[lane] = INFINITY;
-    }
-    __syncthreads();
-    if (!top) again = lams[lane] < INFINITY;
-    if (!top && again) lam = lams[lane];
-    if (pass == 1 || !__syncthreads_or(again)) break;
-  }
+  const bool first = col && (j == 0 || eps[j] - eps[j - 1] > ortol);
+  const bool single = first && (j + 1 >= nocc || eps[j + 1] - eps[j] > ortol);
+  const int jc = col ? j : 0;
+  const double good = twisted_vector<16>(d, e, N, eps[jc], tiny, 64.0 * DBL_EPSILON * onenrm, single, top, w.iw + jc,
+                                         (long long)N * ld, w.Z + jc, ld, &pair[0][lane], &pair[1][lane], &pair[2][lane]);
   if (top && first) {
     double* scale = w.esq;
-    const bool good = single && fabs(best) <= 64.0 * DBL_EPSILON * onenrm * nrm && nrm < 1e200;
-    if (good) scale[j] = 1.0 / sqrt(nrm);
-    if (!good) {
+    if (good > 0.0) {
+      scale[j] = good;
+    } else {
       int jend = j + 1;
       while (jend < nocc && eps[jend] - eps[jend - 1] <= ortol) ++jend;
       if (stats) {
         atomicMax(stats, jend - j);
         if (jend - j > 1) atomicAdd(stats + 1, 1);
       }
-      inverse_iteration(d, e, N, (int)ld, eps, j, jend, onenrm, w.iw, w.Z);
+      inverse_iteration(d, e, N, ld, eps, j, jend, onenrm, w.iw, w.Z);
       for (int q = j; q < jend; ++q) scale[q] = 1.0;
     }
   }
 }
 
 // Modified Gram-Schmidt of the vectors whose eigenvalues are closer than ortol: those
-// of wide_vectors_kernel span the right space (they may overlap by the error of lam
-// over the gap).  The warp's lanes look for the first of a chain, then share its rows.
+// of wide_vectors_kernel span the right space (they may overlap by eps |T| over the gap).
+// The warp's lanes look for the first of a chain, then share its rows.
 __device__ __forceinline__ void orthogonalise_chains(const WideMol& w, int j0, double ortol) {
   const int N = w.N, nocc = w.st->nocc, lane = threadIdx.x & 31;
   const long long ld = w.ld;

@@ -24,9 +24,30 @@ def _defect(calc, z, x):
     return np.abs(P @ S @ P - 2.0 * P).max()
 
 
-@pytest.mark.parametrize("waters, tolerance", [(1, 1e-13), (3, 1e-13), (8, 1e-13), (12, 1e-13), (16, 1e-13), (24, 1e-13)])
+@pytest.mark.parametrize("waters, tolerance", [(1, 1e-13), (3, 1e-13), (8, 1e-13), (12, 1e-13), (16, 1e-13), (24, 1e-13),
+                                                (64, 1e-12), (96, 1e-12), (100, 1e-12), (300, 1e-11)])
 def test_density_is_idempotent(waters, tolerance):
     from gfn1_rs import BatchCalculator, workloads
     z, x = workloads.water_cluster(waters, 1)
     calc = BatchCalculator(electronic_temperature=0.0, energy_tolerance=1e-8, charge_tolerance=1e-6)
     assert _defect(calc, np.asarray(z, dtype=np.uint8), x * A2B) <= tolerance
+
+
+# Dipoles (e bohr) of converged clusters from two pivoted inverse iterations a vector, 11 SCC iterations.
+PIVOTED = {
+    64: (-5.0507841532555195, -2.5011513752365238, -2.242295170734069),
+    96: (-1.0689928934077546, 5.421291680811105, -4.97470914740497),
+    300: (-9.431410176973088, -0.3492062994294059, -8.125087326047243),
+}
+
+
+@pytest.mark.parametrize("waters, tolerance", [(64, 1e-12), (96, 2e-12), (300, 2e-11)])
+def test_dipole_is_that_of_two_pivoted_solves(waters, tolerance):
+    """The charges take the overlap of the orbitals and the SCC's response multiplies it by about ten, so
+    two sets of vectors as orthogonal as above (1e-13, 1e-13, 1e-12) agree in the dipole to ten times that."""
+    from gfn1_rs import BatchCalculator, workloads
+    z, x = workloads.water_cluster(waters, 1)
+    r = BatchCalculator(energy_tolerance=1e-8, charge_tolerance=1e-7).calculate_flat([0, len(z)], z, x * A2B)
+    want = np.array(PIVOTED[waters])
+    assert r.status[0] == 0 and r.iterations[0] == 11
+    assert np.abs(r.dipole[0] - want).max() <= tolerance * np.linalg.norm(want)
