@@ -27,6 +27,7 @@
 namespace gfn1 {
 cudaError_t launch_setup(int max_l, int n, int max_nat, int max_nsh, bool halogens, int num_sms, cudaStream_t st,
                          const Batch& B, const Model& M, int enable_dispersion, const int* mols);
+int setup_max_atoms(size_t smem);
 int setup_launches(int n, int max_nat, bool halogens, int num_sms);
 int grad_launches(int n, int max_nat, int num_sms);
 cudaError_t launch_grad(int max_l, int n, int max_nat, int num_sms, cudaStream_t st, const Batch& B, const Model& M,
@@ -257,6 +258,7 @@ struct gfn1_guess {
 struct gfn1_engine {
   int device = 0;
   int num_sms = 148;
+  int max_atoms = 0;  // of a molecule: what the set-up kernel's shared memory holds
   std::string error;
   ElemTable elem[kNZ];
   bool device_ok[kNZ];
@@ -717,6 +719,12 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
       st = GFN1_E_INVALID_INPUT;
       if (first_err.empty()) first_err = "molecule " + std::to_string(m) + ": invalid electron count";
     }
+    if (st == GFN1_OK && a1 - a0 > eng->max_atoms) {
+      st = GFN1_E_INVALID_INPUT;
+      if (first_err.empty())
+        first_err = "molecule " + std::to_string(m) + ": " + std::to_string(a1 - a0) + " atoms, the device path takes at most " +
+                    std::to_string(eng->max_atoms);
+    }
     if (st == GFN1_OK) {
       const std::string se = spin_multiplicity_error(o.spin_multiplicity, nelec, n);
       if (!se.empty()) {
@@ -733,7 +741,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
     mat_total += (((long long)n * n + 31) / 32) * 32;
     gam_total += (long long)s * s;
     pair_total += (long long)(a1 - a0) * (a1 - a0 - 1) / 2;
-    b->max_nat = std::max(b->max_nat, a1 - a0);
+    if (st == GFN1_OK) b->max_nat = std::max(b->max_nat, a1 - a0);  // (the kernels skip the others)
     b->max_nsh = std::max(b->max_nsh, s);
     b->max_n = std::max(b->max_n, n);
   }
@@ -1219,6 +1227,9 @@ int gfn1_engine_create(const char* param_spec, int device, gfn1_engine** out) {
     return cuda_fail(nullptr, e, "cudaSetDevice");
   }
   cudaDeviceGetAttribute(&eng->num_sms, cudaDevAttrMultiProcessorCount, device);
+  int smem_max = 0;
+  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  eng->max_atoms = setup_max_atoms((size_t)smem_max);
   if ((e = cudaMalloc(&eng->d_elem, sizeof(ElemTable) * kNZ)) != cudaSuccess ||
       (e = cudaMalloc(&eng->d_pair, sizeof(double) * eng->pair_scaling.size())) != cudaSuccess ||
       (e = cudaMalloc(&eng->d_c6, sizeof(double) * eng->c6ref.size())) != cudaSuccess ||

@@ -215,22 +215,28 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
   // the warp's atoms: all of them in one CTA, or shared by the CTAs of the phase
   const int part = all ? 0 : (split >= pair_parts ? split - pair_parts : split);
   const int at0 = part * nw + wid, atn = all ? nw : (nsplit > pair_parts ? nsplit - pair_parts : nsplit) * nw;
+  // Shared memory bounds the size of a molecule (setup_max_atoms), so what is not needed at the same
+  // time shares its words: the coordination numbers serve until the weights are formed, dE/dCN and the
+  // repulsion energies come after them; the tables of the shell pairs stand where the weights come.
   double* xyz = smem;                    // 3*max_nat
   double* cn = xyz + 3 * max_nat;        // max_nat
   double* cnd = cn + max_nat;            // max_nat
-  double* dedcn = cnd + max_nat;         // max_nat
-  double* eat = dedcn + max_nat;         // 2*max_nat: repulsion and dispersion energy of each atom
-  double* gw = eat + 2 * max_nat;        // kMaxRef*max_nat
+  double* dedcn = cn;
+  double* erep = cnd;                    // repulsion and dispersion energy of each atom
+  double* edis = cnd + max_nat;          // max_nat
+  double* gw = edis + max_nat;           // kMaxRef*max_nat
   double* dgw = gw + kMaxRef * max_nat;  // kMaxRef*max_nat
-  double* se = dgw + kMaxRef * max_nat;  // max_nsh
-  int* zs = (int*)(se + max_nsh);        // max_nat
+  int* zs = (int*)(dgw + kMaxRef * max_nat);  // max_nat
   int* atom_sh = zs + max_nat;           // max_nat+1
   int* atom_ao = atom_sh + max_nat + 1;  // max_nat+1
-  int* sh_atom = atom_ao + max_nat + 1;  // max_nsh
+  int* lcount = atom_ao + max_nat + 1;   // 3
+  static_assert(2 * kMaxRef * sizeof(double) >= kMaxShAtom * (sizeof(double) + 4 * sizeof(int)),
+                "the pair tables stand where the weights come");
+  double* se = gw;                       // max_nsh
+  int* sh_atom = (int*)(se + max_nsh);   // max_nsh
   int* sh_k = sh_atom + max_nsh;         // max_nsh
   int* ord = sh_k + max_nsh;             // max_nsh
   int* key = ord + max_nsh;              // max_nsh
-  int* lcount = key + max_nsh;           // 3
 
   for (int i = tid; i < nat; i += nt) {
     zs[i] = B.z[a0 + i];
@@ -328,6 +334,7 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
   }
 
   if (do_classic) {
+    if (do_pairs) __syncthreads();  // the pair tables have served
     if (enable_dispersion) {
       for (int i = tid; i < nat; i += nt) {  // reference weights, src/dispersion.rs:1629-1692
         const ElemTable& e = M.elem[zs[i]];
@@ -419,8 +426,8 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
         B.grad_classic[3 * (a0 + i) + 1] = gy;
         B.grad_classic[3 * (a0 + i) + 2] = gz;
         dedcn[i] = dc;
-        eat[2 * i] = er;
-        eat[2 * i + 1] = ed;
+        erep[i] = er;
+        edis[i] = ed;
         if (!all) {
           B.atom_tmp[4 * (a0 + i) + 1] = dc;
           B.atom_tmp[4 * (a0 + i) + 2] = er;
@@ -435,8 +442,8 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
     if (!all) {
       for (int i = tid; i < nat; i += nt) {
         dedcn[i] = B.atom_tmp[4 * (a0 + i) + 1];
-        eat[2 * i] = B.atom_tmp[4 * (a0 + i) + 2];
-        eat[2 * i + 1] = B.atom_tmp[4 * (a0 + i) + 3];
+        erep[i] = B.atom_tmp[4 * (a0 + i) + 2];
+        edis[i] = B.atom_tmp[4 * (a0 + i) + 3];
       }
       __syncthreads();
     }
@@ -470,8 +477,8 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
     if (part == 0 && wid == 0) {
       double er = 0.0, ed = 0.0;
       for (int i = lane; i < nat; i += 32) {
-        er += eat[2 * i];
-        ed += eat[2 * i + 1];
+        er += erep[i];
+        ed += edis[i];
       }
       er = warp_sum(er);
       ed = warp_sum(ed);
@@ -490,8 +497,15 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
     B.terms[(long long)m * kTerms + 8] = halogen_term(M, zs, xyz, nat, B.grad_classic + 3LL * a0);
 }
 
-size_t setup_smem_bytes(int max_nat, int max_nsh) {
-  return sizeof(double) * (18 * (size_t)max_nat + max_nsh) + sizeof(int) * (3 * (size_t)max_nat + 2 + 4 * (size_t)max_nsh + 4);
+// 140 bytes an atom: 1660 atoms in the 227 KB of a CTA.
+size_t setup_smem_bytes(int max_nat) {
+  return sizeof(double) * (6 + 2 * kMaxRef) * (size_t)max_nat + sizeof(int) * (3 * (size_t)max_nat + 2 + 4);
+}
+// Atoms of the largest molecule whose set-up fits `smem` bytes of shared memory.
+int setup_max_atoms(size_t smem) {
+  int n = (int)(smem / (sizeof(double) * (6 + 2 * kMaxRef) + 3 * sizeof(int)));
+  while (n > 0 && setup_smem_bytes(n) > smem) --n;
+  return n;
 }
 
 // Launches the setup of `n` molecules (`mols`, or the batch when null) whose
@@ -509,7 +523,7 @@ int setup_launches(int n, int max_nat, bool halogens, int num_sms) {
 }
 cudaError_t launch_setup(int max_l, int n, int max_nat, int max_nsh, bool halogens, int num_sms, cudaStream_t st,
                          const Batch& B, const Model& M, int enable_dispersion, const int* mols) {
-  const size_t smem = setup_smem_bytes(max_nat, max_nsh);
+  const size_t smem = setup_smem_bytes(max_nat);
   const bool few = n < 4 * num_sms;
   auto* k = max_l >= 2 ? (few ? setup_kernel<2, 8> : setup_kernel<2, 1>) : (few ? setup_kernel<1, 8> : setup_kernel<1, 1>);
   if (smem > 48 * 1024) {
