@@ -1882,6 +1882,7 @@ struct WideRuntime {
   std::vector<WideMol> mols;  // host copies of the slot descriptors
   WideMol* d_mols = nullptr;
   int* d_act = nullptr;
+  int* d_all = nullptr;  // all slots, in order
   int* h_act = nullptr;
   WideState* d_state = nullptr;
   WideState* h_state = nullptr;
@@ -2319,8 +2320,9 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     }
   }
   // ---- results for every slot: P, W of the last diagonalisation, energies, charges
-  for (int q = 0; q < nslots; ++q) R.h_act[q] = q;
-  if ((e = upload_act(nslots)) != cudaSuccess) return e;
+  // (the list of all slots that wide_bind uploaded: a copy from h_act made here would still be under
+  // way when the next run sorts its own list there)
+  X.act = R.d_all;
   wide_pw_kernel<<<dim3(gx(mt, nslots), nslots), kGemmNT, tsm, st>>>(B, X);
   wide_results_kernel<<<nslots, kWideNT, rsm, st>>>(B, M, X);
   tm.mark("final");
@@ -2348,6 +2350,7 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
   if (n > R.capacity) {
     if (R.d_mols) cudaFree(R.d_mols);
     if (R.d_act) cudaFree(R.d_act);
+    if (R.d_all) cudaFree(R.d_all);
     if (R.d_state) cudaFree(R.d_state);
     if (R.d_sync) cudaFree(R.d_sync);
     if (R.d_flags) cudaFree(R.d_flags);
@@ -2356,6 +2359,7 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
     R.d_flags = nullptr;
     R.d_mols = nullptr;
     R.d_act = nullptr;
+    R.d_all = nullptr;
     R.d_state = nullptr;
     R.d_sync = nullptr;
     R.h_act = nullptr;
@@ -2363,6 +2367,7 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
     R.capacity = 0;
     if ((e = cudaMalloc(&R.d_mols, sizeof(WideMol) * n)) != cudaSuccess ||
         (e = cudaMalloc(&R.d_act, sizeof(int) * n)) != cudaSuccess ||
+        (e = cudaMalloc(&R.d_all, sizeof(int) * n)) != cudaSuccess ||
         (e = cudaMalloc(&R.d_state, sizeof(WideState) * n)) != cudaSuccess ||
         (e = cudaMalloc(&R.d_sync, sizeof(GroupSync) * 2 * n)) != cudaSuccess ||
         (e = cudaMalloc(&R.d_flags, sizeof(unsigned long long) * 2 * kFlagSlots * n)) != cudaSuccess ||
@@ -2372,10 +2377,12 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
     R.capacity = n;
   }
   R.mols.resize(n);
+  std::vector<int> all(n);
   for (int q = 0; q < n; ++q) {
     const WideSlotLayout s = wide_slot_layout(Ns[q], nshs[q], nats[q], cap);
     double* p = base + slot_off[q];
     WideMol& w = R.mols[q];
+    all[q] = q;
     w.m = ids[q];
     w.N = Ns[q];
     w.ld = s.ld;
@@ -2408,6 +2415,7 @@ cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::ve
     w.flags = R.d_flags + (size_t)2 * kFlagSlots * q;
   }
   if ((e = cudaMemcpy(R.d_mols, R.mols.data(), sizeof(WideMol) * n, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+  if ((e = cudaMemcpy(R.d_all, all.data(), sizeof(int) * n, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
   if ((e = cudaMemset(R.d_sync, 0, sizeof(GroupSync) * 2 * n)) != cudaSuccess) return e;
   if ((e = cudaMemset(R.d_flags, 0, sizeof(unsigned long long) * 2 * kFlagSlots * n)) != cudaSuccess) return e;
   return cudaMemset(R.d_state, 0, sizeof(WideState) * n);
@@ -2418,6 +2426,7 @@ void wide_release(WideRuntime& R) {
   if (R.d_flags) cudaFree(R.d_flags);
   if (R.d_mols) cudaFree(R.d_mols);
   if (R.d_act) cudaFree(R.d_act);
+  if (R.d_all) cudaFree(R.d_all);
   if (R.d_state) cudaFree(R.d_state);
   if (R.d_sync) cudaFree(R.d_sync);
   if (R.h_act) cudaFreeHost(R.h_act);

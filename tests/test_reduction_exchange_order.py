@@ -78,3 +78,16 @@ def test_every_run_starts_with_clear_error_flags():
     assert re.search(r"w\.sync\[0\] = w\.sync\[1\] = GroupSync\{0u, 0u, 0, 0\};", body)
     run = text[text.index("cudaError_t run_wide("):]
     assert run.index("wide_begin_kernel<<<") < run.index("wide_autotune(") < run.index("reduce_all(")
+
+
+def test_no_list_is_uploaded_that_the_run_does_not_wait_for():
+    """The lists of active slots are copied from one pinned array that the next run sorts anew; a run that
+    returns right after such a copy would leave it to be read half sorted.  So the copies of run_wide stand
+    before its last synchronisation, and the kernels after it take the list that the binding uploaded."""
+    text = _source("wide.cuh")
+    run = text[text.index("cudaError_t run_wide("):]
+    run = run[:run.index("\n}\n")]
+    last = run.rindex("wide_read_states(")
+    tail = run[run.index("wide_pw_kernel<<<") - 200:]
+    assert "upload_act(" not in tail and "X.act = R.d_all" in tail
+    assert run.index("X.act = R.d_all") > last
