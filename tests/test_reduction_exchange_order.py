@@ -81,13 +81,12 @@ def test_every_run_starts_with_clear_error_flags():
 
 
 def test_no_list_is_uploaded_that_the_run_does_not_wait_for():
-    """The lists of active slots are copied from one pinned array that the next run sorts anew; a run that
-    returns right after such a copy would leave it to be read half sorted.  So the copies of run_wide stand
-    before its last synchronisation, and the kernels after it take the list that the binding uploaded."""
+    """The lists of active slots are copied from one pinned array that the next run sorts anew; a list whose
+    copy is still under way when run_wide returns may be read half sorted.  So the kernels that write the
+    results, after the last synchronisation, take the list that the binding of the slots uploaded."""
     text = _source("wide.cuh")
     run = text[text.index("cudaError_t run_wide("):]
     run = run[:run.index("\n}\n")]
-    last = run.rindex("wide_read_states(")
-    tail = run[run.index("wide_pw_kernel<<<") - 200:]
-    assert "upload_act(" not in tail and "X.act = R.d_all" in tail
-    assert run.index("X.act = R.d_all") > last
+    results = run[run.index("X.act = R.d_all"):]
+    assert "upload_act(" not in results and "wide_pw_kernel<<<" in results and "wide_results_kernel<<<" in results
+    assert "wide_pw_kernel<<<" not in run[:run.index("X.act = R.d_all")]
