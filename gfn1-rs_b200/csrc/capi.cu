@@ -48,8 +48,8 @@ cudaError_t wide_bind_runtime(WideRuntime* r, const std::vector<int>& ids, const
                               const std::vector<long long>& mos, const std::vector<int>& nshs,
                               const std::vector<int>& nats, int cap, double* base,
                               const std::vector<long long>& slot_off);
-cudaError_t wide_run(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime* r, int nslots, int maxn,
-                     int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st);
+cudaError_t wide_run(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime* r, int first, int nslots,
+                     int maxn, int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st);
 void wide_plan_info(const WideRuntime* r, int* nb, int* min_rows, int* group, float* ms, int* tuned);
 size_t dense_table_bytes_host(int maxnsh, int maxn, int maxnat);
 }  // namespace gfn1
@@ -334,6 +334,10 @@ struct gfn1_batch {
   std::vector<int> wide_ids;
   int n_dense = 0;  // leading entries of the processing order above the threshold (their setup and gradient split over CTAs)
   int wide_maxn = 0, wide_maxnsh = 0, wide_maxnat = 0;
+  struct WideGroup {  // molecules of wide_ids that run together
+    int first = 0, count = 0, maxn = 0;
+  };
+  std::vector<WideGroup> wide_groups;
   WideRuntime* wide = nullptr;
   DevBuf<double> wide_buf;
   BlobLayout lay;
@@ -664,6 +668,19 @@ int dense_threshold() {
   return n;
 }
 
+// Large molecules run in groups of at most kWideGroupMax (a dimension of the launch grids) whose slots
+// together take at most these doubles, each group in the memory of the one before.  A slot takes about
+// 100 N^2 bytes and 0.6 MB, so 16 GB are 3400 molecules of 200 AOs or 27 of 2400, many more than advance
+// at a time; without a bound, a batch's workspace was that of all its molecules (200 GB for 40,000 of
+// 200 AOs, whose other matrices take 51).  GFN1_WIDE_SLOT_MB overrides it (the tests' small groups).
+constexpr int kWideGroupMax = 32768;
+long long wide_slot_budget() {
+  long long mb = 16 * 1024;
+  if (const char* v = std::getenv("GFN1_WIDE_SLOT_MB"))
+    if (*v) mb = std::max(1, std::atoi(v));
+  return (mb << 20) / (long long)sizeof(double);
+}
+
 int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t* z, const double* charge,
             const gfn1_options* opt, std::string& first_err, int& worst) {
   gfn1_engine* eng = b->eng;
@@ -828,6 +845,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   while (n_dense < nmol && n_m[h_order[n_dense]] > kDenseN) ++n_dense;
   b->n_dense = n_dense;
   b->wide_ids.clear();
+  b->wide_groups.clear();
   b->wide_maxn = b->wide_maxnsh = b->wide_maxnat = 0;
   for (int q = 0; q < n_dense; ++q) {
     const int mm = h_order[q];
@@ -932,14 +950,24 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   if (!b->wide_ids.empty()) {
     std::vector<int> Ns, nshs, nats;
     std::vector<long long> mos, slot_off;
-    long long tot = 0;
+    long long at = 0, tot = 0;
+    const long long most = wide_slot_budget();
     for (int mm : b->wide_ids) {  // the SCC vectors of every slot use the CtaWs layout of the largest molecule
+      const long long size = wide_slot_doubles(n_m[mm], b->wide_maxnsh, b->wide_maxnat, b->cap);
+      if (b->wide_groups.empty() || at + size > most || b->wide_groups.back().count == kWideGroupMax) {
+        at = 0;
+        b->wide_groups.push_back({(int)Ns.size(), 0, 0});
+      }
+      gfn1_batch::WideGroup& g = b->wide_groups.back();
+      ++g.count;
+      g.maxn = std::max(g.maxn, n_m[mm]);
       Ns.push_back(n_m[mm]);
       nshs.push_back(b->wide_maxnsh);
       nats.push_back(b->wide_maxnat);
       mos.push_back(h_mat[mm]);
-      slot_off.push_back(tot);
-      tot += wide_slot_doubles(n_m[mm], b->wide_maxnsh, b->wide_maxnat, b->cap);
+      slot_off.push_back(at);
+      at += size;
+      tot = std::max(tot, at);
     }
     if (!b->wide) b->wide = wide_runtime_new();
     if (!b->wide_buf.ensure((size_t)std::max<long long>(tot, 1)))
@@ -1064,11 +1092,10 @@ int launch_stage(gfn1_batch* b, int stage, cudaStream_t st) {
       if ((e = launch_scc_robust(R.kind, R.n_cta, R.smem, st, B, M, so, SL)) != cudaSuccess)
         return cuda_fail(eng, e, "scc fallback launch");
     }
-    if (!b->wide_ids.empty()) {  // large molecules on groups of SMs, after the one-SM classes
-      if ((e = wide_run(B, M, so, b->wide, (int)b->wide_ids.size(), b->wide_maxn, b->wide_maxnsh, b->wide_maxnat,
-                        b->cap, eng->num_sms, st)) != cudaSuccess)
+    for (const gfn1_batch::WideGroup& g : b->wide_groups)  // large molecules on groups of SMs, after the one-SM classes
+      if ((e = wide_run(B, M, so, b->wide, g.first, g.count, g.maxn, b->wide_maxnsh, b->wide_maxnat, b->cap,
+                        eng->num_sms, st)) != cudaSuccess)
         return cuda_fail(eng, e, "large-molecule SCC");
-    }
   } else if (stage == 2) {
     if (!b->opt.compute_gradient) return GFN1_OK;
     const int nd = b->n_dense, ns = b->nmol - nd;

@@ -2102,10 +2102,11 @@ static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[kRe
   return cudaSuccess;
 }
 
-// Reads the slots' SCC states back (synchronises the stream).
-static cudaError_t wide_read_states(WideRuntime& R, int n, cudaStream_t st) {
+// Reads the SCC states of n slots from `first` back (synchronises the stream).
+static cudaError_t wide_read_states(WideRuntime& R, int first, int n, cudaStream_t st) {
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(R.h_state, R.d_state, sizeof(WideState) * n, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(R.h_state + first, R.d_state + first, sizeof(WideState) * n, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e;
 }
@@ -2144,11 +2145,11 @@ struct WideTimer {
   }
 };
 
-// One pass of the SCC over the molecules listed in R.h_act[0..na): the whole
-// large-molecule path for a call.  Synchronises `st` once per SCC iteration
+// The SCC of the molecules first .. first + nslots - 1 of the binding, the whole
+// large-molecule path for them.  Synchronises `st` once per SCC iteration
 // (the convergence flags).
-cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime& R, int nslots, int maxn,
-                     int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st) {
+cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime& R, int first, int nslots,
+                     int maxn, int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st) {
   if (nslots == 0) return cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -2209,7 +2210,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   };
   // ---- all slots: orthogonaliser and H0'
   int na = nslots;
-  for (int q = 0; q < na; ++q) R.h_act[q] = q;
+  for (int q = 0; q < na; ++q) R.h_act[q] = first + q;
   by_class(na);
   if ((e = upload_act(na)) != cudaSuccess) return e;
   wide_begin_kernel<<<dim3(gx(((long long)maxn * maxn + 255) / 256, na), na), 256, 0, st>>>(B, X);
@@ -2247,15 +2248,15 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     }
   }
   tm.mark("tune");
-  if ((e = wide_read_states(R, nslots, st)) != cudaSuccess) return e;
+  if ((e = wide_read_states(R, first, nslots, st)) != cudaSuccess) return e;
   std::vector<int> done(nslots, 0);  // converged on an earlier rung, or failed
-  for (int q = 0; q < nslots; ++q) done[q] = R.h_state[q].status != kOk;
+  for (int q = 0; q < nslots; ++q) done[q] = R.h_state[first + q].status != kOk;
   // ---- the fallback ladder (src/electronic.rs:1390-1447): rung 0 with the
   // requested options, then linear mixing with a level shift, then T_el >= 3000 K
   for (int rung = 0; rung <= 3; ++rung) {
     na = 0;
     for (int q = 0; q < nslots; ++q)
-      if (!done[q]) R.h_act[na++] = q;
+      if (!done[q]) R.h_act[na++] = first + q;
     if (na == 0) break;
     by_class(na);
     SccOptions ro = opt;
@@ -2304,12 +2305,12 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       tm.mark("cd");
       wide_energy_mix_kernel<<<na, kWideNT, rsm, st>>>(B, M, X, ro, lshift);
       tm.mark("energy");
-      if ((e = wide_read_states(R, nslots, st)) != cudaSuccess) return e;
+      if ((e = wide_read_states(R, first, nslots, st)) != cudaSuccess) return e;
       int nn = 0;
       for (int a = 0; a < na; ++a) {
         const int q = R.h_act[a];
         const WideState& s = R.h_state[q];
-        if (s.status != kOk || s.converged) done[q] = 1;
+        if (s.status != kOk || s.converged) done[q - first] = 1;
         else R.h_act[nn++] = q;
       }
       if (nn != na) {
@@ -2322,7 +2323,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   // ---- results for every slot: P, W of the last diagonalisation, energies, charges
   // (the list of all slots that wide_bind uploaded: a copy from h_act made here would still be under
   // way when the next run sorts its own list there)
-  X.act = R.d_all;
+  X.act = R.d_all + first;
   wide_pw_kernel<<<dim3(gx(mt, nslots), nslots), kGemmNT, tsm, st>>>(B, X);
   wide_results_kernel<<<nslots, kWideNT, rsm, st>>>(B, M, X);
   tm.mark("final");
@@ -2341,7 +2342,8 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
 }
 
 // Slot descriptors for the large molecules of a batch over one device buffer
-// (`base`, wide_slot_layout(...).total doubles per slot at `slot_off`).
+// (`base`, wide_slot_layout(...).total doubles per slot at `slot_off`; the slots of
+// molecules that do not run together may lie over one another).
 cudaError_t wide_bind(WideRuntime& R, const std::vector<int>& ids, const std::vector<int>& Ns,
                       const std::vector<long long>& mos, const std::vector<int>& nshs, const std::vector<int>& nats,
                       int cap, double* base, const std::vector<long long>& slot_off) {
@@ -2452,9 +2454,9 @@ cudaError_t wide_bind_runtime(WideRuntime* r, const std::vector<int>& ids, const
                               const std::vector<long long>& slot_off) {
   return wide_bind(*r, ids, Ns, mos, nshs, nats, cap, base, slot_off);
 }
-cudaError_t wide_run(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime* r, int nslots, int maxn,
-                     int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st) {
-  return run_wide(B, M, opt, *r, nslots, maxn, maxnsh, maxnat, cap, num_sms, st);
+cudaError_t wide_run(const Batch& B, const Model& M, const SccOptions& opt, WideRuntime* r, int first, int nslots,
+                     int maxn, int maxnsh, int maxnat, int cap, int num_sms, cudaStream_t st) {
+  return run_wide(B, M, opt, *r, first, nslots, maxn, maxnsh, maxnat, cap, num_sms, st);
 }
 void wide_plan_info(const WideRuntime* r, int* nb, int* min_rows, int* group, float* ms, int* tuned) {
   if (nb) *nb = r ? r->plan.nb : 0;
