@@ -2058,6 +2058,11 @@ __global__ void wide_copy_hp_kernel(WideCtx X) {  // A = H0' (a realistic matrix
     w.A[i] = w.Hp[i];
 }
 
+// Whether some molecule has columns for the blocked reduction.
+static bool any_blocked(const int (&ncls)[kReductions], int maxn, int grid_sms) {
+  return ncls[3] || (ncls[2] && maxn > grid_rows(grid_sms));
+}
+
 // Times the reduction of the current H0' matrices for every candidate
 // (panel width x minimum rows per CTA) and keeps the fastest.  Without a molecule
 // that takes the blocked reduction there is nothing to choose: the default plan,
@@ -2070,7 +2075,7 @@ static cudaError_t wide_autotune(const WideCtx& X, int na, const int (&ncls)[kRe
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   if (e != cudaSuccess) return e;
-  const bool blocked = ncls[3] || (ncls[2] && maxn > grid_rows(grid_sms));
+  const bool blocked = any_blocked(ncls, maxn, grid_sms);
   float best = 1e30f;
   WidePlan bestp;
   const dim3 cg((unsigned)std::min<long long>(((long long)maxn * maxn + 255) / 256, 1024), na);
@@ -2232,7 +2237,10 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
   const int gcap = std::min(num_sms, kWideMaxG);
   {
     const int nab = na <= 1 ? 1 : na <= 4 ? 4 : na <= 16 ? 16 : na <= 64 ? 64 : 1024;
-    const long long key = ((long long)dev << 40) | ((long long)((maxn + 127) / 128) << 16) | nab;
+    // (sizes of one class may lie on both sides of what fits on chip: a plan chosen for nothing is
+    // not one for the blocked columns)
+    const long long key = ((long long)dev << 40) | ((long long)((maxn + 127) / 128) << 16) |
+                          (any_blocked(ncls, maxn, grid_sms) ? 1 << 15 : 0) | nab;
     std::lock_guard<std::mutex> lk(g_wide_tune_mu);
     auto it = g_wide_plans.find(key);
     if (fixed_plan) {  // (sweeps)
