@@ -1812,6 +1812,7 @@ __global__ void __launch_bounds__(kWideNT, 1) wide_results_kernel(Batch B, Model
 // ================================================================== host side
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -1936,9 +1937,10 @@ static cudaError_t wide_configure(int dev) {
 }
 
 // Which reduction a molecule of N AOs takes: 0 and 1 the clusters of 8 and 16 CTAs
-// that hold its matrix on chip, 2 the grid that does, 3 the blocked one.  Where a cluster fits it wins at
-// every size and count (a reduction at 320 AOs 0.47 against 3.6 ms, eight at 768 AOs
-// 3.9 against 10.1 ms).
+// that hold its matrix on chip, 2 the grid that does (grid_pays), 3 the blocked one.
+// Where a cluster fits it won at every size and count measured (ms, cluster / blocked):
+//   200 AOs 1: 0.27 / 2.34, 128: 2.30 / 3.38;  320 AOs 1: 0.48 / 4.06, 128: 4.14 / 11.5
+//   480 AOs 1: 0.89 / 5.95, 128: 14.5 / 25.2;  768 AOs 1: 1.98 / 10.5, 8: 3.94 / 12.6, 128: 37.4 / 90.5
 static int reduction_class(int N) {
   return N <= ClusterShape<8>::P ? 0 : N <= ClusterShape<16>::P ? 1 : 2;
 }
@@ -1951,12 +1953,42 @@ static cudaError_t tridiag_all(const WideCtx& X, int na, int maxn, int nb, int m
 // Rows a grid of G CTAs holds on chip.
 static int grid_rows(int G) { return std::min(GridShape::kRows * G, GridShape::P); }
 
+// Molecules of at most maxn AOs that grids hold at a time.
+static int grid_at_a_time(int maxn, int sms) {
+  return std::max(1, sms / std::min((maxn + GridShape::kRows - 1) / GridShape::kRows, sms));
+}
+
+// Whether the n molecules `act`, all beyond a cluster, are reduced sooner by grids, a few at a time, than
+// by the blocked reduction, all together.  A grid of N rows takes N (2.1 + 0.0007 N) us however few or many
+// CTAs share it; the blocked reduction is bound by its latencies, 15.5 N us, for few molecules and by the
+// L2, 1.45e-6 N^3 us a molecule, for many.  (It shares the CTAs out evenly, so that unequal molecules
+// wait for the largest: the geometric mean of the sum of N^3 and n times the largest.)  Measured (B200, ms, grid / blocked with its best plan):
+//   776 AOs   8: 6.4 / 12.2   32: 23.8 / 24.7   64: 47.7 / 46.9
+//   896 AOs   8: 9.6 / 15.1   16: 19.1 / 18.6   24: 28.7 / 26.3   64: 76.5 / 66.7
+//   1000 AOs 16: 22.5 / 23.8  32: 44.8 / 48.2   64: 89.6 / 96.7
+//   1200 AOs  4: 13.3 / 20.8   8: 26.5 / 24.0   16: 52.9 / 40.3   64: 212 / 154
+//   1600 AOs  8: 39.1 / 43.9  16: 78.2 / 83.3;  2000 AOs 16: 110 / 146
+//   mixed (a whole call): 1200 and 24 of 800 AOs 503 / 447, 1600 and 16 of 800 383 / 491,
+//   2400 and 32 of 800 834 / 1232, two of 1200 and 8 of 800 232 / 234
+static bool grid_pays(const std::vector<WideMol>& mols, const int* act, int n, int maxn, int sms) {
+  const int per = grid_at_a_time(maxn, sms);
+  double grid = 0.0, latency = 0.0, sum = 0.0, largest = 0.0;
+  for (int a = 0; a < n; ++a) {  // the largest molecules come first
+    const double N = mols[act[a]].N;
+    if (a % per == 0) grid += N * (2.1 + 0.0007 * N);
+    latency = std::max(latency, 15.5 * N);
+    sum += N * N * N;
+    largest = std::max(largest, N * N * N);
+  }
+  const double volume = 1.45e-6 * std::sqrt(sum * n * largest);
+  return grid <= std::cbrt(latency * latency * latency + volume * volume * volume);
+}
+
 // The reduction on grids of the na molecules of X.act, as many at a time as the
 // resident CTAs hold; the blocked reduction of the columns that none can hold first.
 static cudaError_t grid_all(const WideCtx& X, int na, int maxn, int nb, int min_rows, int capacity, int gcap, size_t smem,
                             int sms, cudaStream_t st, int* group, long long* prof) {
-  const int gmin = std::min((maxn + GridShape::kRows - 1) / GridShape::kRows, sms);
-  const int per = std::max(1, sms / gmin);
+  const int per = grid_at_a_time(maxn, sms);
   for (int a0 = 0; a0 < na; a0 += per) {
     const int nn = std::min(per, na - a0);
     int G = sms / nn, cap = grid_rows(G);
@@ -2212,6 +2244,10 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
     std::stable_sort(R.h_act, R.h_act + na, [&](int a, int b) { return red_class(a) < red_class(b); });
     std::fill(ncls, ncls + kReductions, 0);
     for (int a = 0; a < na; ++a) ++ncls[red_class(R.h_act[a])];
+    if (ncls[2] && !grid_pays(R.mols, R.h_act + ncls[0] + ncls[1], ncls[2], maxn, grid_sms)) {
+      ncls[3] += ncls[2];
+      ncls[2] = 0;
+    }
   };
   // ---- all slots: orthogonaliser and H0'
   int na = nslots;

@@ -1,6 +1,6 @@
 """Large molecules in groups that share the workspace slots one after the other (what bounds the memory
-of a large batch): the same results, bit for bit, as with every molecule in a slot of its own, since a
-molecule's arithmetic does not depend on the others that run beside it; with a fallback ladder in one
+of a large batch): the same results, bit for bit, as with every molecule in a slot of its own, since up
+to 768 AOs a molecule's arithmetic does not depend on the others that run beside it; with a fallback ladder in one
 group and rejected molecules among them."""
 import os
 
