@@ -835,7 +835,7 @@ int prepare(gfn1_batch* b, int nmol, const int32_t* atom_offsets, const uint8_t*
   // most expensive molecules first (cost ~ N^3)
   for (int m = 0; m < nmol; ++m) h_order[m] = m;
   std::stable_sort(h_order, h_order + nmol, [&](int x, int y) { return n_m[x] > n_m[y]; });
-  b->cap = std::max(1, std::min(std::max(o.scc_broyden_size, 2), o.max_scc));
+  b->cap = broyden_slots(o.scc_broyden_size, o.max_scc);
   // above kDenseN AOs one SM per molecule is too slow: those molecules run on
   // groups of SMs (wide.cuh).  GFN1_DENSE_N overrides the threshold (the tests
   // use it to run both paths on the same molecules).

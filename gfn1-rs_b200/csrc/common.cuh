@@ -138,6 +138,16 @@ struct SccKind {
 };
 constexpr SccKind kSccKinds[3] = {{128, 64, 4}, {256, 128, 2}, {256, 192, 1}};
 
+// Iterations of the last rung of the fallback ladder, the only one besides the first that mixes with
+// Broyden vectors, and the vectors a molecule's workspace holds: as many as either rung can have at work
+// (stage_mix addresses vectors, products and system by them).
+constexpr int kLastRungScc = 250;
+__host__ __device__ inline int broyden_slots(int broyden_size, int max_scc) {
+  const int memory = broyden_size > 2 ? broyden_size : 2;
+  const int steps = max_scc > kLastRungScc ? max_scc : kLastRungScc;
+  return memory < steps ? memory : steps;
+}
+
 // SCC stages timed when Batch::stage_cycles is set (the device counterpart of
 // the reference's GFN1_PROFILE scopes, src/electronic.rs:1448, :2089-2157).
 enum Stage : int {

@@ -2095,7 +2095,7 @@ __device__ __forceinline__ void scc_molecule(const SccArgs& A, int m) {
       max_scc = max(A.opt.max_scc, 800);
     } else if (rung == 3) {
       etemp = fmax(A.opt.etemp, 3000.0);
-      max_scc = max(A.opt.max_scc, 250);
+      max_scc = max(A.opt.max_scc, kLastRungScc);
       lshift = 0.0;
     }
     __syncthreads();

@@ -2312,7 +2312,7 @@ cudaError_t run_wide(const Batch& B, const Model& M, const SccOptions& opt, Wide
       ro.max_scc = std::max(opt.max_scc, 800);
     } else if (rung == 3) {
       ro.etemp = std::max(opt.etemp, 3000.0);
-      ro.max_scc = std::max(opt.max_scc, 250);
+      ro.max_scc = std::max(opt.max_scc, kLastRungScc);
       lshift = 0.0;
     }
     if ((e = upload_act(na)) != cudaSuccess) return e;
