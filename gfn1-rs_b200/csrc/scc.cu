@@ -1085,12 +1085,19 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
       if (!one || wid == 0) {
 #pragma unroll 1
         for (int col = 0; col < mact; ++col) {
-          int piv = col;
-          if (one) {  // the first of the largest
+          int piv = lane;
+          if (wid == 0) {  // the first of the largest
             double pabs = lane >= col && lane < mact ? fabs(w.beta[(long long)lane * mact + col]) : -1.0;
-            piv = lane;
+#pragma unroll 4
+            for (int r = lane + 32; r < mact; r += 32) {
+              const double v = r >= col ? fabs(w.beta[(long long)r * mact + col]) : -1.0;
+              if (v > pabs) {
+                pabs = v;
+                piv = r;
+              }
+            }
 #pragma unroll 1
-            for (int o = 8; o > 0; o >>= 1) {
+            for (int o = 16; o > 0; o >>= 1) {
               const double v = __shfl_xor_sync(0xffffffffu, pabs, o);
               const int at = __shfl_xor_sync(0xffffffffu, piv, o);
               if (v > pabs || (v == pabs && at < piv)) {
@@ -1098,20 +1105,12 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
                 piv = at;
               }
             }
-            piv = __shfl_sync(0xffffffffu, pabs < 1e-18 ? -1 : piv, 0);
+            piv = pabs < 1e-18 ? -1 : piv;
+          }
+          if (one) {
+            piv = __shfl_sync(0xffffffffu, piv, 0);
           } else {
-            if (tid == 0) {
-              double pabs = fabs(w.beta[(long long)col * mact + col]);
-#pragma unroll 1
-              for (int r = col + 1; r < mact; ++r) {
-                const double v = fabs(w.beta[(long long)r * mact + col]);
-                if (v > pabs) {
-                  piv = r;
-                  pabs = v;
-                }
-              }
-              sh.iscal[1] = (pabs < 1e-18) ? -1 : piv;
-            }
+            if (tid == 0) sh.iscal[1] = piv;
             __syncthreads();
             piv = sh.iscal[1];
           }
@@ -1145,10 +1144,24 @@ __device__ void stage_mix(const SccOptions& opt, const MolCtx& c, CtaWs& w, int 
           for (int r = t >> 4; r < mact; r += nt >> 4) {  // 16 threads a row; column `col` is zeroed below
             const double f = w.beta[(long long)r * mact + col];
             if (r == col || f == 0.0) continue;
+            const double* from = w.beta + (long long)col * mact;
+            double* to = w.beta + (long long)r * mact;
+            int j = col + 1 + (t & 15);
 #pragma unroll 1
-            for (int j = col + 1 + (t & 15); j <= mact; j += 16) {
+            for (; j + 112 < mact; j += 128) {  // eight entries loaded before the first is stored
+              double a[8], b[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                a[u] = to[j + 16 * u];
+                b[u] = from[j + 16 * u];
+              }
+#pragma unroll
+              for (int u = 0; u < 8; ++u) to[j + 16 * u] = a[u] - f * b[u];
+            }
+#pragma unroll 1
+            for (; j <= mact; j += 16) {
               if (j < mact)
-                w.beta[(long long)r * mact + j] -= f * w.beta[(long long)col * mact + j];
+                to[j] -= f * from[j];
               else
                 w.cvec[r] -= f * w.cvec[col];
             }
