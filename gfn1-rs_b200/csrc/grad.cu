@@ -152,8 +152,8 @@ __device__ __forceinline__ void grad_pair_class(const Model& M, const GradCtx& X
         for (int ka = 0; ka < ea.nsh; ++ka) {
           const double qj = X.q[X.atom_sh[a] + ka];
           const double g = harmonic_avg(eb.hard[kb], ea.hard[ka]);
-          const double rs = rsqrt(r2 + 1.0 / (g * g));
-          const double pref = -(rs * rs) * rs * qi * qj;
+          const double den = r2 + 1.0 / (g * g);
+          const double pref = -1.0 / (den * sqrt(den)) * qi * qj;
           for (int c = 0; c < 3; ++c) gmu[c] += rv[c] * pref;
         }
       }

@@ -52,7 +52,10 @@ constexpr double kSkipExpArg = 64.0;
 constexpr double kSkipPrefBound = 6.235149080811617e14;  // 1e-13 * e^64
 
 // 1/p, 1/sqrt(p) and (pi/p)^3/2 from one reciprocal square root (a divide and two
-// square roots were half of a primitive pair's latency).
+// square roots were half of a primitive pair's latency), a few ulp of each.  That does not show
+// in S: against 80-bit arithmetic the elements of 13 clusters are 1.1e-14 off at most and 5e-16
+// to 2e-15 rms, most of it the contraction coefficients' own rounding, and the same within 2%
+// with the divide and the roots.
 constexpr double kPi32 = 5.568327996831708;  // pi^(3/2)
 
 // Primitive pairs sub, sub + G, ... of na x nb.

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128, 4) setup_kernel(Batch B, Model M, int ena
       else {
         const double dx = xyz[3 * a] - xyz[3 * b], dy = xyz[3 * a + 1] - xyz[3 * b + 1], dz = xyz[3 * a + 2] - xyz[3 * b + 2];
         const double r2 = dx * dx + dy * dy + dz * dz;
-        v = rsqrt(r2 + 1.0 / (g * g));
+        v = rsqrt(r2 + 1.0 / (g * g));  // 1 ulp, as a square root and a divide
       }
       Gm[w] = v;
     }
