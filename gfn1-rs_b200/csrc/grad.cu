@@ -320,13 +320,14 @@ size_t grad_smem_bytes(int max_nat) {
 // largest has max_nat atoms; max_l: the batch's highest shell angular momentum
 // (the s/p instantiation below 2).  One CTA per molecule when they fill the GPU
 // (four CTAs on each SM) or one CTA holds a molecule's pairs at once; otherwise
-// eight lanes per atom pair, as many CTAs per molecule as fill it, and the sums
-// in a second launch (two for molecules of more than kGradOneLaunch atoms).
-constexpr int kGradOneLaunch = 160;
+// eight lanes per atom pair, as many CTAs per molecule as fill it, and a launch
+// each for the sums and the chain, whose warps take an atom at a time.  (The sums and
+// the chain together by one CTA, a launch less, were slower from 18 atoms on: one molecule
+// of 18 atoms 67 against 65 us, of 48 95 / 68, of 159 283 / 79; 64 of 24 atoms 78 / 73.)
 static int grad_steps(int max_nat) { return (max_nat * (max_nat - 1) / 2 + 15) / 16; }  // 16 pairs per CTA and step
 int grad_launches(int n, int max_nat, int num_sms) {
   if (n <= 0) return 0;
-  return n >= 4 * num_sms || grad_steps(max_nat) <= 1 ? 1 : (max_nat <= kGradOneLaunch ? 2 : 3);
+  return n >= 4 * num_sms || grad_steps(max_nat) <= 1 ? 1 : 3;
 }
 cudaError_t launch_grad(int max_l, int n, int max_nat, int num_sms, cudaStream_t st, const Batch& B, const Model& M,
                         const int* mols) {
@@ -343,13 +344,9 @@ cudaError_t launch_grad(int max_l, int n, int max_nat, int num_sms, cudaStream_t
     k<<<dim3(n, 1), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradAll);
   } else {
     k<<<dim3(n, std::min(fill, steps)), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradPairs);
-    if (max_nat <= kGradOneLaunch) {
-      k<<<dim3(n, 1), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradSums | kGradChain);
-    } else {
-      const int y = std::max(1, std::min(fill, (max_nat + 3) / 4));
-      k<<<dim3(n, y), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradSums);
-      k<<<dim3(n, y), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradChain);
-    }
+    const int y = std::max(1, std::min(fill, (max_nat + 3) / 4));
+    k<<<dim3(n, y), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradSums);
+    k<<<dim3(n, y), kGradThreads, smem, st>>>(B, M, max_nat, mols, kGradChain);
   }
   return cudaGetLastError();
 }

@@ -516,7 +516,9 @@ int setup_max_atoms(size_t smem) {
 //  * otherwise eight lanes per shell pair and as many CTAs per molecule as fill
 //    it: one launch for up to kSetupOneLaunch atoms (whose classical terms one CTA
 //    finishes while the others form the pairs), beyond that one launch each for
-//    the coordination numbers, the pair terms and the sums.
+//    the coordination numbers, the pair terms and the sums.  Measured, us, one
+//    launch / three: one molecule of 15 atoms 35 / 43, 18 37 / 42, 24 43 / 41, 48
+//    90 / 46; 8 of 15 32 / 41, 18 37 / 41, 36 89 / 43; 64 of 15 50 / 47, 18 63 / 53.
 constexpr int kSetupOneLaunch = 16;
 int setup_launches(int n, int max_nat, bool halogens, int num_sms) {
   return n <= 0 ? 0 : (n >= 4 * num_sms || max_nat <= kSetupOneLaunch ? 1 : (halogens ? 4 : 3));
