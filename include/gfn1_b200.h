@@ -146,7 +146,10 @@ int gfn1_batch_set_positions(gfn1_batch* b, const double* xyz, int on_device);
 /* Initial shell charges (nshells values) or NULL for the zero guess. */
 int gfn1_batch_set_initial_charges(gfn1_batch* b, const double* q, int on_device);
 /* Enqueues setup, SCC and gradient kernels on `stream` (a cudaStream_t passed as
- * a void pointer; NULL = the engine's stream).  Asynchronous. */
+ * a void pointer; NULL = the engine's stream).  Asynchronous for a batch whose
+ * molecules have at most 192 AOs; with larger ones the host waits for `stream`
+ * once per SCC iteration (their convergence decides what is launched next) and
+ * the call returns when their SCC has finished. */
 int gfn1_batch_launch(gfn1_batch* b, void* stream);
 /* Enqueues one stage: 0 = setup (CN, S, H0, Coulomb matrix, repulsion, D3),
  * 1 = persistent SCC, 2 = gradient; -1 = all three (same as gfn1_batch_launch).
