@@ -1898,7 +1898,8 @@ __device__ __forceinline__ double twisted_vector(const double* d, const double* 
 // their neighbours, a pair of threads each; clusters, and a column that it does not
 // settle, by inverse iteration (a pivoted factorisation and two solves, five dependent
 // passes over global memory, 147k cycles at N = 128, against 30k for the twisted
-// factorisation with its first solve; the second solve adds 1% to the SCC at 128 AOs).
+// factorisation with its first solve; the second solve adds 1.5% to the SCC at 128 AOs
+// and 2% to the 4096-molecule batch).
 template <int KIND>
 __device__ __noinline__ void scc_vectors(const SccArgs& A) {
   constexpr int NT = kSccKinds[KIND].nt, HALF = NT / 2;

@@ -23,8 +23,8 @@
 // Every wait is bounded: after kSpinCycles, or when another CTA has raised the molecule's
 // error flag, the CTA raises it and leaves.
 //
-// Measured on B200 (the blocked reduction before): 2368 AOs 42 -> 8.9 ms, 1300 -> 3.7 ms,
-// 769 -> 1.9 ms.  Of the 7,250 cycles a column at 2368 AOs 1,840 are the products (660
+// Measured on B200 (the blocked reduction before): 2368 AOs 42 -> 9.2 ms, 1296 -> 3.7 ms,
+// 776 -> 2.0 ms.  (The fences of the readers are 3% of that.)  Of the other 7,250 cycles a column at 2368 AOs 1,840 are the products (660
 // of the FP64 units, the rest shared memory), 360 the row sums, 550 the scalars, 2,900
 // the exchange and its spread over the CTAs, 1,490 the vectors of phase C.  Rows singly
 // 8,340 cycles (a line of the ring then has eight writers, each write takes the line
